@@ -130,7 +130,7 @@ System::~System() {
                   d_.mm_a, d_.mm_q, d_.m2d_ri, d_.m2d_src, d_.m2d_sP, d_.m2d_sD, d_.d2d_ri, d_.d2d_src,
                   d_.d2d_s, e_m2d_, ipd_, rhs_, ext_, x_, r_, p_, h_, z_, x32_, r32_, p32_, h32_, z32_,
                   alpha32_, scratch_, scratch32_, partial_, dots_, hist_, cols_, flag_, tmat_, piv_,
-                  info_, diis_x_, diis_e_, d_.tile_box32, ext_buf_, blk_info_, blk_minv_, near_ri_, near_ci_,
+                  info_, diis_x_, diis_e_, d_.tile_box32, d_.pol_split, d_.sub_box32, ext_buf_, blk_info_, blk_minv_, near_ri_, near_ci_,
                   near_blk_};
   for (void *b : bufs) release(b);
   if (flush_buf_) cudaFree(flush_buf_);
@@ -196,16 +196,17 @@ size_t System::device_bytes_estimate() const {
   d.m = (int)m;
   int sms = gpu::sm_count();
   size_t s32 = gpu::tmu_scratch_doubles(d, 2, gpu::tmu32_max_split(d, sms)) + 8 * ((n + 127) / 128);
-  size_t s64 = std::max(gpu::m2d_scratch_doubles(d, gpu::m2d_pick_split(d, sms)),
-                        gpu::tmu_scratch_doubles(d, 2, gpu::tmu_pick_split(d, 2, sms, false)));
-  size_t sym = n >= 2048 ? gpu::tmu_sym_scratch_doubles(d, 4) : 0;
+  size_t s64 = gpu::m2d_scratch_doubles(d, gpu::m2d_pick_split(d, sms));
+  size_t sym = n >= gpu::kSymMinSites ? gpu::tmu_sym_scratch_doubles(d, 2) : 0;
   size_t bytes = 8 * (6 * n + 5 * m + m * m_.ld_cart + 2 * nm2d + nd2d + nv * (2 * nipd + 3 + 10)) +
                  4 * (9 * n + 2 * m + 10 * nv + 2 * (n + 1) + nm2d + nd2d) + 4 * s32 + 8 * s64 + 8 * sym +
                  8 * (gpu::kRedBlocks * 32 + 64 + 2 * (size_t)maxhist_);
   // double-single copies of the positions, static-site tile boxes, and the
   // double-single kernels' split partials (allocated in that mode only)
-  const size_t ds_split = std::max(2 * gpu::tmu_ds_pick_split(d, sms), gpu::m2d_ds_pick_split(d, sms));
+  const size_t ds_split = gpu::m2d_ds_pick_split(d, sms);
   bytes += 16 * (n + 2 * m + 2 * ((m + 127) / 128)) + 8 * ds_split * nv;
+  // coordinate splits and 32-site boxes of the symmetric product
+  bytes += 16 * (3 * n + 2 * ((n + 31) / 32));
   // near-field couplings of the Neumann step (about a dozen per site in water)
   if (inner_precond_ == 2) bytes += 4 * (n + 1) + 40 * 24 * n;
   return bytes + (size_t(4) << 20);  // events, flags, rounding
@@ -248,7 +249,6 @@ int System::upload_static() {
   d_.ld = m.ld_cart;
   int sms = gpu::sm_count();
   nsplit_m2d_ = gpu::m2d_pick_split(d_, sms);
-  nsplit_tmu_ = gpu::tmu_pick_split(d_, 2, sms, false);
   nsplit_tmu32_ = gpu::tmu32_pick_split(d_, sms);
   const int f32_splits = gpu::tmu32_max_split(d_, sms);
   d_.ntile = (n + 127) / 128;
@@ -267,10 +267,11 @@ int System::upload_static() {
   bad |= alloc(x_, nv * 2) | alloc(r_, nv * 2) | alloc(p_, nv * 2) | alloc(h_, nv * 2) | alloc(z_, nv * 2);
   bad |= alloc(x32_, nv * 2) | alloc(r32_, nv * 2) | alloc(p32_, nv * 2) | alloc(h32_, nv * 2) |
          alloc(z32_, nv * 2);
-  scratch_n_ = std::max(gpu::m2d_scratch_doubles(d_, nsplit_m2d_), gpu::tmu_scratch_doubles(d_, 2, nsplit_tmu_));
+  scratch_n_ = gpu::m2d_scratch_doubles(d_, nsplit_m2d_);
   // FP32 scratch for twice the default source split (the autotuner tries both)
   bad |= alloc(scratch_, scratch_n_) | alloc(scratch32_, gpu::tmu_scratch_doubles(d_, 2, f32_splits));
-  bad |= alloc(d_.tile_box32, 2 * (size_t)d_.ntile);
+  bad |= alloc(d_.tile_box32, 2 * (size_t)d_.ntile) | alloc(d_.pol_split, 3 * (size_t)n) |
+         alloc(d_.sub_box32, 2 * (size_t)((n + 31) / 32));
   bad |= alloc(d_.mm_pos32, mm) | alloc(d_.mm_pos32lo, mm) | alloc(d_.mm_tile_box32, 2 * (size_t)((mm + 127) / 128));
   bad |= alloc(partial_, (size_t)gpu::kRedBlocks * 32) | alloc(dots_, 64) | alloc(hist_, 2 * (size_t)maxhist_);
   bad |= alloc(cols_, 2) | alloc(flag_, 1) | alloc(info_, 1);
@@ -381,6 +382,16 @@ int System::upload_geometry() {
   std::vector<float4> boxes(2 * (size_t)d_.ntile);
   gpu::tile_boxes32(pp32.data(), n, boxes.data());
   if (n) h2d(d_.tile_box32, boxes.data(), boxes.size() * sizeof(float4));
+  // symmetric FP64 product: 32-site boxes, and the coordinates about the
+  // centroid rounded to whole bohr (so that the shift is exact) in three floats
+  std::vector<float4> subs(2 * (size_t)((n + 31) / 32)), split(3 * (size_t)n);
+  gpu::tile_boxes32(pp32.data(), n, subs.data(), 32);
+  double whole[3] = {std::nearbyint(c[0]), std::nearbyint(c[1]), std::nearbyint(c[2])};
+  gpu::split_coordinates(cpol_h_.data(), n, whole, split.data());
+  if (n) {
+    h2d(d_.sub_box32, subs.data(), subs.size() * sizeof(float4));
+    h2d(d_.pol_split, split.data(), split.size() * sizeof(float4));
+  }
   // static sites in double-single for the double-single E_M2D
   std::vector<float4> mp32(mm), mp32lo(mm);
   for (int i = 0; i < mm; ++i) {
@@ -663,33 +674,34 @@ int System::matvec64(int matv, int ncol, const double *x, double *y, bool dodiag
     }
   }
   {
-    bool sym = fp64_kernel_ == 2 || (fp64_kernel_ == 0 && d_.n >= 2048);
-    if (sym && ensure_sym_scratch() != kOk) {
-      sym = false;  // not enough memory for the partials: all-ordered-pairs kernel
-      log_msg(kVerbHigh, nullptr, "symmetric T.mu scratch does not fit: using the target-outer kernel");
-    }
     KEv e;
     if (ktime_on_) e = kt_begin(0, ncol);
-    if (sym) {
-      gpu::launch_tmu_f64_sym(d_, ncol, x, y, dodiag, sym_scratch_, st_, 4);
-    } else {
-      // the split partials hold two columns: larger blocks go two at a time
-      const size_t nv = 3 * (size_t)d_.n;
-      for (int c0 = 0; c0 < ncol; c0 += 2)
-        gpu::launch_tmu_f64(d_, std::min(2, ncol - c0), x + c0 * nv, y + c0 * nv, dodiag, scratch_, nsplit_tmu_,
-                            st_);
-    }
+    direct_product(ncol, x, y, dodiag, fp64_kernel_);
     if (ktime_on_) kt_end(e);
     stats_.f64_matvecs += 1;
   }
   return kOk;
 }
 
+// The direct T.mu of FP64 accuracy: each unordered pair once, or for small
+// systems (and when forced) all ordered pairs.
+void System::direct_product(int ncol, const double *x, double *y, bool dodiag, int kernel) {
+  bool sym = kernel == 2 || (kernel == 0 && d_.n >= gpu::kSymMinSites);
+  if (sym && ensure_sym_scratch() != kOk) {
+    sym = false;  // not enough memory for the accumulators: all-ordered-pairs kernel
+    log_msg(kVerbHigh, nullptr, "symmetric T.mu scratch does not fit: using the all-ordered-pairs kernel");
+  }
+  if (sym)
+    gpu::launch_tmu_f64_sym(d_, ncol, x, y, dodiag, sym_scratch_, st_);
+  else
+    gpu::launch_tmu_f64(d_, ncol, x, y, dodiag, st_);
+}
+
 // fixed-point accumulators of the symmetric products (FP64, double-single
 // and FP32 share them: they run one after another on the system's stream)
 int System::ensure_sym_scratch() {
   if (sym_scratch_) return kOk;
-  if (alloc(sym_scratch_, gpu::tmu_sym_scratch_doubles(d_, 4))) {
+  if (alloc(sym_scratch_, gpu::tmu_sym_scratch_doubles(d_, 2))) {
     sym_scratch_ = nullptr;
     cudaGetLastError();
     set_last_error("out of device memory for the symmetric-product accumulators");
@@ -698,13 +710,11 @@ int System::ensure_sym_scratch() {
   return kOk;
 }
 
-// FP64-accurate product for the refinement residual: the FP64 kernel, or in
-// the double-single mode the double-single kernel (one column at a time)
+// split partials of the double-single permanent field
 int System::ensure_ds_scratch() {
   if (ds_scratch_) return kOk;
-  nsplit_ds_ = gpu::tmu_ds_pick_split(d_, gpu::sm_count());
   nsplit_m2d_ds_ = gpu::m2d_ds_pick_split(d_, gpu::sm_count());
-  if (alloc(ds_scratch_, (size_t)std::max(2 * nsplit_ds_, nsplit_m2d_ds_) * 3 * d_.n)) {
+  if (alloc(ds_scratch_, (size_t)nsplit_m2d_ds_ * 3 * d_.n)) {
     ds_scratch_ = nullptr;
     set_last_error("out of device memory for the double-single kernels");
     return kErrMemory;
@@ -712,17 +722,13 @@ int System::ensure_ds_scratch() {
   return kOk;
 }
 
+// product for the refinement residual; mixed-ds takes the direct sums
+// whatever the FMM and kernel settings
 int System::matvec_residual(int ncol, const double *x, double *y) {
   if (precision_ != kPrecMixedDS) return matvec64(kMatvDirect, ncol, x, y, true);
-  int st = ensure_ds_scratch();
-  if (st) return st;
-  // the symmetric double-single kernel shares the FP64 one's fixed-point
-  // scratch (without it: the target-outer double-single kernel)
-  if (d_.n >= 2048 && ensure_sym_scratch() != kOk)
-    log_msg(kVerbHigh, nullptr, "symmetric T.mu scratch does not fit: using the target-outer kernel");
   KEv e;
   if (ktime_on_) e = kt_begin(2, ncol);
-  gpu::launch_tmu_ds(d_, ncol, x, y, true, ds_scratch_, nsplit_ds_, sym_scratch_, st_);
+  direct_product(ncol, x, y, true, 0);
   if (ktime_on_) kt_end(e);
   stats_.ds_matvecs += 1;
   return kOk;

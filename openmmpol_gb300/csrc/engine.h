@@ -166,6 +166,7 @@ class System {
   // consecutive polarizable sites, each within link_bohr of an earlier one
   int set_inner_blocks(int max_sites, double link_bohr);
   int matvec_residual(int ncol, const double *x, double *y);
+  void direct_product(int ncol, const double *x, double *y, bool dodiag, int kernel);
   int ensure_ds_scratch();
   int ensure_sym_scratch();
   int precision() const { return precision_; }
@@ -275,7 +276,7 @@ class System {
   double *ext_buf_ = nullptr;  // external points: coordinates, partials, output, dipoles
   size_t ext_cap_ = 0;
   double *ds_scratch_ = nullptr;  // split partials of the double-single kernels
-  int nsplit_ds_ = 1, nsplit_m2d_ds_ = 1;
+  int nsplit_m2d_ds_ = 1;
   // how the cached E_M2D was computed
   static constexpr int kM2dDirect = 0, kM2dDS = 1, kM2dFMM = 2;
   int m2d_method_ = kM2dDirect;
@@ -293,7 +294,7 @@ class System {
   int *info_ = nullptr;
   bool tmat_ok_ = false, lu_ok_ = false;
   double *diis_x_ = nullptr, *diis_e_ = nullptr;
-  int nsplit_m2d_ = 1, nsplit_tmu_ = 1, nsplit_tmu32_ = 1;
+  int nsplit_m2d_ = 1, nsplit_tmu32_ = 1;
   int maxhist_ = 1024;
   // host mirrors
   std::vector<double> ipd_h_, cpol_h_;

@@ -11,9 +11,10 @@
 //                    the scaled-pair correction pass: for every listed pair
 //                    (s - 1) * f_ij is added, which equals the reference's
 //                    "skip when s == 0, multiply when s != 1" rule.
-//   k_tmu<T,...>     dipole-dipole field T.mu, target-outer like field_extD2D
-//                    (src/mod_electrostatics.F90:2068-2109); FP64 or FP32 with
-//                    compensated (Kahan) cross-tile sums.
+//   k_tmu            FP32 dipole-dipole field T.mu, target-outer like
+//                    field_extD2D (src/mod_electrostatics.F90:2068-2109), with
+//                    compensated (Kahan) cross-tile sums; the products of FP64
+//                    accuracy are in tmu_sym.cu.
 //   k_tmu_finish     partial reduction, u-scale correction, sign and the
 //                    1/alpha diagonal of TMatVec_otf/TMatVec_diag
 //                    (src/mod_polarization.F90:459-504).
@@ -147,30 +148,25 @@ __global__ void k_m2d_finish(int n, int nsplit, const double *__restrict__ parti
 }
 
 // partial[split][rhs][j][3] = E_dd(x)_j over the split's source range.
-template <typename T, int NRHS, bool AMOEBA, bool KAHAN>
-__global__ void __launch_bounds__(TPB) k_tmu(int n, const typename Vec4<T>::type *__restrict__ pos,
-                                             const T *__restrict__ damp, const float2 *__restrict__ wa,
-                                             const T *__restrict__ x, T *__restrict__ partial,
-                                             int per_split, T thr, float thr2m) {
-  using V4 = typename Vec4<T>::type;
-  constexpr bool F64 = std::is_same<T, double>::value;
-  __shared__ V4 s_pos[TILE];
-  __shared__ T s_a[TILE];
-  __shared__ float2 s_wa[TILE];
-  __shared__ T s_mu[NRHS * 3][TILE];
+template <int NRHS, bool AMOEBA>
+__global__ void __launch_bounds__(TPB) k_tmu(int n, const float4 *__restrict__ pos,
+                                             const float *__restrict__ damp, const float *__restrict__ x,
+                                             float *__restrict__ partial, int per_split, float thr) {
+  __shared__ float4 s_pos[TILE];
+  __shared__ float s_a[TILE];
+  __shared__ float s_mu[NRHS * 3][TILE];
   const int j = blockIdx.x * TPB + threadIdx.x;
   const bool valid = j < n;
-  V4 pt;
+  float4 pt;
   if (valid) {
     pt = pos[j];
   } else {
-    pt.x = pt.y = pt.z = pt.w = T(0);
+    pt.x = pt.y = pt.z = pt.w = 0.f;
   }
-  const T at = (valid && AMOEBA) ? damp[j] : T(0);
-  const float2 wat = (F64 && valid) ? wa[j] : make_float2(0.f, 0.f);
-  T acc[NRHS * 3], sum[NRHS * 3], comp[NRHS * 3];
+  const float at = (valid && AMOEBA) ? damp[j] : 0.f;
+  float acc[NRHS * 3], sum[NRHS * 3], comp[NRHS * 3];
 #pragma unroll
-  for (int c = 0; c < NRHS * 3; ++c) sum[c] = comp[c] = T(0);
+  for (int c = 0; c < NRHS * 3; ++c) sum[c] = comp[c] = 0.f;
   const int s0 = blockIdx.y * per_split;
   const int s1 = min(n, s0 + per_split);
   for (int t0 = s0; t0 < s1; t0 += TILE) {
@@ -180,8 +176,7 @@ __global__ void __launch_bounds__(TPB) k_tmu(int n, const typename Vec4<T>::type
       int i = t0 + k;
       if (i < s1) {
         s_pos[k] = pos[i];
-        s_a[k] = AMOEBA ? damp[i] : T(0);
-        if (F64) s_wa[k] = wa[i];
+        s_a[k] = AMOEBA ? damp[i] : 0.f;
 #pragma unroll
         for (int r = 0; r < NRHS; ++r)
 #pragma unroll
@@ -191,37 +186,33 @@ __global__ void __launch_bounds__(TPB) k_tmu(int n, const typename Vec4<T>::type
     __syncthreads();
     const int cnt = min(TILE, s1 - t0);
 #pragma unroll
-    for (int c = 0; c < NRHS * 3; ++c) acc[c] = T(0);
+    for (int c = 0; c < NRHS * 3; ++c) acc[c] = 0.f;
     if (valid) {
 #pragma unroll 2
       for (int k = 0; k < cnt; ++k) {
         if (t0 + k == j) continue;
-        const V4 ps = s_pos[k];
-        T dx = pt.x - ps.x, dy = pt.y - ps.y, dz = pt.z - ps.z;
-        T r2 = dx * dx + dy * dy + dz * dz;
-        T k3, k5x3;
-        dd_pair<T, AMOEBA>(r2, pt.w, ps.w, at, s_a[k], wat, F64 ? s_wa[k] : wat, thr, thr2m, k3, k5x3);
+        const float4 ps = s_pos[k];
+        float dx = pt.x - ps.x, dy = pt.y - ps.y, dz = pt.z - ps.z;
+        float r2 = dx * dx + dy * dy + dz * dz;
+        float k3, k5x3;
+        dd_kernel<float, AMOEBA>(r2, pt.w, ps.w, at, s_a[k], thr, k3, k5x3);
 #pragma unroll
         for (int r = 0; r < NRHS; ++r) {
-          T mx = s_mu[r * 3 + 0][k], my = s_mu[r * 3 + 1][k], mz = s_mu[r * 3 + 2][k];
-          T f = k5x3 * (mx * dx + my * dy + mz * dz);
+          float mx = s_mu[r * 3 + 0][k], my = s_mu[r * 3 + 1][k], mz = s_mu[r * 3 + 2][k];
+          float f = k5x3 * (mx * dx + my * dy + mz * dz);
           acc[r * 3 + 0] += f * dx - k3 * mx;
           acc[r * 3 + 1] += f * dy - k3 * my;
           acc[r * 3 + 2] += f * dz - k3 * mz;
         }
       }
     }
-    // cross-tile accumulation: compensated (Kahan) for FP32
+    // compensated (Kahan) cross-tile accumulation
 #pragma unroll
     for (int c = 0; c < NRHS * 3; ++c) {
-      if (KAHAN) {
-        T y = acc[c] - comp[c];
-        T t = sum[c] + y;
-        comp[c] = (t - sum[c]) - y;
-        sum[c] = t;
-      } else {
-        sum[c] += acc[c];
-      }
+      const float y = acc[c] - comp[c];
+      const float t = sum[c] + y;
+      comp[c] = (t - sum[c]) - y;
+      sum[c] = t;
     }
   }
   if (valid) {
@@ -272,202 +263,6 @@ __global__ void k_tmu_finish(int n, int nrhs, int nsplit, const T *__restrict__ 
   T *yj = &y[((size_t)r * n + j) * 3];
   double ia = dodiag ? 1.0 / alpha[j] : 0.0;
   for (int c = 0; c < 3; ++c) yj[c] = (T)(-e[c] + (dodiag ? (double)xj[c] * ia : 0.0));
-}
-
-// ---------------------------------------------------------------------------
-// Symmetric FP64 dipole field: every unordered pair is evaluated once and
-// both directions are accumulated (T_ij = T_ji), halving the FP64 work of
-// the geometry.  Sites are grouped in super-tiles of 128 (4 warps x 32
-// lanes).  Super-tile I meets the slots k of its half shell
-// J = (I + k) mod ntile, k = 0..K (K = ntile / 2); slot 0 is the diagonal
-// block (target side only, all ordered pairs); for even ntile the slot
-// k = ntile/2 is handled by the lower of the two tiles only.  The work items
-// (I, a chunk of consecutive slots) are handed out by an atomic counter to a
-// persistent grid of as many CTAs as fit on the GPU at once, so that every
-// SM stays busy to the end (a static grid leaves 4 CTAs on some SMs and 5 on
-// others).  Inside a slot a
-// warp pairs its 32 targets with each 32-site sub-tile of J in 32 rotation
-// steps: at step t lane l meets source (l + t) mod 32, read from shared
-// memory, and the source-side accumulators travel one lane per step by
-// shuffle, so no lane ever shares an accumulator.  Source sides are summed
-// over the 4 warps in shared memory; they and the target sides are added to
-// per-site 128-bit fixed-point accumulators (2^-80 resolution) with integer
-// atomics.  Integer addition is exact and associative, so the product is
-// deterministic whatever the order of the CTAs, and the accumulators take
-// O(n) memory.
-// ---------------------------------------------------------------------------
-constexpr int SYM_TILE = 128;
-
-// dynamic shared memory of k_tmu_sym: the staged dipoles s_mu[C][128] and
-// the four warps' source-side sums s_accj[4][C][128] (C = 3 NRHS doubles)
-constexpr size_t sym_smem_bytes(int nrhs) { return (size_t)5 * 3 * nrhs * SYM_TILE * sizeof(double); }
-
-// A launch serves the products of several systems (same column count and
-// damping kind): job j covers the items [item0, item0 + base[j+1] - base[j])
-// of its system's product, whose item space is fixed per system, so that a
-// product may also be spread over several launches (its fixed-point sums add
-// up across them).  A one-job table is the single-system product.
-struct Sym64Job {
-  const Pos64 *pos;
-  const double *damp;
-  const float2 *wa;
-  const double *x;
-  unsigned long long *lo, *hi, *bad;
-  int n, ntile, K, chunk, nchunk, item0;
-  double thr;
-  float thr2m;
-};
-struct Sym64Table {
-  int njobs;
-  int base[kMaxSymSlices + 1];
-  Sym64Job job[kMaxSymSlices];
-};
-
-template <int NRHS, bool AMOEBA>
-__global__ void __launch_bounds__(SYM_TILE) k_tmu_sym(const __grid_constant__ Sym64Table tab,
-                                                       unsigned *__restrict__ next) {
-  constexpr int C = 3 * NRHS;
-  __shared__ double s_x[SYM_TILE], s_y[SYM_TILE], s_z[SYM_TILE], s_w[SYM_TILE], s_a[SYM_TILE];
-  __shared__ float2 s_wa[SYM_TILE];
-  extern __shared__ double sym_dyn[];
-  double(*s_mu)[SYM_TILE] = reinterpret_cast<double(*)[SYM_TILE]>(sym_dyn);
-  double(*s_accj)[C][SYM_TILE] = reinterpret_cast<double(*)[C][SYM_TILE]>(sym_dyn + C * SYM_TILE);
-  __shared__ int s_item;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int total = tab.base[tab.njobs];
-  for (;;) {
-    __syncthreads();  // every thread has read the previous item
-    if (tid == 0) s_item = (int)atomicAdd(next, 1u);
-    __syncthreads();
-    const int item = s_item;
-    if (item >= total) break;
-    int jx = 0;
-    while (jx + 1 < tab.njobs && tab.base[jx + 1] <= item) ++jx;
-    const Sym64Job &jb = tab.job[jx];
-    const int n = jb.n, ntile = jb.ntile, K = jb.K, chunk = jb.chunk, nchunk = jb.nchunk;
-    const Pos64 *__restrict__ pos = jb.pos;
-    const double *__restrict__ damp = jb.damp;
-    const float2 *__restrict__ wa = jb.wa;
-    const double *__restrict__ x = jb.x;
-    unsigned long long *acc_lo = jb.lo, *acc_hi = jb.hi, *bad = jb.bad;
-    const double thr = jb.thr;
-    const float thr2m = jb.thr2m;
-    const int local = jb.item0 + (item - tab.base[jx]);
-    const int I = local / nchunk;
-    const int ti = I * SYM_TILE + tid;
-    const bool vi = ti < n;
-    const Pos64 pi = vi ? pos[ti] : Pos64{0, 0, 0, 0};
-    const double ai = (AMOEBA && vi) ? damp[ti] : 0.0;
-    const float2 wai = vi ? wa[ti] : make_float2(0.f, 0.f);
-    // each side's field 3 sum f d - sum k3 mu (f = k5 mu.d) is accumulated
-    // as its two sums, one FMA per component each
-    double mui[C], afi[C], aki[C];
-#pragma unroll
-    for (int c = 0; c < C; ++c) {
-      mui[c] = vi ? x[((size_t)(c / 3) * n + ti) * 3 + (c % 3)] : 0.0;
-      afi[c] = 0.0;
-      aki[c] = 0.0;
-    }
-    const int k0 = (local - I * nchunk) * chunk;
-    const int k1 = min(K + 1, k0 + chunk);
-    for (int k = k0; k < k1; ++k) {
-      int J = I + k;
-      if (J >= ntile) J -= ntile;
-      if (k > 0 && 2 * k == ntile && I >= ntile / 2) continue;  // the other tile of the pair owns it
-      const bool diag = (k == 0);
-      __syncthreads();
-      {
-        int sj = J * SYM_TILE + tid;
-        bool v = sj < n;
-        Pos64 p = v ? pos[sj] : Pos64{0, 0, 0, 0};
-        s_x[tid] = p.x;
-        s_y[tid] = p.y;
-        s_z[tid] = p.z;
-        s_w[tid] = p.w;
-        s_a[tid] = (AMOEBA && v) ? damp[sj] : 0.0;
-        s_wa[tid] = v ? wa[sj] : make_float2(0.f, 0.f);
-#pragma unroll
-        for (int c = 0; c < C; ++c) s_mu[c][tid] = v ? x[((size_t)(c / 3) * n + sj) * 3 + (c % 3)] : 0.0;
-      }
-      __syncthreads();
-      for (int js = 0; js < 4; ++js) {
-        double afj[C], akj[C];
-#pragma unroll
-        for (int c = 0; c < C; ++c) afj[c] = akj[c] = 0.0;
-        for (int t = 0; t < 32; ++t) {
-          const int jl = js * 32 + ((lane + t) & 31);
-          const int gj = J * SYM_TILE + jl;
-          if (vi && gj < n && gj != ti) {
-            double dx = pi.x - s_x[jl], dy = pi.y - s_y[jl], dz = pi.z - s_z[jl];
-            double r2 = dx * dx + dy * dy + dz * dz;
-            double k3, k5;
-            dd_pair_f64<AMOEBA>(r2, pi.w, s_w[jl], ai, s_a[jl], wai, s_wa[jl], thr, thr2m, k3, k5);
-#pragma unroll
-            for (int r = 0; r < NRHS; ++r) {
-              double mx = s_mu[3 * r][jl], my = s_mu[3 * r + 1][jl], mz = s_mu[3 * r + 2][jl];
-              double f = k5 * (mx * dx + my * dy + mz * dz);
-              afi[3 * r] = fma(f, dx, afi[3 * r]);
-              afi[3 * r + 1] = fma(f, dy, afi[3 * r + 1]);
-              afi[3 * r + 2] = fma(f, dz, afi[3 * r + 2]);
-              aki[3 * r] = fma(k3, mx, aki[3 * r]);
-              aki[3 * r + 1] = fma(k3, my, aki[3 * r + 1]);
-              aki[3 * r + 2] = fma(k3, mz, aki[3 * r + 2]);
-              if (!diag) {
-                double g = k5 * (mui[3 * r] * dx + mui[3 * r + 1] * dy + mui[3 * r + 2] * dz);
-                afj[3 * r] = fma(g, dx, afj[3 * r]);
-                afj[3 * r + 1] = fma(g, dy, afj[3 * r + 1]);
-                afj[3 * r + 2] = fma(g, dz, afj[3 * r + 2]);
-                akj[3 * r] = fma(k3, mui[3 * r], akj[3 * r]);
-                akj[3 * r + 1] = fma(k3, mui[3 * r + 1], akj[3 * r + 1]);
-                akj[3 * r + 2] = fma(k3, mui[3 * r + 2], akj[3 * r + 2]);
-              }
-            }
-          }
-          if (!diag) {
-            // the accumulators of source s move to the lane that meets s next
-#pragma unroll
-            for (int c = 0; c < C; ++c) {
-              afj[c] = __shfl_sync(0xffffffffu, afj[c], (lane + 1) & 31);
-              akj[c] = __shfl_sync(0xffffffffu, akj[c], (lane + 1) & 31);
-            }
-          }
-        }
-        if (!diag) {
-          // after 32 steps lane l holds the accumulators of source js*32 + l
-#pragma unroll
-          for (int c = 0; c < C; ++c) s_accj[warp][c][js * 32 + lane] = fma(3.0, afj[c], -akj[c]);
-        }
-      }
-      if (!diag) {
-        __syncthreads();
-        const int sj = J * SYM_TILE + tid;
-        if (sj < n) {
-#pragma unroll
-          for (int c = 0; c < C; ++c) {
-            const double v = ((s_accj[0][c][tid] + s_accj[1][c][tid]) + s_accj[2][c][tid]) + s_accj[3][c][tid];
-            const size_t o = ((size_t)(c / 3) * n + sj) * 3 + (c % 3);
-            fixed_add(acc_lo + o, acc_hi + o, v, bad);
-          }
-        }
-      }
-    }
-    if (vi) {
-#pragma unroll
-      for (int c = 0; c < C; ++c) {
-        const size_t o = ((size_t)(c / 3) * n + ti) * 3 + (c % 3);
-        fixed_add(acc_lo + o, acc_hi + o, fma(3.0, afi[c], -aki[c]), bad);
-      }
-    }
-  }
-}
-
-// out[k] = the fixed-point accumulator k as a double (NaN when flagged)
-__global__ void k_fixed_to_double(size_t total, const unsigned long long *__restrict__ lo,
-                                  const unsigned long long *__restrict__ hi, const unsigned long long *bad,
-                                  double *__restrict__ out) {
-  const bool nan = *bad != 0ull;
-  for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += (size_t)gridDim.x * blockDim.x)
-    out[k] = nan ? __longlong_as_double(0x7ff8000000000000ll) : fixed_value(lo[k], hi[k]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1033,20 +828,17 @@ size_t tmu_scratch_doubles(const DevSites &s, int nrhs, int nsplit) {
   return (size_t)nsplit * nrhs * s.n * 3;
 }
 
-template <typename T, int NRHS, bool KAHAN>
-static void tmu_allpairs(const DevSites &s, const typename Vec4<T>::type *pos, const T *damp, const T *x,
-                         T *partial, int nsplit, cudaStream_t st) {
+template <int NRHS>
+static void tmu_allpairs(const DevSites &s, const float *x, float *partial, int nsplit, cudaStream_t st) {
   add_launch_count(1);
   int tiles = (s.n + TILE - 1) / TILE;
   int per = ((tiles + nsplit - 1) / nsplit) * TILE;
   dim3 grid((s.n + TPB - 1) / TPB, nsplit);
-  T thr = (T)s.damp_thr;
-  const float2 *wa = std::is_same<T, double>::value ? s.pol_wa32 : nullptr;
-  float thr2m = damp_thr2_margin(s);
+  const float thr = (float)s.damp_thr;
   if (s.amoeba)
-    k_tmu<T, NRHS, true, KAHAN><<<grid, TPB, 0, st>>>(s.n, pos, damp, wa, x, partial, per, thr, thr2m);
+    k_tmu<NRHS, true><<<grid, TPB, 0, st>>>(s.n, s.pol_pos32, s.pol_a32, x, partial, per, thr);
   else
-    k_tmu<T, NRHS, false, KAHAN><<<grid, TPB, 0, st>>>(s.n, pos, damp, wa, x, partial, per, thr, thr2m);
+    k_tmu<NRHS, false><<<grid, TPB, 0, st>>>(s.n, s.pol_pos32, s.pol_a32, x, partial, per, thr);
 }
 
 // Columns per launch: the widest of 8/4/2/1 not above what is left and gmax.
@@ -1055,31 +847,27 @@ inline int column_group(int left, int gmax) {
   return g >= 8 ? 8 : (g >= 4 ? 4 : (g >= 2 ? 2 : 1));
 }
 
-template <typename T, bool KAHAN>
-static void tmu_dispatch(const DevSites &s, int nrhs, const typename Vec4<T>::type *pos, const T *damp,
-                         const T *x, T *partial, int nsplit, int gmax, cudaStream_t st, int kver = 1) {
+static void tmu_dispatch(const DevSites &s, int nrhs, const float *x, float *partial, int nsplit, int gmax,
+                         cudaStream_t st, int kver) {
   // process the columns in groups sharing the pair geometry; every group
   // has its own [split][g][n][3] block of partials, one after the other
   int done = 0;
   while (done < nrhs) {
     int g = column_group(nrhs - done, gmax);
     size_t xo = (size_t)done * s.n * 3;
-    T *pg = partial + (size_t)nsplit * done * s.n * 3;
-    if constexpr (std::is_same<T, float>::value) {
-      if (kver == 2) {
-        add_launch_count(1);
-        launch_tmu32_pairs(s, g, x + xo, pg, nsplit, st);
-        done += g;
-        continue;
-      }
+    float *pg = partial + (size_t)nsplit * done * s.n * 3;
+    done += g;
+    if (kver == 2) {
+      add_launch_count(1);
+      launch_tmu32_pairs(s, g, x + xo, pg, nsplit, st);
+      continue;
     }
     switch (g) {
-      case 8: tmu_allpairs<T, 8, KAHAN>(s, pos, damp, x + xo, pg, nsplit, st); break;
-      case 4: tmu_allpairs<T, 4, KAHAN>(s, pos, damp, x + xo, pg, nsplit, st); break;
-      case 2: tmu_allpairs<T, 2, KAHAN>(s, pos, damp, x + xo, pg, nsplit, st); break;
-      default: tmu_allpairs<T, 1, KAHAN>(s, pos, damp, x + xo, pg, nsplit, st); break;
+      case 8: tmu_allpairs<8>(s, x + xo, pg, nsplit, st); break;
+      case 4: tmu_allpairs<4>(s, x + xo, pg, nsplit, st); break;
+      case 2: tmu_allpairs<2>(s, x + xo, pg, nsplit, st); break;
+      default: tmu_allpairs<1>(s, x + xo, pg, nsplit, st); break;
     }
-    done += g;
   }
 }
 
@@ -1119,173 +907,6 @@ void launch_tmu_finish32(const DevSites &s, int nrhs, const float *partial, cons
   tmu_finish<float>(s, nrhs, 1, partial, s.pol_pos32, s.pol_a32, x, true, y, 2, st);
 }
 
-void launch_tmu_f64(const DevSites &s, int nrhs, const double *x, double *y, bool dodiag, double *scratch,
-                    int nsplit, cudaStream_t st) {
-  if (s.n == 0) return;
-  tmu_dispatch<double, false>(s, nrhs, s.pol_pos, s.pol_a, x, scratch, nsplit, 4, st);
-  tmu_finish<double>(s, nrhs, nsplit, scratch, s.pol_pos, s.pol_a, x, dodiag, y, 4, st);
-}
-
-void launch_tmu_ds(const DevSites &s, int nrhs, const double *x, double *y, bool dodiag, double *scratch,
-                   int nsplit, double *sym_scratch, cudaStream_t st) {
-  if (s.n == 0) return;
-  const size_t nv = 3 * (size_t)s.n;
-  const bool sym = sym_scratch && s.n >= 2048;
-  for (int c = 0; c < nrhs;) {
-    const int g = nrhs - c >= 2 ? 2 : 1;
-    if (sym) {
-      // fixed-point sums (layout of launch_tmu_f64_sym), read out to doubles
-      const size_t C = 3 * (size_t)g;
-      unsigned long long *lo = reinterpret_cast<unsigned long long *>(sym_scratch);
-      unsigned long long *hi = lo + C * s.n;
-      double *e = sym_scratch + 2 * C * s.n;
-      unsigned long long *bad = reinterpret_cast<unsigned long long *>(sym_scratch + 3 * C * s.n);
-      unsigned *next = reinterpret_cast<unsigned *>(bad + 1);
-      cudaMemsetAsync(lo, 0, 2 * C * s.n * sizeof(unsigned long long), st);
-      cudaMemsetAsync(bad, 0, sizeof(unsigned long long), st);
-      launch_tmu_ds_sym_pairs(s, g, x + c * nv, lo, hi, bad, next, st);
-      launch_fixed_to_double(C * s.n, lo, hi, bad, e, st);
-      tmu_finish<double>(s, g, 1, e, s.pol_pos, s.pol_a, x + c * nv, dodiag, y + c * nv, 2, st);
-    } else {
-      add_launch_count(1);
-      launch_tmu_ds_pairs(s, g, x + c * nv, scratch, nsplit, st);
-      tmu_finish<double>(s, g, nsplit, scratch, s.pol_pos, s.pol_a, x + c * nv, dodiag, y + c * nv, 2, st);
-    }
-    c += g;
-  }
-}
-
-namespace {
-struct SymPlan {
-  int ntile, K, chunk, nchunk, nitems, ctas;
-};
-template <int NRHS, bool AMOEBA>
-struct SymLaunch {
-  int resident = 0;
-  SymLaunch() {
-    const int smem = (int)sym_smem_bytes(NRHS);
-    cudaFuncSetAttribute(k_tmu_sym<NRHS, AMOEBA>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_tmu_sym<NRHS, AMOEBA>, SYM_TILE, smem);
-    if (resident < 1) resident = 1;
-  }
-};
-template <int NRHS, bool AMOEBA>
-int sym_resident() {
-  static const SymLaunch<NRHS, AMOEBA> cfg;  // thread-safe one-time set-up
-  return cfg.resident;
-}
-
-// work items: about 16 per resident CTA, each a tile and a chunk of its slots
-// (round_pairs > 0: at most a quarter of a CTA's share of round_pairs)
-SymPlan sym_plan(int n, int ctas, double round_pairs) {
-  SymPlan p;
-  p.ntile = (n + SYM_TILE - 1) / SYM_TILE;
-  p.K = p.ntile / 2;
-  const long long units = (long long)p.ntile * (p.K + 1);
-  long long chunk = units / (16LL * ctas);
-  if (round_pairs > 0.0) {
-    const long long cap = (long long)(round_pairs / (4.0 * ctas * SYM_TILE * SYM_TILE));
-    chunk = std::min(chunk, cap);
-  }
-  if (chunk < 1) chunk = 1;
-  if (chunk > p.K + 1) chunk = p.K + 1;
-  p.chunk = (int)chunk;
-  p.nchunk = (p.K + 1 + p.chunk - 1) / p.chunk;
-  p.nitems = p.ntile * p.nchunk;
-  p.ctas = ctas < p.nitems ? ctas : p.nitems;
-  return p;
-}
-
-int sym64_resident(int g, bool amoeba) {
-  if (g == 4) return amoeba ? sym_resident<4, true>() : sym_resident<4, false>();
-  if (g == 2) return amoeba ? sym_resident<2, true>() : sym_resident<2, false>();
-  return amoeba ? sym_resident<1, true>() : sym_resident<1, false>();
-}
-
-template <int NRHS, bool AMOEBA>
-void launch_sym64_table(const Sym64Table &tab, unsigned *next, cudaStream_t st) {
-  const int total = tab.base[tab.njobs];
-  if (total <= 0) return;
-  const int ctas_max = sym_resident<NRHS, AMOEBA>() * sm_count();
-  const int ctas = ctas_max < total ? ctas_max : total;
-  cudaMemsetAsync(next, 0, sizeof(unsigned), st);
-  k_tmu_sym<NRHS, AMOEBA><<<ctas, SYM_TILE, sym_smem_bytes(NRHS), st>>>(tab, next);
-}
-}  // namespace
-
-int tmu_f64_sym_items(const DevSites &s, int g, double round_pairs) {
-  if (s.n == 0) return 0;
-  return sym_plan(s.n, sym64_resident(g, s.amoeba) * sm_count(), round_pairs).nitems;
-}
-
-void launch_tmu_f64_sym_multi(int g, bool amoeba, const SymSlice *sl, int nsl, unsigned *next, cudaStream_t st) {
-  Sym64Table tab{};
-  int total = 0;
-  for (int k = 0; k < nsl && tab.njobs < kMaxSymSlices; ++k) {
-    const DevSites &s = *sl[k].s;
-    if (sl[k].count <= 0 || s.n == 0) continue;
-    const SymPlan p = sym_plan(s.n, sym64_resident(g, amoeba) * sm_count(), sl[k].round_pairs);
-    Sym64Job &j = tab.job[tab.njobs];
-    j.pos = s.pol_pos, j.damp = s.pol_a, j.wa = s.pol_wa32, j.x = static_cast<const double *>(sl[k].x);
-    j.lo = sl[k].lo, j.hi = sl[k].hi, j.bad = sl[k].bad;
-    j.n = s.n, j.ntile = p.ntile, j.K = p.K, j.chunk = p.chunk, j.nchunk = p.nchunk, j.item0 = sl[k].item0;
-    j.thr = s.damp_thr;
-    j.thr2m = damp_thr2_margin(s);
-    tab.base[tab.njobs] = total;
-    total += sl[k].count;
-    ++tab.njobs;
-  }
-  tab.base[tab.njobs] = total;
-  if (!total) return;
-  add_launch_count(1);
-  if (g == 4)
-    amoeba ? launch_sym64_table<4, true>(tab, next, st) : launch_sym64_table<4, false>(tab, next, st);
-  else if (g == 2)
-    amoeba ? launch_sym64_table<2, true>(tab, next, st) : launch_sym64_table<2, false>(tab, next, st);
-  else
-    amoeba ? launch_sym64_table<1, true>(tab, next, st) : launch_sym64_table<1, false>(tab, next, st);
-}
-
-void launch_fixed_to_double(size_t total, const unsigned long long *lo, const unsigned long long *hi,
-                            const unsigned long long *bad, double *out, cudaStream_t st) {
-  add_launch_count(1);
-  k_fixed_to_double<<<blocks_for(total, 256), 256, 0, st>>>(total, lo, hi, bad, out);
-}
-
-size_t tmu_sym_scratch_doubles(const DevSites &s, int nrhs) {
-  if (s.n == 0) return 0;
-  // two 64-bit accumulator words and one double per value of a column group
-  // (at most four columns), the error flag and the work counter
-  size_t C = 3 * (size_t)(nrhs < 4 ? nrhs : 4);
-  return 3 * C * (size_t)s.n + 2;
-}
-
-void launch_tmu_f64_sym(const DevSites &s, int nrhs, const double *x, double *y, bool dodiag, double *scratch,
-                        cudaStream_t st, int gmax) {
-  if (s.n == 0) return;
-  // columns in groups of 4 or 2 (gmax, what the scratch holds) and a last
-  // single one share the pair geometry
-  int done = 0;
-  while (done < nrhs) {
-    const int left = nrhs - done;
-    int g = (left >= 4 && gmax >= 4) ? 4 : (left >= 2 && gmax >= 2 ? 2 : 1);
-    size_t C = 3 * (size_t)g;
-    unsigned long long *lo = reinterpret_cast<unsigned long long *>(scratch);
-    unsigned long long *hi = lo + C * s.n;
-    double *e = scratch + 2 * C * s.n;
-    unsigned long long *bad = reinterpret_cast<unsigned long long *>(scratch + 3 * C * s.n);
-    unsigned *next = reinterpret_cast<unsigned *>(bad + 1);
-    const double *xg = x + (size_t)done * s.n * 3;
-    cudaMemsetAsync(lo, 0, 2 * C * s.n * sizeof(unsigned long long), st);
-    cudaMemsetAsync(bad, 0, sizeof(unsigned long long), st);
-    SymSlice one{&s, xg, lo, hi, bad, 0, tmu_f64_sym_items(s, g)};
-    launch_tmu_f64_sym_multi(g, s.amoeba, &one, 1, next, st);
-    launch_fixed_to_double(C * s.n, lo, hi, bad, e, st);
-    launch_tmu_finish64(s, g, e, xg, dodiag, y + (size_t)done * s.n * 3, st);
-    done += g;
-  }
-}
-
 void launch_tmu_f32(const DevSites &s, int nrhs, const float *x, float *y, float *scratch, int nsplit,
                     cudaStream_t st, int gmax, int kver, double *sym_scratch) {
   if (s.n == 0) return;
@@ -1307,7 +928,7 @@ void launch_tmu_f32(const DevSites &s, int nrhs, const float *x, float *y, float
     }
     return;
   }
-  tmu_dispatch<float, true>(s, nrhs, s.pol_pos32, s.pol_a32, x, scratch, nsplit, gmax, st, kver);
+  tmu_dispatch(s, nrhs, x, scratch, nsplit, gmax, st, kver);
   tmu_finish<float>(s, nrhs, nsplit, scratch, s.pol_pos32, s.pol_a32, x, true, y, gmax, st);
 }
 

@@ -52,6 +52,9 @@ struct DevSites {
   // pairs, [2*ntile]) and the squared distance beyond which no pair is damped
   float4 *tile_box32 = nullptr;
   int ntile = 0;
+  // symmetric FP64 product: coordinates split into three floats [3][n]
+  // (split_coordinates) and the bounding boxes of 32 sites
+  float4 *pol_split = nullptr, *sub_box32 = nullptr;
   float damp_r2max32 = 0.f;
   // double-single E_M2D: static-site positions (hi with w = 0, lo), their
   // tile boxes and the squared distance beyond which no M2D pair is damped
@@ -73,8 +76,8 @@ void launch_m2d_finish(const DevSites &s, double *out, const double *partial, in
 // y = T x (dodiag) or y = -E_dd(x) (no diagonal); x,y [nrhs][n][3], FP64.
 size_t tmu_scratch_doubles(const DevSites &s, int nrhs, int nsplit);
 int tmu_pick_split(const DevSites &s, int nrhs, int sm_count, bool fp32);
-void launch_tmu_f64(const DevSites &s, int nrhs, const double *x, double *y, bool dodiag,
-                    double *scratch, int nsplit, cudaStream_t st);
+// All ordered pairs in FP64, no scratch (tmu_sym.cu).
+void launch_tmu_f64(const DevSites &s, int nrhs, const double *x, double *y, bool dodiag, cudaStream_t st);
 // The finishing pass alone on a field partial [nrhs][n][3] (one split): the
 // u-scaled pair corrections, the sign and the 1/alpha diagonal
 void launch_tmu_finish64(const DevSites &s, int nrhs, const double *partial, const double *x, bool dodiag,
@@ -83,11 +86,25 @@ void launch_tmu_finish64(const DevSites &s, int nrhs, const double *partial, con
 void launch_tmu_finish32(const DevSites &s, int nrhs, const float *partial, const float *x, float *y,
                          cudaStream_t st);
 // Same product with each unordered pair evaluated once (deterministic
-// half-shell schedule); scratch of tmu_sym_scratch_doubles(s, nrhs_max).
+// half-shell schedule, tmu_sym.cu): near pairs in FP64, the others in
+// double-single; scratch of tmu_sym_scratch_doubles(s, nrhs_max).  The product
+// of every mode from kSymMinSites sites (launch_tmu_f64 below).
+constexpr int kSymMinSites = 1000;
+// squared distances within which a pair always runs in FP64 (AMOEBA pairs
+// also while the damping is strong, a u^3 < 20)
+constexpr float kSymNear2 = 36.f, kSymNear2Wang = 64.f;
 size_t tmu_sym_scratch_doubles(const DevSites &s, int nrhs);
-// gmax (1, 2 or 4): the widest column group the scratch was sized for
 void launch_tmu_f64_sym(const DevSites &s, int nrhs, const double *x, double *y, bool dodiag, double *scratch,
-                        cudaStream_t st, int gmax = 2);
+                        cudaStream_t st);
+// its passes for callers that spread a product over launches: accumulators
+// [g][n][3] (lo, then hi) and the two words from bad zeroed and the scale of x
+// found (before the first share), and the sums read out into y = T x
+void launch_tmu_sym_prepare(const DevSites &s, int g, const double *x, unsigned long long *lo,
+                            unsigned long long *bad, cudaStream_t st);
+void launch_tmu_sym_finish(const DevSites &s, int g, const unsigned long long *lo, const unsigned long long *hi,
+                           const unsigned long long *bad, const double *x, bool dodiag, double *y, cudaStream_t st);
+// coordinates x [n][3] about a centre as three floats each, out [3][n]
+void split_coordinates(const double *x, int n, double centre[3], float4 *out);
 // FP32 inner operator with compensated cross-tile sums; x,y float.  Columns
 // go through the pair kernel in groups of up to gmax (8, 4, 2 or 1) sharing
 // the pair geometry; scratch holds nsplit * nrhs * n * 3 floats.
@@ -130,14 +147,10 @@ int tmu32_sym_items(const DevSites &s, int g, double round_pairs = 0.0);
 void launch_tmu32_sym_multi(int g, const SymSlice *sl, int nsl, unsigned *next, cudaStream_t st);
 void launch_fixed_to_float(size_t total, const unsigned long long *lo, const unsigned long long *hi,
                            const unsigned long long *bad, float *out, cudaStream_t st);
-// FP64 symmetric product (g = 1, 2 or 4; one damping kind per launch)
+// symmetric product of FP64 accuracy (g = 1 or 2; one damping kind per
+// launch; launch_tmu_sym_prepare before a product's first share)
 int tmu_f64_sym_items(const DevSites &s, int g, double round_pairs = 0.0);
 void launch_tmu_f64_sym_multi(int g, bool amoeba, const SymSlice *sl, int nsl, unsigned *next, cudaStream_t st);
-void launch_fixed_to_double(size_t total, const unsigned long long *lo, const unsigned long long *hi,
-                            const unsigned long long *bad, double *out, cudaStream_t st);
-// double-single symmetric product (g = 1 or 2; one damping kind per launch)
-int tmu_ds_sym_items(const DevSites &s, int g, double round_pairs = 0.0);
-void launch_tmu_ds_sym_multi(int g, bool amoeba, const SymSlice *sl, int nsl, unsigned *next, cudaStream_t st);
 void launch_tmu32_pairs(const DevSites &s, int g, const float *x, float *partial, int nsplit, cudaStream_t st);
 // source splits an FP32 scratch must hold (per column) for every shape the
 // autotuner may pick
@@ -145,19 +158,8 @@ int tmu32_max_split(const DevSites &s, int sm_count);
 // Split of the source range for the FP32 operator (tmu32.cu) and its tile
 // boxes / undamped distance, computed on the host from the FP32 positions.
 int tmu32_pick_split(const DevSites &s, int sm_count);
-void tile_boxes32(const float4 *pos32, int n, float4 *boxes /*[2*ceil(n/128)]*/);
+void tile_boxes32(const float4 *pos32, int n, float4 *boxes /*[2*ceil(n/tile)]*/, int tile = 128);
 float damp_r2max32(bool amoeba, double damp_thr, const double *inv_thole, const double *a, int n);
-// Double-single product (ds_kernels.cu): y = T x, columns in groups of two
-// sharing the pair geometry, ~1e-13 relative accuracy on the FP32 pipes;
-// scratch of nsplit * 2 * n * 3.
-int tmu_ds_pick_split(const DevSites &s, int sm_count);
-void launch_tmu_ds_pairs(const DevSites &s, int g, const double *x, double *partial, int nsplit, cudaStream_t st);
-// sym_scratch (tmu_sym_scratch_doubles(s, 2), or null): from 2048 sites
-// each unordered pair is evaluated once (launch_tmu_ds_sym_pairs)
-void launch_tmu_ds(const DevSites &s, int nrhs, const double *x, double *y, bool dodiag, double *scratch,
-                   int nsplit, double *sym_scratch, cudaStream_t st);
-void launch_tmu_ds_sym_pairs(const DevSites &s, int g, const double *x, unsigned long long *lo,
-                             unsigned long long *hi, unsigned long long *bad, unsigned *next, cudaStream_t st);
 // E_M2D with the all-pairs part in double-single (scratch nsplit * n * 3)
 int m2d_ds_pick_split(const DevSites &s, int sm_count);
 void launch_m2d_ds_pairs(const DevSites &s, double *partial, int nsplit, int *err_flag, cudaStream_t st);

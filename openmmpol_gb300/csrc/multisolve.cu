@@ -249,6 +249,11 @@ int MultiSolver::launch_products(std::vector<Job *> &active) {
     if (j->done > 0) continue;
     const size_t C = 3 * (size_t)j->ncol, n = j->s->d_.n;
     double *sym = j->s->sym_scratch_;
+    if (j->kind != kF32) {
+      gpu::launch_tmu_sym_prepare(j->s->d_, j->ncol, j->s->x_, reinterpret_cast<unsigned long long *>(sym),
+                                  reinterpret_cast<unsigned long long *>(sym + 3 * C * n), st_);
+      continue;
+    }
     cudaMemsetAsync(sym, 0, 2 * C * n * sizeof(unsigned long long), st_);
     cudaMemsetAsync(sym + 3 * C * n, 0, sizeof(unsigned long long), st_);
   }
@@ -281,10 +286,8 @@ int MultiSolver::launch_products(std::vector<Job *> &active) {
       const int g = kv.first.g;
       if (kv.first.kind == kF32)
         gpu::launch_tmu32_sym_multi(g, sl.data(), (int)sl.size(), counters_, st_);
-      else if (kv.first.kind == kF64)
-        gpu::launch_tmu_f64_sym_multi(g, kv.first.amoeba != 0, sl.data(), (int)sl.size(), counters_, st_);
       else
-        gpu::launch_tmu_ds_sym_multi(g, kv.first.amoeba != 0, sl.data(), (int)sl.size(), counters_, st_);
+        gpu::launch_tmu_f64_sym_multi(g, kv.first.amoeba != 0, sl.data(), (int)sl.size(), counters_, st_);
       ++nlaunch;
       std::lock_guard<std::mutex> lk(mu_);
       stats_.launches += 1;
@@ -345,9 +348,7 @@ void MultiSolver::enqueue_tail(Job &j, int which) {
     gpu::launch_cg_pupdate_f32(ncol, n, w.p32, w.z32, w.cols, st_);
     cudaMemcpyAsync(w.cols_h, w.cols, ncol * sizeof(gpu::CgCol), cudaMemcpyDeviceToHost, st_);
   } else {
-    double *e = s.sym_scratch_ + 2 * C * n;
-    gpu::launch_fixed_to_double(C * n, lo, hi, bad, e, st_);
-    gpu::launch_tmu_finish64(d, ncol, e, s.x_, true, w.h, st_);
+    gpu::launch_tmu_sym_finish(d, ncol, lo, hi, bad, s.x_, true, w.h, st_);
     gpu::launch_residual(ncol * nv, s.rhs_, w.h, w.r, st_);
     gpu::launch_scale_by_alpha(ncol, n, d.pol_alpha, w.r, w.z, st_);
     gpu::launch_dots(ncol, nv, w.r, w.z, w.partial, st_);
@@ -379,8 +380,7 @@ int MultiSolver::tick() {
           j.stage = kProduct;
           j.kind = s.precision_ == kPrecMixedDS ? kDS : kF64;
           j.round_pairs = round_pairs(j.kind);
-          j.items = j.kind == kDS ? gpu::tmu_ds_sym_items(d, ncol, j.round_pairs)
-                                  : gpu::tmu_f64_sym_items(d, ncol, j.round_pairs);
+          j.items = gpu::tmu_f64_sym_items(d, ncol, j.round_pairs);
           j.done = j.launches = 0;
         } else {
           cudaMemcpyAsync(w.r, s.rhs_, ncol * nv * sizeof(double), cudaMemcpyDeviceToDevice, st_);
@@ -439,8 +439,7 @@ int MultiSolver::tick() {
         } else {
           j.kind = s.precision_ == kPrecMixedDS ? kDS : kF64;
           j.round_pairs = round_pairs(j.kind);
-          j.items = j.kind == kDS ? gpu::tmu_ds_sym_items(d, ncol, j.round_pairs)
-                                  : gpu::tmu_f64_sym_items(d, ncol, j.round_pairs);
+          j.items = gpu::tmu_f64_sym_items(d, ncol, j.round_pairs);
         }
         j.done = j.launches = 0;
         ++j.outer;

@@ -129,13 +129,11 @@ extern "C" int32_t ommp_gpu_tmatvec_noalloc(OMMP_SYSTEM_PRT sp, const double *x_
   double *scratch = nullptr;
   int st = scratch_address(&scratch);
   if (st) return st;
-  if (d.n >= 2048 && ommp::gpu::tmu_sym_scratch_doubles(d, nrhs) <= kNoAllocScratchDoubles) {
+  if (d.n >= ommp::gpu::kSymMinSites && ommp::gpu::tmu_sym_scratch_doubles(d, nrhs) <= kNoAllocScratchDoubles) {
     // each unordered pair once, fixed-point sums in the static scratch
     ommp::gpu::launch_tmu_f64_sym(d, nrhs, x_dev, y_dev, dodiag != 0, scratch, s->stream());
   } else {
-    int nsplit = ommp::gpu::tmu_pick_split(d, nrhs, ommp::gpu::sm_count(), false);
-    if ((size_t)nsplit > fit) nsplit = (int)fit;
-    ommp::gpu::launch_tmu_f64(d, nrhs, x_dev, y_dev, dodiag != 0, scratch, nsplit, s->stream());
+    ommp::gpu::launch_tmu_f64(d, nrhs, x_dev, y_dev, dodiag != 0, s->stream());
   }
   cudaError_t e = cudaStreamSynchronize(s->stream());
   if (e == cudaSuccess) e = cudaGetLastError();

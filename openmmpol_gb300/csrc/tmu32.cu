@@ -761,11 +761,11 @@ int tmu32_pick_split(const DevSites &s, int sms) {
   return split < 1 ? 1 : split;
 }
 
-void tile_boxes32(const float4 *p, int n, float4 *boxes) {
-  const int ntile = (n + T32_TILE - 1) / T32_TILE;
+void tile_boxes32(const float4 *p, int n, float4 *boxes, int tile) {
+  const int ntile = (n + tile - 1) / tile;
   for (int t = 0; t < ntile; ++t) {
     float4 lo = make_float4(INFINITY, INFINITY, INFINITY, 0.f), hi = make_float4(-INFINITY, -INFINITY, -INFINITY, 0.f);
-    for (int i = t * T32_TILE; i < n && i < (t + 1) * T32_TILE; ++i) {
+    for (int i = t * tile; i < n && i < (t + 1) * tile; ++i) {
       lo.x = std::fmin(lo.x, p[i].x), lo.y = std::fmin(lo.y, p[i].y), lo.z = std::fmin(lo.z, p[i].z);
       hi.x = std::fmax(hi.x, p[i].x), hi.y = std::fmax(hi.y, p[i].y), hi.z = std::fmax(hi.z, p[i].z);
     }

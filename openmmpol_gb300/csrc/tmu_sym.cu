@@ -1,0 +1,811 @@
+// Symmetric T.mu of FP64 accuracy (TMatVec_otf / field_extD2D,
+// src/mod_polarization.F90:459-481, src/mod_electrostatics.F90:1954-2111):
+// every unordered pair is evaluated once and both directions are accumulated
+// (T_ij = T_ji).
+//
+// GB300 runs FP64 at 1/64 of its FP32 rate, so a kernel that forms every pair
+// on the FP64 pipe (32 FP64 operations per unordered pair) cannot go below
+// 2,048 FP32 issue slots per pair and lane; it took 230 ms per product at
+// 90,000 sites with that pipe 92 % busy.  Here only the pairs that need FP64
+// use it: those that may be Thole-damped (an exponential or a polynomial in
+// r) or that are close.  All others are formed on the FP32 pipes in
+// double-single arithmetic (ds_math.cuh), ~285 FP32 operations per unordered
+// pair, with
+//   * coordinates split on a grid into three floats (split_coordinates), so
+//     that the difference of two sites is exact and costs 7 operations;
+//   * the unit-length form E = K (mu.n) n - k3 mu of the dipole field
+//     (n = d y, y the FP32 reciprocal distance): |n|^2 is within 2^-22 of 1,
+//     so its deviation is collected exactly by adding the squares to 2 and
+//     r^-3 and 3 r^-5 follow from y^3 by a first- and second-order factor,
+//     with no double-single square root;
+//   * accumulators renormalised once per 32 sources.
+// Errors against extended precision (2-norm, random dipoles): water boxes of
+// 900 to 90,000 sites 3.1e-15 to 4.9e-15 (the FP64 kernel: 8.1e-15 to
+// 8.7e-15), a Wang-AL system of 10,200 sites 2.1e-15 (2.9e-15).
+// Time per product (one column): 917 -> 202 us at 5,001 sites, 2.6 -> 0.50 ms
+// at 9,003, 25.6 -> 4.6 ms at 30,000, 230 -> 40.3 ms at 90,000 (4.05e9 pairs:
+// 29 T FP32 operations/s of a measured FMA-chain rate of 36 T/s); two columns
+// 70.9 ms.  Bound by FP32 issue; 5 CTAs per SM at 96 registers with small
+// spills beat 4 at 128 (40.9 ms).
+//
+// Schedule: sites are grouped in super-tiles of 128 (4 warps x 32 lanes).
+// Super-tile I meets the slots k of its half shell J = (I + k) mod ntile,
+// k = 0..K (K = ntile / 2); for even ntile the slot k = ntile / 2 is handled
+// by the lower of the two tiles only.  Work items (I, a chunk of slots; for
+// small systems a quarter of one slot) are handed out by an atomic counter
+// to a persistent grid.  Inside a slot each warp tests the bounding boxes of
+// its own 32 sites and of each 32-site sub-tile of J: far apart, the 32 x 32
+// pairs run without a test; otherwise an FP32 test masks the pairs that may
+// be damped or are close and queues them, and the warp then forms the queued
+// pairs in FP64, 32 at a time (whole sub-tiles in FP64 kept that pipe busy for
+// half of a 9,000-site product: 810 us), so that the FP64 pipe works
+// beside the FP32 ones.  A warp meets the 32 sources in 32 rotation steps:
+// at step t lane l meets source (l + t) mod 32, the source-side accumulators
+// travelling one lane per step by shuffle.  Both sides end in per-site
+// 128-bit fixed-point accumulators (2^-80 resolution) with integer atomics:
+// the sums do not depend on the order of the CTAs.
+//
+// The dipoles are scaled by a power of two per product (sym_prepare: largest
+// magnitude in [2^-12, 2^-11)), so that neither the FP32 range nor the
+// fixed-point resolution depends on their size; k_tmu_sym_finish scales back.
+//
+// Built with --fmad=false -ftz=true: every FMA is explicit.
+#include <algorithm>
+#include <cmath>
+
+#include "ds_math.cuh"
+#include "kernels.h"
+#include "pair_math.cuh"
+
+namespace ommp {
+namespace gpu {
+
+namespace {
+
+constexpr int SYM_TILE = 128;
+constexpr int SYM_SUB = 32;
+// padding sites: no finite distance is 0 and their dipoles are 0
+constexpr float SYM_FAR = 1.0e6f;
+
+// A launch serves the products of several systems (same column count and
+// damping kind): job j covers the items [item0, item0 + base[j+1] - base[j])
+// of its system's product, whose item space is fixed per system, so that a
+// product may also be spread over several launches (its fixed-point sums add
+// up across them).  A one-job table is the single-system product.
+struct SymJob {
+  const float4 *g;        // [3][n] coordinate splits
+  const Pos64 *pos;
+  const double *damp;
+  const float2 *wa;
+  const float4 *boxes, *subs;  // bounding boxes of 128 and of 32 sites
+  const double *x;
+  unsigned long long *lo, *hi, *bad;
+  int n, ntile, K, chunk, nchunk, quarters, item0;
+  double thr;
+  float thr2m, r2near;
+};
+struct SymTable {
+  int njobs;
+  int base[kMaxSymSlices + 1];
+  SymJob job[kMaxSymSlices];
+};
+
+// floats of a staged source: 9 coordinate parts, 6 per column
+template <int G>
+__host__ __device__ constexpr int sym_records() {
+  return (9 + 6 * G + 3) / 4;
+}
+
+template <int G>
+struct SymSmem {
+  float4 rec[sym_records<G>()][SYM_TILE];
+  double accj[4][3 * G][SYM_TILE];
+  float2 wa[SYM_TILE];                         // damping test of the near loops
+  unsigned short queue[4][SYM_SUB * SYM_SUB];  // per warp: target lane * 32 + source
+};
+
+__device__ __forceinline__ float box_dist2(const float4 &alo, const float4 &ahi, const float4 &blo, const float4 &bhi) {
+  const float gx = fmaxf(0.f, fmaxf(blo.x - ahi.x, alo.x - bhi.x));
+  const float gy = fmaxf(0.f, fmaxf(blo.y - ahi.y, alo.y - bhi.y));
+  const float gz = fmaxf(0.f, fmaxf(blo.z - ahi.z, alo.z - bhi.z));
+  return fmaf(gx, gx, fmaf(gy, gy, gz * gz));
+}
+
+// 2^e of the scaling of a product's dipoles from the largest high word of
+// |x| (0 when all are zero: no scaling)
+__device__ __forceinline__ int sym_exponent(unsigned emax) {
+  const int e = (int)(emax >> 20);
+  return e == 0 ? 0 : e - 1023 + 12;
+}
+__device__ __forceinline__ double pow2(int e) {  // |e| <= 1022
+  return __hiloint2double((1023 + e) << 20, 0);
+}
+// v 2^-e without leaving the range of a double's exponent
+__device__ __forceinline__ double scale_down(double v, int e) {
+  const int h = e / 2;
+  return v * pow2(-h) * pow2(-(e - h));
+}
+__device__ __forceinline__ double scale_up(double v, int e) {
+  const int h = e / 2;
+  return v * pow2(h) * pow2(e - h);
+}
+
+// exact addition into the fixed-point words like fixed_add, with integer
+// operations instead of FP64 ones
+__device__ __forceinline__ void fixed_add_int(unsigned long long *lo, unsigned long long *hi, double v,
+                                              unsigned long long *bad) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  const int e = (int)((b >> 52) & 2047);
+  if (e >= 1023 + 36) {  // not below 2^36 (or not finite)
+    atomicOr(bad, 1ull);
+    return;
+  }
+  if (e < 1023 - 80) return;  // below the resolution
+  const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+  // value = m 2^(e - 1075); units of 2^-80: m 2^s
+  const int s = e - 1075 + 80;
+  unsigned long long l, h;
+  if (s >= 64) {
+    l = 0;
+    h = m << (s - 64);
+  } else if (s > 0) {
+    l = m << s;
+    h = m >> (64 - s);
+  } else {
+    l = m >> (-s);
+    h = 0;
+  }
+  if (b >> 63) {
+    l = ~l + 1ull;
+    h = ~h + (l == 0 ? 1ull : 0ull);
+  }
+  const unsigned long long old = atomicAdd(lo, l);
+  atomicAdd(hi, h + (old + l < old ? 1ull : 0ull));
+}
+
+// One side of a double-single pair: (ah, al) += K (mu.n) n - k3 mu.
+struct SymGeom {
+  float xh, xl, yh, yl, zh, zl;  // n = d y
+  float kh, kl;                  // -k3
+  float Kh, Kl;                  // 3 r^-5 / y^2
+};
+
+__device__ __forceinline__ void sym_diff(float th, float tm, float tl, float sh, float sm, float sl, float &h,
+                                         float &l) {
+  // grid splits: the two leading differences are exact and |th - sh| is 0 or
+  // at least |tm - sm|, so the fast sum is exact too
+  const float dh = th - sh, dm = tm - sm;
+  h = dh + dm;
+  l = (dm - (h - dh)) + (tl - sl);
+}
+
+// MASKED: pairs left to FP64 and the site itself give nothing here (masked is
+// set): the close ones and those whose damping reaches the leading float.
+// AMOEBA damping 1 - (1 + x) exp(-x) with x = a u^3 > 20 (from about 6.6 bohr
+// of 9 in water) differs from 1 by less than 2^-24, so an FP32 exponential in
+// the low parts is enough.  The radii keep the double-single share of the
+// product's error below that of the FP64 kernel this one replaced.
+template <bool MASKED, bool AMOEBA>
+__device__ __forceinline__ SymGeom sym_geometry(const float (&t)[9], const float (&s)[9], float2 wat, float2 was,
+                                                bool &masked) {
+  float dx, dy, dz, ex, ey, ez;
+  sym_diff(t[0], t[3], t[6], s[0], s[3], s[6], dx, ex);
+  sym_diff(t[1], t[4], t[7], s[1], s[4], s[7], dy, ey);
+  sym_diff(t[2], t[5], t[8], s[2], s[5], s[8], dz, ez);
+  const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+  const float y0 = rsqrtf(r2);
+  float y = fmaf(0.5f * y0, fmaf(-(r2 * y0), y0, 1.f), y0);
+  float damp3 = 0.f, damp5 = 0.f;
+  if (MASKED) {
+    if (AMOEBA) {
+      const float u2 = r2 * wat.x * was.x;
+      const float x2 = fminf(wat.y, was.y) * (u2 * u2 * u2);
+      masked = !(r2 >= kSymNear2) || !(x2 >= 400.1f);
+      if (!masked) {
+        const float x = x2 * rsqrtf(x2);
+        damp3 = __expf(-x);
+        damp5 = fmaf(x, damp3, damp3);
+      }
+    } else {
+      masked = !(r2 >= kSymNear2Wang) || maybe_damped_wang(r2, wat, was);
+    }
+    if (masked) y = 0.f;
+  }
+  SymGeom g;
+  g.xh = dx * y;
+  g.yh = dy * y;
+  g.zh = dz * y;
+  g.xl = fmaf(ex, y, fmaf(dx, y, -g.xh));
+  g.yl = fmaf(ey, y, fmaf(dy, y, -g.yh));
+  g.zl = fmaf(ez, y, fmaf(dz, y, -g.zh));
+  // eps = 1 - |n|^2: the squares added to 2 in exact fast sums
+  const float px = g.xh * g.xh, py = g.yh * g.yh, pz = g.zh * g.zh;
+  const float qx = fmaf(g.xh + g.xh, g.xl, fmaf(g.xh, g.xh, -px));
+  const float qy = fmaf(g.yh + g.yh, g.yl, fmaf(g.yh, g.yh, -py));
+  const float qz = fmaf(g.zh + g.zh, g.zl, fmaf(g.zh, g.zh, -pz));
+  const float s1 = 2.f + px, s2 = s1 + py, s3 = s2 + pz;
+  const float rx = px - (s1 - 2.f), ry = py - (s2 - s1), rz = pz - (s3 - s2);
+  const float eps = (3.f - s3) - (((qx + qy) + qz) + ((rx + ry) + rz));
+  // r^-3 = y^3 (1 - eps)^(-3/2), 3 r^-5 d d = 3 y^3 (1 - eps)^(-5/2) n n
+  const float w3 = eps * fmaf(1.875f, eps, 1.5f);
+  const float w5 = eps * fmaf(4.375f, eps, 2.5f);
+  const float y2 = y * y, y2l = fmaf(y, y, -y2);
+  const float Y = y2 * y, Yl = fmaf(y2l, y, fmaf(y2, y, -Y));
+  g.kh = -Y;
+  g.kl = -fmaf(Y, w3, Yl);
+  g.Kh = 3.f * Y;
+  g.Kl = fmaf(g.Kh, w5, fmaf(3.f, Yl, fmaf(3.f, Y, -g.Kh)));
+  if (MASKED && AMOEBA) {
+    g.kl = fmaf(-g.kh, damp3, g.kl);
+    g.Kl = fmaf(-g.Kh, damp5, g.Kl);
+  }
+  return g;
+}
+
+__device__ __forceinline__ void sym_acc(float &ah, float &al, float xh, float xl, float yh, float yl) {
+  const float p = xh * yh;
+  const float q = fmaf(xl, yh, fmaf(xh, yl, fmaf(xh, yh, -p)));
+  const dsf s = two_sum(ah, p);
+  ah = s.h;
+  al += s.l + q;
+}
+
+__device__ __forceinline__ void sym_column(const SymGeom &g, const float (&mh)[3], const float (&ml)[3],
+                                           float (&ah)[3], float (&al)[3]) {
+  const float q0 = mh[0] * g.xh, q1 = mh[1] * g.yh, q2 = mh[2] * g.zh;
+  const float f0 = fmaf(ml[0], g.xh, fmaf(mh[0], g.xl, fmaf(mh[0], g.xh, -q0)));
+  const float f1 = fmaf(ml[1], g.yh, fmaf(mh[1], g.yl, fmaf(mh[1], g.yh, -q1)));
+  const float f2 = fmaf(ml[2], g.zh, fmaf(mh[2], g.zl, fmaf(mh[2], g.zh, -q2)));
+  const dsf u1 = two_sum(q0, q1);
+  const dsf u2 = two_sum(u1.h, q2);
+  const float t = ((f0 + f1) + f2) + (u1.l + u2.l);
+  const float fh = g.Kh * u2.h;
+  const float fl = fmaf(g.Kl, u2.h, fmaf(g.Kh, t, fmaf(g.Kh, u2.h, -fh)));
+  sym_acc(ah[0], al[0], fh, fl, g.xh, g.xl);
+  sym_acc(ah[0], al[0], g.kh, g.kl, mh[0], ml[0]);
+  sym_acc(ah[1], al[1], fh, fl, g.yh, g.yl);
+  sym_acc(ah[1], al[1], g.kh, g.kl, mh[1], ml[1]);
+  sym_acc(ah[2], al[2], fh, fl, g.zh, g.zl);
+  sym_acc(ah[2], al[2], g.kh, g.kl, mh[2], ml[2]);
+}
+
+// the 32 x 32 pairs of a warp's sites and the sub-tile js in double-single;
+// NEAR: returns the number of pairs left to FP64 in the warp's queue
+template <int G, bool NEAR, bool AMOEBA>
+__device__ __forceinline__ int sym_pairs(SymSmem<G> &sm, int js, int warp, int lane, bool self, const float (&tg)[9], float2 wai,
+                                         const float (&mih)[G][3], const float (&mil)[G][3],
+                                         float (&aih)[G][3], float (&ail)[G][3], float (&ajh)[G][3],
+                                         float (&ajl)[G][3]) {
+  constexpr int R = sym_records<G>();
+  int queued = 0;
+#pragma unroll
+  for (int c = 0; c < G; ++c)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) ajh[c][k] = ajl[c][k] = 0.f;
+#pragma unroll 1
+  for (int t = 0; t < SYM_SUB; ++t) {
+    const int jl = js * SYM_SUB + ((lane + t) & 31);
+    float f[4 * R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const float4 v = sm.rec[r][jl];
+      f[4 * r] = v.x, f[4 * r + 1] = v.y, f[4 * r + 2] = v.z, f[4 * r + 3] = v.w;
+    }
+    float s[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) s[k] = f[k];
+    bool masked = false;
+    const SymGeom g = sym_geometry<NEAR, AMOEBA>(tg, s, wai, NEAR ? sm.wa[jl] : wai, masked);
+    if (NEAR) {
+      // a sub-tile with itself meets every pair twice: queued once
+      if (self) masked = masked && ((lane + t) & 31) > lane;
+      const unsigned m = __ballot_sync(0xffffffffu, masked);
+      if (masked)
+        sm.queue[warp][queued + __popc(m & ((1u << lane) - 1u))] = (unsigned short)(lane * 32 + ((lane + t) & 31));
+      queued += __popc(m);
+    }
+#pragma unroll
+    for (int c = 0; c < G; ++c) {
+      const float mh[3] = {f[9 + 6 * c], f[10 + 6 * c], f[11 + 6 * c]};
+      const float ml[3] = {f[12 + 6 * c], f[13 + 6 * c], f[14 + 6 * c]};
+      sym_column(g, mh, ml, aih[c], ail[c]);
+      sym_column(g, mih[c], mil[c], ajh[c], ajl[c]);
+    }
+    // the accumulators of source s move to the lane that meets s next
+#pragma unroll
+    for (int c = 0; c < G; ++c)
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        ajh[c][k] = __shfl_sync(0xffffffffu, ajh[c][k], (lane + 1) & 31);
+        ajl[c][k] = __shfl_sync(0xffffffffu, ajl[c][k], (lane + 1) & 31);
+      }
+  }
+  // the target sums' low parts stay small against the high ones
+#pragma unroll
+  for (int c = 0; c < G; ++c)
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const dsf r = two_sum(aih[c][k], ail[c][k]);
+      aih[c][k] = r.h;
+      ail[c][k] = r.l;
+    }
+  return queued;
+}
+
+// the queued pairs of target sub-tile at i0 and source sub-tile at j0 in FP64,
+// one per lane, both sides straight into the fixed-point sums
+template <int G, bool AMOEBA>
+__device__ __noinline__ void sym_queued(const unsigned short *queue, int count, int lane, int i0, int j0,
+                                        const SymJob &jb, int ex) {
+  const int n = jb.n;
+  for (int e = lane; e < count; e += 32) {
+    const int q = queue[e], i = i0 + (q >> 5), j = j0 + (q & 31);
+    if (i >= n || j >= n || i == j) continue;
+    const Pos64 pi = jb.pos[i], pj = jb.pos[j];
+    const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
+    const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+    double k3, k5;
+    dd_pair_f64<AMOEBA, true>(r2, pi.w, pj.w, AMOEBA ? jb.damp[i] : 0.0, AMOEBA ? jb.damp[j] : 0.0, jb.wa[i], jb.wa[j],
+                        jb.thr, jb.thr2m, k3, k5);
+    k5 *= 3.0;
+#pragma unroll
+    for (int r = 0; r < G; ++r) {
+      for (int side = 0; side < 2; ++side) {
+        const size_t o = ((size_t)r * n + (side ? i : j)) * 3, d = ((size_t)r * n + (side ? j : i)) * 3;
+        const double mx = scale_down(jb.x[o], ex), my = scale_down(jb.x[o + 1], ex), mz = scale_down(jb.x[o + 2], ex);
+        const double f = k5 * fma(mx, dx, fma(my, dy, mz * dz));
+        fixed_add_int(jb.lo + d, jb.hi + d, fma(f, dx, -(k3 * mx)), jb.bad);
+        fixed_add_int(jb.lo + d + 1, jb.hi + d + 1, fma(f, dy, -(k3 * my)), jb.bad);
+        fixed_add_int(jb.lo + d + 2, jb.hi + d + 2, fma(f, dz, -(k3 * mz)), jb.bad);
+      }
+    }
+  }
+}
+
+template <int G, bool AMOEBA>
+__global__ void __launch_bounds__(SYM_TILE, G == 1 ? 5 : 3) k_tmu_sym(const __grid_constant__ SymTable tab,
+                                                       unsigned *__restrict__ next) {
+  constexpr int C = 3 * G, R = sym_records<G>();
+  extern __shared__ float4 sym_dyn[];
+  SymSmem<G> &sm = *reinterpret_cast<SymSmem<G> *>(sym_dyn);
+  __shared__ int s_item;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int total = tab.base[tab.njobs];
+  for (;;) {
+    __syncthreads();  // every thread has read the previous item
+    if (tid == 0) s_item = (int)atomicAdd(next, 1u);
+    __syncthreads();
+    const int item = s_item;
+    if (item >= total) break;
+    int jx = 0;
+    while (jx + 1 < tab.njobs && tab.base[jx + 1] <= item) ++jx;
+    const SymJob &jb = tab.job[jx];
+    const int n = jb.n, ntile = jb.ntile, nsub = (n + SYM_SUB - 1) / SYM_SUB;
+    const float4 *__restrict__ gc = jb.g;
+    const double *__restrict__ x = jb.x;
+    const int local = jb.item0 + (item - tab.base[jx]);
+    const int q = local % jb.quarters, unit = local / jb.quarters;
+    const int js0 = q * (4 / jb.quarters), js1 = js0 + 4 / jb.quarters;
+    const int I = unit / jb.nchunk;
+    const int ti = I * SYM_TILE + tid;
+    const bool vi = ti < n;
+    const int ex = sym_exponent(*reinterpret_cast<const unsigned *>(jb.bad + 1));
+    float tg[9], mih[G][3], mil[G][3];
+    {
+      const float4 h = vi ? gc[ti] : make_float4(SYM_FAR, SYM_FAR, SYM_FAR, 0.f);
+      const float4 m = vi ? gc[(size_t)n + ti] : make_float4(0.f, 0.f, 0.f, 0.f);
+      const float4 l = vi ? gc[2 * (size_t)n + ti] : make_float4(0.f, 0.f, 0.f, 0.f);
+      tg[0] = h.x, tg[1] = h.y, tg[2] = h.z, tg[3] = m.x, tg[4] = m.y, tg[5] = m.z, tg[6] = l.x, tg[7] = l.y,
+      tg[8] = l.z;
+    }
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const double m = vi ? scale_down(x[((size_t)(c / 3) * n + ti) * 3 + (c % 3)], ex) : 0.0;
+      const dsf d = to_ds(m);
+      mih[c / 3][c % 3] = d.h;
+      mil[c / 3][c % 3] = d.l;
+    }
+    double sumi[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) sumi[c] = 0.0;
+    const float4 ilo = jb.boxes[2 * I], ihi = jb.boxes[2 * I + 1];
+    const int k0 = (unit - I * jb.nchunk) * jb.chunk;
+    const int k1 = min(jb.K + 1, k0 + jb.chunk);
+    for (int k = k0; k < k1; ++k) {
+      int J = I + k;
+      if (J >= ntile) J -= ntile;
+      if (k > 0 && 2 * k == ntile && I >= ntile / 2) continue;  // the other tile of the pair owns it
+      const bool diag = (k == 0);
+      // uniform over the CTA: may the slot hold near pairs?
+      const bool near_slot = !(box_dist2(ilo, ihi, jb.boxes[2 * J], jb.boxes[2 * J + 1]) > jb.r2near);
+      __syncthreads();
+      if (warp >= js0 && warp < js1) {
+        const int sj = J * SYM_TILE + tid;
+        const bool v = sj < n;
+        const float4 h = v ? gc[sj] : make_float4(-SYM_FAR, -SYM_FAR, -SYM_FAR, 0.f);
+        const float4 m = v ? gc[(size_t)n + sj] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float4 l = v ? gc[2 * (size_t)n + sj] : make_float4(0.f, 0.f, 0.f, 0.f);
+        float f[4 * R] = {h.x, h.y, h.z, m.x, m.y, m.z, l.x, l.y, l.z};
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          const double mu = v ? scale_down(x[((size_t)(c / 3) * n + sj) * 3 + (c % 3)], ex) : 0.0;
+          const dsf d = to_ds(mu);
+          f[9 + 6 * (c / 3) + c % 3] = d.h;
+          f[12 + 6 * (c / 3) + c % 3] = d.l;
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) sm.rec[r][tid] = make_float4(f[4 * r], f[4 * r + 1], f[4 * r + 2], f[4 * r + 3]);
+        if (near_slot) sm.wa[tid] = v ? jb.wa[sj] : make_float2(0.f, 0.f);
+      }
+      __syncthreads();
+      const int si = 4 * I + warp;  // the warp's own sub-tile
+      float aih[G][3], ail[G][3];
+#pragma unroll
+      for (int c = 0; c < G; ++c)
+#pragma unroll
+        for (int d = 0; d < 3; ++d) aih[c][d] = ail[c][d] = 0.f;
+      for (int js = js0; js < js1; ++js) {
+        const int sj = 4 * J + js;
+        const bool skip = si >= nsub || sj >= nsub || (diag && js < warp);
+        const bool self = diag && js == warp;
+        bool near = false;
+        if (!skip && near_slot)
+          near = self || !(box_dist2(jb.subs[2 * si], jb.subs[2 * si + 1], jb.subs[2 * sj], jb.subs[2 * sj + 1]) >
+                           jb.r2near);
+        double outj[C];
+        if (skip) {
+#pragma unroll
+          for (int c = 0; c < C; ++c) outj[c] = 0.0;
+        } else {
+          float ajh[G][3], ajl[G][3];
+          if (near) {
+            const float2 wai = vi ? jb.wa[ti] : make_float2(0.f, 0.f);
+            const int queued =
+                sym_pairs<G, true, AMOEBA>(sm, js, warp, lane, self, tg, wai, mih, mil, aih, ail, ajh, ajl);
+            __syncwarp();
+            sym_queued<G, AMOEBA>(sm.queue[warp], queued, lane, I * SYM_TILE + warp * 32, J * SYM_TILE + js * 32, jb, ex);
+            __syncwarp();
+          } else {
+            sym_pairs<G, false, AMOEBA>(sm, js, warp, lane, false, tg, make_float2(0.f, 0.f), mih, mil, aih, ail, ajh,
+                                        ajl);
+          }
+#pragma unroll
+          for (int c = 0; c < C; ++c) outj[c] = self ? 0.0 : (double)ajh[c / 3][c % 3] + (double)ajl[c / 3][c % 3];
+        }
+        // after 32 steps lane l holds the sums of source js*32 + l
+#pragma unroll
+        for (int c = 0; c < C; ++c) sm.accj[warp][c][js * SYM_SUB + lane] = outj[c];
+      }
+#pragma unroll
+      for (int c = 0; c < C; ++c) sumi[c] += (double)aih[c / 3][c % 3] + (double)ail[c / 3][c % 3];
+      __syncthreads();
+      const int sj = J * SYM_TILE + tid;
+      if (warp >= js0 && warp < js1 && sj < n) {
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          const double v = ((sm.accj[0][c][tid] + sm.accj[1][c][tid]) + sm.accj[2][c][tid]) + sm.accj[3][c][tid];
+          const size_t o = ((size_t)(c / 3) * n + sj) * 3 + (c % 3);
+          fixed_add_int(jb.lo + o, jb.hi + o, v, jb.bad);
+        }
+      }
+    }
+    if (vi) {
+#pragma unroll
+      for (int c = 0; c < C; ++c) {
+        const size_t o = ((size_t)(c / 3) * n + ti) * 3 + (c % 3);
+        fixed_add_int(jb.lo + o, jb.hi + o, sumi[c], jb.bad);
+      }
+    }
+  }
+}
+
+// accumulators to zero and the largest high word of |x| (ctl[1]; the flag and
+// ctl were zeroed before)
+__global__ void __launch_bounds__(256) k_sym_prepare(size_t total, const double *__restrict__ x,
+                                                     unsigned long long *__restrict__ acc, unsigned *ctl) {
+  unsigned m = 0;
+  for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += (size_t)gridDim.x * blockDim.x) {
+    acc[k] = 0ull;
+    acc[total + k] = 0ull;
+    m = max(m, (unsigned)__double2hiint(x[k]) & 0x7FFFFFFFu);
+  }
+  m = __reduce_max_sync(0xffffffffu, m);
+  if ((threadIdx.x & 31) == 0 && m) atomicMax(ctl, m);
+}
+
+// y = -(pair sums + scaled-pair corrections) (+ x / alpha): the fixed-point
+// sums read out (NaN when flagged) and scaled back
+template <bool AMOEBA>
+__global__ void __launch_bounds__(128) k_tmu_sym_finish(
+    int n, const unsigned long long *__restrict__ lo, const unsigned long long *__restrict__ hi,
+    const unsigned long long *__restrict__ bad, const Pos64 *__restrict__ pos, const double *__restrict__ damp,
+    const float2 *__restrict__ wa, const double *__restrict__ x, const double *__restrict__ alpha, bool dodiag,
+    const int *__restrict__ ri, const int *__restrict__ src, const double *__restrict__ scale, double thr, float thr2m,
+    double *__restrict__ y) {
+  const int j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= n) return;
+  const size_t col = (size_t)blockIdx.y * n, o = (col + j) * 3;
+  const bool nan = *bad != 0ull;
+  const int ex = sym_exponent(*reinterpret_cast<const unsigned *>(bad + 1));
+  double e[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c)
+    e[c] = nan ? __longlong_as_double(0x7ff8000000000000ll) : scale_up(fixed_value(lo[o + c], hi[o + c]), ex);
+  if (ri) {
+    const Pos64 pt = pos[j];
+    const double at = AMOEBA ? damp[j] : 0.0;
+    const float2 wat = wa[j];
+    for (int k = ri[j]; k < ri[j + 1]; ++k) {
+      const int i = src[k];
+      const Pos64 ps = pos[i];
+      const double dx = pt.x - ps.x, dy = pt.y - ps.y, dz = pt.z - ps.z;
+      const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+      double k3, k5;
+      dd_pair_f64<AMOEBA, true>(r2, pt.w, ps.w, at, AMOEBA ? damp[i] : 0.0, wat, wa[i], thr, thr2m, k3, k5);
+      const double *mu = &x[(col + i) * 3];
+      const double f = 3.0 * k5 * fma(mu[0], dx, fma(mu[1], dy, mu[2] * dz));
+      const double cs = scale[k] - 1.0;
+      e[0] = fma(cs, fma(f, dx, -(k3 * mu[0])), e[0]);
+      e[1] = fma(cs, fma(f, dy, -(k3 * mu[1])), e[1]);
+      e[2] = fma(cs, fma(f, dz, -(k3 * mu[2])), e[2]);
+    }
+  }
+  const double ia = dodiag ? 1.0 / alpha[j] : 0.0;
+#pragma unroll
+  for (int c = 0; c < 3; ++c) y[o + c] = dodiag ? fma(x[o + c], ia, -e[c]) : -e[c];
+}
+
+// ---------------------------------------------------------------------------
+// All ordered pairs in FP64, one target per CTA, its 128 threads striding over
+// the sources (and the scaled pairs), the sums reduced in a fixed order.
+// Bound by the FP64 pipe at every size: the work of even the smallest system
+// spreads over all SMs (one target per thread left a 192-site system on two
+// SMs, 250 us per product; see launch_tmu_f64 for the sizes it serves).
+// ---------------------------------------------------------------------------
+template <int G, bool AMOEBA>
+__global__ void __launch_bounds__(128) k_tmu_rows(int n, const Pos64 *__restrict__ pos,
+                                                  const double *__restrict__ damp, const float2 *__restrict__ wa,
+                                                  const double *__restrict__ x, const double *__restrict__ alpha,
+                                                  bool dodiag, const int *__restrict__ ri,
+                                                  const int *__restrict__ src, const double *__restrict__ scale,
+                                                  double thr, float thr2m, double *__restrict__ y) {
+  constexpr int C = 3 * G;
+  __shared__ double s_sum[4][C];
+  const int j = blockIdx.x;
+  const Pos64 pt = pos[j];
+  const double at = AMOEBA ? damp[j] : 0.0;
+  const float2 wat = wa[j];
+  double acc[C];
+#pragma unroll
+  for (int c = 0; c < C; ++c) acc[c] = 0.0;
+  auto pair = [&](int i, double w) {
+    const Pos64 ps = pos[i];
+    const double dx = pt.x - ps.x, dy = pt.y - ps.y, dz = pt.z - ps.z;
+    const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+    double k3, k5;
+    dd_pair_f64<AMOEBA, true>(r2, pt.w, ps.w, at, AMOEBA ? damp[i] : 0.0, wat, wa[i], thr, thr2m, k3, k5);
+    const double k3w = k3 * w, k5w = 3.0 * w * k5;
+#pragma unroll
+    for (int r = 0; r < G; ++r) {
+      const double *mu = &x[((size_t)r * n + i) * 3];
+      const double mx = mu[0], my = mu[1], mz = mu[2];
+      const double f = k5w * fma(mx, dx, fma(my, dy, mz * dz));
+      acc[3 * r] = fma(f, dx, fma(-k3w, mx, acc[3 * r]));
+      acc[3 * r + 1] = fma(f, dy, fma(-k3w, my, acc[3 * r + 1]));
+      acc[3 * r + 2] = fma(f, dz, fma(-k3w, mz, acc[3 * r + 2]));
+    }
+  };
+  for (int i = threadIdx.x; i < n; i += 128)
+    if (i != j) pair(i, 1.0);
+  if (ri)
+    for (int k = ri[j] + threadIdx.x; k < ri[j + 1]; k += 128) pair(src[k], scale[k] - 1.0);
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
+    if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5][c] = acc[c];
+  }
+  __syncthreads();
+  if (threadIdx.x < C) {
+    const int c = threadIdx.x;
+    const double e = ((s_sum[0][c] + s_sum[1][c]) + s_sum[2][c]) + s_sum[3][c];
+    const size_t o = ((size_t)(c / 3) * n + j) * 3 + (c % 3);
+    y[o] = dodiag ? x[o] / alpha[j] - e : -e;
+  }
+}
+
+template <int G, bool AMOEBA>
+struct SymLaunch {
+  int resident = 0;
+  SymLaunch() {
+    const int smem = (int)sizeof(SymSmem<G>);
+    cudaFuncSetAttribute(k_tmu_sym<G, AMOEBA>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_tmu_sym<G, AMOEBA>, SYM_TILE, smem);
+    if (resident < 1) resident = 1;
+  }
+};
+template <int G, bool AMOEBA>
+int sym_resident() {
+  static const SymLaunch<G, AMOEBA> cfg;  // thread-safe one-time set-up
+  return cfg.resident;
+}
+int sym_ctas(int g, bool amoeba) {
+  if (g == 2) return (amoeba ? sym_resident<2, true>() : sym_resident<2, false>()) * sm_count();
+  return (amoeba ? sym_resident<1, true>() : sym_resident<1, false>()) * sm_count();
+}
+
+struct SymPlan {
+  int ntile, K, chunk, nchunk, quarters;
+  int items() const { return ntile * nchunk * quarters; }
+};
+
+// work items: about 16 per resident CTA, each a tile and a chunk of its slots
+// (round_pairs > 0: at most a quarter of a CTA's share of round_pairs); with
+// fewer than 8 slots per CTA an item is a quarter of one slot
+SymPlan sym_plan(int n, int ctas, double round_pairs) {
+  SymPlan p;
+  p.ntile = (n + SYM_TILE - 1) / SYM_TILE;
+  p.K = p.ntile / 2;
+  const long long units = (long long)p.ntile * (p.K + 1);
+  long long chunk = units / (16LL * ctas);
+  if (round_pairs > 0.0) chunk = std::min(chunk, (long long)(round_pairs / (4.0 * ctas * SYM_TILE * SYM_TILE)));
+  chunk = std::max(1LL, std::min(chunk, (long long)p.K + 1));
+  p.chunk = (int)chunk;
+  p.nchunk = (p.K + 1 + p.chunk - 1) / p.chunk;
+  p.quarters = units < 8LL * ctas ? 4 : 1;
+  return p;
+}
+
+template <int G, bool AMOEBA>
+void launch_table(const SymTable &tab, unsigned *next, cudaStream_t st) {
+  const int total = tab.base[tab.njobs];
+  const int ctas = std::min(sym_resident<G, AMOEBA>() * sm_count(), total);
+  cudaMemsetAsync(next, 0, sizeof(unsigned), st);
+  k_tmu_sym<G, AMOEBA><<<ctas, SYM_TILE, sizeof(SymSmem<G>), st>>>(tab, next);
+}
+
+// thr^2 with the relative safety margin of the FP32 damping pre-test
+float thr2_margin(const DevSites &s) { return (float)(s.damp_thr * s.damp_thr * (1.0 + 1e-5)); }
+
+template <int G>
+void launch_rows(const DevSites &s, const double *x, double *y, bool dodiag, cudaStream_t st) {
+  const int *ri = s.d2d_nnz ? s.d2d_ri : nullptr;
+  if (s.amoeba)
+    k_tmu_rows<G, true><<<s.n, 128, 0, st>>>(s.n, s.pol_pos, s.pol_a, s.pol_wa32, x, s.pol_alpha, dodiag, ri,
+                                             s.d2d_src, s.d2d_s, s.damp_thr, thr2_margin(s), y);
+  else
+    k_tmu_rows<G, false><<<s.n, 128, 0, st>>>(s.n, s.pol_pos, s.pol_a, s.pol_wa32, x, s.pol_alpha, dodiag, ri,
+                                              s.d2d_src, s.d2d_s, s.damp_thr, thr2_margin(s), y);
+}
+
+}  // namespace
+
+int tmu_f64_sym_items(const DevSites &s, int g, double round_pairs) {
+  if (s.n == 0) return 0;
+  return sym_plan(s.n, sym_ctas(g, s.amoeba), round_pairs).items();
+}
+
+void launch_tmu_f64_sym_multi(int g, bool amoeba, const SymSlice *sl, int nsl, unsigned *next, cudaStream_t st) {
+  SymTable tab{};
+  int total = 0;
+  for (int k = 0; k < nsl && tab.njobs < kMaxSymSlices; ++k) {
+    const DevSites &s = *sl[k].s;
+    if (sl[k].count <= 0 || s.n == 0) continue;
+    const SymPlan p = sym_plan(s.n, sym_ctas(g, amoeba), sl[k].round_pairs);
+    SymJob &j = tab.job[tab.njobs];
+    j.g = s.pol_split, j.pos = s.pol_pos, j.damp = s.pol_a, j.wa = s.pol_wa32;
+    j.boxes = s.tile_box32, j.subs = s.sub_box32;
+    j.x = static_cast<const double *>(sl[k].x);
+    j.lo = sl[k].lo, j.hi = sl[k].hi, j.bad = sl[k].bad;
+    j.n = s.n, j.ntile = p.ntile, j.K = p.K, j.chunk = p.chunk, j.nchunk = p.nchunk, j.quarters = p.quarters;
+    j.item0 = sl[k].item0;
+    j.thr = s.damp_thr;
+    j.thr2m = thr2_margin(s);
+    j.r2near = std::max(s.damp_r2max32, s.amoeba ? kSymNear2 : kSymNear2Wang);
+    tab.base[tab.njobs] = total;
+    total += sl[k].count;
+    ++tab.njobs;
+  }
+  tab.base[tab.njobs] = total;
+  if (!total) return;
+  add_launch_count(1);
+  if (g == 2)
+    amoeba ? launch_table<2, true>(tab, next, st) : launch_table<2, false>(tab, next, st);
+  else
+    amoeba ? launch_table<1, true>(tab, next, st) : launch_table<1, false>(tab, next, st);
+}
+
+void launch_tmu_sym_prepare(const DevSites &s, int g, const double *x, unsigned long long *lo, unsigned long long *bad,
+                            cudaStream_t st) {
+  const size_t total = 3 * (size_t)g * s.n;
+  add_launch_count(1);
+  cudaMemsetAsync(bad, 0, 2 * sizeof(unsigned long long), st);
+  const int blocks = (int)std::min<size_t>((total + 255) / 256, 1216);
+  k_sym_prepare<<<blocks, 256, 0, st>>>(total, x, lo, reinterpret_cast<unsigned *>(bad + 1));
+}
+
+void launch_tmu_sym_finish(const DevSites &s, int g, const unsigned long long *lo, const unsigned long long *hi,
+                           const unsigned long long *bad, const double *x, bool dodiag, double *y, cudaStream_t st) {
+  add_launch_count(1);
+  const dim3 grid((s.n + 127) / 128, g);
+  const int *ri = s.d2d_nnz ? s.d2d_ri : nullptr;
+  if (s.amoeba)
+    k_tmu_sym_finish<true><<<grid, 128, 0, st>>>(s.n, lo, hi, bad, s.pol_pos, s.pol_a, s.pol_wa32, x, s.pol_alpha,
+                                                 dodiag, ri, s.d2d_src, s.d2d_s, s.damp_thr, thr2_margin(s), y);
+  else
+    k_tmu_sym_finish<false><<<grid, 128, 0, st>>>(s.n, lo, hi, bad, s.pol_pos, s.pol_a, s.pol_wa32, x, s.pol_alpha,
+                                                  dodiag, ri, s.d2d_src, s.d2d_s, s.damp_thr, thr2_margin(s), y);
+}
+
+size_t tmu_sym_scratch_doubles(const DevSites &s, int nrhs) {
+  if (s.n == 0) return 0;
+  // two 64-bit accumulator words and one value read out (FP32 product) per
+  // value of a column group (at most two columns), the error flag, the scale
+  // and the work counter
+  const size_t C = 3 * (size_t)(nrhs < 2 ? nrhs : 2);
+  return 3 * C * (size_t)s.n + 3;
+}
+
+void launch_tmu_f64_sym(const DevSites &s, int nrhs, const double *x, double *y, bool dodiag, double *scratch,
+                        cudaStream_t st) {
+  if (s.n == 0) return;
+  // two columns share the pair geometry
+  for (int done = 0; done < nrhs;) {
+    const int g = nrhs - done >= 2 ? 2 : 1;
+    const size_t C = 3 * (size_t)g;
+    unsigned long long *lo = reinterpret_cast<unsigned long long *>(scratch);
+    unsigned long long *hi = lo + C * s.n;
+    unsigned long long *bad = lo + 3 * C * s.n;
+    unsigned *next = reinterpret_cast<unsigned *>(bad + 2);
+    const double *xg = x + (size_t)done * s.n * 3;
+    launch_tmu_sym_prepare(s, g, xg, lo, bad, st);
+    SymSlice one{&s, xg, lo, hi, bad, 0, tmu_f64_sym_items(s, g)};
+    launch_tmu_f64_sym_multi(g, s.amoeba, &one, 1, next, st);
+    launch_tmu_sym_finish(s, g, lo, hi, bad, xg, dodiag, y + (size_t)done * s.n * 3, st);
+    done += g;
+  }
+}
+
+// Below kSymMinSites a symmetric product is bound by the latency of its few
+// items (67 us at 900 and at 1,200 sites, 92 us at 2,001) and all ordered
+// pairs in FP64 are faster: 12 us at 192 sites, 61 at 900, 92 at 1,200,
+// 233 at 2,001 (one target per thread: 250 us at 192).
+void launch_tmu_f64(const DevSites &s, int nrhs, const double *x, double *y, bool dodiag, cudaStream_t st) {
+  if (s.n == 0) return;
+  for (int c = 0; c < nrhs;) {
+    const int g = nrhs - c >= 2 ? 2 : 1;
+    const size_t o = (size_t)c * s.n * 3;
+    add_launch_count(1);
+    if (g == 2)
+      launch_rows<2>(s, x + o, y + o, dodiag, st);
+    else
+      launch_rows<1>(s, x + o, y + o, dodiag, st);
+    c += g;
+  }
+}
+
+// x = h + m + l with h a multiple of g and m of g 2^-23 (g = 2^-23 of the
+// power of two that bounds every coordinate), so that differences of h and of
+// m are exact in FP32
+void split_coordinates(const double *x, int n, double centre[3], float4 *out) {
+  double big = 1.0;
+  for (int i = 0; i < n; ++i)
+    for (int k = 0; k < 3; ++k) big = std::max(big, std::fabs(x[3 * (size_t)i + k] - centre[k]));
+  int e = 0;
+  std::frexp(big, &e);  // big < 2^e
+  const double g1 = std::ldexp(1.0, e - 23), g2 = std::ldexp(g1, -23);
+  for (int i = 0; i < n; ++i) {
+    float h[3], m[3], l[3];
+    for (int k = 0; k < 3; ++k) {
+      const double v = x[3 * (size_t)i + k] - centre[k];
+      const double hk = std::nearbyint(v / g1) * g1;
+      const double mk = std::nearbyint((v - hk) / g2) * g2;
+      h[k] = (float)hk, m[k] = (float)mk, l[k] = (float)((v - hk) - mk);
+    }
+    out[i] = make_float4(h[0], h[1], h[2], 0.f);
+    out[(size_t)n + i] = make_float4(m[0], m[1], m[2], 0.f);
+    out[2 * (size_t)n + i] = make_float4(l[0], l[1], l[2], 0.f);
+  }
+}
+
+}  // namespace gpu
+}  // namespace ommp
