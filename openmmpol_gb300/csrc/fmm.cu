@@ -19,9 +19,10 @@
 //                 shared-memory accumulator summed per target term in a
 //                 fixed order (deterministic)
 //   k_fmm_l2l     children's local expansions from the parent's
+//   k_fmm_near    (fmm_near.cu) the near field of the 27 neighbouring leaves,
+//                 direct, with the Thole damping of the direct kernels
 //   k_fmm_l2p     far field of the leaf's local expansion at each site plus
-//                 the near field of the 27 neighbouring leaves, direct, with
-//                 the Thole damping of the direct kernels
+//                 the near field's partial sums
 // then the finishing pass of the direct product (scaled-pair corrections
 // with exact pair terms, sign, 1/alpha diagonal).  Sites are kept in leaf
 // order on the device (a counting sort per geometry).
@@ -52,6 +53,7 @@ struct FmmTree {
   gpu::Pos64 *spos = nullptr, *spos_t = nullptr;       // w = 1/thole (inf without Thole factor)
   double *sa = nullptr, *sa_t = nullptr;               // Thole damping a
   float2 *swa = nullptr, *swa_t = nullptr;             // FP32 damping pre-test data
+  float4 *split = nullptr;                             // T.mu: split coordinates [3][n] (fmm_near.cu)
   double *sq = nullptr;                                // sorted multipoles [n][ld] (M2D sources)
   int *tmm = nullptr;                                  // targets' static index (M2D self pair)
   double *M = nullptr, *Lc = nullptr;                  // [2][ncell][K]
@@ -73,12 +75,14 @@ struct FmmState {
   int *mm_off = nullptr, *ll_off = nullptr;
   FmmTree d2d, m2d;            // polarizable sites; static sources with polarizable targets
   double *field = nullptr;     // [2][n][3]
+  double *near = nullptr;      // T.mu near-field partials [kFmmNearSplit][2][n][3], after field
+  unsigned *word = nullptr;    // after near
   size_t field_n = 0;
   bool built = false;          // d2d tree for the current geometry
 };
 
 void free_tree(FmmTree &t) {
-  void *b[] = {t.cnt, t.leaf_start, t.perm, t.spos, t.sa, t.swa, t.sq, t.M, t.Lc};
+  void *b[] = {t.cnt, t.leaf_start, t.perm, t.spos, t.sa, t.swa, t.sq, t.M, t.Lc, t.split};
   for (void *p : b)
     if (p) cudaFree(p);
   if (!t.shared) {
@@ -149,61 +153,62 @@ __device__ __forceinline__ int cell_idx(int l, int x, int y, int z) {
 }
 __device__ __forceinline__ int level_off(int l) { return ((1 << (3 * l)) - 1) / 7; }
 
-// leaf multipoles of the dipoles x [col][n][3]
-__global__ void __launch_bounds__(FT) k_fmm_p2m(FmmArgs a, const double *__restrict__ x, int n) {
-  __shared__ double s_p[3][fmm::kMaxOrder + 1][FCH];
-  __shared__ double s_mu[3][FCH];
+// leaf multipoles of the dipoles x [col][n][3], one term per thread (blockDim
+// covers K): with the powers v^m / m! of a site and the same shifted by one
+// and times the dipole (A), a term's share is
+//   Ax[a] Y[b] Z[c] + X[a] (Ay[b] Z[c] + Y[b] Az[c]),
+// five FP64 operations (the three products formed apart: 12; 502 -> 283 us
+// at 60,000 sites, order 10).  FP64 pipe.
+__global__ void __launch_bounds__(512) k_fmm_p2m(FmmArgs a, const double *__restrict__ x, int n) {
+  __shared__ double s_p[3][fmm::kMaxOrder + 1][FCH + 1], s_a[3][fmm::kMaxOrder + 1][FCH + 1];
   const int c = blockIdx.x, col = blockIdx.y;
   const int s0 = a.leaf_start[c], s1 = a.leaf_start[c + 1];
   if (s0 == s1) return;
   int cx, cy, cz;
   cell_xyz(c, a.L, cx, cy, cz);
   const double h = a.h0 / (1 << a.L);
-  const double ctr[3] = {a.ox + (cx + 0.5) * h, a.oy + (cy + 0.5) * h, a.oz + (cz + 0.5) * h};
-  double acc[kMaxTermsPerThread];
-  for (int j = 0; j < kMaxTermsPerThread; ++j) acc[j] = 0.0;
+  const int t = threadIdx.x;
+  const short4 e = t < a.K ? a.terms[t] : make_short4(0, 0, 0, 0);
+  double acc = 0.0;
   for (int b0 = s0; b0 < s1; b0 += FCH) {
     __syncthreads();
-    const int k = threadIdx.x;
-    if (k < FCH && b0 + k < s1) {
+    for (int i = threadIdx.x; i < 3 * FCH; i += blockDim.x) {
+      const int d = i / FCH, k = i % FCH;
+      if (b0 + k >= s1) continue;
       const Pos64 ps = a.spos[b0 + k];
-      const int pi = a.perm[b0 + k];
-      const double v[3] = {ps.x - ctr[0], ps.y - ctr[1], ps.z - ctr[2]};
-      for (int d = 0; d < 3; ++d) {
-        double pw = 1.0;
-        s_p[d][0][k] = 1.0;
-        for (int m = 1; m <= a.p; ++m) {
-          pw = pw * v[d] / m;
-          s_p[d][m][k] = pw;
-        }
-        s_mu[d][k] = x[((size_t)col * n + pi) * 3 + d];
+      const double v = d == 0 ? ps.x - (a.ox + (cx + 0.5) * h) : d == 1 ? ps.y - (a.oy + (cy + 0.5) * h)
+                                                                        : ps.z - (a.oz + (cz + 0.5) * h);
+      const double mu = x[((size_t)col * n + a.perm[b0 + k]) * 3 + d];
+      double pw = 1.0;
+      s_p[d][0][k] = 1.0;
+      s_a[d][0][k] = 0.0;
+      for (int m = 1; m <= a.p; ++m) {
+        s_a[d][m][k] = mu * pw;
+        pw = pw * v * (1.0 / m);
+        s_p[d][m][k] = pw;
       }
     }
     __syncthreads();
     const int cnt = min(FCH, s1 - b0);
-    for (int j = 0; j < kMaxTermsPerThread; ++j) {
-      const int t = threadIdx.x + j * FT;
-      if (t >= a.K) break;
-      const short4 e = a.terms[t];
-      double w = 0.0;
-      for (int q = 0; q < cnt; ++q) {
-        if (e.x) w += s_mu[0][q] * s_p[0][e.x - 1][q] * s_p[1][e.y][q] * s_p[2][e.z][q];
-        if (e.y) w += s_mu[1][q] * s_p[0][e.x][q] * s_p[1][e.y - 1][q] * s_p[2][e.z][q];
-        if (e.z) w += s_mu[2][q] * s_p[0][e.x][q] * s_p[1][e.y][q] * s_p[2][e.z - 1][q];
-      }
-      acc[j] += w;
+    if (t >= a.K) continue;
+    double w = 0.0;
+    for (int q = 0; q < cnt; ++q) {
+      const double Y = s_p[1][e.y][q], Z = s_p[2][e.z][q];
+      w = fma(s_a[0][e.x][q], Y * Z, w);
+      w = fma(s_p[0][e.x][q], fma(s_a[1][e.y][q], Z, Y * s_a[2][e.z][q]), w);
     }
+    acc += w;
   }
-  double *Mc = a.M + ((size_t)col * a.ncell + level_off(a.L) + c) * a.K;
-  for (int j = 0; j < kMaxTermsPerThread; ++j) {
-    const int t = threadIdx.x + j * FT;
-    if (t < a.K) Mc[t] = acc[j];
-  }
+  if (t < a.K) a.M[((size_t)col * a.ncell + level_off(a.L) + c) * a.K + t] = acc;
 }
 
 // parents at level l - 1 from their children at level l:
 // M_g(parent) = sum_children sum_(k <= g) M_k(child) s^(g - k) / (g - k)!
-__global__ void __launch_bounds__(FT) k_fmm_m2m(FmmArgs a, int l) {
+// The eight children are worked on side by side (FT threads each) and added
+// in order: one after another they were a chain of 8 K loads (256 -> 167 us at
+// order 10, 64 parents; latency of the longest term's list).
+__global__ void __launch_bounds__(8 * FT) k_fmm_m2m(FmmArgs a, int l) {
+  extern __shared__ double s_w[];  // [8][K]
   const int pc = blockIdx.x, col = blockIdx.y;
   if (a.cnt[level_off(l - 1) + pc] == 0) return;
   int px, py, pz;
@@ -211,28 +216,26 @@ __global__ void __launch_bounds__(FT) k_fmm_m2m(FmmArgs a, int l) {
   double hp[fmm::kMaxOrder + 1];  // (h_c / 2)^k
   hp[0] = 1.0;
   for (int k = 1; k <= a.p; ++k) hp[k] = hp[k - 1] * 0.5 * a.h0 / (1 << l);
-  double acc[kMaxTermsPerThread];
-  for (int j = 0; j < kMaxTermsPerThread; ++j) acc[j] = 0.0;
-  for (int ch = 0; ch < 8; ++ch) {
-    const int bx = ch >> 2, by = (ch >> 1) & 1, bz = ch & 1;
-    const int cc = cell_idx(l, 2 * px + bx, 2 * py + by, 2 * pz + bz);
-    if (a.cnt[level_off(l) + cc] == 0) continue;
-    const double *Mc = a.M + ((size_t)col * a.ncell + level_off(l) + cc) * a.K;
-    for (int j = 0; j < kMaxTermsPerThread; ++j) {
-      const int t = threadIdx.x + j * FT;
-      if (t >= a.K) break;
-      double w = 0.0;
+  const int ch = threadIdx.x / FT, lane = threadIdx.x % FT;
+  const int bx = ch >> 2, by = (ch >> 1) & 1, bz = ch & 1;
+  const int cc = cell_idx(l, 2 * px + bx, 2 * py + by, 2 * pz + bz);
+  const bool any = a.cnt[level_off(l) + cc] != 0;
+  const double *Mc = a.M + ((size_t)col * a.ncell + level_off(l) + cc) * a.K;
+  for (int t = lane; t < a.K; t += FT) {
+    double w = 0.0;
+    if (any)
       for (int e = a.mm_off[t]; e < a.mm_off[t + 1]; ++e) {
         const int2 ent = a.mm_e[e];
         w += Mc[ent.x] * a.mm_c[e] * hp[ent.y & 255] * child_sign(ent.y, bx, by, bz);
       }
-      acc[j] += w;
-    }
+    s_w[ch * a.K + t] = w;
   }
+  __syncthreads();
   double *Mp = a.M + ((size_t)col * a.ncell + level_off(l - 1) + pc) * a.K;
-  for (int j = 0; j < kMaxTermsPerThread; ++j) {
-    const int t = threadIdx.x + j * FT;
-    if (t < a.K) Mp[t] = acc[j];
+  for (int t = threadIdx.x; t < a.K; t += 8 * FT) {
+    double s = 0.0;
+    for (int k = 0; k < 8; ++k) s += s_w[k * a.K + t];
+    Mp[t] = s;
   }
 }
 
@@ -311,44 +314,70 @@ __global__ void k_fmm_m32(FmmArgs a, int first_cell, int ncells) {
   }
 }
 
-// the unit-offset derivative table of the arithmetic type
-template <typename T>
-__device__ __forceinline__ const T *tables(const FmmArgs &a);
-template <>
-__device__ __forceinline__ const double *tables<double>(const FmmArgs &a) {
-  return a.dunit;
-}
-template <>
-__device__ __forceinline__ const float *tables<float>(const FmmArgs &a) {
-  return a.dunit32;
+// The same M2L in FP32 for the cells of all levels in one launch, the (target
+// term, source term) pairs of each thread held in registers (PJ pairs per
+// thread of NT; 256 x 12 serve orders <= 8, 512 x 16 orders <= 10): the
+// multipoles (scaled to the cell size), the unit-offset derivatives and the
+// pair sums in FP32, the sum over source terms of each local term and the
+// local expansion in FP64.  The FP32 rounding (~1e-6 of a local coefficient)
+// is far below the expansion's own truncation error (~1e-4 at order 10), and
+// GB300 issues FP32 at 64x its FP64 rate.
+// A step (one source cell) is 16 multiply-adds per thread and column, less
+// than the latency of fetching the next cell's multipoles and derivatives, so
+// the sources are listed first and M2L_NB of them are fetched ahead with
+// asynchronous copies while the previous ones are used (both levels of a
+// 60,000-site box at order 10: 1.03 -> 0.74 ms).
+constexpr int M2L_NB = 4;
+
+__device__ __forceinline__ void copy_async4(float *dst, const float *src) {
+  const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
 }
 
-// The same M2L with the (target term, source term) pairs of each thread
-// held in registers (PJ pairs per thread of NT), both columns in one CTA
-// sharing the derivative row staged in shared memory.
-// instantiations: 256 threads x 12 pairs (orders <= 8), 512 x 16 (<= 10).
-// T = float: the multipoles (scaled to the cell size), the unit-offset
-// derivatives and the pair sums in FP32, the sum over source terms of each
-// local term and the local expansion in FP64.  The FP32 rounding (~1e-6
-// of a local coefficient) is far below the expansion's own truncation
-// error (~1e-4 at order 10), and GB300 issues FP32 at 64x its FP64 rate.
-template <typename T, int NT, int PJ>
-__global__ void __launch_bounds__(NT) k_fmm_m2l_reg(FmmArgs a, int l) {
-  extern __shared__ __align__(16) unsigned char sh_raw[];
-  T *sh = reinterpret_cast<T *>(sh_raw);
-  T *s_m = sh;                // [2][K]
-  T *s_d = sh + 2 * a.K;      // [KD]
-  T *s_acc = s_d + a.KD;      // [npairs]
-  const T *dunit = tables<T>(a);
+template <int NT, int PJ, int NCOL>
+__global__ void __launch_bounds__(NT) k_fmm_m2l_reg(FmmArgs a) {
+  extern __shared__ __align__(16) float sh32[];
+  __shared__ int s_src[192], s_off[192], s_n;
+  const int rec = (NCOL + 1) * a.K;  // K == KD: multipoles of the columns, derivatives
+  float *s_buf = sh32;               // [2][M2L_NB][rec]
+  float *s_acc = sh32;               // [npairs], after the last step
   const int npairs = a.hoff[a.K];
-  const int tc = blockIdx.x;
+  int l = 2;
+  while (level_off(l + 1) - level_off(2) <= (int)blockIdx.x) ++l;
+  const int tc = blockIdx.x - (level_off(l) - level_off(2));
   if (a.cnt_t[level_off(l) + tc] == 0) return;
   int tx, ty, tz;
   cell_xyz(tc, l, tx, ty, tz);
   const int n = 1 << l;
   const double hinv = (1 << l) / a.h0;
+  // the well-separated cells with sources, in a fixed order
+  if (threadIdx.x < 32) {
+    int cnt = 0;
+    for (int b = 0; b < 27 * 8; b += 32) {
+      const int i = b + threadIdx.x;
+      const int o = i >> 3, ch = i & 7;
+      const int sx = 2 * ((tx >> 1) + o / 9 - 1) + (ch >> 2), sy = 2 * ((ty >> 1) + (o / 3) % 3 - 1) + ((ch >> 1) & 1),
+                sz = 2 * ((tz >> 1) + o % 3 - 1) + (ch & 1);
+      const int dx = tx - sx, dy = ty - sy, dz = tz - sz;
+      bool take = i < 27 * 8 && sx >= 0 && sy >= 0 && sz >= 0 && sx < n && sy < n && sz < n &&
+                  !(abs(dx) <= 1 && abs(dy) <= 1 && abs(dz) <= 1);
+      int sc = 0;
+      if (take) {
+        sc = cell_idx(l, sx, sy, sz);
+        take = a.cnt[level_off(l) + sc] != 0;
+      }
+      const unsigned m = __ballot_sync(0xffffffffu, take);
+      if (take) {
+        const int k = cnt + __popc(m & ((1u << threadIdx.x) - 1u));
+        s_src[k] = sc;
+        s_off[k] = ((dx + 3) * 7 + (dy + 3)) * 7 + (dz + 3);
+      }
+      cnt += __popc(m);
+    }
+    if (threadIdx.x == 0) s_n = cnt;
+  }
   int pk[PJ];
-  T acc0[PJ], acc1[PJ];
+  float acc[NCOL][PJ];
 #pragma unroll
   for (int j = 0; j < PJ; ++j) {
     const int q = threadIdx.x + j * NT;
@@ -357,50 +386,49 @@ __global__ void __launch_bounds__(NT) k_fmm_m2l_reg(FmmArgs a, int l) {
       const int4 pr = a.pairs[q];
       pk[j] = pr.x | (pr.y << 10) | (pr.w << 20);
     }
-    acc0[j] = acc1[j] = T(0);
-  }
-  for (int ox = -1; ox <= 1; ++ox)
-    for (int oy = -1; oy <= 1; ++oy)
-      for (int oz = -1; oz <= 1; ++oz) {
-        const int PX = (tx >> 1) + ox, PY = (ty >> 1) + oy, PZ = (tz >> 1) + oz;
-        if (PX < 0 || PY < 0 || PZ < 0 || 2 * PX >= n || 2 * PY >= n || 2 * PZ >= n) continue;
-        for (int ch = 0; ch < 8; ++ch) {
-          const int sx = 2 * PX + (ch >> 2), sy = 2 * PY + ((ch >> 1) & 1), sz = 2 * PZ + (ch & 1);
-          const int dx = tx - sx, dy = ty - sy, dz = tz - sz;
-          if (abs(dx) <= 1 && abs(dy) <= 1 && abs(dz) <= 1) continue;
-          const int sc = cell_idx(l, sx, sy, sz);
-          if (a.cnt[level_off(l) + sc] == 0) continue;  // uniform over the CTA
-          __syncthreads();
-          for (int i = threadIdx.x; i < a.ncol * a.K; i += NT) {
-            const int col = i / a.K, g = i - col * a.K;
-            if constexpr (std::is_same<T, float>::value) {
-              s_m[i] = a.M32[((size_t)col * a.ncell + level_off(l) + sc) * a.K + g];  // k_fmm_m32
-            } else {
-              const int ng = a.terms[g].w;
-              double f = 1.0;
-              for (int r = 0; r < ng; ++r) f *= hinv;
-              s_m[i] = a.M[((size_t)col * a.ncell + level_off(l) + sc) * a.K + g] * f;
-            }
-          }
-          const T *D = dunit + (size_t)(((dx + 3) * 7 + (dy + 3)) * 7 + (dz + 3)) * a.KD;
-          for (int i = threadIdx.x; i < a.KD; i += NT) s_d[i] = D[i];
-          __syncthreads();
 #pragma unroll
-          for (int j = 0; j < PJ; ++j) {
-            if (pk[j] < 0) continue;
-            const int g = pk[j] & 1023;
-            const T d = (pk[j] >> 20) ? -s_d[(pk[j] >> 10) & 1023] : s_d[(pk[j] >> 10) & 1023];
-            acc0[j] += s_m[g] * d;
-            acc1[j] += s_m[a.K + g] * d;
-          }
-        }
+    for (int c = 0; c < NCOL; ++c) acc[c][j] = 0.f;
+  }
+  __syncthreads();
+  const int ns = s_n;
+  auto fetch = [&](int b0, int buf) {
+    for (int i = threadIdx.x; i < M2L_NB * rec; i += NT) {
+      const int k = i / rec, r = i - k * rec;
+      if (b0 + k >= ns) break;
+      const int col = r / a.K, g = r - col * a.K;
+      const float *src = col < NCOL ? a.M32 + ((size_t)col * a.ncell + level_off(l) + s_src[b0 + k]) * a.K + g
+                                    : a.dunit32 + (size_t)s_off[b0 + k] * a.KD + g;
+      copy_async4(&s_buf[(buf * M2L_NB + k) * rec + r], src);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  fetch(0, 0);
+  for (int b0 = 0, buf = 0; b0 < ns; b0 += M2L_NB, buf ^= 1) {
+    fetch(b0 + M2L_NB, buf ^ 1);  // an empty group after the last batch
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    const int kn = min(M2L_NB, ns - b0);
+    for (int k = 0; k < kn; ++k) {
+      const float *s_m = &s_buf[(buf * M2L_NB + k) * rec], *s_d = s_m + NCOL * a.K;
+#pragma unroll
+      for (int j = 0; j < PJ; ++j) {
+        if (pk[j] < 0) continue;
+        const int g = pk[j] & 1023;
+        const float d = (pk[j] >> 20) ? -s_d[(pk[j] >> 10) & 1023] : s_d[(pk[j] >> 10) & 1023];
+#pragma unroll
+        for (int c = 0; c < NCOL; ++c) acc[c][j] += s_m[c * a.K + g] * d;
       }
-  for (int col = 0; col < a.ncol; ++col) {
+    }
+    __syncthreads();  // the buffer is filled again by the next fetch
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+#pragma unroll
+  for (int col = 0; col < NCOL; ++col) {
     __syncthreads();
 #pragma unroll
     for (int j = 0; j < PJ; ++j) {
       const int q = threadIdx.x + j * NT;
-      if (q < npairs) s_acc[q] = col ? acc1[j] : acc0[j];
+      if (q < npairs) s_acc[q] = acc[col][j];
     }
     __syncthreads();
     double *Lt = a.Lc + ((size_t)col * a.ncell + level_off(l) + tc) * a.K;
@@ -441,94 +469,68 @@ __global__ void __launch_bounds__(FT) k_fmm_l2l(FmmArgs a, int l) {
   }
 }
 
-// far field of the leaf's local expansion plus the direct near field of the
-// 27 neighbouring leaves at each site of the leaf; field [col][n][3]
-template <bool AMOEBA>
-__global__ void __launch_bounds__(FT) k_fmm_l2p(FmmArgs a, const double *__restrict__ x, int n, double thr,
-                                                 float thr2m, double *__restrict__ field) {
-  __shared__ Pos64 s_pos[FT];
-  __shared__ double s_a[FT];
-  __shared__ float2 s_wa[FT];
-  __shared__ double s_mu[FT * 3];
-  __shared__ double s_L[fmm::nterms(fmm::kMaxOrder)];
+// position of the term (a, b, c) in the order of nested Horner schemes (a, then
+// b, then c from high to low)
+__device__ __forceinline__ int horner_pos(int p, int a, int b, int c) {
+  const int u = p - a, v = u - b;
+  return u * (u + 1) * (u + 2) / 6 + v * (v + 1) / 2 + (v - c);
+}
+// -grad sum_abc L_abc u^(abc) by nested Horner schemes over s_H (terms in
+// horner_pos order): about 3 FP64 operations per term instead of 12 with
+// the powers of each component formed apart (791 -> 154 us at 60,000 sites)
+__device__ __forceinline__ void horner_field(int p, const double *s_H, double X, double Y, double Z, double *e) {
+  double w = 0.0, wx = 0.0, wy = 0.0, wz = 0.0;
+  int i = 0;
+  for (int a = p; a >= 0; --a) {
+    double v = 0.0, vy = 0.0, vz = 0.0;
+    for (int b = p - a; b >= 0; --b) {
+      double s = 0.0, sz = 0.0;
+      for (int c = p - a - b; c >= 0; --c) {
+        sz = fma(sz, Z, s);
+        s = fma(s, Z, s_H[i++]);
+      }
+      vy = fma(vy, Y, v);
+      vz = fma(vz, Y, sz);
+      v = fma(v, Y, s);
+    }
+    wx = fma(wx, X, w);
+    wy = fma(wy, X, vy);
+    wz = fma(wz, X, vz);
+    w = fma(w, X, v);
+  }
+  e[0] -= wx;
+  e[1] -= wy;
+  e[2] -= wz;
+}
+
+// far field of the leaf's local expansion at each site of the leaf plus the
+// near field's partial sums (near [kFmmNearSplit][ncol][n][3], fmm_near.cu);
+// field [col][n][3]
+__global__ void __launch_bounds__(FT) k_fmm_l2p(FmmArgs a, int n, const double *__restrict__ near,
+                                                 double *__restrict__ field) {
+  __shared__ double s_H[fmm::nterms(fmm::kMaxOrder)];
   const int c = blockIdx.x, col = blockIdx.y;
   const int s0 = a.leaf_start[c], s1 = a.leaf_start[c + 1];
   if (s0 == s1) return;
   int cx, cy, cz;
   cell_xyz(c, a.L, cx, cy, cz);
-  const int nl = 1 << a.L;
-  const double h = a.h0 / nl;
-  const double ctr[3] = {a.ox + (cx + 0.5) * h, a.oy + (cy + 0.5) * h, a.oz + (cz + 0.5) * h};
+  const double h = a.h0 / (1 << a.L);
   const double *Lt = a.Lc + ((size_t)col * a.ncell + level_off(a.L) + c) * a.K;
-  for (int t = threadIdx.x; t < a.K; t += FT) s_L[t] = Lt[t];
-  for (int b0 = s0; b0 < s1; b0 += FT) {
-    const int si = b0 + threadIdx.x;
-    const bool valid = si < s1;
-    Pos64 pt = valid ? a.spos[si] : Pos64{0, 0, 0, 0};
-    const double at = valid && AMOEBA ? a.sa[si] : 0.0;
-    const float2 wat = valid ? a.swa[si] : make_float2(0.f, 0.f);
+  for (int t = threadIdx.x; t < a.K; t += FT) {
+    const short4 e = a.terms[t];
+    s_H[horner_pos(a.p, e.x, e.y, e.z)] = Lt[t];
+  }
+  __syncthreads();
+  for (int si = s0 + threadIdx.x; si < s1; si += FT) {
+    const Pos64 pt = a.spos[si];
     double e[3] = {0.0, 0.0, 0.0};
-    // near field 3 sum f d - sum k3 mu (f = k5 mu.d) as its two sums
-    double nf[3] = {0.0, 0.0, 0.0}, nk[3] = {0.0, 0.0, 0.0};
-    __syncthreads();
-    if (valid) {
-      const double u[3] = {pt.x - ctr[0], pt.y - ctr[1], pt.z - ctr[2]};
-      double pu[3][fmm::kMaxOrder + 1];
-      for (int d = 0; d < 3; ++d) {
-        pu[d][0] = 1.0;
-        for (int m = 1; m <= a.p; ++m) pu[d][m] = pu[d][m - 1] * u[d];
-      }
-      for (int t = 0; t < a.K; ++t) {
-        const short4 ex = a.terms[t];
-        const double Lv = s_L[t];
-        if (ex.x) e[0] -= Lv * ex.x * pu[0][ex.x - 1] * pu[1][ex.y] * pu[2][ex.z];
-        if (ex.y) e[1] -= Lv * ex.y * pu[0][ex.x] * pu[1][ex.y - 1] * pu[2][ex.z];
-        if (ex.z) e[2] -= Lv * ex.z * pu[0][ex.x] * pu[1][ex.y] * pu[2][ex.z - 1];
-      }
-    }
-    for (int ox = -1; ox <= 1; ++ox)
-      for (int oy = -1; oy <= 1; ++oy)
-        for (int oz = -1; oz <= 1; ++oz) {
-          const int X = cx + ox, Y = cy + oy, Z = cz + oz;
-          if (X < 0 || Y < 0 || Z < 0 || X >= nl || Y >= nl || Z >= nl) continue;
-          const int nc = cell_idx(a.L, X, Y, Z);
-          const int r0 = a.leaf_start[nc], r1 = a.leaf_start[nc + 1];
-          for (int t0 = r0; t0 < r1; t0 += FT) {
-            __syncthreads();
-            const int k = t0 + threadIdx.x;
-            if (k < r1) {
-              s_pos[threadIdx.x] = a.spos[k];
-              s_a[threadIdx.x] = AMOEBA ? a.sa[k] : 0.0;
-              s_wa[threadIdx.x] = a.swa[k];
-              const int pi = a.perm[k];
-              for (int d = 0; d < 3; ++d) s_mu[threadIdx.x * 3 + d] = x[((size_t)col * n + pi) * 3 + d];
-            }
-            __syncthreads();
-            if (!valid) continue;
-            const int cnt = min(FT, r1 - t0);
-            for (int q = 0; q < cnt; ++q) {
-              if (t0 + q == si) continue;
-              const Pos64 ps = s_pos[q];
-              const double dx = pt.x - ps.x, dy = pt.y - ps.y, dz = pt.z - ps.z;
-              const double r2 = dx * dx + dy * dy + dz * dz;
-              if (coincident(r2)) continue;
-              double k3, k5;
-              dd_pair_f64<AMOEBA>(r2, pt.w, ps.w, at, s_a[q], wat, s_wa[q], thr, thr2m, k3, k5);
-              const double *mu = &s_mu[q * 3];
-              const double f = k5 * (mu[0] * dx + mu[1] * dy + mu[2] * dz);
-              nf[0] = fma(f, dx, nf[0]);
-              nf[1] = fma(f, dy, nf[1]);
-              nf[2] = fma(f, dz, nf[2]);
-              nk[0] = fma(k3, mu[0], nk[0]);
-              nk[1] = fma(k3, mu[1], nk[1]);
-              nk[2] = fma(k3, mu[2], nk[2]);
-            }
-          }
-        }
-    if (valid) {
-      for (int d = 0; d < 3; ++d) e[d] += fma(3.0, nf[d], -nk[d]);
-      const int pi = a.perm[si];
-      for (int d = 0; d < 3; ++d) field[((size_t)col * n + pi) * 3 + d] = e[d];
+    horner_field(a.p, s_H, pt.x - (a.ox + (cx + 0.5) * h), pt.y - (a.oy + (cy + 0.5) * h),
+                 pt.z - (a.oz + (cz + 0.5) * h), e);
+    const size_t o = ((size_t)col * n + a.perm[si]) * 3;
+    for (int d = 0; d < 3; ++d) {
+      double s = 0.0;
+      for (int k = 0; k < kFmmNearSplit; ++k) s += near[(size_t)k * a.ncol * n * 3 + o + d];
+      field[o + d] = e[d] + s;
     }
   }
 }
@@ -620,7 +622,7 @@ __global__ void __launch_bounds__(FT) k_fmm_l2p_m2d(FmmArgs a, const int *__rest
   __shared__ float2 s_wa[FT];
   __shared__ int s_mm[FT];
   __shared__ double s_q[FT * LD];
-  __shared__ double s_L[fmm::nterms(fmm::kMaxOrder)];
+  __shared__ double s_H[fmm::nterms(fmm::kMaxOrder)];
   const int c = blockIdx.x;
   const int s0 = leaf_start_t[c], s1 = leaf_start_t[c + 1];
   if (s0 == s1) return;
@@ -630,7 +632,10 @@ __global__ void __launch_bounds__(FT) k_fmm_l2p_m2d(FmmArgs a, const int *__rest
   const double h = a.h0 / nl;
   const double ctr[3] = {a.ox + (cx + 0.5) * h, a.oy + (cy + 0.5) * h, a.oz + (cz + 0.5) * h};
   const double *Lt = a.Lc + ((size_t)level_off(a.L) + c) * a.K;
-  for (int t = threadIdx.x; t < a.K; t += FT) s_L[t] = Lt[t];
+  for (int t = threadIdx.x; t < a.K; t += FT) {
+    const short4 ex = a.terms[t];
+    s_H[horner_pos(a.p, ex.x, ex.y, ex.z)] = Lt[t];
+  }
   int bad = 0;
   for (int b0 = s0; b0 < s1; b0 += FT) {
     const int si = b0 + threadIdx.x;
@@ -641,21 +646,7 @@ __global__ void __launch_bounds__(FT) k_fmm_l2p_m2d(FmmArgs a, const int *__rest
     const int self = valid ? tmm[si] : -1;
     double e[3] = {0.0, 0.0, 0.0};
     __syncthreads();
-    if (valid) {
-      const double u[3] = {pt.x - ctr[0], pt.y - ctr[1], pt.z - ctr[2]};
-      double pu[3][fmm::kMaxOrder + 1];
-      for (int d = 0; d < 3; ++d) {
-        pu[d][0] = 1.0;
-        for (int m = 1; m <= a.p; ++m) pu[d][m] = pu[d][m - 1] * u[d];
-      }
-      for (int t = 0; t < a.K; ++t) {
-        const short4 ex = a.terms[t];
-        const double Lv = s_L[t];
-        if (ex.x) e[0] -= Lv * ex.x * pu[0][ex.x - 1] * pu[1][ex.y] * pu[2][ex.z];
-        if (ex.y) e[1] -= Lv * ex.y * pu[0][ex.x] * pu[1][ex.y - 1] * pu[2][ex.z];
-        if (ex.z) e[2] -= Lv * ex.z * pu[0][ex.x] * pu[1][ex.y] * pu[2][ex.z - 1];
-      }
-    }
+    if (valid) horner_field(a.p, s_H, pt.x - ctr[0], pt.y - ctr[1], pt.z - ctr[2], e);
     for (int ox = -1; ox <= 1; ++ox)
       for (int oy = -1; oy <= 1; ++oy)
         for (int oz = -1; oz <= 1; ++oz) {
@@ -790,6 +781,11 @@ void System::fmm_invalidate() {
 
 namespace {
 
+// shared memory of k_fmm_m2l_reg: two batches of sources, or the pair sums
+size_t m2l_smem(const FmmState &f, int ncol) {
+  return sizeof(float) * std::max<size_t>(2 * gpu::M2L_NB * (size_t)(ncol + 1) * f.K, f.npairs);
+}
+
 // per-order tables: terms, M2L pairs sorted by target term, unit-offset
 // derivative tensors, M2M / L2L translation lists
 int build_tables(FmmState &f, int p, cudaStream_t st) {
@@ -866,12 +862,12 @@ int build_tables(FmmState &f, int p, cudaStream_t st) {
   }
   const size_t smem = (f.K + (size_t)f.npairs) * sizeof(double);
   if (smem > 48 * 1024) cudaFuncSetAttribute(gpu::k_fmm_m2l, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  const size_t smem_reg = (2 * (size_t)f.K + f.KD + f.npairs) * sizeof(float);
-  if (smem_reg > 48 * 1024) {
-    cudaFuncSetAttribute(gpu::k_fmm_m2l_reg<float, 256, 12>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem_reg);
-    cudaFuncSetAttribute(gpu::k_fmm_m2l_reg<float, 512, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem_reg);
+  for (int ncol = 1; ncol <= 2; ++ncol) {
+    const int b = (int)m2l_smem(f, ncol);
+    const void *k[2] = {ncol == 2 ? (const void *)gpu::k_fmm_m2l_reg<256, 12, 2> : (const void *)gpu::k_fmm_m2l_reg<256, 12, 1>,
+                        ncol == 2 ? (const void *)gpu::k_fmm_m2l_reg<512, 16, 2> : (const void *)gpu::k_fmm_m2l_reg<512, 16, 1>};
+    if (b > 48 * 1024)
+      for (const void *fn : k) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
   }
   return cudaStreamSynchronize(st) == cudaSuccess ? kOk : kErrCuda;  // host vectors die here
 }
@@ -1015,25 +1011,33 @@ void tree_args(const FmmState &f, const FmmTree &t, int ncol, gpu::FmmArgs &a) {
 // upward pass from the leaf multipoles, M2L, downward pass (columns of a)
 void run_tree(const FmmState &f, const FmmTree &t, const gpu::FmmArgs &a, int ncol, cudaStream_t st) {
   const size_t smem = (f.K + (size_t)f.npairs) * sizeof(double);
-  for (int l = t.L; l >= 1; --l) gpu::k_fmm_m2m<<<dim3(1 << (3 * (l - 1)), ncol), gpu::FT, 0, st>>>(a, l);
-  const size_t smem_reg = (2 * (size_t)f.K + f.KD + f.npairs) * sizeof(float);
+  // no cell above level 2 has well-separated neighbours: their multipoles are not needed
+  for (int l = t.L; l >= 3; --l)
+    gpu::k_fmm_m2m<<<dim3(1 << (3 * (l - 1)), ncol), 8 * gpu::FT, 8 * (size_t)f.K * sizeof(double), st>>>(a, l);
+  const size_t smem_reg = m2l_smem(f, ncol);
   const bool reg = f.npairs <= 16 * 512;
+  const int c0 = ((1 << 6) - 1) / 7, nc = t.ncell - c0;  // the cells of levels 2..L
   if (reg && t.L >= 2) {
-    const int c0 = ((1 << 6) - 1) / 7, nc = t.ncell - c0;  // the cells of levels 2..L
     gpu::k_fmm_m32<<<gpu::sm_count() * 8, 256, 0, st>>>(a, c0, nc);
     gpu::add_launch_count(1);
   }
+  int launches = 1;
   if (f.npairs <= 12 * 256) {
-    for (int l = 2; l <= t.L; ++l)
-      gpu::k_fmm_m2l_reg<float, 256, 12><<<dim3(1 << (3 * l), 1), 256, smem_reg, st>>>(a, l);
-  } else if (f.npairs <= 16 * 512) {
-    for (int l = 2; l <= t.L; ++l)
-      gpu::k_fmm_m2l_reg<float, 512, 16><<<dim3(1 << (3 * l), 1), 512, smem_reg, st>>>(a, l);
+    if (ncol == 2)
+      gpu::k_fmm_m2l_reg<256, 12, 2><<<nc, 256, smem_reg, st>>>(a);
+    else
+      gpu::k_fmm_m2l_reg<256, 12, 1><<<nc, 256, smem_reg, st>>>(a);
+  } else if (reg) {
+    if (ncol == 2)
+      gpu::k_fmm_m2l_reg<512, 16, 2><<<nc, 512, smem_reg, st>>>(a);
+    else
+      gpu::k_fmm_m2l_reg<512, 16, 1><<<nc, 512, smem_reg, st>>>(a);
   } else {
     for (int l = 2; l <= t.L; ++l) gpu::k_fmm_m2l<<<dim3(1 << (3 * l), ncol), gpu::FT, smem, st>>>(a, l);
+    launches = t.L - 1;
   }
   for (int l = 2; l < t.L; ++l) gpu::k_fmm_l2l<<<dim3(1 << (3 * (l + 1)), ncol), gpu::FT, 0, st>>>(a, l);
-  gpu::add_launch_count(t.L + (t.L - 1) + std::max(0, t.L - 2));
+  gpu::add_launch_count(std::max(0, t.L - 2) + launches + std::max(0, t.L - 2));
 }
 
 }  // namespace
@@ -1075,6 +1079,14 @@ int System::fmm_prepare() {
     sa[s] = m_.damping[j];
     swa[s] = make_float2((float)(w * w), (float)(m_.damping[j] * m_.damping[j]));
   }
+  std::vector<float4> split(3 * (size_t)n);
+  {
+    std::vector<double> xs(3 * (size_t)n);
+    for (int s = 0; s < n; ++s) std::copy_n(&xp[3 * (size_t)o.perm_s[s]], 3, &xs[3 * (size_t)s]);
+    double whole[3];
+    for (int d = 0; d < 3; ++d) whole[d] = std::nearbyint(o.lo[d] + 0.5 * o.side);
+    gpu::split_coordinates(xs.data(), n, whole, split.data());
+  }
   t.L = o.L;
   t.h0 = o.side;
   t.ox = o.lo[0], t.oy = o.lo[1], t.oz = o.lo[2];
@@ -1082,7 +1094,7 @@ int System::fmm_prepare() {
   t.ncell = o.ncell;
   t.shared = true;
   int bad = upload(t.cnt, o.cnt_s, st_) | upload(t.leaf_start, o.start_s, st_) | upload(t.perm, o.perm_s, st_) |
-            upload(t.spos, spos, st_) | upload(t.sa, sa, st_) | upload(t.swa, swa, st_);
+            upload(t.spos, spos, st_) | upload(t.sa, sa, st_) | upload(t.swa, swa, st_) | upload(t.split, split, st_);
   t.cnt_t = t.cnt, t.leaf_start_t = t.leaf_start, t.perm_t = t.perm, t.spos_t = t.spos, t.sa_t = t.sa, t.swa_t = t.swa;
   if (t.nalloc_cell < t.ncell) {
     if (t.M) cudaFree(t.M);
@@ -1094,9 +1106,13 @@ int System::fmm_prepare() {
     t.nalloc_cell = t.ncell;
   }
   if (f.field_n < 6 * (size_t)n) {
+    // field, near-field partials and the scale of their dipoles
     if (f.field) cudaFree(f.field);
     f.field = nullptr;
-    bad |= cudaMalloc((void **)&f.field, 6 * (size_t)n * sizeof(double)) != cudaSuccess;
+    const size_t v = 6 * (size_t)n;
+    bad |= cudaMalloc((void **)&f.field, ((1 + gpu::kFmmNearSplit) * v + 1) * sizeof(double)) != cudaSuccess;
+    f.near = f.field ? f.field + v : nullptr;
+    f.word = f.field ? reinterpret_cast<unsigned *>(f.field + (1 + gpu::kFmmNearSplit) * v) : nullptr;
     f.field_n = 6 * (size_t)n;
   }
   if (bad) {
@@ -1134,12 +1150,12 @@ int System::fmm_tmu(int ncol, const double *x, double *y, bool dodiag) {
     cudaMemsetAsync(t.M, 0, 2 * (size_t)t.ncell * f.K * sizeof(double), st_);
     cudaMemsetAsync(t.Lc, 0, 2 * (size_t)t.ncell * f.K * sizeof(double), st_);
     const int nleaf = 1 << (3 * t.L);
-    gpu::k_fmm_p2m<<<dim3(nleaf, g), gpu::FT, 0, st_>>>(a, xg, n);
+    gpu::k_fmm_p2m<<<dim3(nleaf, g), (f.K + 31) / 32 * 32, 0, st_>>>(a, xg, n);
     run_tree(f, t, a, g, st_);
-    if (m_.amoeba)
-      gpu::k_fmm_l2p<true><<<dim3(nleaf, g), gpu::FT, 0, st_>>>(a, xg, n, d_.damp_thr, thr2m, f.field);
-    else
-      gpu::k_fmm_l2p<false><<<dim3(nleaf, g), gpu::FT, 0, st_>>>(a, xg, n, d_.damp_thr, thr2m, f.field);
+    gpu::launch_max_word(g * nv, xg, f.word, st_);
+    gpu::launch_fmm_near({n, t.L, g, m_.amoeba, t.leaf_start, t.perm, t.split, t.spos, t.sa, t.swa, d_.damp_thr, thr2m},
+                         xg, f.word, f.near, st_);
+    gpu::k_fmm_l2p<<<dim3(nleaf, g), gpu::FT, 0, st_>>>(a, n, f.near, f.field);
     gpu::add_launch_count(2);
     gpu::launch_tmu_finish64(d_, g, f.field, xg, dodiag, y + c0 * nv, st_);
   }

@@ -103,6 +103,25 @@ void launch_tmu_sym_prepare(const DevSites &s, int g, const double *x, unsigned 
                             unsigned long long *bad, cudaStream_t st);
 void launch_tmu_sym_finish(const DevSites &s, int g, const unsigned long long *lo, const unsigned long long *hi,
                            const unsigned long long *bad, const double *x, bool dodiag, double *y, cudaStream_t st);
+// the largest high word of |x| (the scale of the double-single products)
+void launch_max_word(size_t total, const double *x, unsigned *word, cudaStream_t st);
+// near field of the FMM (fmm_near.cu): the dipoles x [col][n][3] of the 27
+// neighbouring leaves at every site, sites sorted by leaf (split coordinates
+// [3][n], spos, sa, swa; perm the polarizable index); partial
+// [kFmmNearSplit][col][n][3] in polarizable order, word from launch_max_word
+struct FmmNearArgs {
+  int n, L, ncol;
+  bool amoeba;
+  const int *leaf_start, *perm;
+  const float4 *split;
+  const Pos64 *spos;
+  const double *sa;
+  const float2 *swa;
+  double thr;
+  float thr2m;
+};
+constexpr int kFmmNearSplit = 9;
+void launch_fmm_near(const FmmNearArgs &a, const double *x, const unsigned *word, double *partial, cudaStream_t st);
 // coordinates x [n][3] about a centre as three floats each, out [3][n]
 void split_coordinates(const double *x, int n, double centre[3], float4 *out);
 // FP32 inner operator with compensated cross-tile sums; x,y float.  Columns

@@ -53,7 +53,7 @@
 #include <algorithm>
 #include <cmath>
 
-#include "ds_math.cuh"
+#include "ds_pair.cuh"
 #include "kernels.h"
 #include "pair_math.cuh"
 
@@ -111,25 +111,6 @@ __device__ __forceinline__ float box_dist2(const float4 &alo, const float4 &ahi,
   return fmaf(gx, gx, fmaf(gy, gy, gz * gz));
 }
 
-// 2^e of the scaling of a product's dipoles from the largest high word of
-// |x| (0 when all are zero: no scaling)
-__device__ __forceinline__ int sym_exponent(unsigned emax) {
-  const int e = (int)(emax >> 20);
-  return e == 0 ? 0 : e - 1023 + 12;
-}
-__device__ __forceinline__ double pow2(int e) {  // |e| <= 1022
-  return __hiloint2double((1023 + e) << 20, 0);
-}
-// v 2^-e without leaving the range of a double's exponent
-__device__ __forceinline__ double scale_down(double v, int e) {
-  const int h = e / 2;
-  return v * pow2(-h) * pow2(-(e - h));
-}
-__device__ __forceinline__ double scale_up(double v, int e) {
-  const int h = e / 2;
-  return v * pow2(h) * pow2(e - h);
-}
-
 // exact addition into the fixed-point words like fixed_add, with integer
 // operations instead of FP64 ones
 __device__ __forceinline__ void fixed_add_int(unsigned long long *lo, unsigned long long *hi, double v,
@@ -163,112 +144,6 @@ __device__ __forceinline__ void fixed_add_int(unsigned long long *lo, unsigned l
   atomicAdd(hi, h + (old + l < old ? 1ull : 0ull));
 }
 
-// One side of a double-single pair: (ah, al) += K (mu.n) n - k3 mu.
-struct SymGeom {
-  float xh, xl, yh, yl, zh, zl;  // n = d y
-  float kh, kl;                  // -k3
-  float Kh, Kl;                  // 3 r^-5 / y^2
-};
-
-__device__ __forceinline__ void sym_diff(float th, float tm, float tl, float sh, float sm, float sl, float &h,
-                                         float &l) {
-  // grid splits: the two leading differences are exact and |th - sh| is 0 or
-  // at least |tm - sm|, so the fast sum is exact too
-  const float dh = th - sh, dm = tm - sm;
-  h = dh + dm;
-  l = (dm - (h - dh)) + (tl - sl);
-}
-
-// MASKED: pairs left to FP64 and the site itself give nothing here (masked is
-// set): the close ones and those whose damping reaches the leading float.
-// AMOEBA damping 1 - (1 + x) exp(-x) with x = a u^3 > 20 (from about 6.6 bohr
-// of 9 in water) differs from 1 by less than 2^-24, so an FP32 exponential in
-// the low parts is enough.  The radii keep the double-single share of the
-// product's error below that of the FP64 kernel this one replaced.
-template <bool MASKED, bool AMOEBA>
-__device__ __forceinline__ SymGeom sym_geometry(const float (&t)[9], const float (&s)[9], float2 wat, float2 was,
-                                                bool &masked) {
-  float dx, dy, dz, ex, ey, ez;
-  sym_diff(t[0], t[3], t[6], s[0], s[3], s[6], dx, ex);
-  sym_diff(t[1], t[4], t[7], s[1], s[4], s[7], dy, ey);
-  sym_diff(t[2], t[5], t[8], s[2], s[5], s[8], dz, ez);
-  const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-  const float y0 = rsqrtf(r2);
-  float y = fmaf(0.5f * y0, fmaf(-(r2 * y0), y0, 1.f), y0);
-  float damp3 = 0.f, damp5 = 0.f;
-  if (MASKED) {
-    if (AMOEBA) {
-      const float u2 = r2 * wat.x * was.x;
-      const float x2 = fminf(wat.y, was.y) * (u2 * u2 * u2);
-      masked = !(r2 >= kSymNear2) || !(x2 >= 400.1f);
-      if (!masked) {
-        const float x = x2 * rsqrtf(x2);
-        damp3 = __expf(-x);
-        damp5 = fmaf(x, damp3, damp3);
-      }
-    } else {
-      masked = !(r2 >= kSymNear2Wang) || maybe_damped_wang(r2, wat, was);
-    }
-    if (masked) y = 0.f;
-  }
-  SymGeom g;
-  g.xh = dx * y;
-  g.yh = dy * y;
-  g.zh = dz * y;
-  g.xl = fmaf(ex, y, fmaf(dx, y, -g.xh));
-  g.yl = fmaf(ey, y, fmaf(dy, y, -g.yh));
-  g.zl = fmaf(ez, y, fmaf(dz, y, -g.zh));
-  // eps = 1 - |n|^2: the squares added to 2 in exact fast sums
-  const float px = g.xh * g.xh, py = g.yh * g.yh, pz = g.zh * g.zh;
-  const float qx = fmaf(g.xh + g.xh, g.xl, fmaf(g.xh, g.xh, -px));
-  const float qy = fmaf(g.yh + g.yh, g.yl, fmaf(g.yh, g.yh, -py));
-  const float qz = fmaf(g.zh + g.zh, g.zl, fmaf(g.zh, g.zh, -pz));
-  const float s1 = 2.f + px, s2 = s1 + py, s3 = s2 + pz;
-  const float rx = px - (s1 - 2.f), ry = py - (s2 - s1), rz = pz - (s3 - s2);
-  const float eps = (3.f - s3) - (((qx + qy) + qz) + ((rx + ry) + rz));
-  // r^-3 = y^3 (1 - eps)^(-3/2), 3 r^-5 d d = 3 y^3 (1 - eps)^(-5/2) n n
-  const float w3 = eps * fmaf(1.875f, eps, 1.5f);
-  const float w5 = eps * fmaf(4.375f, eps, 2.5f);
-  const float y2 = y * y, y2l = fmaf(y, y, -y2);
-  const float Y = y2 * y, Yl = fmaf(y2l, y, fmaf(y2, y, -Y));
-  g.kh = -Y;
-  g.kl = -fmaf(Y, w3, Yl);
-  g.Kh = 3.f * Y;
-  g.Kl = fmaf(g.Kh, w5, fmaf(3.f, Yl, fmaf(3.f, Y, -g.Kh)));
-  if (MASKED && AMOEBA) {
-    g.kl = fmaf(-g.kh, damp3, g.kl);
-    g.Kl = fmaf(-g.Kh, damp5, g.Kl);
-  }
-  return g;
-}
-
-__device__ __forceinline__ void sym_acc(float &ah, float &al, float xh, float xl, float yh, float yl) {
-  const float p = xh * yh;
-  const float q = fmaf(xl, yh, fmaf(xh, yl, fmaf(xh, yh, -p)));
-  const dsf s = two_sum(ah, p);
-  ah = s.h;
-  al += s.l + q;
-}
-
-__device__ __forceinline__ void sym_column(const SymGeom &g, const float (&mh)[3], const float (&ml)[3],
-                                           float (&ah)[3], float (&al)[3]) {
-  const float q0 = mh[0] * g.xh, q1 = mh[1] * g.yh, q2 = mh[2] * g.zh;
-  const float f0 = fmaf(ml[0], g.xh, fmaf(mh[0], g.xl, fmaf(mh[0], g.xh, -q0)));
-  const float f1 = fmaf(ml[1], g.yh, fmaf(mh[1], g.yl, fmaf(mh[1], g.yh, -q1)));
-  const float f2 = fmaf(ml[2], g.zh, fmaf(mh[2], g.zl, fmaf(mh[2], g.zh, -q2)));
-  const dsf u1 = two_sum(q0, q1);
-  const dsf u2 = two_sum(u1.h, q2);
-  const float t = ((f0 + f1) + f2) + (u1.l + u2.l);
-  const float fh = g.Kh * u2.h;
-  const float fl = fmaf(g.Kl, u2.h, fmaf(g.Kh, t, fmaf(g.Kh, u2.h, -fh)));
-  sym_acc(ah[0], al[0], fh, fl, g.xh, g.xl);
-  sym_acc(ah[0], al[0], g.kh, g.kl, mh[0], ml[0]);
-  sym_acc(ah[1], al[1], fh, fl, g.yh, g.yl);
-  sym_acc(ah[1], al[1], g.kh, g.kl, mh[1], ml[1]);
-  sym_acc(ah[2], al[2], fh, fl, g.zh, g.zl);
-  sym_acc(ah[2], al[2], g.kh, g.kl, mh[2], ml[2]);
-}
-
 // the 32 x 32 pairs of a warp's sites and the sub-tile js in double-single;
 // NEAR: returns the number of pairs left to FP64 in the warp's queue
 template <int G, bool NEAR, bool AMOEBA>
@@ -295,7 +170,7 @@ __device__ __forceinline__ int sym_pairs(SymSmem<G> &sm, int js, int warp, int l
 #pragma unroll
     for (int k = 0; k < 9; ++k) s[k] = f[k];
     bool masked = false;
-    const SymGeom g = sym_geometry<NEAR, AMOEBA>(tg, s, wai, NEAR ? sm.wa[jl] : wai, masked);
+    const DsPair g = dsp_geometry<NEAR, AMOEBA>(tg, s, wai, NEAR ? sm.wa[jl] : wai, masked);
     if (NEAR) {
       // a sub-tile with itself meets every pair twice: queued once
       if (self) masked = masked && ((lane + t) & 31) > lane;
@@ -308,8 +183,8 @@ __device__ __forceinline__ int sym_pairs(SymSmem<G> &sm, int js, int warp, int l
     for (int c = 0; c < G; ++c) {
       const float mh[3] = {f[9 + 6 * c], f[10 + 6 * c], f[11 + 6 * c]};
       const float ml[3] = {f[12 + 6 * c], f[13 + 6 * c], f[14 + 6 * c]};
-      sym_column(g, mh, ml, aih[c], ail[c]);
-      sym_column(g, mih[c], mil[c], ajh[c], ajl[c]);
+      dsp_column(g, mh, ml, aih[c], ail[c]);
+      dsp_column(g, mih[c], mil[c], ajh[c], ajl[c]);
     }
     // the accumulators of source s move to the lane that meets s next
 #pragma unroll
@@ -389,7 +264,7 @@ __global__ void __launch_bounds__(SYM_TILE, G == 1 ? 5 : 3) k_tmu_sym(const __gr
     const int I = unit / jb.nchunk;
     const int ti = I * SYM_TILE + tid;
     const bool vi = ti < n;
-    const int ex = sym_exponent(*reinterpret_cast<const unsigned *>(jb.bad + 1));
+    const int ex = dsp_exponent(*reinterpret_cast<const unsigned *>(jb.bad + 1));
     float tg[9], mih[G][3], mil[G][3];
     {
       const float4 h = vi ? gc[ti] : make_float4(SYM_FAR, SYM_FAR, SYM_FAR, 0.f);
@@ -499,14 +374,16 @@ __global__ void __launch_bounds__(SYM_TILE, G == 1 ? 5 : 3) k_tmu_sym(const __gr
   }
 }
 
-// accumulators to zero and the largest high word of |x| (ctl[1]; the flag and
-// ctl were zeroed before)
+// accumulators (if any) to zero and the largest high word of |x| (ctl, zeroed
+// before)
 __global__ void __launch_bounds__(256) k_sym_prepare(size_t total, const double *__restrict__ x,
                                                      unsigned long long *__restrict__ acc, unsigned *ctl) {
   unsigned m = 0;
   for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += (size_t)gridDim.x * blockDim.x) {
-    acc[k] = 0ull;
-    acc[total + k] = 0ull;
+    if (acc) {
+      acc[k] = 0ull;
+      acc[total + k] = 0ull;
+    }
     m = max(m, (unsigned)__double2hiint(x[k]) & 0x7FFFFFFFu);
   }
   m = __reduce_max_sync(0xffffffffu, m);
@@ -526,7 +403,7 @@ __global__ void __launch_bounds__(128) k_tmu_sym_finish(
   if (j >= n) return;
   const size_t col = (size_t)blockIdx.y * n, o = (col + j) * 3;
   const bool nan = *bad != 0ull;
-  const int ex = sym_exponent(*reinterpret_cast<const unsigned *>(bad + 1));
+  const int ex = dsp_exponent(*reinterpret_cast<const unsigned *>(bad + 1));
   double e[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c)
@@ -721,6 +598,13 @@ void launch_tmu_sym_prepare(const DevSites &s, int g, const double *x, unsigned 
   cudaMemsetAsync(bad, 0, 2 * sizeof(unsigned long long), st);
   const int blocks = (int)std::min<size_t>((total + 255) / 256, 1216);
   k_sym_prepare<<<blocks, 256, 0, st>>>(total, x, lo, reinterpret_cast<unsigned *>(bad + 1));
+}
+
+void launch_max_word(size_t total, const double *x, unsigned *word, cudaStream_t st) {
+  add_launch_count(1);
+  cudaMemsetAsync(word, 0, sizeof(unsigned), st);
+  const int blocks = (int)std::min<size_t>((total + 255) / 256, 1216);
+  k_sym_prepare<<<blocks, 256, 0, st>>>(total, x, nullptr, word);
 }
 
 void launch_tmu_sym_finish(const DevSites &s, int g, const unsigned long long *lo, const unsigned long long *hi,
