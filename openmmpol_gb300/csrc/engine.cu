@@ -124,7 +124,7 @@ System::~System() {
   if (st_) cudaStreamSynchronize(st_);
   free_ws(ws_);
   free_ws(wsb_);
-  void *bufs[] = {d_.pol_pos, d_.pol_a, d_.pol_alpha, d_.polar_mm, d_.pol_pos32, d_.pol_pos32lo, d_.pol_a32,
+  void *bufs[] = {inv32_, sqrt_alpha_, d_.pol_pos, d_.pol_a, d_.pol_alpha, d_.polar_mm, d_.pol_pos32, d_.pol_pos32lo, d_.pol_a32,
                   d_.pol_wa32, ds_scratch_, d_.mm_pos32, d_.mm_pos32lo, d_.mm_tile_box32,
                   d_.mm_wa32, d_.mm_pos,
                   d_.mm_a, d_.mm_q, d_.m2d_ri, d_.m2d_src, d_.m2d_sP, d_.m2d_sD, d_.d2d_ri, d_.d2d_src,
@@ -651,7 +651,7 @@ int System::ensure_tmat() {
   }
   gpu::launch_build_tmat(d_, tmat_, st_);
   tmat_ok_ = true;
-  lu_ok_ = false;
+  lu_ok_ = inv_ok_ = inv_failed_ = false;
   return check(cudaGetLastError(), "T matrix");
 }
 
@@ -866,9 +866,79 @@ int System::diis64(int matv, const double *rhs, double *x, int set) {
   return kOk;
 }
 
+// The inversion solver: the FP32 inverse of T refined in FP64 (dense.cu), or
+// the FP64 LU factors where that is not enough.
 int System::inversion64(const double *rhs, double *x) {
+  // without T its LU factors are in its place: this geometry needs them
+  if (!tmat_ok_ && lu_ok_) return lu64(rhs, x);
   int st = ensure_tmat();
   if (st) return st;
+  bool done = false;
+  st = refine_inverse(rhs, x, done);
+  if (st || done) return st;
+  return lu64(rhs, x);
+}
+
+// done: x is the solution to FP64 accuracy (the residual, relative to rhs,
+// below 1e-13 and no longer decreasing)
+int System::refine_inverse(const double *rhs, double *x, bool &done) {
+  done = false;
+  const int nn = 3 * d_.n;
+  if (!inv_ok_) {
+    if (inv_failed_) return kOk;
+    if (!inv32_ && (alloc(inv32_, gpu::inverse32_floats(nn)) || alloc(sqrt_alpha_, (size_t)nn))) {
+      cudaGetLastError();
+      release(inv32_);
+      inv32_ = nullptr;
+      inv_failed_ = true;  // the LU factorisation reports its own memory
+      return kOk;
+    }
+    gpu::launch_inverse32(nn, tmat_, d_.pol_alpha, sqrt_alpha_, inv32_, info_, st_);
+    int info = 0;
+    cudaMemcpyAsync(&info, info_, sizeof(int), cudaMemcpyDeviceToHost, st_);
+    const int st = check(cudaStreamSynchronize(st_), "inverse of T");
+    if (st) return st;
+    if (info) {  // not positive definite
+      inv_failed_ = true;
+      return kOk;
+    }
+    inv_ok_ = true;
+  }
+  // x and r of this solve: best so far in x, the next iterate in h_
+  double *xn = h_, *r = r_;
+  const size_t bytes = (size_t)nn * sizeof(double);
+  cudaMemsetAsync(xn, 0, bytes, st_);
+  cudaMemcpyAsync(r, rhs, bytes, cudaMemcpyDeviceToDevice, st_);
+  double first = 0.0, prev = 0.0;
+  for (int it = 0; it < 20; ++it) {
+    gpu::launch_dots(1, nn, r, r, partial_, st_);
+    gpu::launch_reduce_partials(1, partial_, dots_, st_);
+    cudaMemcpyAsync(scal_h_, dots_, sizeof(double), cudaMemcpyDeviceToHost, st_);
+    const int st = check(cudaStreamSynchronize(st_), "refinement of the inverse");
+    if (st) return st;
+    const double rms = std::sqrt(scal_h_[0] / nn);
+    if (it == 0) {
+      first = rms;
+      if (rms == 0.0) {
+        cudaMemsetAsync(x, 0, bytes, st_);
+        done = true;
+        return kOk;
+      }
+    }
+    if (!std::isfinite(rms)) return kOk;
+    if (it == 0 || rms < prev) cudaMemcpyAsync(x, xn, bytes, cudaMemcpyDeviceToDevice, st_);
+    if (it > 0 && !(rms < 0.25 * prev)) {
+      done = std::min(rms, prev) <= 1e-13 * first;
+      return kOk;
+    }
+    prev = rms;
+    gpu::launch_inverse32_step(nn, inv32_, sqrt_alpha_, r, 1.0 / rms, xn, st_);
+    gpu::launch_dense_residual(nn, tmat_, xn, rhs, r, st_);
+  }
+  return kOk;
+}
+
+int System::lu64(const double *rhs, double *x) {
   size_t nn = 3 * (size_t)d_.n;
   if (!lu_ok_) {
     double *lu = nullptr;
@@ -880,7 +950,7 @@ int System::inversion64(const double *rhs, double *x) {
     gpu::launch_lu_factor((int)nn, lu, piv_, info_, nullptr, st_);
     int info = 0;
     cudaMemcpyAsync(&info, info_, sizeof(int), cudaMemcpyDeviceToHost, st_);
-    st = check(cudaStreamSynchronize(st_), "LU");
+    const int st = check(cudaStreamSynchronize(st_), "LU");
     if (st) {
       cudaFree(lu);
       return st;
@@ -890,7 +960,8 @@ int System::inversion64(const double *rhs, double *x) {
       set_last_error("inversion solver: singular interaction matrix");
       return kErrNumeric;
     }
-    // the factors replace T; an in-core matvec rebuilds T on demand
+    // the factors replace T; an in-core matvec rebuilds T on demand, and the
+    // solver stays with the factors for this geometry
     std::swap(lu, tmat_);
     cudaFree(lu);
     tmat_ok_ = false;
@@ -1068,7 +1139,7 @@ int System::update_coordinates(const double *c) {
   m2d_done_ = ipd_done_ = ipd_use_guess_ = false;
   fixedelec_done_ = false;
   fixedelec_grad_done_ = false;
-  tmat_ok_ = lu_ok_ = false;
+  tmat_ok_ = lu_ok_ = inv_ok_ = inv_failed_ = false;
   return upload_geometry();
 }
 

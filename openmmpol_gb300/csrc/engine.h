@@ -217,6 +217,8 @@ class System {
   int cg64(int matv, int ncol, const double *rhs, double *x, int set0) { return cg64_ws(ws_, matv, ncol, rhs, x, set0); }
   int diis64(int matv, const double *rhs, double *x, int set);
   int inversion64(const double *rhs, double *x);
+  int refine_inverse(const double *rhs, double *x, bool &done);
+  int lu64(const double *rhs, double *x);
   int mixed_ir(int ncol, const double *rhs, double *x, int set0, bool have_guess) {
     return mixed_ir_ws(ws_, ncol, rhs, x, set0, have_guess);
   }
@@ -292,7 +294,10 @@ class System {
   double *tmat_ = nullptr;
   int *piv_ = nullptr;
   int *info_ = nullptr;
-  bool tmat_ok_ = false, lu_ok_ = false;
+  // FP32 inverse of T for the inversion solver and the square roots of alpha
+  float *inv32_ = nullptr;
+  double *sqrt_alpha_ = nullptr;
+  bool tmat_ok_ = false, lu_ok_ = false, inv_ok_ = false, inv_failed_ = false;
   double *diis_x_ = nullptr, *diis_e_ = nullptr;
   int nsplit_m2d_ = 1, nsplit_tmu32_ = 1;
   int maxhist_ = 1024;

@@ -307,19 +307,6 @@ __global__ void k_scale_tmat(int n, const int *__restrict__ ri, const int *__res
   }
 }
 
-// y = A x (- diag(A) x when !dodiag), column major, nrhs columns
-__global__ void k_gemv(int nn, const double *__restrict__ A, const double *__restrict__ x,
-                       double *__restrict__ y, bool dodiag, const double *__restrict__ alpha) {
-  int r = blockIdx.x * blockDim.x + threadIdx.x;
-  int c0 = blockIdx.y;  // rhs
-  if (r >= nn) return;
-  const double *xv = x + (size_t)c0 * nn;
-  double acc = 0.0;
-  for (int c = 0; c < nn; ++c) acc += A[(size_t)c * nn + r] * xv[c];
-  if (!dodiag) acc -= xv[r] / alpha[r / 3];
-  y[(size_t)c0 * nn + r] = acc;
-}
-
 // LU: pivot search in column k (one block), swap, update, scale
 __global__ void k_lu_pivot(int nn, int k, double *A, int *piv, int *info) {
   __shared__ double sv[1024];
@@ -1066,13 +1053,6 @@ void launch_build_tmat(const DevSites &s, double *tmat, cudaStream_t st) {
   else
     k_build_tmat<false><<<grid, 128, 0, st>>>(s.n, s.pol_pos, s.pol_a, s.pol_alpha, s.damp_thr, tmat);
   if (s.d2d_nnz) k_scale_tmat<<<(s.n + 127) / 128, 128, 0, st>>>(s.n, s.d2d_ri, s.d2d_src, s.d2d_s, tmat);
-}
-
-void launch_gemv(int nn, const double *A, const double *x, double *y, bool dodiag, const double *alpha,
-                 int nrhs, cudaStream_t st) {
-  add_launch_count(1);
-  dim3 grid((nn + 127) / 128, nrhs);
-  k_gemv<<<grid, 128, 0, st>>>(nn, A, x, y, dodiag, alpha);
 }
 
 void launch_lu_factor(int nn, double *A, int *piv, int *info, double *work, cudaStream_t st) {

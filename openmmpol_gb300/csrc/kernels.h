@@ -224,6 +224,17 @@ void launch_scale_alpha32(int ncol, int n, const float *alpha, const float *r, f
 void launch_build_tmat(const DevSites &s, double *tmat, cudaStream_t st);  // [3n][3n] col-major
 void launch_gemv(int nn, const double *A, const double *x, double *y, bool dodiag,
                  const double *alpha, int nrhs, cudaStream_t st);
+// r = rhs - T x
+void launch_dense_residual(int nn, const double *T, const double *x, const double *rhs, double *r, cudaStream_t st);
+// FP32 inverse of the symmetric positive definite T (dense.cu): buf of
+// inverse32_floats(nn), s [nn] the square roots of the polarizabilities; info
+// (device int) 0 = ok.  launch_inverse32_step: x += T^-1 r with it (scale:
+// about the inverse of r's size, so that r fits FP32).
+size_t inverse32_floats(int nn);
+void launch_inverse32(int nn, const double *T, const double *alpha, double *s, float *buf, int *info,
+                      cudaStream_t st);
+void launch_inverse32_step(int nn, float *buf, const double *s, const double *r, double scale, double *x,
+                           cudaStream_t st);
 // LU with partial pivoting in place (column major); info (device int) 0 = ok.
 void launch_lu_factor(int nn, double *A, int *piv, int *info, double *work, cudaStream_t st);
 void launch_lu_solve(int nn, const double *A, const int *piv, double *b, cudaStream_t st);
