@@ -51,22 +51,24 @@ __device__ __forceinline__ dsf ds_mulf(dsf x, float y) {
   e = fmaf(x.l, y, e);
   return fast_two_sum(p, e);
 }
-// (ah + al) - (bh + bl): the hi difference is exact, the lo difference
-// rounds once; absolute error ~2^-48 of the operands (coordinates)
-__device__ __forceinline__ dsf ds_diff(float ah, float al, float bh, float bl) {
-  dsf s = two_sum(ah, -bh);
-  return fast_two_sum(s.h, s.l + (al - bl));
+// t - s of two coordinates split on a common grid (split_coordinates): the two
+// leading differences are exact and |th - sh| is 0 or at least |tm - sm|, so
+// the fast sum is exact too
+__device__ __forceinline__ dsf ds_delta(float th, float tm, float tl, float sh, float sm, float sl) {
+  const float dh = th - sh, dm = tm - sm;
+  const float h = dh + dm;
+  return {h, (dm - (h - dh)) + (tl - sl)};
 }
-// 1/sqrt(a): FP32 estimate y, one Newton step y (1 + (1 - a y^2) / 2) with
-// 1 - a y^2 formed in double-single (the estimate's 2^-22 error squares)
+// 1/sqrt(a): FP32 estimate refined by one FP32 Newton step to y, then
+// y (1 + e / 2 + 3 e^2 / 8), e = 1 - a y^2 formed in double-single
 __device__ __forceinline__ dsf ds_rsqrt(dsf a) {
-  float y = rsqrtf(a.h);
-  float p = y * y;
-  dsf y2{p, fmaf(y, y, -p)};
-  dsf t = ds_mul(a, y2);
-  float e = (1.0f - t.h) - t.l;  // 1 - t.h is exact: t.h is within 2^-21 of 1
-  float c = (0.5f * y) * e;
-  return fast_two_sum(y, c);
+  const float y0 = rsqrtf(a.h);
+  const float y = fmaf(0.5f * y0, fmaf(-(a.h * y0), y0, 1.f), y0);
+  const float p = y * y;
+  const float th = a.h * p;
+  const float tl = fmaf(a.l, p, fmaf(a.h, fmaf(y, y, -p), fmaf(a.h, p, -th)));
+  const float e = (1.0f - th) - tl;  // 1 - th is exact: th is within 2^-21 of 1
+  return fast_two_sum(y, (y * e) * fmaf(0.375f, e, 0.5f));
 }
 // acc += p_exact(x * y) with x, y double-single, lazily (acc.l collects the
 // low-order parts; the caller renormalises)

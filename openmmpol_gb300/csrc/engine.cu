@@ -124,8 +124,8 @@ System::~System() {
   if (st_) cudaStreamSynchronize(st_);
   free_ws(ws_);
   free_ws(wsb_);
-  void *bufs[] = {inv32_, sqrt_alpha_, d_.pol_pos, d_.pol_a, d_.pol_alpha, d_.polar_mm, d_.pol_pos32, d_.pol_pos32lo, d_.pol_a32,
-                  d_.pol_wa32, ds_scratch_, d_.mm_pos32, d_.mm_pos32lo, d_.mm_tile_box32,
+  void *bufs[] = {inv32_, sqrt_alpha_, d_.pol_pos, d_.pol_a, d_.pol_alpha, d_.polar_mm, d_.pol_pos32, d_.pol_a32,
+                  d_.pol_wa32, d_.mm_split, d_.mm_tile_box32,
                   d_.mm_wa32, d_.mm_pos,
                   d_.mm_a, d_.mm_q, d_.m2d_ri, d_.m2d_src, d_.m2d_sP, d_.m2d_sD, d_.d2d_ri, d_.d2d_src,
                   d_.d2d_s, e_m2d_, ipd_, rhs_, ext_, x_, r_, p_, h_, z_, x32_, r32_, p32_, h32_, z32_,
@@ -201,12 +201,9 @@ size_t System::device_bytes_estimate() const {
   size_t bytes = 8 * (6 * n + 5 * m + m * m_.ld_cart + 2 * nm2d + nd2d + nv * (2 * nipd + 3 + 10)) +
                  4 * (9 * n + 2 * m + 10 * nv + 2 * (n + 1) + nm2d + nd2d) + 4 * s32 + 8 * s64 + 8 * sym +
                  8 * (gpu::kRedBlocks * 32 + 64 + 2 * (size_t)maxhist_);
-  // double-single copies of the positions, static-site tile boxes, and the
-  // double-single kernels' split partials (allocated in that mode only)
-  const size_t ds_split = gpu::m2d_ds_pick_split(d, sms);
-  bytes += 16 * (n + 2 * m + 2 * ((m + 127) / 128)) + 8 * ds_split * nv;
-  // coordinate splits and 32-site boxes of the symmetric product
-  bytes += 16 * (3 * n + 2 * ((n + 31) / 32));
+  bytes += 16 * (n + 2 * ((m + 127) / 128));
+  // coordinate splits and 32-site boxes of the double-single kernels
+  bytes += 16 * (3 * n + 3 * m + 2 * ((n + 31) / 32));
   // near-field couplings of the Neumann step (about a dozen per site in water)
   if (inner_precond_ == 2) bytes += 4 * (n + 1) + 40 * 24 * n;
   return bytes + (size_t(4) << 20);  // events, flags, rounding
@@ -256,7 +253,7 @@ int System::upload_static() {
   int nipd = m.n_ipd;
   int bad = 0;
   bad |= alloc(d_.pol_pos, n) | alloc(d_.pol_a, n) | alloc(d_.pol_alpha, n) | alloc(d_.polar_mm, n);
-  bad |= alloc(d_.pol_pos32, n) | alloc(d_.pol_pos32lo, n) | alloc(d_.pol_a32, n) | alloc(alpha32_, n);
+  bad |= alloc(d_.pol_pos32, n) | alloc(d_.pol_a32, n) | alloc(alpha32_, n);
   bad |= alloc(d_.pol_wa32, n) | alloc(d_.mm_wa32, mm);
   bad |= alloc(d_.mm_pos, mm) | alloc(d_.mm_a, mm) | alloc(d_.mm_q, (size_t)mm * m.ld_cart);
   bad |= alloc(d_.m2d_ri, n + 1) | alloc(d_.m2d_src, m2d_pairs_.src.size()) |
@@ -272,7 +269,7 @@ int System::upload_static() {
   bad |= alloc(scratch_, scratch_n_) | alloc(scratch32_, gpu::tmu_scratch_doubles(d_, 2, f32_splits));
   bad |= alloc(d_.tile_box32, 2 * (size_t)d_.ntile) | alloc(d_.pol_split, 3 * (size_t)n) |
          alloc(d_.sub_box32, 2 * (size_t)((n + 31) / 32));
-  bad |= alloc(d_.mm_pos32, mm) | alloc(d_.mm_pos32lo, mm) | alloc(d_.mm_tile_box32, 2 * (size_t)((mm + 127) / 128));
+  bad |= alloc(d_.mm_split, 3 * (size_t)mm) | alloc(d_.mm_tile_box32, 2 * (size_t)((mm + 127) / 128));
   bad |= alloc(partial_, (size_t)gpu::kRedBlocks * 32) | alloc(dots_, 64) | alloc(hist_, 2 * (size_t)maxhist_);
   bad |= alloc(cols_, 2) | alloc(flag_, 1) | alloc(info_, 1);
   if (bad || pinned_alloc((void **)&cols_h_, 2 * sizeof(gpu::CgCol)) != cudaSuccess ||
@@ -353,7 +350,7 @@ int System::upload_geometry() {
   int n = m.npol, mm = m.mm;
   const double inf = std::numeric_limits<double>::infinity();
   std::vector<gpu::Pos64> pp(n), mp(mm);
-  std::vector<float4> pp32(n), pp32lo(n);
+  std::vector<float4> pp32(n);
   std::vector<double> ma(mm, 0.0);
   double c[3] = {0, 0, 0};
   for (int i = 0; i < mm; ++i)
@@ -366,8 +363,6 @@ int System::upload_geometry() {
     pp[j] = gpu::Pos64{x[0], x[1], x[2], w};
     const double xc[3] = {x[0] - c[0], x[1] - c[1], x[2] - c[2]};
     pp32[j] = make_float4((float)xc[0], (float)xc[1], (float)xc[2], (float)w);
-    pp32lo[j] = make_float4((float)(xc[0] - (double)pp32[j].x), (float)(xc[1] - (double)pp32[j].y),
-                            (float)(xc[2] - (double)pp32[j].z), 0.f);
     for (int k = 0; k < 3; ++k) cpol_h_[3 * (size_t)j + k] = x[k];
   }
   for (int i = 0; i < mm; ++i) {
@@ -378,34 +373,32 @@ int System::upload_geometry() {
   }
   h2d(d_.pol_pos, pp.data(), n * sizeof(gpu::Pos64));
   h2d(d_.pol_pos32, pp32.data(), n * sizeof(float4));
-  h2d(d_.pol_pos32lo, pp32lo.data(), n * sizeof(float4));
   std::vector<float4> boxes(2 * (size_t)d_.ntile);
   gpu::tile_boxes32(pp32.data(), n, boxes.data());
   if (n) h2d(d_.tile_box32, boxes.data(), boxes.size() * sizeof(float4));
-  // symmetric FP64 product: 32-site boxes, and the coordinates about the
+  // double-single kernels: 32-site boxes, and the coordinates about the
   // centroid rounded to whole bohr (so that the shift is exact) in three floats
-  std::vector<float4> subs(2 * (size_t)((n + 31) / 32)), split(3 * (size_t)n);
+  std::vector<float4> subs(2 * (size_t)((n + 31) / 32)), msplit(3 * (size_t)mm), split(3 * (size_t)n);
   gpu::tile_boxes32(pp32.data(), n, subs.data(), 32);
   double whole[3] = {std::nearbyint(c[0]), std::nearbyint(c[1]), std::nearbyint(c[2])};
-  gpu::split_coordinates(cpol_h_.data(), n, whole, split.data());
+  gpu::split_coordinates(m.cmm.data(), mm, whole, msplit.data());
+  for (int p = 0; p < 3; ++p)
+    for (int j = 0; j < n; ++j) split[(size_t)p * n + j] = msplit[(size_t)p * mm + m.polar_mm[j]];
+  if (mm) h2d(d_.mm_split, msplit.data(), msplit.size() * sizeof(float4));
   if (n) {
     h2d(d_.sub_box32, subs.data(), subs.size() * sizeof(float4));
     h2d(d_.pol_split, split.data(), split.size() * sizeof(float4));
   }
-  // static sites in double-single for the double-single E_M2D
-  std::vector<float4> mp32(mm), mp32lo(mm);
+  // tile boxes of the static sites
+  std::vector<float4> mp32(mm);
   for (int i = 0; i < mm; ++i) {
     const double *x = &m.cmm[3 * (size_t)i];
     const double xc[3] = {x[0] - c[0], x[1] - c[1], x[2] - c[2]};
     mp32[i] = make_float4((float)xc[0], (float)xc[1], (float)xc[2], 0.f);
-    mp32lo[i] = make_float4((float)(xc[0] - (double)mp32[i].x), (float)(xc[1] - (double)mp32[i].y),
-                            (float)(xc[2] - (double)mp32[i].z), 0.f);
   }
   std::vector<float4> mboxes(2 * (size_t)((mm + 127) / 128));
   gpu::tile_boxes32(mp32.data(), mm, mboxes.data());
   if (mm) {
-    h2d(d_.mm_pos32, mp32.data(), mm * sizeof(float4));
-    h2d(d_.mm_pos32lo, mp32lo.data(), mm * sizeof(float4));
     h2d(d_.mm_tile_box32, mboxes.data(), mboxes.size() * sizeof(float4));
   }
   h2d(d_.mm_pos, mp.data(), mm * sizeof(gpu::Pos64));
@@ -589,30 +582,23 @@ int System::flush_l2(size_t bytes) {
 }
 
 int System::ensure_m2d() {
-  // the method the mode asks for: double-single in the mixed-ds mode, the
-  // FMM when it is switched on, else the direct FP64 sums; a cached field
-  // serves if it came from that method or from the direct FP64 sums
-  const bool ds = precision_ == kPrecMixedDS;
-  const int want = ds ? kM2dDS : (fmm_on_ ? kM2dFMM : kM2dDirect);
+  // the method the mode asks for: the FMM when it is switched on (mixed-ds
+  // takes the direct sums), else the direct sums; a cached field serves if it
+  // came from that method or from the direct sums
+  const bool fmm = fmm_on_ && precision_ != kPrecMixedDS;
+  const int want = fmm ? kM2dFMM : kM2dDirect;
   if (m2d_done_ && (m2d_method_ == want || m2d_method_ == kM2dDirect)) return kOk;
   cudaMemsetAsync(flag_, 0, sizeof(int), st_);
   int method = kM2dDirect;
-  if (ds) {
-    int st = ensure_ds_scratch();
+  bool done = false;
+  if (fmm) {  // the fast multipole method (too small a system: direct)
+    int st = fmm_m2d(e_m2d_, done);
     if (st) return st;
-    gpu::launch_m2d_ds(d_, e_m2d_, ds_scratch_, nsplit_m2d_ds_, flag_, st_);
-    method = kM2dDS;
-  } else {
-    bool done = false;
-    if (fmm_on_) {  // the fast multipole method (too small a system: direct)
-      int st = fmm_m2d(e_m2d_, done);
-      if (st) return st;
-    }
-    if (done)
-      method = kM2dFMM;
-    else
-      gpu::launch_m2d(d_, e_m2d_, scratch_, nsplit_m2d_, flag_, st_);
   }
+  if (done)
+    method = kM2dFMM;
+  else
+    gpu::launch_m2d(d_, e_m2d_, scratch_, nsplit_m2d_, flag_, st_);
   m2d_method_ = method;
   int flag = 0;
   cudaMemcpyAsync(&flag, flag_, sizeof(int), cudaMemcpyDeviceToHost, st_);
@@ -705,18 +691,6 @@ int System::ensure_sym_scratch() {
     sym_scratch_ = nullptr;
     cudaGetLastError();
     set_last_error("out of device memory for the symmetric-product accumulators");
-    return kErrMemory;
-  }
-  return kOk;
-}
-
-// split partials of the double-single permanent field
-int System::ensure_ds_scratch() {
-  if (ds_scratch_) return kOk;
-  nsplit_m2d_ds_ = gpu::m2d_ds_pick_split(d_, gpu::sm_count());
-  if (alloc(ds_scratch_, (size_t)nsplit_m2d_ds_ * 3 * d_.n)) {
-    ds_scratch_ = nullptr;
-    set_last_error("out of device memory for the double-single kernels");
     return kErrMemory;
   }
   return kOk;

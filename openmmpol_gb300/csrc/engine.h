@@ -167,7 +167,6 @@ class System {
   int set_inner_blocks(int max_sites, double link_bohr);
   int matvec_residual(int ncol, const double *x, double *y);
   void direct_product(int ncol, const double *x, double *y, bool dodiag, int kernel);
-  int ensure_ds_scratch();
   int ensure_sym_scratch();
   int precision() const { return precision_; }
   double tol() const { return tol_; }
@@ -277,10 +276,8 @@ class System {
   int build_blocks();
   double *ext_buf_ = nullptr;  // external points: coordinates, partials, output, dipoles
   size_t ext_cap_ = 0;
-  double *ds_scratch_ = nullptr;  // split partials of the double-single kernels
-  int nsplit_m2d_ds_ = 1;
   // how the cached E_M2D was computed
-  static constexpr int kM2dDirect = 0, kM2dDS = 1, kM2dFMM = 2;
+  static constexpr int kM2dDirect = 0, kM2dFMM = 1;
   int m2d_method_ = kM2dDirect;
   int fp32_kernel_ = 0;  // 0 autotuned, else the forced kernel version
   float *scratch32_ = nullptr;

@@ -675,7 +675,7 @@ __global__ void __launch_bounds__(FT) k_fmm_l2p_m2d(FmmArgs a, const int *__rest
                 bad = 1;
                 continue;
               }
-              m2d_pair_f64<AMOEBA>(dx, dy, dz, pt.w, ps.w, at, s_a[q], wat, s_wa[q], &s_q[q * LD], thr, thr2m, e[0],
+              m2d_pair_f64<AMOEBA, true>(dx, dy, dz, pt.w, ps.w, at, s_a[q], wat, s_wa[q], &s_q[q * LD], thr, thr2m, e[0],
                                    e[1], e[2]);
             }
           }

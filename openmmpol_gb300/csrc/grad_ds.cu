@@ -67,12 +67,13 @@ struct DsK {
 // d = target - source and the (damped) inverse powers; false for coincident
 // sites (NEAR only: far tiles hold none)
 template <bool NEAR, bool AMOEBA>
-__device__ __forceinline__ bool ds_grad_geom(const float4 &th, const float4 &tl, const float4 &sh, const float4 &sl,
+__device__ __forceinline__ bool ds_grad_geom(const float4 &th, const float4 &tm, const float4 &tl, const float4 &sh,
+                                             const float4 &sm, const float4 &sl,
                                              double wt, double ws, double at, double as, float2 wat, float2 was,
                                              double thr, float thr2m, DsK &g) {
-  g.dx = ds_diff(th.x, tl.x, sh.x, sl.x);
-  g.dy = ds_diff(th.y, tl.y, sh.y, sl.y);
-  g.dz = ds_diff(th.z, tl.z, sh.z, sl.z);
+  g.dx = ds_delta(th.x, tm.x, tl.x, sh.x, sm.x, sl.x);
+  g.dy = ds_delta(th.y, tm.y, tl.y, sh.y, sm.y, sl.y);
+  g.dz = ds_delta(th.z, tm.z, tl.z, sh.z, sm.z, sl.z);
   const dsf dx = g.dx, dy = g.dy, dz = g.dz;
   float px = dx.h * dx.h, py = dy.h * dy.h, pz = dz.h * dz.h;
   float ex = fmaf(dx.h + dx.h, dx.l, fmaf(dx.h, dx.h, -px));
@@ -120,14 +121,15 @@ template <bool AMOEBA>
 __global__ void __launch_bounds__(GD_TPB) k_grad_ds_mp(DevSites s, double *__restrict__ partial, int per_split,
                                                        float thr2m, int *err) {
   constexpr int LD = AMOEBA ? 10 : 1;
-  __shared__ float4 s_ph[GD_TILE], s_pl[GD_TILE];
+  __shared__ float4 s_ph[GD_TILE], s_pm2[GD_TILE], s_pl[GD_TILE];
   __shared__ float s_qh[GD_TILE * LD], s_ql[GD_TILE * LD];
   __shared__ double s_w[GD_TILE], s_a[GD_TILE];
   __shared__ float2 s_wa[GD_TILE];
   const int j = blockIdx.x * GD_TPB + threadIdx.x;
   const bool valid = j < s.n;
-  const float4 th = valid ? s.pol_pos32[j] : make_float4(0.f, 0.f, 0.f, 0.f);
-  const float4 tl = valid ? s.pol_pos32lo[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 th = valid ? s.pol_split[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 td = valid ? s.pol_split[(size_t)s.n + j] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 tl = valid ? s.pol_split[2 * (size_t)s.n + j] : make_float4(0.f, 0.f, 0.f, 0.f);
   const int tm = valid ? s.polar_mm[j] : -1;
   const double wt = valid ? s.pol_pos[j].w : 0.0, at = valid && AMOEBA ? s.pol_a[j] : 0.0;
   const float2 wat = valid ? s.pol_wa32[j] : make_float2(0.f, 0.f);
@@ -140,8 +142,9 @@ __global__ void __launch_bounds__(GD_TPB) k_grad_ds_mp(DevSites s, double *__res
     {
       const int k = threadIdx.x, i = t0 + k;
       if (i < s1) {
-        s_ph[k] = s.mm_pos32[i];
-        s_pl[k] = s.mm_pos32lo[i];
+        s_ph[k] = s.mm_split[i];
+        s_pm2[k] = s.mm_split[(size_t)s.m + i];
+        s_pl[k] = s.mm_split[2 * (size_t)s.m + i];
         s_w[k] = s.mm_pos[i].w;
         s_a[k] = AMOEBA ? s.mm_a[i] : 0.0;
         s_wa[k] = s.mm_wa32[i];
@@ -165,10 +168,10 @@ __global__ void __launch_bounds__(GD_TPB) k_grad_ds_mp(DevSites s, double *__res
       for (int k = 0; k < cnt; ++k) {
         DsK g;
         if (far_tile) {
-          ds_grad_geom<false, AMOEBA>(th, tl, s_ph[k], s_pl[k], 0.0, 0.0, 0.0, 0.0, wat, wat, 0.0, 0.f, g);
+          ds_grad_geom<false, AMOEBA>(th, td, tl, s_ph[k], s_pm2[k], s_pl[k], 0.0, 0.0, 0.0, 0.0, wat, wat, 0.0, 0.f, g);
         } else {
           if (t0 + k == tm) continue;
-          if (!ds_grad_geom<true, AMOEBA>(th, tl, s_ph[k], s_pl[k], wt, s_w[k], at, s_a[k], wat, s_wa[k], s.damp_thr,
+          if (!ds_grad_geom<true, AMOEBA>(th, td, tl, s_ph[k], s_pm2[k], s_pl[k], wt, s_w[k], at, s_a[k], wat, s_wa[k], s.damp_thr,
                                           thr2m, g)) {
             bad = 1;
             continue;
@@ -198,7 +201,7 @@ __global__ void __launch_bounds__(GD_TPB) k_grad_ds_dip(DevSites s, const double
                                                         int *err) {
   constexpr int NS = AMOEBA ? 2 : 1;        // dipole sets
   constexpr int ND = AMOEBA ? 18 : 9;       // hd[6] (hp[6]) e[3] (h[3])
-  __shared__ float4 s_ph[GD_TILE], s_pl[GD_TILE];
+  __shared__ float4 s_ph[GD_TILE], s_pm2[GD_TILE], s_pl[GD_TILE];
   __shared__ float s_mh[GD_TILE * 3 * NS], s_ml[GD_TILE * 3 * NS];
   __shared__ double s_w[GD_TILE], s_a[GD_TILE];
   __shared__ float2 s_wa[GD_TILE];
@@ -206,8 +209,9 @@ __global__ void __launch_bounds__(GD_TPB) k_grad_ds_dip(DevSites s, const double
   __shared__ double s_sum[ND * GD_TPB];
   const int t = blockIdx.x * GD_TPB + threadIdx.x;
   const bool valid = t < s.m;
-  const float4 th = valid ? s.mm_pos32[t] : make_float4(0.f, 0.f, 0.f, 0.f);
-  const float4 tl = valid ? s.mm_pos32lo[t] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 th = valid ? s.mm_split[t] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 td = valid ? s.mm_split[(size_t)s.m + t] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 tl = valid ? s.mm_split[2 * (size_t)s.m + t] : make_float4(0.f, 0.f, 0.f, 0.f);
   const double wt = valid ? s.mm_pos[t].w : 0.0, at = valid && AMOEBA ? s.mm_a[t] : 0.0;
   const float2 wat = valid ? s.mm_wa32[t] : make_float2(0.f, 0.f);
   dsf Q[6], trq{0.f, 0.f};
@@ -226,8 +230,9 @@ __global__ void __launch_bounds__(GD_TPB) k_grad_ds_dip(DevSites s, const double
     {
       const int k = threadIdx.x, i = t0 + k;
       if (i < s1) {
-        s_ph[k] = s.pol_pos32[i];
-        s_pl[k] = s.pol_pos32lo[i];
+        s_ph[k] = s.pol_split[i];
+        s_pm2[k] = s.pol_split[(size_t)s.n + i];
+        s_pl[k] = s.pol_split[2 * (size_t)s.n + i];
         s_w[k] = s.pol_pos[i].w;
         s_a[k] = AMOEBA ? s.pol_a[i] : 0.0;
         s_wa[k] = s.pol_wa32[i];
@@ -257,10 +262,10 @@ __global__ void __launch_bounds__(GD_TPB) k_grad_ds_dip(DevSites s, const double
       for (int k = 0; k < cnt; ++k) {
         DsK g;
         if (far_tile) {
-          ds_grad_geom<false, AMOEBA>(th, tl, s_ph[k], s_pl[k], 0.0, 0.0, 0.0, 0.0, wat, wat, 0.0, 0.f, g);
+          ds_grad_geom<false, AMOEBA>(th, td, tl, s_ph[k], s_pm2[k], s_pl[k], 0.0, 0.0, 0.0, 0.0, wat, wat, 0.0, 0.f, g);
         } else {
           if (s_pm[k] == t) continue;
-          if (!ds_grad_geom<true, AMOEBA>(th, tl, s_ph[k], s_pl[k], wt, s_w[k], at, s_a[k], wat, s_wa[k], s.damp_thr,
+          if (!ds_grad_geom<true, AMOEBA>(th, td, tl, s_ph[k], s_pm2[k], s_pl[k], wt, s_w[k], at, s_a[k], wat, s_wa[k], s.damp_thr,
                                           thr2m, g)) {
             bad = 1;
             continue;

@@ -2,11 +2,6 @@
 //
 // Pair kernels (all-pairs, CUDA cores; the pair tensor math is not a dense
 // contraction, so no tensor cores):
-//   k_m2d_allpairs   field of the permanent multipoles at the polarizable
-//                    sites, unscaled, Thole-damped (AMOEBA exp / Wang linear).
-//                    Restates elec_prop_M2D + damped_coulomb_kernel + the
-//                    q/mu/quad field formulas (src/mod_electrostatics.F90:
-//                    1018-1095, 1097-1405, 2579-2731).
 //   k_m2d_finish     fixed-order reduction of the source-split partials plus
 //                    the scaled-pair correction pass: for every listed pair
 //                    (s - 1) * f_ij is added, which equals the reference's
@@ -36,70 +31,6 @@ namespace {
 constexpr int TPB = 128;   // targets per CTA
 constexpr int TILE = 128;  // sources per shared-memory tile
 
-template <bool AMOEBA>
-__global__ void __launch_bounds__(TPB) k_m2d_allpairs(int n, int m, const Pos64 *__restrict__ pol_pos,
-                                                      const double *__restrict__ pol_a,
-                                                      const int *__restrict__ polar_mm,
-                                                      const Pos64 *__restrict__ mm_pos,
-                                                      const double *__restrict__ mm_a,
-                                                      const double *__restrict__ mm_q, int ld,
-                                                      const float2 *__restrict__ pol_wa,
-                                                      const float2 *__restrict__ mm_wa,
-                                                      double *__restrict__ partial, int per_split,
-                                                      double thr, float thr2m, int *err_flag) {
-  constexpr int LD = AMOEBA ? 10 : 1;         // multipole record in memory
-  constexpr int SLD = AMOEBA ? M2D_SLD : 1;    // staged record (m2d_stage)
-  constexpr int NA = AMOEBA ? 9 : 3;          // field sums (m2d_pair_acc)
-  __shared__ Pos64 s_pos[TILE];
-  __shared__ double s_a[TILE];
-  __shared__ float2 s_wa[TILE];
-  __shared__ double s_q[TILE * SLD];
-  const int j = blockIdx.x * TPB + threadIdx.x;
-  const bool valid = j < n;
-  Pos64 pt = valid ? pol_pos[j] : Pos64{0, 0, 0, 0};
-  // the target's own mm index and its thole (pol_pos stores 1/thole)
-  const int tm = valid ? polar_mm[j] : -1;
-  const double at = valid && AMOEBA ? pol_a[j] : 0.0;
-  const float2 wat = valid ? pol_wa[j] : make_float2(0.f, 0.f);
-  double acc[NA];
-#pragma unroll
-  for (int c = 0; c < NA; ++c) acc[c] = 0.0;
-  int bad = 0;
-  const int s0 = blockIdx.y * per_split;
-  const int s1 = min(m, s0 + per_split);
-  for (int t0 = s0; t0 < s1; t0 += TILE) {
-    __syncthreads();
-    for (int k = threadIdx.x; k < TILE; k += TPB) {
-      int i = t0 + k;
-      if (i < s1) {
-        s_pos[k] = mm_pos[i];
-        s_a[k] = AMOEBA ? mm_a[i] : 0.0;
-        s_wa[k] = mm_wa[i];
-        m2d_stage<AMOEBA>(&mm_q[(size_t)i * LD], &s_q[k * SLD]);
-      }
-    }
-    __syncthreads();
-    const int cnt = min(TILE, s1 - t0);
-    if (!valid) continue;
-    for (int k = 0; k < cnt; ++k) {
-      const int i = t0 + k;
-      if (i == tm) continue;
-      const Pos64 ps = s_pos[k];
-      double dx = pt.x - ps.x, dy = pt.y - ps.y, dz = pt.z - ps.z;
-      if (coincident(dx * dx + dy * dy + dz * dz)) {
-        bad = 1;
-        continue;
-      }
-      m2d_pair_acc<AMOEBA>(dx, dy, dz, pt.w, ps.w, at, s_a[k], wat, s_wa[k], &s_q[k * SLD], thr, thr2m, acc);
-    }
-  }
-  if (bad) atomicOr(err_flag, 1);
-  if (valid) {
-    double *o = partial + ((size_t)blockIdx.y * n + j) * 3;
-    m2d_field<AMOEBA>(acc, o[0], o[1], o[2]);
-  }
-}
-
 // Reduce partials and apply the scaled-pair corrections; out [n_ipd][n][3]
 // with set 0 = D (direct field, d-scale) and set 1 = P (p-scale) for AMOEBA.
 template <bool AMOEBA>
@@ -127,7 +58,9 @@ __global__ void k_m2d_finish(int n, int nsplit, const double *__restrict__ parti
     double q[LD];
     for (int c = 0; c < LD; ++c) q[c] = mm_q[(size_t)i * LD + c];
     double fx = 0, fy = 0, fz = 0;
-    m2d_pair_f64<AMOEBA>(pt.x - ps.x, pt.y - ps.y, pt.z - ps.z, pt.w, ps.w, at,
+    // the same reciprocal distance as the pair pass: the excluded pairs are
+    // the largest terms and have to cancel
+    m2d_pair_f64<AMOEBA, true>(pt.x - ps.x, pt.y - ps.y, pt.z - ps.z, pt.w, ps.w, at,
                          AMOEBA ? mm_a[i] : 0.0, wat, mm_wa[i], q, thr, thr2m, fx, fy, fz);
     double cp = sP[k] - 1.0, cd = sD[k] - 1.0;
     eP[0] += cp * fx;
@@ -724,29 +657,6 @@ int sm_count() {
 }
 
 // ---- M2D -----------------------------------------------------------------
-// Source splits of the FP64 permanent field: about 16 waves of CTAs, so
-// that the last, partly filled wave idles few SMs (one wave of ~4.6 CTAs
-// per SM left the SMs with 4 idle while those with 5 finished), with the
-// split partials kept below 64 MiB.
-int m2d_pick_split(const DevSites &s, int sms) {
-  static int resident = 0;
-  if (!resident) {
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_m2d_allpairs<true>, TPB, 0);
-    if (resident < 1) resident = 1;
-  }
-  const long long tblocks = (s.n + TPB - 1) / TPB;
-  const long long want = 16LL * resident * sms;
-  long long split = (want + tblocks - 1) / tblocks;
-  const long long maxsplit = (s.m + TILE - 1) / TILE;
-  const long long maxmem = (64LL << 20) / (24LL * (s.n > 0 ? s.n : 1));
-  if (split > maxmem) split = maxmem;
-  if (split > maxsplit) split = maxsplit;
-  if (split < 1) split = 1;
-  return (int)split;
-}
-
-size_t m2d_scratch_doubles(const DevSites &s, int nsplit) { return (size_t)nsplit * s.n * 3; }
-
 // split partials -> FP64 scaled-pair corrections -> D and P sets
 static void m2d_finish(const DevSites &s, double *out, const double *scratch, int nsplit, cudaStream_t st) {
   int fb = (s.n + 127) / 128;
@@ -763,31 +673,6 @@ static void m2d_finish(const DevSites &s, double *out, const double *scratch, in
 void launch_m2d_finish(const DevSites &s, double *out, const double *partial, int nsplit, cudaStream_t st) {
   add_launch_count(1);
   m2d_finish(s, out, partial, nsplit, st);
-}
-
-void launch_m2d(const DevSites &s, double *out, double *scratch, int nsplit, int *err_flag,
-                cudaStream_t st) {
-  if (s.n == 0) return;
-  add_launch_count(2);
-  int tiles = (s.m + TILE - 1) / TILE;
-  int per = ((tiles + nsplit - 1) / nsplit) * TILE;
-  dim3 grid((s.n + TPB - 1) / TPB, nsplit);
-  if (s.amoeba)
-    k_m2d_allpairs<true><<<grid, TPB, 0, st>>>(s.n, s.m, s.pol_pos, s.pol_a, s.polar_mm, s.mm_pos, s.mm_a,
-                                               s.mm_q, s.ld, s.pol_wa32, s.mm_wa32, scratch, per, s.damp_thr,
-                                               damp_thr2_margin(s), err_flag);
-  else
-    k_m2d_allpairs<false><<<grid, TPB, 0, st>>>(s.n, s.m, s.pol_pos, s.pol_a, s.polar_mm, s.mm_pos, s.mm_a,
-                                                s.mm_q, s.ld, s.pol_wa32, s.mm_wa32, scratch, per, s.damp_thr,
-                                                damp_thr2_margin(s), err_flag);
-  m2d_finish(s, out, scratch, nsplit, st);
-}
-
-void launch_m2d_ds(const DevSites &s, double *out, double *scratch, int nsplit, int *err_flag, cudaStream_t st) {
-  if (s.n == 0) return;
-  add_launch_count(2);
-  launch_m2d_ds_pairs(s, scratch, nsplit, err_flag, st);
-  m2d_finish(s, out, scratch, nsplit, st);
 }
 
 // ---- T.mu -----------------------------------------------------------------

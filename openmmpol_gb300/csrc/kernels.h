@@ -31,7 +31,6 @@ struct DevSites {
   double *pol_alpha = nullptr;  // polarizability
   int *polar_mm = nullptr;      // mm index of each polarizable site
   float4 *pol_pos32 = nullptr;  // centred FP32 copy: x, y, z, 1/thole
-  float4 *pol_pos32lo = nullptr;  // x, y, z - pol_pos32 (double-single low parts), w = 0
   float *pol_a32 = nullptr;
   float2 *pol_wa32 = nullptr;   // (1/thole)^2, a^2 in FP32: damping pre-test of the FP64 kernels
   float2 *mm_wa32 = nullptr;    // same for the static sites (inf when not polarizable)
@@ -55,10 +54,12 @@ struct DevSites {
   // symmetric FP64 product: coordinates split into three floats [3][n]
   // (split_coordinates) and the bounding boxes of 32 sites
   float4 *pol_split = nullptr, *sub_box32 = nullptr;
+  // the same split of the static sites [3][m] (one grid for both)
+  float4 *mm_split = nullptr;
   float damp_r2max32 = 0.f;
-  // double-single E_M2D: static-site positions (hi with w = 0, lo), their
-  // tile boxes and the squared distance beyond which no M2D pair is damped
-  float4 *mm_pos32 = nullptr, *mm_pos32lo = nullptr, *mm_tile_box32 = nullptr;
+  // tile boxes of the static sites and the squared distance beyond which no
+  // M2D pair is damped
+  float4 *mm_tile_box32 = nullptr;
   float m2d_r2max32 = 0.f;
 };
 
@@ -179,12 +180,12 @@ int tmu32_max_split(const DevSites &s, int sm_count);
 int tmu32_pick_split(const DevSites &s, int sm_count);
 void tile_boxes32(const float4 *pos32, int n, float4 *boxes /*[2*ceil(n/tile)]*/, int tile = 128);
 float damp_r2max32(bool amoeba, double damp_thr, const double *inv_thole, const double *a, int n);
-// E_M2D with the all-pairs part in double-single (scratch nsplit * n * 3)
-int m2d_ds_pick_split(const DevSites &s, int sm_count);
-void launch_m2d_ds_pairs(const DevSites &s, double *partial, int nsplit, int *err_flag, cudaStream_t st);
-void launch_m2d_ds(const DevSites &s, double *out, double *scratch, int nsplit, int *err_flag, cudaStream_t st);
 float m2d_r2max32(bool amoeba, double damp_thr, const double *pol_w, const double *pol_a, int n, const double *mm_w,
                   const double *mm_a, int m);
+// Static-static pair sums (m2m.cu), energy or gradient: partial
+// [nsplit][10 or 12 (Wang-AL 1 or 3)][m]
+int m2m_pick_split(const DevSites &s, bool grad, int sm_count);
+void launch_m2m(const DevSites &s, bool grad, double *partial, int nsplit, int *err, cudaStream_t st);
 // Polarization-gradient pair sums in double-single (grad_ds.cu): the static
 // multipoles' field gradient at the polarizable sites (partial [nsplit][6]
 // [m], at each site's static index; which 0) and the induced dipoles' field

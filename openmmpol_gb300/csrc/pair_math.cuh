@@ -175,14 +175,14 @@ __device__ __forceinline__ void dd_pair(T r2, T wt, T ws, T at, T as, float2 wat
 // Field of a static multipole (charge; + dipole and quadrupole for AMOEBA,
 // q[0..9]) at a polarizable target, d = target - source, Thole-damped
 // (elec_prop_M2D pair term, src/mod_electrostatics.F90:2579-2731).
-template <bool AMOEBA>
+template <bool AMOEBA, bool FULL = false>
 __device__ __forceinline__ void m2d_pair_f64(double dx, double dy, double dz, double wt, double ws,
                                              double at, double as, float2 wat, float2 was,
                                              const double *q, double thr, float thr2m,
                                              double &ex, double &ey, double &ez) {
   double r2 = dx * dx + dy * dy + dz * dz;
   float r2f = r2_f32(r2);
-  double rinv = rinv_f64(r2, r2f);
+  double rinv = FULL ? rinv_f64_full(r2, r2f) : rinv_f64(r2, r2f);
   double ir2 = rinv * rinv;
   double k3 = rinv * ir2;
   if (AMOEBA) {
@@ -241,13 +241,13 @@ __device__ __forceinline__ void m2d_stage(const double *q, double *o) {
   for (int c = 0; c < 6; ++c) o[7 + c] = 15.0 * q[4 + c];
 }
 
-template <bool AMOEBA>
+template <bool AMOEBA, bool FULL = false>
 __device__ __forceinline__ void m2d_pair_acc(double dx, double dy, double dz, double wt, double ws, double at,
                                              double as, float2 wat, float2 was, const double *q, double thr,
                                              float thr2m, double *acc) {
   const double r2 = dx * dx + dy * dy + dz * dz;
   const float r2f = r2_f32(r2);
-  const double rinv = rinv_f64(r2, r2f);
+  const double rinv = FULL ? rinv_f64_full(r2, r2f) : rinv_f64(r2, r2f);
   const double ir2 = rinv * rinv;
   double k3 = rinv * ir2;
   if (AMOEBA) {
