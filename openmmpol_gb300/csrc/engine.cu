@@ -125,7 +125,7 @@ System::~System() {
   free_ws(ws_);
   free_ws(wsb_);
   void *bufs[] = {inv32_, sqrt_alpha_, d_.pol_pos, d_.pol_a, d_.pol_alpha, d_.polar_mm, d_.pol_pos32, d_.pol_a32,
-                  d_.pol_wa32, d_.mm_split, d_.mm_tile_box32,
+                  d_.pol_wa32, d_.mm_split, d_.mm_sub_box32, d_.mm_tile_box32,
                   d_.mm_wa32, d_.mm_pos,
                   d_.mm_a, d_.mm_q, d_.m2d_ri, d_.m2d_src, d_.m2d_sP, d_.m2d_sD, d_.d2d_ri, d_.d2d_src,
                   d_.d2d_s, e_m2d_, ipd_, rhs_, ext_, x_, r_, p_, h_, z_, x32_, r32_, p32_, h32_, z32_,
@@ -203,7 +203,7 @@ size_t System::device_bytes_estimate() const {
                  8 * (gpu::kRedBlocks * 32 + 64 + 2 * (size_t)maxhist_);
   bytes += 16 * (n + 2 * ((m + 127) / 128));
   // coordinate splits and 32-site boxes of the double-single kernels
-  bytes += 16 * (3 * n + 3 * m + 2 * ((n + 31) / 32));
+  bytes += 16 * (3 * n + 3 * m + 2 * ((n + 31) / 32) + 2 * ((m + 31) / 32));
   // near-field couplings of the Neumann step (about a dozen per site in water)
   if (inner_precond_ == 2) bytes += 4 * (n + 1) + 40 * 24 * n;
   return bytes + (size_t(4) << 20);  // events, flags, rounding
@@ -269,7 +269,7 @@ int System::upload_static() {
   bad |= alloc(scratch_, scratch_n_) | alloc(scratch32_, gpu::tmu_scratch_doubles(d_, 2, f32_splits));
   bad |= alloc(d_.tile_box32, 2 * (size_t)d_.ntile) | alloc(d_.pol_split, 3 * (size_t)n) |
          alloc(d_.sub_box32, 2 * (size_t)((n + 31) / 32));
-  bad |= alloc(d_.mm_split, 3 * (size_t)mm) | alloc(d_.mm_tile_box32, 2 * (size_t)((mm + 127) / 128));
+  bad |= alloc(d_.mm_split, 3 * (size_t)mm) | alloc(d_.mm_sub_box32, 2 * (size_t)((mm + 31) / 32)) | alloc(d_.mm_tile_box32, 2 * (size_t)((mm + 127) / 128));
   bad |= alloc(partial_, (size_t)gpu::kRedBlocks * 32) | alloc(dots_, 64) | alloc(hist_, 2 * (size_t)maxhist_);
   bad |= alloc(cols_, 2) | alloc(flag_, 1) | alloc(info_, 1);
   if (bad || pinned_alloc((void **)&cols_h_, 2 * sizeof(gpu::CgCol)) != cudaSuccess ||
@@ -396,10 +396,12 @@ int System::upload_geometry() {
     const double xc[3] = {x[0] - c[0], x[1] - c[1], x[2] - c[2]};
     mp32[i] = make_float4((float)xc[0], (float)xc[1], (float)xc[2], 0.f);
   }
-  std::vector<float4> mboxes(2 * (size_t)((mm + 127) / 128));
+  std::vector<float4> mboxes(2 * (size_t)((mm + 127) / 128)), msubs(2 * (size_t)((mm + 31) / 32));
   gpu::tile_boxes32(mp32.data(), mm, mboxes.data());
+  gpu::tile_boxes32(mp32.data(), mm, msubs.data(), 32);
   if (mm) {
     h2d(d_.mm_tile_box32, mboxes.data(), mboxes.size() * sizeof(float4));
+    h2d(d_.mm_sub_box32, msubs.data(), msubs.size() * sizeof(float4));
   }
   h2d(d_.mm_pos, mp.data(), mm * sizeof(gpu::Pos64));
   h2d(d_.mm_a, ma.data(), mm * sizeof(double));

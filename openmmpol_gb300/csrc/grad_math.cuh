@@ -171,8 +171,11 @@ OMMP_HD void cross3(const double *a, const double *b, double *o) {
 // gradient on c, cz, cx, cy.  Frames: 0 none, 1 z-then-x, 2 bisector,
 // 3 z-only, 4 z-bisector, 5 3-fold (the construction of rotate_multipoles,
 // src/rotate_multipoles.F90:3-230).  Returns false for a degenerate frame.
+// tau: a torque on the site, added (the derivative of Phi with respect to a
+// rotation of the lab-frame multipoles).
 OMMP_HD bool frame_pullback(int frame, const double *c, const double *cz, const double *cx, const double *cy,
-                            const double *q0, const double *E, const double *G, double out[4][3]) {
+                            const double *q0, const double *E, const double *G, double out[4][3],
+                            const double *tau = nullptr) {
   for (int w = 0; w < 4; ++w) out[w][0] = out[w][1] = out[w][2] = 0.0;
   if (frame < 1 || frame > 5) return true;
   double a[3], b[3], d[3];
@@ -229,6 +232,13 @@ OMMP_HD bool frame_pullback(int frame, const double *c, const double *cz, const 
   for (int i = 0; i < 3; ++i)
     for (int j = 0; j < 3; ++j)
       W[i][j] = -E[i] * q0[1 + j] + 2.0 * (Gm[i][0] * RQ[0][j] + Gm[i][1] * RQ[1][j] + Gm[i][2] * RQ[2][j]);
+  // dPhi = tau.omega for dR = omega x R: W = (tau x R) / 2
+  if (tau)
+    for (int j = 0; j < 3; ++j) {
+      W[0][j] += 0.5 * (tau[1] * R[2][j] - tau[2] * R[1][j]);
+      W[1][j] += 0.5 * (tau[2] * R[0][j] - tau[0] * R[2][j]);
+      W[2][j] += 0.5 * (tau[0] * R[1][j] - tau[1] * R[0][j]);
+    }
   double gx[3] = {W[0][0], W[1][0], W[2][0]}, gy[3] = {W[0][1], W[1][1], W[2][1]},
          gz[3] = {W[0][2], W[1][2], W[2][2]};
   // ey = ez x ex

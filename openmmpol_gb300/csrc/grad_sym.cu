@@ -19,15 +19,14 @@
 // s = n.T, R = Q p'; K = y^3, G = 3 y^3, F = 3 y^4, C = 15 y^4, F5 = 3 y^5,
 // H = 15 y^5, D = 105 y^5 with the damping factors of r^-3 (K), r^-5 (G, F,
 // F5), r^-7 (C, H) and r^-9 (D)):
-//   force on t = n [a_s (-G q_t + C b_t + H tr_t - D s_t)
-//                   + a_t (G q_s + C b_s - H tr_s + D s_s)
+//   force on t = n [a_s (-G q_t + C b_t - D s_t) + a_t (G q_s + C b_s + D s_s)
 //                   - F (m_t.p_s + m_s.p_t) + 2 H (T_t.p_s - T_s.p_t)]
-//              + p_s (K q_t - F b_t - F5 tr_t + H s_t)
-//              - p_t (K q_s + F b_s - F5 tr_s + H s_s)
+//              + p_s (K q_t - F b_t + H s_t) - p_t (K q_s + F b_s + H s_s)
 //              + a_s (2 H T_t - F m_t) - a_t (2 H T_s + F m_s) + 2 F5 (R_s - R_t)
 //   torque on t = [a_s (2 C T_t - G m_t) - 2 F R_t] x n + [K m_t - 2 F T_t] x p_s
 //   torque on s = [2 F R_s - a_t (G m_s + 2 C T_s)] x n + [K m_s + 2 F T_s] x p_t
-// (R_t = Q_t p_s, R_s = Q_s p_t; the torques with m alone).  The formulas are
+// (R_t = Q_t p_s, R_s = Q_s p_t; the torques with m alone), and for
+// quadrupoles that are not traceless the terms of trace_force.  The formulas are
 // written once for double and for double-single numbers.
 //
 // Schedule, near pairs and accumulation are those of the symmetric T.mu
@@ -36,6 +35,11 @@
 // damping reaches farther) queued for FP64, fixed-point sums.  Sub-tile pairs
 // without a polarizable site are skipped.  The dipoles are scaled by a power
 // of two as in the products.
+//
+// 30,000 sites: 76 -> 37 ms in the mixed modes, 330 ms in FP64 before; 90,000:
+// 668 -> 332 ms (2.95 s in FP64).  Error against 64 bits 7e-15 to 8e-15 (before
+// 2.7e-14 in FP64, 3e-14 to 6e-14 in double-single).  255 registers without
+// spills at 2 CTAs per SM: bound by FP32 issue and its latency at 8 warps.
 //
 // Built with --fmad=false -ftz=true: every FMA is explicit.
 #include <algorithm>
@@ -54,7 +58,7 @@ constexpr float FAR = 1.0e6f;
 struct GradSymJob {
   DevSites s;
   const double *p, *d;    // [m][3] scaled mean dipole and half difference
-  const int *any_d;       // some d is not zero
+  const int *any;         // [0] some d is not zero, [1] some quadrupole has a trace
   const unsigned *word;   // largest high word of the dipoles
   const unsigned *polar;  // [ceil(m / 32)] sites of the sub-tile that are polarizable
   unsigned long long *lo, *hi, *bad;
@@ -132,10 +136,8 @@ __device__ __forceinline__ void pair_force(const Site<T, true> &t, const Site<T,
   // n
   T x1 = mul(neg(k.G), t.q), x2 = mul(k.G, s.q);
   mad(x1, k.C, bt);
-  mad(x1, k.H, t.tr);
   mad(x1, neg(k.D), st);
   mad(x2, k.C, bs);
-  mad(x2, neg(k.H), s.tr);
   mad(x2, k.D, ss);
   T X = mul(as, norm(x1));
   mad(X, at, norm(x2));
@@ -147,10 +149,8 @@ __device__ __forceinline__ void pair_force(const Site<T, true> &t, const Site<T,
   // p_s, p_t
   T ws = mul(k.K, t.q), wt = mul(neg(k.K), s.q);
   mad(ws, nF, bt);
-  mad(ws, neg(k.F5), t.tr);
   mad(ws, k.H, st);
   mad(wt, nF, bs);
-  mad(wt, k.F5, s.tr);
   mad(wt, neg(k.H), ss);
   ws = norm(ws);
   wt = norm(wt);
@@ -197,6 +197,20 @@ __device__ __forceinline__ void pair_force(const Site<T, true> &t, const Site<T,
   }
   add_cross(u, n, tau_s);
   add_cross(w, t.p, tau_s);
+}
+
+// The trace of the quadrupole of a site in the field of the dipole p of the
+// other: the reference keeps it in the Hessian contraction (the force on the
+// static site) and drops it in the field of the quadrupole, so it acts on one
+// side only.  n and p.n change sign together: the same form for either site.
+template <typename T>
+__device__ __forceinline__ void trace_force(T tr, const T *p, const T *n, const Powers<T> &k, T *f) {
+  const T x = mul(mul(k.H, tr), dot(p, n)), w = mul(neg(k.F5), tr);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    mad(f[c], x, n[c]);
+    mad(f[c], w, p[c]);
+  }
 }
 
 // charges and dipoles only; p2 the unscaled dipole of t (the dipole-dipole
@@ -297,7 +311,7 @@ __device__ __forceinline__ void fixed_add_to(const GradSymJob &jb, size_t o, dou
 // the queued pairs in FP64, one per lane
 template <bool AMOEBA>
 __device__ __noinline__ void grad_queued(const GradSymJob &jb, const unsigned short *queue, int count, int lane,
-                                         int i0, int j0, int ex, bool delta) {
+                                         int i0, int j0, int ex, bool delta, bool trace) {
   constexpr int NO = GradSmem<AMOEBA>::NO;
   const DevSites &s = jb.s;
   for (int e = lane; e < count; e += 32) {
@@ -330,12 +344,16 @@ __device__ __noinline__ void grad_queued(const GradSymJob &jb, const unsigned sh
     double vi[NV], vj[NV];
     site_values<AMOEBA>(jb, i, ex, vi);
     site_values<AMOEBA>(jb, j, ex, vj);
-    double f[3] = {0.0, 0.0, 0.0}, tt[3] = {0.0, 0.0, 0.0}, ts[3] = {0.0, 0.0, 0.0};
+    double f[3] = {0.0, 0.0, 0.0}, gi[3] = {0.0, 0.0, 0.0}, gj[3] = {0.0, 0.0, 0.0}, tt[3] = {0.0, 0.0, 0.0}, ts[3] = {0.0, 0.0, 0.0};
     Site<double, AMOEBA> a, b;
     fill(a, vi);
     fill(b, vj);
     if constexpr (AMOEBA) {
       pair_force(a, b, n, k, f, tt, ts);
+      if (trace) {
+        trace_force(a.tr, b.p, n, k, gi);
+        trace_force(b.tr, a.p, n, k, gj);
+      }
       if (delta) {
         const double du[3] = {scale_up(vi[17], ex), scale_up(vi[18], ex), scale_up(vi[19], ex)};
         delta_force(du, vj + 17, n, k, f);
@@ -346,8 +364,8 @@ __device__ __noinline__ void grad_queued(const GradSymJob &jb, const unsigned sh
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      fixed_add_to(jb, (size_t)i * NO + c, f[c]);
-      fixed_add_to(jb, (size_t)j * NO + c, -f[c]);
+      fixed_add_to(jb, (size_t)i * NO + c, f[c] + gi[c]);
+      fixed_add_to(jb, (size_t)j * NO + c, gj[c] - f[c]);
       if (AMOEBA) {
         fixed_add_to(jb, (size_t)i * NO + 3 + c, tt[c]);
         fixed_add_to(jb, (size_t)j * NO + 3 + c, ts[c]);
@@ -374,7 +392,7 @@ __global__ void __launch_bounds__(TILE, AMOEBA ? 2 : 4) k_grad_sym(const __grid_
   const DevSites &s = jb.s;
   const int m = s.m, nsub = (m + SUB - 1) / SUB;
   const int ex = dsp_exponent(*jb.word);
-  const bool delta = AMOEBA && *jb.any_d != 0;
+  const bool delta = AMOEBA && jb.any[0] != 0, trace = AMOEBA && jb.any[1] != 0;
   for (;;) {
     __syncthreads();
     if (tid == 0) s_item = (int)atomicAdd(next, 1u);
@@ -522,6 +540,10 @@ __global__ void __launch_bounds__(TILE, AMOEBA ? 2 : 4) k_grad_sym(const __grid_
           dsf g[3] = {{0.f, 0.f}, {0.f, 0.f}, {0.f, 0.f}};
           if constexpr (AMOEBA) {
             pair_force(st, ss, n, k, g, ai + 3, aj + 3);
+            if (trace) {
+              trace_force(st.tr, ss.p, n, k, ai);
+              trace_force(ss.tr, st.p, n, k, aj);
+            }
             if (delta) delta_force(tv + 17, sv + 17, n, k, g);
           } else {
             pair_force(st, p2, ss, n, k, g);
@@ -542,7 +564,8 @@ __global__ void __launch_bounds__(TILE, AMOEBA ? 2 : 4) k_grad_sym(const __grid_
         }
         if (near) {
           __syncwarp();
-          grad_queued<AMOEBA>(jb, sm.queue[warp], queued, lane, I * TILE + warp * SUB, J * TILE + js * SUB, ex, delta);
+          grad_queued<AMOEBA>(jb, sm.queue[warp], queued, lane, I * TILE + warp * SUB, J * TILE + js * SUB, ex, delta,
+                              trace);
           __syncwarp();
         }
 #pragma unroll
@@ -567,11 +590,11 @@ __global__ void __launch_bounds__(TILE, AMOEBA ? 2 : 4) k_grad_sym(const __grid_
   }
 }
 
-// scaled mean dipoles and half differences in static-site order, and whether
-// any difference is not zero
+// scaled mean dipoles and half differences in static-site order, whether any
+// difference is not zero and whether any quadrupole has a trace beyond rounding
 __global__ void k_grad_dipoles(int m, int n, int nset, const int *__restrict__ mm_polar, const double *__restrict__ ipd,
                                const unsigned *__restrict__ word, double *__restrict__ p, double *__restrict__ d,
-                               int *any_d) {
+                               const double *__restrict__ q, int *any) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= m) return;
   const int j = mm_polar[i], ex = dsp_exponent(*word);
@@ -583,7 +606,12 @@ __global__ void k_grad_dipoles(int m, int n, int nset, const int *__restrict__ m
     d[3 * (size_t)i + c] = 0.5 * (a - b);
     diff = diff || a != b;
   }
-  if (diff) *any_d = 1;
+  if (diff) any[0] = 1;
+  if (nset == 2) {
+    const double *Q = q + (size_t)i * 10 + 4;
+    const double big = fmax(fmax(fabs(Q[0]), fabs(Q[2])), fabs(Q[5]));
+    if (fabs((Q[0] + Q[2]) + Q[5]) > 2e-15 * big) any[1] = 1;
+  }
 }
 
 template <bool AMOEBA>
@@ -621,7 +649,7 @@ void launch_grad_sym(const DevSites &s, const double *ipd, const int *mm_polar, 
   double *p = reinterpret_cast<double *>(j.bad + 4);
   j.p = p;
   j.d = p + 3 * (size_t)s.m;
-  j.any_d = any;
+  j.any = any;
   j.word = word;
   j.polar = polar;
   j.err = err;
@@ -640,7 +668,7 @@ void launch_grad_sym(const DevSites &s, const double *ipd, const int *mm_polar, 
   launch_max_word(nset * 3 * (size_t)s.n, ipd, word, st);
   add_launch_count(2);
   k_grad_dipoles<<<(s.m + 255) / 256, 256, 0, st>>>(s.m, s.n, (int)nset, mm_polar, ipd, word, p,
-                                                    p + 3 * (size_t)s.m, any);
+                                                    p + 3 * (size_t)s.m, s.mm_q, any);
   const int grid = std::min(ctas, j.items);
   if (s.amoeba)
     k_grad_sym<true><<<grid, TILE, sizeof(GradSmem<true>), st>>>(j, next);

@@ -55,7 +55,7 @@ struct DevSites {
   // (split_coordinates) and the bounding boxes of 32 sites
   float4 *pol_split = nullptr, *sub_box32 = nullptr;
   // the same split of the static sites [3][m] (one grid for both)
-  float4 *mm_split = nullptr;
+  float4 *mm_split = nullptr, *mm_sub_box32 = nullptr;  // and their 32-site boxes
   float damp_r2max32 = 0.f;
   // tile boxes of the static sites and the squared distance beyond which no
   // M2D pair is damped
@@ -186,15 +186,13 @@ float m2d_r2max32(bool amoeba, double damp_thr, const double *pol_w, const doubl
 // [nsplit][10 or 12 (Wang-AL 1 or 3)][m]
 int m2m_pick_split(const DevSites &s, bool grad, int sm_count);
 void launch_m2m(const DevSites &s, bool grad, double *partial, int nsplit, int *err, cudaStream_t st);
-// Polarization-gradient pair sums in double-single (grad_ds.cu): the static
-// multipoles' field gradient at the polarizable sites (partial [nsplit][6]
-// [m], at each site's static index; which 0) and the induced dipoles' field
-// gradients, field and quadrupole-contracted Hessian at the static sites
-// (partial [nsplit][18 or 9][m]; which 1), unscaled
-int grad_ds_pick_split(const DevSites &s, int which, int sm_count);
-void launch_grad_ds_mp(const DevSites &s, double *partial, int nsplit, int *err, cudaStream_t st);
-void launch_grad_ds_dip(const DevSites &s, const double *ipd, double *partial, int nsplit, int *err,
-                        cudaStream_t st);
+// Pair pass of the polarization gradient (grad_sym.cu): buf of
+// grad_sym_doubles(s) receives fixed-point sums lo [m][6 or 3] (force, for
+// AMOEBA torque), hi, then the non-finite flag, the work counter and the
+// scale word; polar one bit per static site
+size_t grad_sym_doubles(const DevSites &s);
+void launch_grad_sym(const DevSites &s, const double *ipd, const int *mm_polar, const unsigned *polar, double *buf,
+                     int *err, cudaStream_t st);
 // z = M^-1 r for the block-Jacobi preconditioner (info / minv as built by
 // build_block_jacobi), columns [ncol][n][3], FP32
 void launch_block_apply(int ncol, int n, const int4 *info, const float *minv, const float *r, float *z,

@@ -314,23 +314,36 @@ __device__ __forceinline__ bool coincident(double r2) { return __double2hiint(r2
 // (kernels.cu, ds_kernels.cu): integer addition is exact and associative,
 // so the sums do not depend on the order of the CTAs.
 // v added exactly into the two-word fixed-point value hi * 2^-16 + lo * 2^-80
-// (hi two's complement, lo unsigned).  A value that is not finite or not
-// below 2^36 in magnitude sets *bad instead (the whole product is then NaN).
-__device__ __forceinline__ void fixed_add(unsigned long long *lo, unsigned long long *hi, double v,
-                                          unsigned long long *bad) {
-  if (!(fabs(v) < 68719476736.0)) {
+// (hi two's complement, lo unsigned), with integer operations instead of FP64
+// ones.  A value that is not finite or not below 2^36 in magnitude sets *bad
+// instead (the whole product is then NaN).
+__device__ __forceinline__ void fixed_add_int(unsigned long long *lo, unsigned long long *hi, double v,
+                                              unsigned long long *bad) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  const int e = (int)((b >> 52) & 2047);
+  if (e >= 1023 + 36) {  // not below 2^36 (or not finite)
     atomicOr(bad, 1ull);
     return;
   }
-  const double s = v * 65536.0;  // exact
-  double fl = floor(s);
-  double fr = s - fl;  // exact, in [0, 1]
-  if (fr >= 1.0) {     // s - floor(s) rounded up to 1 for tiny negative s
-    fr = 0.0;
-    fl += 1.0;
+  if (e < 1023 - 80) return;  // below the resolution
+  const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
+  // value = m 2^(e - 1075); units of 2^-80: m 2^s
+  const int s = e - 1075 + 80;
+  unsigned long long l, h;
+  if (s >= 64) {
+    l = 0;
+    h = m << (s - 64);
+  } else if (s > 0) {
+    l = m << s;
+    h = m >> (64 - s);
+  } else {
+    l = m >> (-s);
+    h = 0;
   }
-  const unsigned long long h = (unsigned long long)(long long)fl;
-  const unsigned long long l = (unsigned long long)(fr * 18446744073709551616.0);
+  if (b >> 63) {
+    l = ~l + 1ull;
+    h = ~h + (l == 0 ? 1ull : 0ull);
+  }
   const unsigned long long old = atomicAdd(lo, l);
   atomicAdd(hi, h + (old + l < old ? 1ull : 0ull));
 }

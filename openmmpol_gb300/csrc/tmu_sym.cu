@@ -111,39 +111,6 @@ __device__ __forceinline__ float box_dist2(const float4 &alo, const float4 &ahi,
   return fmaf(gx, gx, fmaf(gy, gy, gz * gz));
 }
 
-// exact addition into the fixed-point words like fixed_add, with integer
-// operations instead of FP64 ones
-__device__ __forceinline__ void fixed_add_int(unsigned long long *lo, unsigned long long *hi, double v,
-                                              unsigned long long *bad) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-  const int e = (int)((b >> 52) & 2047);
-  if (e >= 1023 + 36) {  // not below 2^36 (or not finite)
-    atomicOr(bad, 1ull);
-    return;
-  }
-  if (e < 1023 - 80) return;  // below the resolution
-  const unsigned long long m = (b & 0xFFFFFFFFFFFFFull) | 0x10000000000000ull;
-  // value = m 2^(e - 1075); units of 2^-80: m 2^s
-  const int s = e - 1075 + 80;
-  unsigned long long l, h;
-  if (s >= 64) {
-    l = 0;
-    h = m << (s - 64);
-  } else if (s > 0) {
-    l = m << s;
-    h = m >> (64 - s);
-  } else {
-    l = m >> (-s);
-    h = 0;
-  }
-  if (b >> 63) {
-    l = ~l + 1ull;
-    h = ~h + (l == 0 ? 1ull : 0ull);
-  }
-  const unsigned long long old = atomicAdd(lo, l);
-  atomicAdd(hi, h + (old + l < old ? 1ull : 0ull));
-}
-
 // the 32 x 32 pairs of a warp's sites and the sub-tile js in double-single;
 // NEAR: returns the number of pairs left to FP64 in the warp's queue
 template <int G, bool NEAR, bool AMOEBA>
