@@ -26,7 +26,7 @@ CU_SOURCES = ["kernels.cu", "engine.cu", "solvers.cu", "noalloc.cu", "tmu32.cu",
 # the double-single kernel fuses nothing implicitly (its FMAs are explicit)
 CU_EXTRA = {"tmu32.cu": ["-ftz=true"], "m2d.cu": ["-ftz=true", "--fmad=false"], "m2m.cu": ["-ftz=true", "--fmad=false"],
             "tmu_sym.cu": ["-ftz=true", "--fmad=false"], "fmm_near.cu": ["-ftz=true", "--fmad=false"],
-            "grad_sym.cu": ["-ftz=true", "--fmad=false"]}
+            "grad_sym.cu": ["-ftz=true", "--fmad=false"], "external.cu": ["-ftz=true", "--fmad=false"]}
 CXX_SOURCES = ["setup.cpp", "capi.cpp", "log.cpp", "server.cpp", "precond.cpp"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 

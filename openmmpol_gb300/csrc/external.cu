@@ -10,148 +10,242 @@
 // otherwise.  The results are ADDED into the caller's array, as the
 // reference's routines do.
 //
-// One CTA of 128 threads owns 128 points; sources stream through shared
-// memory in tiles of 128 records, split over blockIdx.y with the partials
-// summed in a fixed order: FP64 throughout, deterministic.
+// The sums were FP64-bound: at 20,001 points and 9,000 sites 12.8 ms for the
+// static multipoles and 6.3 ms for the induced dipoles.  They run in
+// double-single on the FP32 pipes (ds_pair.cuh; about 350 FP32 operations per
+// point and AMOEBA site), static and induced dipole of a site added first so
+// that one pass serves both.  Points and sites are split on one grid per call;
+// one thread owns a point, sources stream through shared memory in tiles of
+// 128; pairs closer than 5 bohr go to a list of the point's own and are formed
+// in FP64 by its thread.  The source range is split over blockIdx.y (quarters
+// of a tile: a few QM nuclei alone fill the GPU) and the partials are summed in
+// a fixed order: deterministic.
+//
+// Built with --fmad=false -ftz=true: every FMA of a pair is explicit.
+#include <algorithm>
 #include <cmath>
+#include <vector>
 
+#include "ds_pair.cuh"
 #include "engine.h"
 #include "log.h"
-#include "pair_math.cuh"
 
 namespace ommp {
 namespace gpu {
 namespace {
 
-constexpr int EXT_TPB = 128;
+constexpr int NT = 128;
+constexpr int NLIST = 24;       // listed sources per point before they are formed
+constexpr float CLOSE2 = 25.f;  // bohr^2
 
-// SRC 0: AMOEBA multipoles (10 per site), 1: charges, 2: dipoles (3 per site)
-template <int SRC>
-struct SrcWidth;
-template <>
-struct SrcWidth<0> {
-  static constexpr int value = 10;
+// values of a source: q, dipole (3), with QUAD the quadrupole (6)
+template <bool QUAD>
+struct ExtRec {
+  static constexpr int NV = QUAD ? 10 : 4;
+  static constexpr int R = (9 + 2 * NV + 3) / 4;
 };
-template <>
-struct SrcWidth<1> {
-  static constexpr int value = 1;
+
+// x - c as three floats on the grid g1, g1 2^-23 (split_coordinates)
+__device__ __forceinline__ void split3(double v, double g1, float *o) {
+  const double g2 = g1 * 1.1920928955078125e-7;
+  const double h = rint(v / g1) * g1, m = rint((v - h) / g2) * g2;
+  o[0] = (float)h;
+  o[3] = (float)m;
+  o[6] = (float)((v - h) - m);
+}
+
+struct ExtArgs {
+  int n, m, nv;        // points, sources, polarizable sites (dipole sets)
+  const double *cext;
+  const Pos64 *pos;    // sources
+  const double *q;     // [m][ld] multipoles, or null (induced dipoles alone)
+  int ld;
+  const int *polar;    // [m] polarizable index of a source or -1; null: the source itself
+  const double *mu, *mu2;  // induced dipoles added (null: none) and a second set averaged with them
+  double c[3], g1;
+  const unsigned *word;  // scale of the dipoles, or null
+  double *val;         // [m][NV] FP64 values
+  float4 *rec;         // [R][m]
 };
-template <>
-struct SrcWidth<2> {
-  static constexpr int value = 3;
-};
+
+template <bool QUAD>
+__global__ void k_ext_sources(ExtArgs a) {
+  constexpr int NV = ExtRec<QUAD>::NV, R = ExtRec<QUAD>::R;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= a.m) return;
+  double v[NV];
+  for (int c = 0; c < NV; ++c) v[c] = a.q && c < a.ld ? a.q[(size_t)i * a.ld + c] : 0.0;
+  const int p = a.mu ? (a.polar ? a.polar[i] : i) : -1;
+  if (p >= 0) {
+    const int ex = a.word ? dsp_exponent(*a.word) : 0;
+    for (int c = 0; c < 3; ++c) {
+      const double d = a.mu[3 * (size_t)p + c];
+      v[1 + c] += scale_down(a.mu2 ? 0.5 * (a.mu2[3 * (size_t)p + c] + d) : d, ex);
+    }
+  }
+  const Pos64 x = a.pos[i];
+  float f[4 * R] = {};
+  split3(x.x - a.c[0], a.g1, f);
+  split3(x.y - a.c[1], a.g1, f + 1);
+  split3(x.z - a.c[2], a.g1, f + 2);
+  for (int c = 0; c < NV; ++c) {
+    a.val[(size_t)i * NV + c] = v[c];
+    const dsf d = to_ds(v[c]);
+    f[9 + 2 * c] = d.h;
+    f[10 + 2 * c] = d.l;
+  }
+#pragma unroll
+  for (int r = 0; r < R; ++r) a.rec[(size_t)r * a.m + i] = make_float4(f[4 * r], f[4 * r + 1], f[4 * r + 2], f[4 * r + 3]);
+}
 
 // partial[split][n][C] (C = 1 potential, 3 field)
-template <bool FIELD, int SRC>
-__global__ void __launch_bounds__(EXT_TPB) k_ext(int n, const double *__restrict__ cext, int m,
-                                                 const Pos64 *__restrict__ spos, const double *__restrict__ sdata,
-                                                 double *__restrict__ partial, int per_split, int *bad_flag) {
-  constexpr int LD = SrcWidth<SRC>::value;
-  constexpr int C = FIELD ? 3 : 1;
-  __shared__ double s_x[EXT_TPB], s_y[EXT_TPB], s_z[EXT_TPB];
-  __shared__ double s_d[EXT_TPB * LD];
-  const int j = blockIdx.x * EXT_TPB + threadIdx.x;
-  const bool valid = j < n;
-  double px = 0, py = 0, pz = 0;
-  if (valid) {
-    px = cext[3 * (size_t)j];
-    py = cext[3 * (size_t)j + 1];
-    pz = cext[3 * (size_t)j + 2];
-  }
-  double acc[C];
+template <bool FIELD, bool QUAD>
+__global__ void __launch_bounds__(NT, 4) k_ext(const __grid_constant__ ExtArgs a, double *__restrict__ partial,
+                                               int per_split, int *bad_flag) {
+  constexpr int NV = ExtRec<QUAD>::NV, R = ExtRec<QUAD>::R, C = FIELD ? 3 : 1;
+  __shared__ float4 s_rec[R][NT];
+  __shared__ int s_list[NLIST][NT];
+  const int j = blockIdx.x * NT + threadIdx.x;
+  const bool valid = j < a.n;
+  const int tj = valid ? j : a.n - 1;
+  const double px = a.cext[3 * (size_t)tj], py = a.cext[3 * (size_t)tj + 1], pz = a.cext[3 * (size_t)tj + 2];
+  float tg[9];
+  split3(px - a.c[0], a.g1, tg);
+  split3(py - a.c[1], a.g1, tg + 1);
+  split3(pz - a.c[2], a.g1, tg + 2);
+  double sum[C];
 #pragma unroll
-  for (int c = 0; c < C; ++c) acc[c] = 0.0;
-  int bad = 0;
-  const int s0 = blockIdx.y * per_split;
-  const int s1 = min(m, s0 + per_split);
-  for (int t0 = s0; t0 < s1; t0 += EXT_TPB) {
-    __syncthreads();
-    {
-      const int i = t0 + threadIdx.x;
-      if (i < s1) {
-        const Pos64 p = spos[i];
-        s_x[threadIdx.x] = p.x;
-        s_y[threadIdx.x] = p.y;
-        s_z[threadIdx.x] = p.z;
-      }
-      for (int k = threadIdx.x; k < EXT_TPB * LD; k += EXT_TPB) {
-        const size_t g = (size_t)t0 * LD + k;
-        if (g < (size_t)s1 * LD) s_d[k] = sdata[g];
-      }
-    }
-    __syncthreads();
-    if (!valid) continue;
-    const int cnt = min(EXT_TPB, s1 - t0);
-    for (int k = 0; k < cnt; ++k) {
-      const double dx = px - s_x[k], dy = py - s_y[k], dz = pz - s_z[k];
+  for (int c = 0; c < C; ++c) sum[c] = 0.0;
+  int listed = 0, bad = 0;
+  // the listed pairs in FP64
+  auto form = [&]() {
+    for (int e = 0; e < listed; ++e) {
+      const int i = s_list[e][threadIdx.x];
+      const Pos64 ps = a.pos[i];
+      const double dx = px - ps.x, dy = py - ps.y, dz = pz - ps.z;
       const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
       if (r2 < 4.930380657631324e-28) {  // |r| < 100 eps: the reference stops here
         bad = 1;
         continue;
       }
-      const double k1 = rinv_f64(r2, r2_f32(r2));
-      const double ir2 = k1 * k1;
-      const double k2 = k1 * ir2;  // r^-3
-      const double *q = &s_d[k * LD];
-      if (SRC == 2) {
-        const double mdr = fma(q[0], dx, fma(q[1], dy, q[2] * dz));
-        if (!FIELD) {
-          acc[0] = fma(mdr, k2, acc[0]);
-        } else {
-          const double f = 3.0 * mdr * (k2 * ir2);
-          acc[0] += fma(f, dx, -q[0] * k2);
-          acc[C > 1 ? 1 : 0] += fma(f, dy, -q[1] * k2);
-          acc[C > 2 ? 2 : 0] += fma(f, dz, -q[2] * k2);
-        }
-      } else if (SRC == 1) {
-        if (!FIELD) {
-          acc[0] = fma(q[0], k1, acc[0]);
-        } else {
-          const double c = q[0] * k2;
-          acc[0] = fma(c, dx, acc[0]);
-          acc[C > 1 ? 1 : 0] = fma(c, dy, acc[C > 1 ? 1 : 0]);
-          acc[C > 2 ? 2 : 0] = fma(c, dz, acc[C > 2 ? 2 : 0]);
-        }
+      const double *q = a.val + (size_t)i * NV;
+      const double k1 = rinv_f64_full(r2, r2_f32(r2)), ir2 = k1 * k1, k3 = k1 * ir2, k5 = k3 * ir2;
+      const double md = fma(q[1], dx, fma(q[2], dy, q[3] * dz));
+      double tx = 0.0, ty = 0.0, tz = 0.0, s = 0.0;
+      if (QUAD) {
+        tx = fma(q[4], dx, fma(q[5], dy, q[7 % NV] * dz));
+        ty = fma(q[5 % NV], dx, fma(q[6 % NV], dy, q[8 % NV] * dz));
+        tz = fma(q[7 % NV], dx, fma(q[8 % NV], dy, q[9 % NV] * dz));
+        s = fma(tx, dx, fma(ty, dy, tz * dz));
+      }
+      if (!FIELD) {
+        sum[0] += fma(q[0], k1, fma(md, k3, 3.0 * s * k5));
       } else {
-        const double k3 = k2 * ir2;  // r^-5
-        const double mdr = fma(q[1], dx, fma(q[2], dy, q[3] * dz));
-        const double qx = fma(q[4], dx, fma(q[5], dy, q[7] * dz));
-        const double qy = fma(q[5], dx, fma(q[6], dy, q[8] * dz));
-        const double qz = fma(q[7], dx, fma(q[8], dy, q[9] * dz));
-        const double qxr = fma(qx, dx, fma(qy, dy, qz * dz));
-        if (!FIELD) {
-          acc[0] += q[0] * k1 + mdr * k2 + 3.0 * qxr * k3;
-        } else {
-          const double k4 = k3 * ir2;  // r^-7
-          const double c = q[0] * k2 + 3.0 * mdr * k3 + 15.0 * qxr * k4;
-          const double k3x6 = 6.0 * k3;
-          acc[0] += c * dx - q[1] * k2 - k3x6 * qx;
-          acc[C > 1 ? 1 : 0] += c * dy - q[2] * k2 - k3x6 * qy;
-          acc[C > 2 ? 2 : 0] += c * dz - q[3] * k2 - k3x6 * qz;
-        }
+        const double c = fma(q[0], k3, fma(3.0 * md, k5, 15.0 * s * (k5 * ir2)));
+        const double k6 = 6.0 * k5;
+        sum[0] += fma(c, dx, -fma(q[1], k3, k6 * tx));
+        sum[C > 1 ? 1 : 0] += fma(c, dy, -fma(q[2], k3, k6 * ty));
+        sum[C > 2 ? 2 : 0] += fma(c, dz, -fma(q[3], k3, k6 * tz));
       }
     }
-  }
-  if (bad) atomicOr(bad_flag, 1);
-  if (valid) {
+    listed = 0;
+  };
+  const int s0 = blockIdx.y * per_split, s1 = min(a.m, s0 + per_split);
+  for (int t0 = s0; t0 < s1; t0 += NT) {
+    const int cnt = min(NT, s1 - t0);
+    __syncthreads();
+    if (threadIdx.x < cnt)
 #pragma unroll
-    for (int c = 0; c < C; ++c) partial[((size_t)blockIdx.y * n + j) * C + c] = acc[c];
+      for (int r = 0; r < R; ++r) s_rec[r][threadIdx.x] = a.rec[(size_t)r * a.m + t0 + threadIdx.x];
+    __syncthreads();
+    dsf acc[C];
+#pragma unroll
+    for (int c = 0; c < C; ++c) acc[c] = dsf{0.f, 0.f};
+#pragma unroll 1
+    for (int k = 0; k < cnt; ++k) {
+      float f[4 * R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const float4 v = s_rec[r][k];
+        f[4 * r] = v.x, f[4 * r + 1] = v.y, f[4 * r + 2] = v.z, f[4 * r + 3] = v.w;
+      }
+      float sc[9];
+#pragma unroll
+      for (int c = 0; c < 9; ++c) sc[c] = f[c];
+      const DspDelta d = dsp_delta(tg, sc);
+      float y = d.ri;
+      if (!(d.r2 >= CLOSE2)) {
+        y = 0.f;
+        if (listed == NLIST) form();
+        s_list[listed++][threadIdx.x] = t0 + k;
+      }
+      auto q = [&](int c) { return dsf{f[9 + 2 * c], f[10 + 2 * c]}; };
+      // the charges cancel between sites: their factor is kept to 2^-48
+      const DspUnit n = dsp_unit<true>(d, y);
+      const float w3 = dsp_power<3>(n.eps), w5 = dsp_power<5>(n.eps);
+      const float y2 = y * y, y2l = fmaf(y, y, -y2);
+      const float y3 = y2 * y, y3l = fmaf(y2l, y, fmaf(y2, y, -y3));
+      const dsf m = dsp_dot(q(1), q(2), q(3), n.x, n.y, n.z);
+      dsf t[3], nqn{0.f, 0.f};
+      if (QUAD) {
+        t[0] = dsp_norm(dsp_dot(q(4), q(5), q(7), n.x, n.y, n.z));
+        t[1] = dsp_norm(dsp_dot(q(5), q(6), q(8), n.x, n.y, n.z));
+        t[2] = dsp_norm(dsp_dot(q(7), q(8), q(9), n.x, n.y, n.z));
+        nqn = dsp_dot(t[0], t[1], t[2], n.x, n.y, n.z);
+      }
+      if (!FIELD) {
+        const dsf V = dsp_scaled<1>(y, 0.f, n);
+        dsp_acc(acc[0], V, q(0));
+        dsp_acc(acc[0], dsf{y2, fmaf(y2, w3, y2l)}, m);
+        if (QUAD) dsp_acc(acc[0], dsp_coef(3.f, y3, y3l, w5), nqn);
+      } else {
+        const dsf K = {-y3, -fmaf(y3, w3, y3l)};
+        dsf c = dsp_mul(dsp_scaled<3>(y2, y2l, n), q(0));
+        dsp_acc(c, dsp_coef(3.f, y3, y3l, w5), m);
+        if (QUAD) {
+          const float y4 = y3 * y, y4l = fmaf(y3l, y, fmaf(y3, y, -y4));
+          dsp_acc(c, dsp_coef(15.f, y4, y4l, dsp_power<7>(n.eps)), nqn);
+          const dsf H = dsp_coef(-6.f, y4, y4l, w5);
+#pragma unroll
+          for (int u = 0; u < C; ++u) dsp_acc(acc[u], H, t[u]);
+        }
+        c = dsp_norm(c);
+        const dsf nn[3] = {n.x, n.y, n.z};
+#pragma unroll
+        for (int u = 0; u < C; ++u) {
+          dsp_acc(acc[u], c, nn[u]);
+          dsp_acc(acc[u], K, q(1 + u));
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < C; ++c) acc[c] = dsp_norm(acc[c]);
+      if (!FIELD && (k & 3) == 3) {
+        // the potential is a small remainder of the charges' partial sums:
+        // they go into the FP64 sum every four sources (error of a Wang-AL
+        // system's potential 1.0e-14 with whole tiles)
+        sum[0] += (double)acc[0].h + (double)acc[0].l;
+        acc[0] = dsf{0.f, 0.f};
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < C; ++c) sum[c] += (double)acc[c].h + (double)acc[c].l;
   }
+  form();
+  if (!valid) return;
+  if (bad) atomicOr(bad_flag, 1);
+#pragma unroll
+  for (int c = 0; c < C; ++c) partial[((size_t)blockIdx.y * a.n + j) * C + c] = sum[c];
 }
 
-// out[j][c] = sum over the nsplit partial blocks, in order
-__global__ void k_ext_sum(size_t total, int nsplit, const double *__restrict__ partial, double *__restrict__ out) {
+// out[j][c] = sum over the nsplit partial blocks, in order, scaled back
+__global__ void k_ext_sum(size_t total, int nsplit, const double *__restrict__ partial, const unsigned *word,
+                          double *__restrict__ out) {
+  const int ex = word ? dsp_exponent(*word) : 0;
   for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += (size_t)gridDim.x * blockDim.x) {
     double s = 0.0;
     for (int p = 0; p < nsplit; ++p) s += partial[(size_t)p * total + k];
-    out[k] = s;
+    out[k] = scale_up(s, ex);
   }
-}
-
-__global__ void k_half_sum(size_t n, const double *__restrict__ a, const double *__restrict__ b,
-                           double *__restrict__ out) {
-  for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x)
-    out[k] = 0.5 * (a[k] + b[k]);
 }
 
 int blocks_for_ext(size_t n) {
@@ -161,27 +255,22 @@ int blocks_for_ext(size_t n) {
   return (int)b;
 }
 
+// about four waves of CTAs, at least 32 sources per split
 int ext_split(int n, int m, int sms) {
-  const int blocks = (n + EXT_TPB - 1) / EXT_TPB;
-  const int tiles = (m + EXT_TPB - 1) / EXT_TPB;
-  int split = (4 * sms + blocks - 1) / blocks;
-  if (split > tiles) split = tiles;
-  return split < 1 ? 1 : split;
+  const int blocks = (n + NT - 1) / NT;
+  return std::max(1, std::min((m + 31) / 32, (16 * sms + blocks - 1) / blocks));
 }
 
-template <bool FIELD>
-void launch_src(int src, int n, const double *cext, int m, const Pos64 *spos, const double *sdata, double *partial,
-                int nsplit, int *bad, cudaStream_t st) {
-  const int tiles = (m + EXT_TPB - 1) / EXT_TPB;
-  const int per = ((tiles + nsplit - 1) / nsplit) * EXT_TPB;
-  dim3 grid((n + EXT_TPB - 1) / EXT_TPB, nsplit);
-  add_launch_count(1);
-  if (src == 0)
-    k_ext<FIELD, 0><<<grid, EXT_TPB, 0, st>>>(n, cext, m, spos, sdata, partial, per, bad);
-  else if (src == 1)
-    k_ext<FIELD, 1><<<grid, EXT_TPB, 0, st>>>(n, cext, m, spos, sdata, partial, per, bad);
+template <bool QUAD>
+void launch_ext(bool field, const ExtArgs &a, double *partial, int nsplit, int *bad, cudaStream_t st) {
+  const int per = ((a.m + nsplit - 1) / nsplit + 31) / 32 * 32;
+  const dim3 grid((a.n + NT - 1) / NT, nsplit);
+  add_launch_count(2);
+  k_ext_sources<QUAD><<<(a.m + 127) / 128, 128, 0, st>>>(a);
+  if (field)
+    k_ext<true, QUAD><<<grid, NT, 0, st>>>(a, partial, per, bad);
   else
-    k_ext<FIELD, 2><<<grid, EXT_TPB, 0, st>>>(n, cext, m, spos, sdata, partial, per, bad);
+    k_ext<false, QUAD><<<grid, NT, 0, st>>>(a, partial, per, bad);
 }
 
 }  // namespace
@@ -200,10 +289,15 @@ int System::ext_props(int which, bool field, int n, const double *cext_h, double
   }
   if (n == 0 || (!do_mm && !do_pol)) return kOk;
   const int C = field ? 3 : 1;
-  const int sms = gpu::sm_count();
-  const int smm = do_mm ? gpu::ext_split(n, d_.m, sms) : 0;
-  const int spol = do_pol ? gpu::ext_split(n, d_.n, sms) : 0;
-  const size_t need = 3 * (size_t)n + (size_t)(smm + spol) * n * C + (size_t)n * C + 3 * (size_t)d_.n;
+  // sources: the static sites (with the induced dipoles of the polarizable
+  // ones), or the polarizable sites alone
+  const int m = do_mm ? d_.m : d_.n;
+  const bool quad = do_mm && m_.amoeba;
+  const int nsplit = gpu::ext_split(n, m, gpu::sm_count());
+  const size_t nval = quad ? gpu::ExtRec<true>::NV : gpu::ExtRec<false>::NV;
+  const size_t nrec = quad ? gpu::ExtRec<true>::R : gpu::ExtRec<false>::R;
+  const size_t need = 3 * (size_t)n + (size_t)(nsplit + 1) * n * C + (size_t)m * (nval + 2 * nrec) +
+                      ((size_t)m + 1) / 2 + 4;
   if (need > ext_cap_) {
     if (ext_buf_) cudaFree(ext_buf_);
     ext_buf_ = nullptr;
@@ -215,34 +309,50 @@ int System::ext_props(int which, bool field, int n, const double *cext_h, double
     }
     ext_cap_ = need;
   }
-  double *cext = ext_buf_;
+  // the source records first: 16-byte aligned
+  gpu::ExtArgs a{};
+  a.rec = reinterpret_cast<float4 *>(ext_buf_);
+  a.val = ext_buf_ + 2 * nrec * m;
+  double *cext = a.val + nval * m;
   double *partial = cext + 3 * (size_t)n;
-  double *out = partial + (size_t)(smm + spol) * n * C;
-  double *mu = out + (size_t)n * C;
+  double *out = partial + (size_t)nsplit * n * C;
+  unsigned *word = reinterpret_cast<unsigned *>(out + (size_t)n * C);
+  int *polar = reinterpret_cast<int *>(word + 2);
+  a.n = n, a.m = m, a.nv = d_.n;
+  a.cext = cext;
+  a.pos = do_mm ? d_.mm_pos : d_.pol_pos;
+  a.q = do_mm ? d_.mm_q : nullptr;
+  a.ld = d_.ld;
+  if (do_pol) {
+    // the D set for the potential, the mean of both for the field (AMOEBA)
+    a.mu = ipd_;
+    a.mu2 = field && m_.amoeba ? ipd_ + 3 * (size_t)d_.n : nullptr;
+    if (do_mm) {
+      a.polar = polar;
+      cudaMemcpyAsync(polar, m_.mm_polar.data(), (size_t)m * sizeof(int), cudaMemcpyHostToDevice, st_);
+    }
+  }
+  // one grid for the points and the sites: about the first site, rounded to
+  // whole bohr (an exact shift), as wide as the farthest of them
+  double big = 1.0;
+  for (int c = 0; c < 3; ++c) a.c[c] = std::nearbyint(m_.cmm[c]);
+  for (int i = 0; i < d_.m; ++i)
+    for (int c = 0; c < 3; ++c) big = std::max(big, std::fabs(m_.cmm[3 * (size_t)i + c] - a.c[c]));
+  for (size_t k = 0; k < 3 * (size_t)n; ++k) big = std::max(big, std::fabs(cext_h[k] - a.c[k % 3]));
+  int e = 0;
+  std::frexp(std::isfinite(big) ? big : 1.0, &e);
+  a.g1 = std::ldexp(1.0, e - 23);
   cudaMemcpyAsync(cext, cext_h, 3 * (size_t)n * sizeof(double), cudaMemcpyHostToDevice, st_);
   cudaMemsetAsync(flag_, 0, sizeof(int), st_);
-  if (do_mm) {
-    const int src = m_.amoeba ? 0 : 1;
-    if (field)
-      gpu::launch_src<true>(src, n, cext, d_.m, d_.mm_pos, d_.mm_q, partial, smm, flag_, st_);
-    else
-      gpu::launch_src<false>(src, n, cext, d_.m, d_.mm_pos, d_.mm_q, partial, smm, flag_, st_);
+  if (!do_mm) {
+    a.word = word;
+    gpu::launch_max_word((a.mu2 ? 2 : 1) * 3 * (size_t)d_.n, ipd_, word, st_);
   }
-  if (do_pol) {
-    const size_t nv = 3 * (size_t)d_.n;
-    const double *dip = ipd_;  // D set (AMOEBA) or the only set
-    if (field && m_.amoeba) {
-      gpu::k_half_sum<<<gpu::blocks_for_ext(nv), 256, 0, st_>>>(nv, ipd_ + nv, ipd_, mu);
-      gpu::add_launch_count(1);
-      dip = mu;
-    }
-    double *pp = partial + (size_t)smm * n * C;
-    if (field)
-      gpu::launch_src<true>(2, n, cext, d_.n, d_.pol_pos, dip, pp, spol, flag_, st_);
-    else
-      gpu::launch_src<false>(2, n, cext, d_.n, d_.pol_pos, dip, pp, spol, flag_, st_);
-  }
-  gpu::k_ext_sum<<<gpu::blocks_for_ext((size_t)n * C), 256, 0, st_>>>((size_t)n * C, smm + spol, partial, out);
+  if (quad)
+    gpu::launch_ext<true>(field, a, partial, nsplit, flag_, st_);
+  else
+    gpu::launch_ext<false>(field, a, partial, nsplit, flag_, st_);
+  gpu::k_ext_sum<<<gpu::blocks_for_ext((size_t)n * C), 256, 0, st_>>>((size_t)n * C, nsplit, partial, a.word, out);
   gpu::add_launch_count(1);
   std::vector<double> h((size_t)n * C);
   int flag = 0;
