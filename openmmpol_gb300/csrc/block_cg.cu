@@ -39,6 +39,8 @@ constexpr int GT = 32;          // output tile of the Gram kernel (rows and colu
 constexpr int GE = 64;          // elements per staged tile
 constexpr int kGramChunks = 152;  // element chunks (blocks along x)
 constexpr int CK = 16;          // output columns per block of the combine kernel
+constexpr int CT = 64;         // threads per block of the combine kernel (one element each: 3,003
+                               // sites fill the SMs, 256 left them on 36 blocks)
 constexpr int kMaxBlock = 128;  // widest block (columns)
 
 // partial[c][a][b] = sum over chunk c of U[ua[a]][i] V[vb[b]][i]
@@ -79,18 +81,28 @@ __global__ void __launch_bounds__(256) k_gram(size_t nv, int sa, const float *__
       if (b0 + tb + c < sb) partial[((size_t)blockIdx.x * sa + a) * sb + b0 + tb + c] = acc[c];
 }
 
-// out[k] = sum over chunks of partial[c][k], in chunk order
-__global__ void k_gram_reduce(int nchunk, int total, const double *__restrict__ partial, double *__restrict__ out) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= total) return;
+// out[k] = sum over chunks of partial[c][k]: 32 outputs per block, its 8 warps
+// take every eighth chunk (one thread per output was a chain of 152 loads, 22
+// us), summed in warp order
+__global__ void __launch_bounds__(256) k_gram_reduce(int nchunk, int total, const double *__restrict__ partial,
+                                                     double *__restrict__ out) {
+  __shared__ double sh[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, k = blockIdx.x * 32 + lane;
   double s = 0.0;
-  for (int c = 0; c < nchunk; ++c) s += partial[(size_t)c * total + k];
+  if (k < total) {
+#pragma unroll 4
+    for (int c = w; c < nchunk; c += 8) s += partial[(size_t)c * total + k];
+  }
+  sh[w][lane] = s;
+  __syncthreads();
+  if (w || k >= total) return;
+  for (int v = 1; v < 8; ++v) s += sh[v][lane];
   out[k] = s;
 }
 
 // out[oc[k]][i] = base[bc[k]][i] + sum_j in[ic[j]][i] C[j][k]  (k < nout;
 // C is [nin][nout]); out may be base (in-place update), never in
-__global__ void __launch_bounds__(256) k_combine(size_t nv, int nin, const float *__restrict__ in,
+__global__ void __launch_bounds__(CT) k_combine(size_t nv, int nin, const float *__restrict__ in,
                                                  const int *__restrict__ ic, int nout, float *out,
                                                  const int *__restrict__ oc, const float *base,
                                                  const int *__restrict__ bc, const float *__restrict__ C) {
@@ -106,6 +118,7 @@ __global__ void __launch_bounds__(256) k_combine(size_t nv, int nin, const float
     float acc[CK];
 #pragma unroll
     for (int kk = 0; kk < CK; ++kk) acc[kk] = kk < kn ? base[(size_t)bc[k0 + kk] * nv + i] : 0.f;
+#pragma unroll 8
     for (int j = 0; j < nin; ++j) {
       const float x = in[(size_t)ic[j] * nv + i];
 #pragma unroll
@@ -136,16 +149,16 @@ void launch_gram(size_t nv, int sa, const float *U, const int *ua, int sb, const
   dim3 grid(kGramChunks, (sa + GT - 1) / GT, (sb + GT - 1) / GT);
   k_gram<<<grid, 256, 0, st>>>(nv, sa, U, ua, sb, V, vb, partial);
   const int total = sa * sb;
-  k_gram_reduce<<<(total + 255) / 256, 256, 0, st>>>(kGramChunks, total, partial, out);
+  k_gram_reduce<<<(total + 31) / 32, 256, 0, st>>>(kGramChunks, total, partial, out);
 }
 
 void launch_combine(size_t nv, int nin, const float *in, const int *ic, int nout, float *out, const int *oc,
                     const float *base, const int *bc, const float *C, cudaStream_t st) {
   if (nout < 1) return;
   add_launch_count(1);
-  int bx = (int)std::min<size_t>((nv + 255) / 256, 4 * 152);
+  int bx = (int)std::min<size_t>((nv + CT - 1) / CT, 16 * 152);
   dim3 grid(bx < 1 ? 1 : bx, (nout + CK - 1) / CK);
-  k_combine<<<grid, 256, 0, st>>>(nv, nin, in, ic, nout, out, oc, base, bc, C);
+  k_combine<<<grid, CT, 0, st>>>(nv, nin, in, ic, nout, out, oc, base, bc, C);
 }
 
 void launch_scale_alpha32(int ncol, int n, const float *alpha, const float *r, float *z, cudaStream_t st) {
@@ -241,17 +254,11 @@ int System::bpcg32_ws(Workspace &w, int ncol, int max_it, double eta) {
   F32Shape shape{1, 1, 2};
   int st = tune_f32(w, std::min(ncol, 8), shape);
   if (st) return st;
-  const bool blocks = inner_precond_ >= 1 && blk_info_;
-  const bool near = blocks && near_precond();
-  auto precondition = [&](int nc) {
-    if (blocks) {
-      gpu::launch_block_apply(nc, n, blk_info_, blk_minv_, w.r32, w.z32, st_);
-      // the next direction block (w.t32) is written only after this: scratch
-      if (near)
-        gpu::launch_near_correct(nc, n, blk_info_, blk_minv_, near_ri_, near_ci_, near_blk_, w.z32, w.t32, st_);
-    } else {
-      gpu::launch_scale_alpha32(nc, n, alpha32_, w.r32, w.z32, st_);
-    }
+  // Z = M^-1 R of all columns and rho = r.z of each in w.scal_h
+  const gpu::CgJob<float> job = inner_job(w, ncol, false);
+  auto precondition = [&]() {
+    if (job.mode == 0) gpu::launch_scale_alpha32(ncol, n, alpha32_, w.r32, w.z32, st_);
+    gpu::launch_precondition(job, w.scal_h, st_);
   };
   // index maps in w.bidx: [0, smax) identity, then the active columns
   std::vector<int> idx(2 * (size_t)smax);
@@ -259,10 +266,7 @@ int System::bpcg32_ws(Workspace &w, int ncol, int max_it, double eta) {
   int *ident = w.bidx, *actd = w.bidx + smax;
   double *gpart = w.gram, *gout = w.gram + (size_t)gpu::block_cg_gram_doubles(smax) - 2 * (size_t)smax * smax;
   cudaMemsetAsync(w.x32, 0, ncol * nv * sizeof(float), st_);
-  precondition(ncol);
-  gpu::launch_dots_f32(ncol, nv, w.r32, w.z32, w.partial, st_);
-  gpu::launch_reduce_partials(ncol, w.partial, w.dots, st_);
-  cudaMemcpyAsync(w.scal_h, w.dots, ncol * sizeof(double), cudaMemcpyDeviceToHost, st_);
+  precondition();
   st = check(cudaStreamSynchronize(st_), "block CG init");
   if (st) return st;
   std::vector<int> act;
@@ -313,17 +317,14 @@ int System::bpcg32_ws(Workspace &w, int ncol, int max_it, double eta) {
     cudaMemcpyAsync(w.bcoef, C.data(), 2 * (size_t)s * sa * sizeof(float), cudaMemcpyHostToDevice, st_);
     gpu::launch_combine(nv, s, w.p32, ident, sa, w.x32, actd, w.x32, actd, w.bcoef, st_);
     gpu::launch_combine(nv, s, w.h32, ident, sa, w.r32, actd, w.r32, actd, w.bcoef + (size_t)s * sa, st_);
-    precondition(ncol);
+    precondition();
     // convergence of each column, and K = Q^T Z
-    gpu::launch_dots_f32(ncol, nv, w.r32, w.z32, w.partial, st_);
-    gpu::launch_reduce_partials(ncol, w.partial, w.dots, st_);
     gpu::launch_gram(nv, s, w.h32, ident, sa, w.z32, actd, gpart, gout, st_);
     cudaMemcpyAsync(w.bscal_h, gout, (size_t)s * sa * sizeof(double), cudaMemcpyDeviceToHost, st_);
-    cudaMemcpyAsync(w.bscal_h + (size_t)s * sa, w.dots, ncol * sizeof(double), cudaMemcpyDeviceToHost, st_);
     st = check(cudaStreamSynchronize(st_), "block CG update");
     if (st) return st;
     K.assign(w.bscal_h, w.bscal_h + (size_t)s * sa);
-    const double *rho = w.bscal_h + (size_t)s * sa;
+    const double *rho = w.scal_h;
     std::vector<int> keep;  // positions in act of the columns still above eta
     for (int k = 0; k < sa; ++k) {
       const double rms = std::sqrt(std::max(rho[act[k]], 0.0) / (double)nv);

@@ -124,7 +124,7 @@ System::~System() {
   if (st_) cudaStreamSynchronize(st_);
   free_ws(ws_);
   free_ws(wsb_);
-  void *bufs[] = {inv32_, sqrt_alpha_, d_.pol_pos, d_.pol_a, d_.pol_alpha, d_.polar_mm, d_.pol_pos32, d_.pol_a32,
+  void *bufs[] = {inv32_, sqrt_alpha_, d_.pol_pos, d_.pol_a, d_.pol_alpha, d_.pol_ialpha, d_.polar_mm, d_.pol_pos32, d_.pol_a32,
                   d_.pol_wa32, d_.mm_split, d_.mm_sub_box32, d_.mm_tile_box32,
                   d_.mm_wa32, d_.mm_pos,
                   d_.mm_a, d_.mm_q, d_.m2d_ri, d_.m2d_src, d_.m2d_sP, d_.m2d_sD, d_.d2d_ri, d_.d2d_src,
@@ -252,7 +252,7 @@ int System::upload_static() {
   size_t nv = 3 * (size_t)n;
   int nipd = m.n_ipd;
   int bad = 0;
-  bad |= alloc(d_.pol_pos, n) | alloc(d_.pol_a, n) | alloc(d_.pol_alpha, n) | alloc(d_.polar_mm, n);
+  bad |= alloc(d_.pol_pos, n) | alloc(d_.pol_a, n) | alloc(d_.pol_alpha, n) | alloc(d_.pol_ialpha, n) | alloc(d_.polar_mm, n);
   bad |= alloc(d_.pol_pos32, n) | alloc(d_.pol_a32, n) | alloc(alpha32_, n);
   bad |= alloc(d_.pol_wa32, n) | alloc(d_.mm_wa32, mm);
   bad |= alloc(d_.mm_pos, mm) | alloc(d_.mm_a, mm) | alloc(d_.mm_q, (size_t)mm * m.ld_cart);
@@ -282,7 +282,7 @@ int System::upload_static() {
   ws_.x32 = x32_, ws_.r32 = r32_, ws_.p32 = p32_, ws_.h32 = h32_, ws_.z32 = z32_;
   ws_.scratch32 = scratch32_;
   ws_.scratch32_nsplit = f32_splits;
-  ws_.partial = partial_, ws_.dots = dots_, ws_.hist = hist_;
+  ws_.partial = partial_, ws_.partial_len = (size_t)gpu::kRedBlocks * 8, ws_.dots = dots_, ws_.hist = hist_;
   ws_.cols = cols_, ws_.cols_h = cols_h_, ws_.scal_h = scal_h_;
   ws_.owned = false;
   d_.m2d_nnz = (int)m2d_pairs_.src.size();
@@ -302,6 +302,8 @@ int System::upload_static() {
     a32[k] = (float)a[k];
   }
   up(d_.pol_alpha, alpha.data(), n * sizeof(double));
+  for (double &a : alpha) a = 1.0 / a;
+  up(d_.pol_ialpha, alpha.data(), n * sizeof(double));
   up(d_.pol_a, a.data(), n * sizeof(double));
   up(alpha32_, alpha32.data(), n * sizeof(float));
   up(d_.pol_a32, a32.data(), n * sizeof(float));
@@ -683,6 +685,13 @@ void System::direct_product(int ncol, const double *x, double *y, bool dodiag, i
     gpu::launch_tmu_f64_sym(d_, ncol, x, y, dodiag, sym_scratch_, st_);
   else
     gpu::launch_tmu_f64(d_, ncol, x, y, dodiag, st_);
+}
+
+// matvec64 would take the symmetric direct product in one column group
+bool System::direct_symmetric(int matv, int ncol) {
+  if ((matv == kMatvIncore && tmat_ok_) || fmm_on_ || ncol > 2) return false;
+  if (fp64_kernel_ != 2 && !(fp64_kernel_ == 0 && d_.n >= gpu::kSymMinSites)) return false;
+  return ensure_sym_scratch() == kOk;
 }
 
 // fixed-point accumulators of the symmetric products (FP64, double-single

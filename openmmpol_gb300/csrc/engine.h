@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "kernels.h"
+#include "pcg.h"
 #include "ommp_internal.h"
 
 namespace ommp {
@@ -33,7 +34,8 @@ struct Workspace {
   float *x32 = nullptr, *r32 = nullptr, *p32 = nullptr, *h32 = nullptr, *z32 = nullptr;
   float *scratch32 = nullptr;
   int scratch32_nsplit = 0;  // source splits the FP32 scratch holds for cap columns
-  double *partial = nullptr;  // kRedBlocks x cap
+  double *partial = nullptr;  // partial sums of the reductions
+  size_t partial_len = 0;     // at least kRedBlocks x cap
   double *dots = nullptr;     // 3 x cap (+ fcap)
   double *hist = nullptr;     // cap x maxhist, or none
   // block CG of the batch (block_cg.cu): next directions, Gram partials and
@@ -231,7 +233,10 @@ class System {
   };
   int tune_f32(Workspace &w, int ncol, F32Shape &shape);
   bool update_allowed(const std::vector<double> &rms) const;
-  void f32_product(Workspace &w, int ncol, const F32Shape &shape);
+  int f32_product(Workspace &w, int ncol, const F32Shape &shape, bool prepared = false, double *part = nullptr,
+                  int max_part = 0);
+  gpu::CgJob<float> inner_job(Workspace &w, int ncol, bool prepared);
+  bool direct_symmetric(int matv, int ncol);
   int ensure_batch_ws(int ncol, int nf);
   void free_ws(Workspace &w);
   int check(cudaError_t e, const char *what);

@@ -23,6 +23,7 @@
 
 #include "kernels.h"
 #include "pair_math.cuh"
+#include "pcg.h"
 
 namespace ommp {
 namespace gpu {
@@ -157,45 +158,41 @@ __global__ void __launch_bounds__(TPB) k_tmu(int n, const float4 *__restrict__ p
   }
 }
 
-// y[r][j] = -(sum_split partial + scaled-pair corrections) (+ x/alpha)
-template <typename T, bool AMOEBA>
-__global__ void k_tmu_finish(int n, int nrhs, int nsplit, const T *__restrict__ partial,
-                             const typename Vec4<T>::type *__restrict__ pos,
-                             const T *__restrict__ damp, const float2 *__restrict__ wa,
-                             const T *__restrict__ x, const double *__restrict__ alpha, bool dodiag,
+// y[r][j] = -(field + scaled-pair corrections) (+ x/alpha): the FMM's finishing pass
+template <bool AMOEBA>
+__global__ void k_tmu_finish(int n, const double *__restrict__ field, const Pos64 *__restrict__ pos,
+                             const double *__restrict__ damp, const float2 *__restrict__ wa,
+                             const double *__restrict__ x, const double *__restrict__ alpha, bool dodiag,
                              const int *__restrict__ ri, const int *__restrict__ src,
-                             const double *__restrict__ scale, T thr, float thr2m, T *__restrict__ y) {
-  constexpr bool F64 = std::is_same<T, double>::value;
+                             const double *__restrict__ scale, double thr, float thr2m, double *__restrict__ y) {
   int j = blockIdx.x * blockDim.x + threadIdx.x;
   int r = blockIdx.y;
   if (j >= n) return;
-  double e[3] = {0, 0, 0};
-  for (int s = 0; s < nsplit; ++s)
-    for (int c = 0; c < 3; ++c) e[c] += (double)partial[(((size_t)s * nrhs + r) * n + j) * 3 + c];
+  double e[3];
+  for (int c = 0; c < 3; ++c) e[c] = field[((size_t)r * n + j) * 3 + c];
   if (ri) {
-    auto pt = pos[j];
-    T at = AMOEBA ? damp[j] : T(0);
-    float2 wat = F64 ? wa[j] : make_float2(0.f, 0.f);
+    const Pos64 pt = pos[j];
+    const double at = AMOEBA ? damp[j] : 0.0;
+    const float2 wat = wa[j];
     for (int k = ri[j]; k < ri[j + 1]; ++k) {
       int i = src[k];
-      auto ps = pos[i];
-      T dx = pt.x - ps.x, dy = pt.y - ps.y, dz = pt.z - ps.z;
-      T r2 = dx * dx + dy * dy + dz * dz;
-      T k3, k5x3;
-      dd_pair<T, AMOEBA>(r2, pt.w, ps.w, at, AMOEBA ? damp[i] : T(0), wat, F64 ? wa[i] : wat, thr, thr2m, k3,
-                         k5x3);
-      const T *mu = &x[((size_t)r * n + i) * 3];
-      T f = k5x3 * (mu[0] * dx + mu[1] * dy + mu[2] * dz);
+      const Pos64 ps = pos[i];
+      double dx = pt.x - ps.x, dy = pt.y - ps.y, dz = pt.z - ps.z;
+      double r2 = dx * dx + dy * dy + dz * dz;
+      double k3, k5;
+      dd_pair_f64<AMOEBA>(r2, pt.w, ps.w, at, AMOEBA ? damp[i] : 0.0, wat, wa[i], thr, thr2m, k3, k5);
+      const double *mu = &x[((size_t)r * n + i) * 3];
+      double f = 3.0 * k5 * (mu[0] * dx + mu[1] * dy + mu[2] * dz);
       double cs = scale[k] - 1.0;
-      e[0] += cs * (double)(f * dx - k3 * mu[0]);
-      e[1] += cs * (double)(f * dy - k3 * mu[1]);
-      e[2] += cs * (double)(f * dz - k3 * mu[2]);
+      e[0] += cs * (f * dx - k3 * mu[0]);
+      e[1] += cs * (f * dy - k3 * mu[1]);
+      e[2] += cs * (f * dz - k3 * mu[2]);
     }
   }
-  const T *xj = &x[((size_t)r * n + j) * 3];
-  T *yj = &y[((size_t)r * n + j) * 3];
+  const double *xj = &x[((size_t)r * n + j) * 3];
+  double *yj = &y[((size_t)r * n + j) * 3];
   double ia = dodiag ? 1.0 / alpha[j] : 0.0;
-  for (int c = 0; c < 3; ++c) yj[c] = (T)(-e[c] + (dodiag ? (double)xj[c] * ia : 0.0));
+  for (int c = 0; c < 3; ++c) yj[c] = -e[c] + (dodiag ? xj[c] * ia : 0.0);
 }
 
 // ---------------------------------------------------------------------------
@@ -405,111 +402,11 @@ __global__ void k_to_f32_cols(size_t nv, size_t tot, const double *x, const doub
     y[i] = (float)(x[i] * scale[i / nv]);
 }
 
-// start of the inner PCG with the first r.z on the device (no host read)
-__global__ void k_cg_init(int ncol, const double *dots, CgCol *cols, double tol) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= ncol) return;
-  CgCol c{};
-  c.gold = dots[k];
-  c.tol = tol;
-  c.active = dots[k] > 0.0 ? 1 : 0;
-  cols[k] = c;
-}
-
-__global__ void k_cg_alpha(int ncol, const double *dots, CgCol *cols, double eps) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= ncol) return;
-  CgCol c = cols[k];
-  if (!c.active) return;
-  c.gama = dots[k];
-  if (fabs(c.gama) < eps) {
-    c.quick = 1;
-    c.active = 0;
-    c.alpha = 0.0;
-  } else {
-    c.alpha = c.gold / c.gama;
-  }
-  cols[k] = c;
-}
-
-// one column per blockIdx.y (see k_dots)
-template <typename T>
-__global__ void k_cg_update(int ncol, int n, T *x, T *r, const T *p, const T *h, T *z,
-                            const T *alpha_pol, const CgCol *cols, double *partial) {
-  __shared__ double sh[kRedThreads / 32];
-  size_t nv = 3 * (size_t)n;
-  const int k = blockIdx.y;
-  double acc = 0.0;
-  if (cols[k].active) {
-    double al = cols[k].alpha;
-    T a = (T)al;
-    size_t off = (size_t)k * nv;
-    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += (size_t)gridDim.x * blockDim.x) {
-      if (sizeof(T) == 8) {
-        x[off + i] += a * p[off + i];
-        r[off + i] -= a * h[off + i];
-      } else {
-        x[off + i] = (T)((double)x[off + i] + al * (double)p[off + i]);
-        r[off + i] = (T)((double)r[off + i] - al * (double)h[off + i]);
-      }
-      T zi = alpha_pol[i / 3] * r[off + i];
-      z[off + i] = zi;
-      acc += (double)r[off + i] * (double)zi;
-    }
-  }
-  for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = acc;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double s = 0.0;
-    for (int w = 0; w < kRedThreads / 32; ++w) s += sh[w];
-    partial[(size_t)blockIdx.x * ncol + k] = s;
-  }
-}
-
-__global__ void k_cg_gnew(int ncol, int n, const double *dots, CgCol *cols, double *hist, int hist_stride) {
-  int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= ncol) return;
-  CgCol c = cols[k];
-  if (!c.active) return;
-  c.gnew = dots[k];
-  c.rms = sqrt(c.gnew / (3.0 * n));
-  c.iters += 1;
-  if (hist && c.iters <= hist_stride) hist[(size_t)k * hist_stride + c.iters - 1] = c.rms;
-  if (c.rms < c.tol) {
-    c.converged = 1;
-    c.active = 0;
-  } else {
-    c.beta = c.gnew / c.gold;
-    c.gama = c.beta;  // the reference reuses gama for the beta ratio
-    c.gold = c.gnew;
-  }
-  cols[k] = c;
-}
-
-template <typename T>
-__global__ void k_cg_pupdate(int ncol, int n, T *p, const T *z, const CgCol *cols) {
-  size_t nv = 3 * (size_t)n;
-  const int k = blockIdx.y;
-  if (!cols[k].active) return;
-  T b = (T)cols[k].beta;
-  size_t off = (size_t)k * nv;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nv; i += (size_t)gridDim.x * blockDim.x)
-    p[off + i] = b * p[off + i] + z[off + i];
-}
-
 __global__ void k_ir_accumulate(int ncol, int n, double *mu, const float *d32, const double *scale) {
   size_t nv = 3 * (size_t)n;
   size_t tot = nv * ncol;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < tot; i += (size_t)gridDim.x * blockDim.x)
     mu[i] += scale[i / nv] * (double)d32[i];
-}
-
-__global__ void k_residual_update(int ncol, int n, double *r, const float *t32, const double *scale) {
-  size_t nv = 3 * (size_t)n;
-  size_t tot = nv * ncol;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < tot; i += (size_t)gridDim.x * blockDim.x)
-    r[i] -= scale[i / nv] * (double)t32[i];
 }
 
 __global__ void k_residual(size_t tot, const double *rhs, const double *tmu, double *r) {
@@ -743,153 +640,54 @@ static void tmu_dispatch(const DevSites &s, int nrhs, const float *x, float *par
   }
 }
 
-template <typename T>
-static void tmu_finish(const DevSites &s, int nrhs, int nsplit, const T *partial,
-                       const typename Vec4<T>::type *pos, const T *damp, const T *x, bool dodiag, T *y,
-                       int gmax, cudaStream_t st) {
-  // the same column groups as tmu_dispatch, each with its own block
-  int done = 0;
-  while (done < nrhs) {
-    int g = column_group(nrhs - done, gmax);
-    const T *pg = partial + (size_t)nsplit * done * s.n * 3;
-    add_launch_count(1);
-    dim3 grid((s.n + 127) / 128, g);
-    size_t xo = (size_t)done * s.n * 3;
-    const float2 *wa = std::is_same<T, double>::value ? s.pol_wa32 : nullptr;
-    float thr2m = damp_thr2_margin(s);
-    if (s.amoeba)
-      k_tmu_finish<T, true><<<grid, 128, 0, st>>>(s.n, g, nsplit, pg, pos, damp, wa, x + xo, s.pol_alpha,
-                                                  dodiag, s.d2d_nnz ? s.d2d_ri : nullptr, s.d2d_src, s.d2d_s,
-                                                  (T)s.damp_thr, thr2m, y + xo);
-    else
-      k_tmu_finish<T, false><<<grid, 128, 0, st>>>(s.n, g, nsplit, pg, pos, damp, wa, x + xo, s.pol_alpha,
-                                                   dodiag, s.d2d_nnz ? s.d2d_ri : nullptr, s.d2d_src, s.d2d_s,
-                                                   (T)s.damp_thr, thr2m, y + xo);
-    done += g;
-  }
-}
-
 void launch_tmu_finish64(const DevSites &s, int nrhs, const double *partial, const double *x, bool dodiag,
                          double *y, cudaStream_t st) {
-  tmu_finish<double>(s, nrhs, 1, partial, s.pol_pos, s.pol_a, x, dodiag, y, 2, st);
+  add_launch_count(1);
+  const dim3 grid((s.n + 127) / 128, nrhs);
+  const int *ri = s.d2d_nnz ? s.d2d_ri : nullptr;
+  if (s.amoeba)
+    k_tmu_finish<true><<<grid, 128, 0, st>>>(s.n, partial, s.pol_pos, s.pol_a, s.pol_wa32, x, s.pol_alpha, dodiag, ri,
+                                             s.d2d_src, s.d2d_s, s.damp_thr, damp_thr2_margin(s), y);
+  else
+    k_tmu_finish<false><<<grid, 128, 0, st>>>(s.n, partial, s.pol_pos, s.pol_a, s.pol_wa32, x, s.pol_alpha, dodiag,
+                                              ri, s.d2d_src, s.d2d_s, s.damp_thr, damp_thr2_margin(s), y);
 }
 
-void launch_tmu_finish32(const DevSites &s, int nrhs, const float *partial, const float *x, float *y,
-                         cudaStream_t st) {
-  tmu_finish<float>(s, nrhs, 1, partial, s.pol_pos32, s.pol_a32, x, true, y, 2, st);
-}
-
-void launch_tmu_f32(const DevSites &s, int nrhs, const float *x, float *y, float *scratch, int nsplit,
-                    cudaStream_t st, int gmax, int kver, double *sym_scratch) {
-  if (s.n == 0) return;
-  if (kver == 3 && sym_scratch) {
-    // symmetric kernel: fixed-point sums read out as floats into the third
-    // block of the symmetric scratch, then the shared finishing pass
-    const size_t nv = 3 * (size_t)s.n;
-    for (int c = 0; c < nrhs;) {
-      const int g = (nrhs - c >= 2 && gmax >= 2) ? 2 : 1;
+int launch_tmu_f32(const DevSites &s, int nrhs, const float *x, float *y, float *scratch, int nsplit, cudaStream_t st,
+                   int gmax, int kver, double *sym_scratch, bool prepared, double *part, int max_part) {
+  if (s.n == 0) return 0;
+  const size_t nv = 3 * (size_t)s.n;
+  const bool sym = kver == 3 && sym_scratch;
+  if (!sym) tmu_dispatch(s, nrhs, x, scratch, nsplit, gmax, st, kver);
+  int npart = 0;
+  for (int c = 0; c < nrhs;) {
+    const int g = column_group(nrhs - c, sym ? std::min(gmax, 2) : gmax);
+    F32Finish fin = f32_finish(s, g, x + c * nv, y + c * nv);
+    if (sym) {
+      // fixed-point sums, read out by the finishing pass
       const size_t C = 3 * (size_t)g;
       unsigned long long *lo = reinterpret_cast<unsigned long long *>(sym_scratch);
       unsigned long long *hi = lo + C * s.n;
-      float *e = reinterpret_cast<float *>(sym_scratch + 2 * C * s.n);
-      unsigned long long *bad = reinterpret_cast<unsigned long long *>(sym_scratch + 3 * C * s.n);
-      unsigned *next = reinterpret_cast<unsigned *>(bad + 1);
-      launch_tmu32_sym_pairs(s, g, x + c * nv, lo, hi, bad, next, e, st);
-      tmu_finish<float>(s, g, 1, e, s.pol_pos32, s.pol_a32, x + c * nv, true, y + c * nv, 2, st);
-      c += g;
+      unsigned long long *bad = lo + 3 * C * s.n;
+      if (!prepared) {
+        cudaMemsetAsync(lo, 0, 2 * C * s.n * sizeof(unsigned long long), st);
+        cudaMemsetAsync(bad, 0, 2 * sizeof(unsigned long long), st);
+      }
+      SymSlice one{&s, x + c * nv, lo, hi, bad, 0, tmu32_sym_items(s, g)};
+      launch_tmu32_sym_multi(g, &one, 1, reinterpret_cast<unsigned *>(bad + 1), st, true);
+      fin.lo = lo, fin.hi = hi, fin.bad = bad;
+    } else {
+      fin.partial = scratch + (size_t)nsplit * c * nv;
+      fin.nsplit = nsplit;
     }
-    return;
+    if (part) {
+      npart = fin.nblk = std::min(fin.nblk, max_part);
+      fin.part = part + (size_t)c * npart;
+    }
+    launch_f32_finish(&fin, 1, st);
+    c += g;
   }
-  tmu_dispatch(s, nrhs, x, scratch, nsplit, gmax, st, kver);
-  tmu_finish<float>(s, nrhs, nsplit, scratch, s.pol_pos32, s.pol_a32, x, true, y, gmax, st);
-}
-
-// z = M^-1 r, one thread per site and column: the three rows of the site's
-// block times the run's slice of r
-__global__ void k_block_apply(int n, const int4 *__restrict__ info, const float *__restrict__ minv,
-                              const float *__restrict__ r, float *__restrict__ z) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  const size_t co = (size_t)blockIdx.y * 3 * n;
-  const int4 b = info[j];
-  const int w = 3 * b.y;
-  const float *rr = r + co + 3 * (size_t)b.x;
-  const float *m0 = minv + b.z + (size_t)(3 * b.w) * w;
-  const float *m1 = m0 + w, *m2 = m1 + w;
-  float z0 = 0.f, z1 = 0.f, z2 = 0.f;
-  for (int l = 0; l < w; ++l) {
-    const float v = rr[l];
-    z0 = fmaf(m0[l], v, z0);
-    z1 = fmaf(m1[l], v, z1);
-    z2 = fmaf(m2[l], v, z2);
-  }
-  float *zz = z + co + 3 * (size_t)j;
-  zz[0] = z0;
-  zz[1] = z1;
-  zz[2] = z2;
-}
-
-// z -= B^-1 w, the second half of the Neumann step (w read over the run,
-// z[j] read and written by its own thread, so z may hold z0 in place)
-__global__ void k_block_apply_sub(int n, const int4 *__restrict__ info, const float *__restrict__ minv,
-                                  const float *__restrict__ w, float *__restrict__ z) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  const size_t co = (size_t)blockIdx.y * 3 * n;
-  const int4 b = info[j];
-  const int wd = 3 * b.y;
-  const float *ww = w + co + 3 * (size_t)b.x;
-  const float *m0 = minv + b.z + (size_t)(3 * b.w) * wd;
-  const float *m1 = m0 + wd, *m2 = m1 + wd;
-  float t0 = 0.f, t1 = 0.f, t2 = 0.f;
-  for (int l = 0; l < wd; ++l) {
-    const float v = ww[l];
-    t0 = fmaf(m0[l], v, t0);
-    t1 = fmaf(m1[l], v, t1);
-    t2 = fmaf(m2[l], v, t2);
-  }
-  float *zz = z + co + 3 * (size_t)j;
-  zz[0] -= t0;
-  zz[1] -= t1;
-  zz[2] -= t2;
-}
-
-// y[j] = sum over the near-field row j of N_ji x[i] (3x3 FP32 blocks)
-__global__ void k_near_apply(int n, const int *__restrict__ ri, const int *__restrict__ ci,
-                             const float *__restrict__ blk, const float *__restrict__ x, float *__restrict__ y) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  const size_t co = (size_t)blockIdx.y * 3 * n;
-  float y0 = 0.f, y1 = 0.f, y2 = 0.f;
-  for (int e = ri[j]; e < ri[j + 1]; ++e) {
-    const float *b = blk + 9 * (size_t)e;
-    const float *xi = x + co + 3 * (size_t)ci[e];
-    const float a = xi[0], c = xi[1], d = xi[2];
-    y0 = fmaf(b[0], a, fmaf(b[1], c, fmaf(b[2], d, y0)));
-    y1 = fmaf(b[3], a, fmaf(b[4], c, fmaf(b[5], d, y1)));
-    y2 = fmaf(b[6], a, fmaf(b[7], c, fmaf(b[8], d, y2)));
-  }
-  float *yy = y + co + 3 * (size_t)j;
-  yy[0] = y0;
-  yy[1] = y1;
-  yy[2] = y2;
-}
-
-void launch_near_correct(int ncol, int n, const int4 *info, const float *minv, const int *ri, const int *ci,
-                         const float *blk, float *z, float *w, cudaStream_t st) {
-  if (n == 0) return;
-  add_launch_count(2);
-  dim3 grid((n + 127) / 128, ncol);
-  k_near_apply<<<grid, 128, 0, st>>>(n, ri, ci, blk, z, w);
-  k_block_apply_sub<<<grid, 128, 0, st>>>(n, info, minv, w, z);
-}
-
-void launch_block_apply(int ncol, int n, const int4 *info, const float *minv, const float *r, float *z,
-                        cudaStream_t st) {
-  if (n == 0) return;
-  add_launch_count(1);
-  dim3 grid((n + 127) / 128, ncol);
-  k_block_apply<<<grid, 128, 0, st>>>(n, info, minv, r, z);
+  return npart;
 }
 
 // Batched right-hand sides, set-major columns: rhs[s*nf + f] = E_M2D[s] + field[f]
@@ -973,11 +771,6 @@ void launch_dots_bcast(int ncol, size_t n, const double *a, const double *b, dou
   add_launch_count(1);
   k_dots<double><<<dim3(dots_blocks(n), ncol), kRedThreads, 0, st>>>(ncol, n, a, b, 0, partial);
 }
-void launch_dots_f32(int ncol, size_t n, const float *a, const float *b, double *partial, cudaStream_t st) {
-  if (ncol < 1) return;
-  add_launch_count(1);
-  k_dots<float><<<dim3(dots_blocks(n), ncol), kRedThreads, 0, st>>>(ncol, n, a, b, n, partial);
-}
 void launch_reduce_partials(int ncol, const double *partial, double *result, cudaStream_t st) {
   add_launch_count(1);
   k_reduce_partials<<<ncol, 32, 0, st>>>(ncol, kRedBlocks, partial, result);
@@ -1004,50 +797,9 @@ void launch_to_f32(size_t n, const double *x, const double *scale, float *y, cud
   add_launch_count(1);
   k_to_f32<<<blocks_for(n, 256), 256, 0, st>>>(n, x, scale, y);
 }
-void launch_cg_init(int ncol, const double *dots, CgCol *cols, double tol, cudaStream_t st) {
-  add_launch_count(1);
-  k_cg_init<<<(ncol + 127) / 128, 128, 0, st>>>(ncol, dots, cols, tol);
-}
-void launch_cg_alpha(int ncol, const double *dots, CgCol *cols, double eps, cudaStream_t st) {
-  add_launch_count(1);
-  k_cg_alpha<<<(ncol + 127) / 128, 128, 0, st>>>(ncol, dots, cols, eps);
-}
-void launch_cg_update(int ncol, int n, double *x, double *r, const double *p, const double *h, double *z,
-                      const double *alpha_pol, const CgCol *cols, double *partial, cudaStream_t st) {
-  if (ncol < 1) return;
-  add_launch_count(1);
-  k_cg_update<double><<<dim3(kRedBlocks, ncol), kRedThreads, 0, st>>>(ncol, n, x, r, p, h, z, alpha_pol, cols,
-                                                                      partial);
-}
-void launch_cg_update_f32(int ncol, int n, float *x, float *r, const float *p, const float *h, float *z,
-                          const float *alpha_pol, const CgCol *cols, double *partial, cudaStream_t st) {
-  if (ncol < 1) return;
-  add_launch_count(1);
-  k_cg_update<float><<<dim3(kRedBlocks, ncol), kRedThreads, 0, st>>>(ncol, n, x, r, p, h, z, alpha_pol, cols,
-                                                                     partial);
-}
-void launch_cg_gnew(int ncol, int n, const double *dots, CgCol *cols, double *hist, int hist_stride,
-                    cudaStream_t st) {
-  add_launch_count(1);
-  k_cg_gnew<<<(ncol + 127) / 128, 128, 0, st>>>(ncol, n, dots, cols, hist, hist_stride);
-}
-void launch_cg_pupdate(int ncol, int n, double *p, const double *z, const CgCol *cols, cudaStream_t st) {
-  if (ncol < 1) return;
-  add_launch_count(1);
-  k_cg_pupdate<double><<<dim3(blocks_for(3 * (size_t)n, 256), ncol), 256, 0, st>>>(ncol, n, p, z, cols);
-}
-void launch_cg_pupdate_f32(int ncol, int n, float *p, const float *z, const CgCol *cols, cudaStream_t st) {
-  if (ncol < 1) return;
-  add_launch_count(1);
-  k_cg_pupdate<float><<<dim3(blocks_for(3 * (size_t)n, 256), ncol), 256, 0, st>>>(ncol, n, p, z, cols);
-}
 void launch_ir_accumulate(int ncol, int n, double *mu, const float *d32, const double *scale, cudaStream_t st) {
   add_launch_count(1);
   k_ir_accumulate<<<blocks_for((size_t)ncol * n * 3, 256), 256, 0, st>>>(ncol, n, mu, d32, scale);
-}
-void launch_residual_update(int ncol, int n, double *r, const float *t32, const double *scale, cudaStream_t st) {
-  add_launch_count(1);
-  k_residual_update<<<blocks_for((size_t)ncol * n * 3, 256), 256, 0, st>>>(ncol, n, r, t32, scale);
 }
 void launch_residual(size_t total, const double *rhs, const double *tmu, double *r, cudaStream_t st) {
   add_launch_count(1);

@@ -29,6 +29,7 @@ struct DevSites {
   Pos64 *pol_pos = nullptr;   // x, y, z, 1/thole
   double *pol_a = nullptr;      // Thole damping a
   double *pol_alpha = nullptr;  // polarizability
+  double *pol_ialpha = nullptr;  // and its reciprocal
   int *polar_mm = nullptr;      // mm index of each polarizable site
   float4 *pol_pos32 = nullptr;  // centred FP32 copy: x, y, z, 1/thole
   float *pol_a32 = nullptr;
@@ -83,14 +84,13 @@ void launch_tmu_f64(const DevSites &s, int nrhs, const double *x, double *y, boo
 // u-scaled pair corrections, the sign and the 1/alpha diagonal
 void launch_tmu_finish64(const DevSites &s, int nrhs, const double *partial, const double *x, bool dodiag,
                          double *y, cudaStream_t st);
-// FP32 finishing pass (partial [nrhs][n][3], one split; diagonal included)
-void launch_tmu_finish32(const DevSites &s, int nrhs, const float *partial, const float *x, float *y,
-                         cudaStream_t st);
 // Same product with each unordered pair evaluated once (deterministic
 // half-shell schedule, tmu_sym.cu): near pairs in FP64, the others in
 // double-single; scratch of tmu_sym_scratch_doubles(s, nrhs_max).  The product
 // of every mode from kSymMinSites sites (launch_tmu_f64 below).
 constexpr int kSymMinSites = 1000;
+// the finishing passes give a site four lanes below this many sites, one above
+constexpr int kFinishLanesSites = 32768;
 // squared distances within which a pair always runs in FP64 (AMOEBA pairs
 // also while the damping is strong, a u^3 < 20)
 constexpr float kSymNear2 = 36.f, kSymNear2Wang = 64.f;
@@ -99,11 +99,13 @@ void launch_tmu_f64_sym(const DevSites &s, int nrhs, const double *x, double *y,
                         cudaStream_t st);
 // its passes for callers that spread a product over launches: accumulators
 // [g][n][3] (lo, then hi) and the two words from bad zeroed and the scale of x
-// found (before the first share), and the sums read out into y = T x
+// found (before the first share), and the sums read out into y = T x, with
+// at most max_part partial sums of x.y per column (part [g][*npart])
 void launch_tmu_sym_prepare(const DevSites &s, int g, const double *x, unsigned long long *lo,
                             unsigned long long *bad, cudaStream_t st);
 void launch_tmu_sym_finish(const DevSites &s, int g, const unsigned long long *lo, const unsigned long long *hi,
-                           const unsigned long long *bad, const double *x, bool dodiag, double *y, cudaStream_t st);
+                           const unsigned long long *bad, const double *x, bool dodiag, double *y, cudaStream_t st,
+                           double *part = nullptr, int max_part = 0, int *npart = nullptr);
 // the largest high word of |x| (the scale of the double-single products)
 void launch_max_word(size_t total, const double *x, unsigned *word, cudaStream_t st);
 // near field of the FMM (fmm_near.cu): the dipoles x [col][n][3] of the 27
@@ -133,13 +135,12 @@ void split_coordinates(const double *x, int n, double centre[3], float4 *out);
 // kver 3: the symmetric kernel of tmu32.cu (each unordered pair once),
 // columns in groups of gmax (1 or 2), sums in sym_scratch (laid out as for
 // launch_tmu_f64_sym, tmu_sym_scratch_doubles(s, 2)); scratch unused.
-void launch_tmu_f32(const DevSites &s, int nrhs, const float *x, float *y, float *scratch,
-                    int nsplit, cudaStream_t st, int gmax = 4, int kver = 2, double *sym_scratch = nullptr);
-// symmetric FP32 pair sums of g (1 or 2) columns into the fixed-point
-// accumulators lo / hi [g][n][3] (zeroed here), read out into out [g][n][3]
-void launch_tmu32_sym_pairs(const DevSites &s, int g, const float *x, unsigned long long *lo,
-                            unsigned long long *hi, unsigned long long *bad, unsigned *next, float *out,
-                            cudaStream_t st);
+// prepared: the accumulators of a kver-3 product in one column group are
+// zero already.  part: partial sums of x.y, at most max_part per column; their
+// number is returned (part [nrhs][number]).
+int launch_tmu_f32(const DevSites &s, int nrhs, const float *x, float *y, float *scratch, int nsplit, cudaStream_t st,
+                   int gmax = 4, int kver = 2, double *sym_scratch = nullptr, bool prepared = false,
+                   double *part = nullptr, int max_part = 0);
 int tmu32_sym_resident(int g, bool amoeba);
 
 // ---- multi-system symmetric products --------------------------------------
@@ -163,14 +164,14 @@ struct SymSlice {
 };
 constexpr int kMaxSymSlices = 32;  // systems per launch
 int tmu32_sym_items(const DevSites &s, int g, double round_pairs = 0.0);
-// next: a device counter of the launch (zeroed by the launcher)
-void launch_tmu32_sym_multi(int g, const SymSlice *sl, int nsl, unsigned *next, cudaStream_t st);
-void launch_fixed_to_float(size_t total, const unsigned long long *lo, const unsigned long long *hi,
-                           const unsigned long long *bad, float *out, cudaStream_t st);
+// next: a device counter of the launch (zeroed by the launcher unless it is
+// zero already)
+void launch_tmu32_sym_multi(int g, const SymSlice *sl, int nsl, unsigned *next, cudaStream_t st, bool zeroed = false);
 // symmetric product of FP64 accuracy (g = 1 or 2; one damping kind per
 // launch; launch_tmu_sym_prepare before a product's first share)
 int tmu_f64_sym_items(const DevSites &s, int g, double round_pairs = 0.0);
-void launch_tmu_f64_sym_multi(int g, bool amoeba, const SymSlice *sl, int nsl, unsigned *next, cudaStream_t st);
+void launch_tmu_f64_sym_multi(int g, bool amoeba, const SymSlice *sl, int nsl, unsigned *next, cudaStream_t st,
+                              bool zeroed = false);
 void launch_tmu32_pairs(const DevSites &s, int g, const float *x, float *partial, int nsplit, cudaStream_t st);
 // source splits an FP32 scratch must hold (per column) for every shape the
 // autotuner may pick
@@ -193,15 +194,6 @@ void launch_m2m(const DevSites &s, bool grad, double *partial, int nsplit, int *
 size_t grad_sym_doubles(const DevSites &s);
 void launch_grad_sym(const DevSites &s, const double *ipd, const int *mm_polar, const unsigned *polar, double *buf,
                      int *err, cudaStream_t st);
-// z = M^-1 r for the block-Jacobi preconditioner (info / minv as built by
-// build_block_jacobi), columns [ncol][n][3], FP32
-void launch_block_apply(int ncol, int n, const int4 *info, const float *minv, const float *r, float *z,
-                        cudaStream_t st);
-// the Neumann step of the near-field preconditioner on z = B^-1 r:
-// w = N z (near-field rows ri/ci/blk of build_near_field), z -= B^-1 w;
-// w is a scratch of the same shape as z
-void launch_near_correct(int ncol, int n, const int4 *info, const float *minv, const int *ri, const int *ci,
-                         const float *blk, float *z, float *w, cudaStream_t st);
 // batched fields: rhs[s*nf+f] = E_M2D[s] + field[f]; solution scatter to [f][s]
 void launch_batch_rhs(int n, int nf, int nset, const double *e_m2d, const double *fields, double *rhs,
                       cudaStream_t st);
@@ -247,8 +239,6 @@ void launch_dots(int ncol, size_t n, const double *a, const double *b, double *p
 // partial[b][k] = sum_i a[k*n+i] * v[i]  (one vector against ncol columns)
 void launch_dots_bcast(int ncol, size_t n, const double *a, const double *v, double *partial,
                        cudaStream_t st);
-void launch_dots_f32(int ncol, size_t n, const float *a, const float *b, double *partial,
-                     cudaStream_t st);
 // result[k] = sum_b partial[b][k]  (fixed order)
 void launch_reduce_partials(int ncol, const double *partial, double *result, cudaStream_t st);
 
@@ -272,34 +262,12 @@ struct CgCol {
   int iters;
 };
 // cols[k] = {gold = dots[k], tol, active = dots[k] > 0} (inner PCG start)
-void launch_cg_init(int ncol, const double *dots, CgCol *cols, double tol, cudaStream_t st);
-// gama_k = (h.p)_k from reduced dots; alpha = gold/gama; quick-exit flags.
-void launch_cg_alpha(int ncol, const double *dots, CgCol *cols, double eps, cudaStream_t st);
-// x += alpha p; r -= alpha h; z = alpha_pol r; partial r.z per column
-void launch_cg_update(int ncol, int n, double *x, double *r, const double *p, const double *h,
-                      double *z, const double *alpha_pol, const CgCol *cols, double *partial,
-                      cudaStream_t st);
-// gnew = (r.z)_k, rms, convergence against cols[k].tol, beta; history
-void launch_cg_gnew(int ncol, int n, const double *dots, CgCol *cols, double *hist, int hist_stride,
-                    cudaStream_t st);
-void launch_cg_pupdate(int ncol, int n, double *p, const double *z, const CgCol *cols,
-                       cudaStream_t st);
-// FP32 vectors, FP64 scalars (inner solver of the mixed-precision path)
-void launch_cg_update_f32(int ncol, int n, float *x, float *r, const float *p, const float *h,
-                          float *z, const float *alpha_pol, const CgCol *cols, double *partial,
-                          cudaStream_t st);
-void launch_cg_pupdate_f32(int ncol, int n, float *p, const float *z, const CgCol *cols,
-                           cudaStream_t st);
 // mu[k] += scale[k] * dmu32[k]  (IR correction, FP64 accumulate)
 void launch_ir_accumulate(int ncol, int n, double *mu, const float *d32, const double *scale,
                           cudaStream_t st);
 // r = rhs - Tmu (all columns), into r; and r32 = r / scale
 void launch_residual(size_t total, const double *rhs, const double *tmu, double *r,
                      cudaStream_t st);
-// r[k] -= scale[k] * t32[k]  (refinement residual updated by the FP32
-// product of the correction instead of a recomputed product)
-void launch_residual_update(int ncol, int n, double *r, const float *t32, const double *scale,
-                            cudaStream_t st);
 // DIIS: x_new = sum_i c_i X[:, i]
 void launch_lincomb(int nvec, size_t n, const double *X, size_t ldx, const double *c, double *out,
                     cudaStream_t st);

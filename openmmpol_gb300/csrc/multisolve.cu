@@ -73,6 +73,7 @@ struct MultiSolver::Job {
   int kind = kNone, items = 0, done = 0, launches = 0;
   double round_pairs = 0.0;  // item size of the product in flight (SymSlice::round_pairs)
   bool update = false;       // the FP32 product in flight updates the residual
+  bool prepared = false;     // the CG steps cleared the FP32 product's accumulators
   std::vector<double> rms;   // residual rms of the last check, per column
   int outer = 0, inner = 0;
   double eta = 1e-5;
@@ -249,6 +250,11 @@ int MultiSolver::launch_products(std::vector<Job *> &active) {
     if (j->done > 0) continue;
     const size_t C = 3 * (size_t)j->ncol, n = j->s->d_.n;
     double *sym = j->s->sym_scratch_;
+    if (j->kind == kF32 && j->prepared) {  // cleared by the CG steps
+      j->prepared = false;
+      continue;
+    }
+    j->prepared = false;
     if (j->kind != kF32) {
       gpu::launch_tmu_sym_prepare(j->s->d_, j->ncol, j->s->x_, reinterpret_cast<unsigned long long *>(sym),
                                   reinterpret_cast<unsigned long long *>(sym + 3 * C * n), st_);
@@ -302,58 +308,48 @@ int MultiSolver::launch_products(std::vector<Job *> &active) {
   return nlaunch;
 }
 
-// The bookkeeping after a system's product (which 0: the rest of the FP32
-// inner PCG iteration; 1: the refinement residual and its rms; 2: the
-// residual updated by the FP32 product of the correction), on the engine
-// stream, launched directly.  Capturing it as a CUDA graph per system and
-// column count was measured slower in a request stream: every new system
-// paid the graph's instantiation, more than its replays saved.
-void MultiSolver::enqueue_tail(Job &j, int which) {
-  System &s = *j.s;
-  const gpu::DevSites &d = s.d_;
-  const int n = d.n, ncol = j.ncol;
-  const size_t nv = 3 * (size_t)n, C = 3 * (size_t)ncol;
-  Workspace &w = s.ws_;
-  unsigned long long *lo = reinterpret_cast<unsigned long long *>(s.sym_scratch_);
-  unsigned long long *hi = lo + C * n;
-  unsigned long long *bad = reinterpret_cast<unsigned long long *>(s.sym_scratch_ + 3 * C * n);
-  if (which == 2) {
-    // r -= rms T32 d: the FP32 product of the correction (System::update_allowed)
-    float *e = reinterpret_cast<float *>(s.sym_scratch_ + 2 * C * n);
-    gpu::launch_fixed_to_float(C * n, lo, hi, bad, e, st_);
-    gpu::launch_tmu_finish32(d, ncol, e, w.p32, w.h32, st_);
-    gpu::launch_residual_update(ncol, n, w.r, w.h32, w.dots + 2 * w.cap, st_);
-    gpu::launch_scale_by_alpha(ncol, n, d.pol_alpha, w.r, w.z, st_);
-    gpu::launch_dots(ncol, nv, w.r, w.z, w.partial, st_);
-    gpu::launch_reduce_partials(ncol, w.partial, w.dots, st_);
-    cudaMemcpyAsync(w.scal_h, w.dots, ncol * sizeof(double), cudaMemcpyDeviceToHost, st_);
-  } else if (which == 0) {
-    float *e = reinterpret_cast<float *>(s.sym_scratch_ + 2 * C * n);
-    gpu::launch_fixed_to_float(C * n, lo, hi, bad, e, st_);
-    gpu::launch_tmu_finish32(d, ncol, e, w.p32, w.h32, st_);
-    // the rest of pcg32_ws's iteration
-    gpu::launch_dots_f32(ncol, nv, w.h32, w.p32, w.partial, st_);
-    gpu::launch_reduce_partials(ncol, w.partial, w.dots, st_);
-    gpu::launch_cg_alpha(ncol, w.dots, w.cols, 1e-300, st_);
-    gpu::launch_cg_update_f32(ncol, n, w.x32, w.r32, w.p32, w.h32, w.z32, s.alpha32_, w.cols, w.partial, st_);
-    if (s.inner_precond_ >= 1 && s.blk_info_) {
-      gpu::launch_block_apply(ncol, n, s.blk_info_, s.blk_minv_, w.r32, w.z32, st_);
-      if (s.near_precond())
-        gpu::launch_near_correct(ncol, n, s.blk_info_, s.blk_minv_, s.near_ri_, s.near_ci_, s.near_blk_, w.z32, w.h32,
-                                 st_);
-      gpu::launch_dots_f32(ncol, nv, w.r32, w.z32, w.partial, st_);
+// The bookkeeping after the products that completed this round, on the engine
+// stream: one launch per step for all systems in the inner PCG (the finishing
+// pass and the CG steps take a table of systems), then the refinement
+// residual and its rms of those that ended a solve or its update.
+void MultiSolver::enqueue_tails(const std::vector<Job *> &inner, const std::vector<Job *> &residual) {
+  std::vector<gpu::F32Finish> fin;
+  std::vector<gpu::CgJob<float>> steps;
+  auto finish32 = [&](Job &j, double *part, int max_part) {
+    System &s = *j.s;
+    const size_t C = 3 * (size_t)j.ncol, n = s.d_.n;
+    gpu::F32Finish f = gpu::f32_finish(s.d_, j.ncol, s.ws_.p32, s.ws_.h32);
+    unsigned long long *lo = reinterpret_cast<unsigned long long *>(s.sym_scratch_);
+    f.lo = lo, f.hi = lo + C * n, f.bad = lo + 3 * C * n;
+    if (part) f.nblk = std::min(f.nblk, max_part);
+    f.part = part;
+    fin.push_back(f);
+    return f.nblk;
+  };
+  for (Job *j : inner) {
+    gpu::CgJob<float> job = j->s->inner_job(j->s->ws_, j->ncol, true);
+    job.na = finish32(*j, job.pa, (int)(j->s->ws_.partial_len / (2 * (size_t)j->ncol)));
+    steps.push_back(job);
+    j->prepared = true;
+  }
+  for (Job *j : residual)
+    if (j->update) finish32(*j, nullptr, 0);
+  gpu::launch_f32_finish(fin.data(), (int)fin.size(), st_);
+  gpu::launch_cg_steps(steps.data(), (int)steps.size(), st_);
+  for (Job *j : residual) {
+    System &s = *j->s;
+    Workspace &w = s.ws_;
+    const int n = s.d_.n, nb = gpu::cg_blocks(n, j->ncol, w.partial_len);
+    const size_t nv = 3 * (size_t)n, C = 3 * (size_t)j->ncol;
+    if (j->update) {
+      // r -= rms T32 d: the FP32 product of the correction (System::update_allowed)
+      gpu::launch_refine(j->ncol, nb, nv, s.rhs_, nullptr, w.h32, w.dots + 2 * w.cap, s.d_.pol_alpha, w.r, w.partial,
+                         w.scal_h, st_);
+    } else {
+      unsigned long long *lo = reinterpret_cast<unsigned long long *>(s.sym_scratch_);
+      gpu::launch_tmu_sym_finish(s.d_, j->ncol, lo, lo + C * n, lo + 3 * C * n, s.x_, true, w.h, st_);
+      gpu::launch_refine(j->ncol, nb, nv, s.rhs_, w.h, nullptr, nullptr, s.d_.pol_alpha, w.r, w.partial, w.scal_h, st_);
     }
-    gpu::launch_reduce_partials(ncol, w.partial, w.dots, st_);
-    gpu::launch_cg_gnew(ncol, n, w.dots, w.cols, nullptr, 0, st_);
-    gpu::launch_cg_pupdate_f32(ncol, n, w.p32, w.z32, w.cols, st_);
-    cudaMemcpyAsync(w.cols_h, w.cols, ncol * sizeof(gpu::CgCol), cudaMemcpyDeviceToHost, st_);
-  } else {
-    gpu::launch_tmu_sym_finish(d, ncol, lo, hi, bad, s.x_, true, w.h, st_);
-    gpu::launch_residual(ncol * nv, s.rhs_, w.h, w.r, st_);
-    gpu::launch_scale_by_alpha(ncol, n, d.pol_alpha, w.r, w.z, st_);
-    gpu::launch_dots(ncol, nv, w.r, w.z, w.partial, st_);
-    gpu::launch_reduce_partials(ncol, w.partial, w.dots, st_);
-    cudaMemcpyAsync(w.scal_h, w.dots, ncol * sizeof(double), cudaMemcpyDeviceToHost, st_);
   }
 }
 
@@ -366,6 +362,7 @@ int MultiSolver::tick() {
   if (jobs_.empty()) return 0;
   const auto wall0 = std::chrono::steady_clock::now();
   bool work = false;
+  std::vector<gpu::CgJob<float>> starts;
   // ---- steps decided in the previous round ----------------------------------
   for (Job *jp : jobs_) {
     Job &j = *jp;
@@ -383,40 +380,21 @@ int MultiSolver::tick() {
           j.items = gpu::tmu_f64_sym_items(d, ncol, j.round_pairs);
           j.done = j.launches = 0;
         } else {
-          cudaMemcpyAsync(w.r, s.rhs_, ncol * nv * sizeof(double), cudaMemcpyDeviceToDevice, st_);
-          gpu::launch_scale_by_alpha(ncol, n, d.pol_alpha, w.r, w.z, st_);
-          gpu::launch_dots(ncol, nv, w.r, w.z, w.partial, st_);
-          gpu::launch_reduce_partials(ncol, w.partial, w.dots, st_);
-          cudaMemcpyAsync(w.scal_h, w.dots, ncol * sizeof(double), cudaMemcpyDeviceToHost, st_);
+          gpu::launch_refine(ncol, gpu::cg_blocks(n, ncol, w.partial_len), nv, s.rhs_, nullptr, nullptr, nullptr,
+                             d.pol_alpha, w.r, w.partial, w.scal_h, st_);
           j.stage = kAwaitCheck;
           work = true;
         }
         break;
       case kInnerInit: {
-        // pcg32_ws's start, with the first r.z kept on the device
+        // pcg32_ws's start
         cudaMemcpyAsync(w.dots + cap, w.scal_h + cap, 2 * cap * sizeof(double), cudaMemcpyHostToDevice, st_);
         gpu::launch_to_f32_cols(ncol, nv, w.r, w.dots + cap, w.r32, st_);
-        cudaMemsetAsync(w.x32, 0, ncol * nv * sizeof(float), st_);
-        cudaMemsetAsync(w.p32, 0, ncol * nv * sizeof(float), st_);
-        cudaMemsetAsync(w.h32, 0, ncol * nv * sizeof(float), st_);
-        for (int k = 0; k < ncol; ++k) {
-          gpu::CgCol c{};
-          c.active = 1;
-          c.tol = j.eta;
-          w.cols_h[k] = c;
-        }
-        cudaMemcpyAsync(w.cols, w.cols_h, ncol * sizeof(gpu::CgCol), cudaMemcpyHostToDevice, st_);
-        gpu::launch_cg_update_f32(ncol, n, w.x32, w.r32, w.p32, w.h32, w.z32, s.alpha32_, w.cols, w.partial, st_);
-        if (s.inner_precond_ >= 1 && s.blk_info_) {
-          gpu::launch_block_apply(ncol, n, s.blk_info_, s.blk_minv_, w.r32, w.z32, st_);
-          if (s.near_precond())
-            gpu::launch_near_correct(ncol, n, s.blk_info_, s.blk_minv_, s.near_ri_, s.near_ci_, s.near_blk_, w.z32,
-                                     w.h32, st_);
-          gpu::launch_dots_f32(ncol, nv, w.r32, w.z32, w.partial, st_);
-        }
-        gpu::launch_reduce_partials(ncol, w.partial, w.dots, st_);
-        cudaMemcpyAsync(w.p32, w.z32, ncol * nv * sizeof(float), cudaMemcpyDeviceToDevice, st_);
-        gpu::launch_cg_init(ncol, w.dots, w.cols, j.eta, st_);
+        gpu::CgJob<float> job = s.inner_job(w, ncol, true);
+        job.tol = j.eta;
+        job.init = gpu::kCgInitZero;
+        starts.push_back(job);
+        j.prepared = true;
         j.stage = kProduct;
         j.kind = kF32;
         j.round_pairs = round_pairs(kF32);
@@ -466,12 +444,14 @@ int MultiSolver::tick() {
         break;
     }
   }
+  gpu::launch_cg_steps(starts.data(), (int)starts.size(), st_);
   // ---- this round's share of every product -----------------------------------
   cudaEventRecord(ev_[0], st_);
   const bool launched = launch_products(jobs_) > 0;
   if (launched) work = true;
   cudaEventRecord(ev_[1], st_);
   // ---- bookkeeping of the products that completed ----------------------------
+  std::vector<Job *> inner, residual;
   for (Job *jp : jobs_) {
     Job &j = *jp;
     if (j.stage != kProduct || j.done < j.items) continue;
@@ -483,24 +463,25 @@ int MultiSolver::tick() {
     if (j.kind == kF32 && j.update) {
       s.stats_.f32_matvecs += 1;
       s.stats_.updates += 1;
-      enqueue_tail(j, 2);
-      j.update = false;
+      residual.push_back(&j);
       j.stage = kAwaitCheck;
     } else if (j.kind == kF32) {
       s.stats_.f32_matvecs += 1;
-      enqueue_tail(j, 0);
+      inner.push_back(&j);
       j.stage = kAwaitInner;
     } else {
       if (j.kind == kDS)
         s.stats_.ds_matvecs += 1;
       else
         s.stats_.f64_matvecs += 1;
-      enqueue_tail(j, 1);
+      residual.push_back(&j);
       j.stage = kAwaitCheck;
     }
     j.kind = kNone;
     work = true;
   }
+  enqueue_tails(inner, residual);
+  for (Job *j : residual) j->update = false;
   cudaEventRecord(ev_[2], st_);
   if (work) {
     cudaError_t e = cudaStreamSynchronize(st_);

@@ -59,7 +59,7 @@ class MultiSolver {
  private:
   struct Job;
   int launch_products(std::vector<Job *> &active);
-  void enqueue_tail(Job &j, int which);
+  void enqueue_tails(const std::vector<Job *> &inner, const std::vector<Job *> &residual);
   double round_pairs(int kind);  // pairs of one round's budget for a product kind
   void fail(Job &j, int status, const std::string &err);
 

@@ -63,7 +63,8 @@ int System::ensure_batch_ws(int ncol, int nf) {
   bad |= walloc(w.x32, ncol * nv) | walloc(w.r32, ncol * nv) | walloc(w.p32, ncol * nv) |
          walloc(w.h32, ncol * nv) | walloc(w.z32, ncol * nv);
   bad |= walloc(w.scratch32, (size_t)s0 * ncol * nv);
-  bad |= walloc(w.partial, (size_t)gpu::kRedBlocks * std::max(ncol, nf)) |
+  w.partial_len = (size_t)gpu::kRedBlocks * std::max(ncol, nf);
+  bad |= walloc(w.partial, w.partial_len) |
          walloc(w.dots, 3 * (size_t)ncol + nf) | walloc(w.cols, ncol);
   // block CG buffers (sized for the widest block)
   const int smax = gpu::block_cg_max_columns();
@@ -117,33 +118,45 @@ int System::cg64_ws(Workspace &w, int matv, int ncol, const double *rhs, double 
     if (st) return st;
     gpu::launch_residual(ncol * nv, rhs, w.z, w.r, st_);
   }
-  gpu::launch_scale_by_alpha(ncol, n, d_.pol_alpha, w.r, w.z, st_);
-  cudaMemcpyAsync(w.p, w.z, ncol * nv * sizeof(double), cudaMemcpyDeviceToDevice, st_);
-  gpu::launch_dots(ncol, nv, w.r, w.z, w.partial, st_);
-  gpu::launch_reduce_partials(ncol, w.partial, w.dots, st_);
-  cudaMemcpyAsync(w.scal_h, w.dots, ncol * sizeof(double), cudaMemcpyDeviceToHost, st_);
-  st = check(cudaStreamSynchronize(st_), "CG init");
-  if (st) return st;
-  for (int k = 0; k < ncol; ++k) {
-    gpu::CgCol c{};
-    c.gold = w.scal_h[k];
-    c.tol = tol_;
-    c.active = 1;
-    w.cols_h[k] = c;
-  }
-  cudaMemcpyAsync(w.cols, w.cols_h, ncol * sizeof(gpu::CgCol), cudaMemcpyHostToDevice, st_);
+  // z = alpha r, p = z, the first r.z
+  const size_t share = w.partial_len / (2 * (size_t)ncol);
   double *hist = (set0 >= 0) ? w.hist : nullptr;
+  gpu::CgJob<double> job{};
+  job.n = n, job.ncol = ncol;
+  job.nb = gpu::cg_blocks(n, ncol, w.partial_len);
+  job.eps = kEpsRp, job.tol = tol_;
+  job.x = x, job.r = w.r, job.p = w.p, job.h = w.h, job.alpha = d_.pol_alpha;
+  job.pa = w.partial, job.pb = w.partial + share * ncol;
+  job.cols = w.cols, job.cols_h = w.cols_h;
+  job.hist = hist, job.nhist = maxhist_;
+  // the direct symmetric product of one column group: its accumulators and
+  // scale are prepared by the steps, its finishing pass sums p.h
+  const bool sym = direct_symmetric(matv, ncol);
+  const size_t C = 3 * (size_t)ncol;
+  unsigned long long *lo = reinterpret_cast<unsigned long long *>(sym_scratch_);
+  if (sym) job.acc = lo, job.nacc = 2 * C * n, job.words = lo + 3 * C * n;
+  const bool small = !sym && n <= gpu::kCgSmallSites;
+  job.init = gpu::kCgInitKeep;
+  gpu::launch_cg_steps(&job, 1, st_);
+  job.init = 0;
   for (int it = 1; it <= maxiter_; ++it) {
-    st = matvec64(matv, ncol, w.p, w.h, true);
-    if (st) return st;
-    gpu::launch_dots(ncol, nv, w.h, w.p, w.partial, st_);
-    gpu::launch_reduce_partials(ncol, w.partial, w.dots, st_);
-    gpu::launch_cg_alpha(ncol, w.dots, w.cols, kEpsRp, st_);
-    gpu::launch_cg_update(ncol, n, x, w.r, w.p, w.h, w.z, d_.pol_alpha, w.cols, w.partial, st_);
-    gpu::launch_reduce_partials(ncol, w.partial, w.dots, st_);
-    gpu::launch_cg_gnew(ncol, n, w.dots, w.cols, hist, maxhist_, st_);
-    gpu::launch_cg_pupdate(ncol, n, w.p, w.z, w.cols, st_);
-    cudaMemcpyAsync(w.cols_h, w.cols, ncol * sizeof(gpu::CgCol), cudaMemcpyDeviceToHost, st_);
+    if (sym) {
+      KEv e;
+      if (ktime_on_) e = kt_begin(0, ncol);
+      gpu::SymSlice one{&d_, w.p, lo, lo + C * n, job.words, 0, gpu::tmu_f64_sym_items(d_, ncol)};
+      gpu::launch_tmu_f64_sym_multi(ncol, d_.amoeba, &one, 1, reinterpret_cast<unsigned *>(job.words + 2), st_, true);
+      gpu::launch_tmu_sym_finish(d_, ncol, lo, lo + C * n, job.words, w.p, true, w.h, st_, job.pa, (int)share, &job.na);
+      if (ktime_on_) kt_end(e);
+      stats_.f64_matvecs += 1;
+    } else {
+      st = matvec64(matv, ncol, w.p, w.h, true);
+      if (st) return st;
+      if (!small) gpu::launch_cg_dot(ncol, job.na = job.nb, nv, w.h, w.p, job.pa, st_);
+    }
+    if (small)
+      gpu::launch_cg_small(job, st_);
+    else
+      gpu::launch_cg_steps(&job, 1, st_);
     st = check(cudaStreamSynchronize(st_), "CG iteration");
     if (st) return st;
     bool any = false;
@@ -182,8 +195,9 @@ int System::cg64_ws(Workspace &w, int matv, int ncol, const double *rhs, double 
 // ---------------------------------------------------------------------------
 // FP32 product with the tuned launch shape
 // ---------------------------------------------------------------------------
-void System::f32_product(Workspace &w, int ncol, const F32Shape &sh) {
-  gpu::launch_tmu_f32(d_, ncol, w.p32, w.h32, w.scratch32, sh.nsplit, st_, sh.g, sh.kver, sym_scratch_);
+int System::f32_product(Workspace &w, int ncol, const F32Shape &sh, bool prepared, double *part, int max_part) {
+  return gpu::launch_tmu_f32(d_, ncol, w.p32, w.h32, w.scratch32, sh.nsplit, st_, sh.g, sh.kver, sym_scratch_, prepared,
+                             part, max_part);
 }
 
 int System::tune_f32(Workspace &w, int ncol, F32Shape &shape) {
@@ -247,68 +261,55 @@ int System::tune_f32(Workspace &w, int ncol, F32Shape &shape) {
   return kOk;
 }
 
+// the CG steps on the FP32 columns of a workspace; prepared: they also clear
+// the accumulators of the symmetric product
+gpu::CgJob<float> System::inner_job(Workspace &w, int ncol, bool prepared) {
+  gpu::CgJob<float> job{};
+  job.n = d_.n, job.ncol = ncol;
+  // z = M^-1 r: the diagonal, the block-Jacobi blocks, or those with the
+  // Neumann step over the near blocks
+  job.mode = inner_precond_ >= 1 && blk_info_ ? (near_precond() ? 2 : 1) : 0;
+  job.nb = gpu::cg_blocks(d_.n, ncol, w.partial_len);
+  job.eps = 1e-300;
+  job.x = w.x32, job.r = w.r32, job.p = w.p32, job.h = w.h32, job.z = w.z32;
+  job.w = reinterpret_cast<float *>(w.z);  // free during the inner solve
+  job.alpha = alpha32_;
+  job.info = blk_info_, job.minv = blk_minv_;
+  job.ri = near_ri_, job.ci = near_ci_, job.blk = near_blk_;
+  job.pa = w.partial, job.pb = w.partial + w.partial_len / (2 * (size_t)ncol) * ncol;
+  job.cols = w.cols, job.cols_h = w.cols_h;
+  if (prepared) {
+    unsigned long long *lo = reinterpret_cast<unsigned long long *>(sym_scratch_);
+    job.acc = lo, job.nacc = 2 * 3 * (size_t)ncol * d_.n, job.words = lo + 3 * 3 * (size_t)ncol * d_.n;
+  }
+  return job;
+}
+
 // ---------------------------------------------------------------------------
 // FP32 inner PCG on w.r32 (columns normalised to unit rms); result in w.x32
 // ---------------------------------------------------------------------------
 int System::pcg32_ws(Workspace &w, int ncol, int max_it, double eta) {
   const int n = d_.n;
-  const size_t nv = 3 * (size_t)n;
   F32Shape shape{1, 1, 2};
   int st = tune_f32(w, ncol, shape);
   if (st) return st;
-  // x = 0; p = h = 0 so that an update step with alpha = 0 only forms
-  // z = alpha_pol r and the partial r.z
-  cudaMemsetAsync(w.x32, 0, ncol * nv * sizeof(float), st_);
-  cudaMemsetAsync(w.p32, 0, ncol * nv * sizeof(float), st_);
-  cudaMemsetAsync(w.h32, 0, ncol * nv * sizeof(float), st_);
-  for (int k = 0; k < ncol; ++k) {
-    gpu::CgCol c{};
-    c.active = 1;
-    c.tol = eta;
-    w.cols_h[k] = c;
-  }
-  cudaMemcpyAsync(w.cols, w.cols_h, ncol * sizeof(gpu::CgCol), cudaMemcpyHostToDevice, st_);
-  // z = M^-1 r: the diagonal (fused in the update) or the block-Jacobi blocks
-  const bool blocks = inner_precond_ >= 1 && blk_info_;
-  const bool near = blocks && near_precond();
-  auto precondition = [&]() {
-    if (!blocks) return;
-    gpu::launch_block_apply(ncol, n, blk_info_, blk_minv_, w.r32, w.z32, st_);
-    // h32 (T p) is spent by the update above: scratch of the Neumann step
-    if (near) gpu::launch_near_correct(ncol, n, blk_info_, blk_minv_, near_ri_, near_ci_, near_blk_, w.z32, w.h32, st_);
-    gpu::launch_dots_f32(ncol, nv, w.r32, w.z32, w.partial, st_);
-  };
-  gpu::launch_cg_update_f32(ncol, n, w.x32, w.r32, w.p32, w.h32, w.z32, alpha32_, w.cols, w.partial, st_);
-  precondition();
-  gpu::launch_reduce_partials(ncol, w.partial, w.dots, st_);
-  cudaMemcpyAsync(w.p32, w.z32, ncol * nv * sizeof(float), cudaMemcpyDeviceToDevice, st_);
-  cudaMemcpyAsync(w.scal_h, w.dots, ncol * sizeof(double), cudaMemcpyDeviceToHost, st_);
-  st = check(cudaStreamSynchronize(st_), "inner CG init");
-  if (st) return st;
-  for (int k = 0; k < ncol; ++k) {
-    gpu::CgCol c{};
-    c.gold = w.scal_h[k];
-    c.tol = eta;
-    c.active = w.scal_h[k] > 0.0 ? 1 : 0;
-    w.cols_h[k] = c;
-  }
-  cudaMemcpyAsync(w.cols, w.cols_h, ncol * sizeof(gpu::CgCol), cudaMemcpyHostToDevice, st_);
+  // the symmetric product of one column group: its accumulators are cleared
+  // by the steps
+  const bool prepared = shape.kver == 3 && (ncol == 1 || (ncol == 2 && shape.g >= 2));
+  gpu::CgJob<float> job = inner_job(w, ncol, prepared);
+  const int share = (int)(w.partial_len / (2 * (size_t)ncol));
+  job.tol = eta;
+  job.init = gpu::kCgInitZero;
+  gpu::launch_cg_steps(&job, 1, st_);
+  job.init = 0;
   auto iteration = [&]() {
-    f32_product(w, ncol, shape);
-    gpu::launch_dots_f32(ncol, nv, w.h32, w.p32, w.partial, st_);
-    gpu::launch_reduce_partials(ncol, w.partial, w.dots, st_);
-    gpu::launch_cg_alpha(ncol, w.dots, w.cols, 1e-300, st_);
-    gpu::launch_cg_update_f32(ncol, n, w.x32, w.r32, w.p32, w.h32, w.z32, alpha32_, w.cols, w.partial, st_);
-    precondition();
-    gpu::launch_reduce_partials(ncol, w.partial, w.dots, st_);
-    gpu::launch_cg_gnew(ncol, n, w.dots, w.cols, nullptr, 0, st_);
-    gpu::launch_cg_pupdate_f32(ncol, n, w.p32, w.z32, w.cols, st_);
-    cudaMemcpyAsync(w.cols_h, w.cols, ncol * sizeof(gpu::CgCol), cudaMemcpyDeviceToHost, st_);
+    job.na = f32_product(w, ncol, shape, prepared, job.pa, share);
+    gpu::launch_cg_steps(&job, 1, st_);
   };
   // capture one iteration as a graph (kernel arguments and buffers are fixed
   // per workspace, width and launch shape; the tolerance lives in w.cols)
   if (use_graphs_ && (w.graph_ncol != ncol || w.graph_gmax != shape.g || w.graph_nsplit != shape.nsplit ||
-                     w.graph_kver != shape.kver || w.graph_prec != (near ? 2 : blocks ? 1 : 0))) {
+                     w.graph_kver != shape.kver || w.graph_prec != job.mode)) {
     if (w.graph) cudaGraphExecDestroy(w.graph);
     w.graph = nullptr;
     w.graph_ncol = -1;
@@ -324,7 +325,7 @@ int System::pcg32_ws(Workspace &w, int ncol, int max_it, double eta) {
         w.graph_gmax = shape.g;
         w.graph_nsplit = shape.nsplit;
         w.graph_kver = shape.kver;
-        w.graph_prec = near ? 2 : blocks ? 1 : 0;
+        w.graph_prec = job.mode;
         w.graph_kernels = kernels;
       } else {
         w.graph = nullptr;
@@ -386,24 +387,21 @@ int System::mixed_ir_ws(Workspace &w, int ncol, const double *rhs, double *x, in
     const int pst = ensure_near();
     if (pst) return pst;
   }
+  const int nb = gpu::cg_blocks(n, ncol, w.partial_len);
   if (have_guess) {
     int st0 = matvec_residual(ncol, x, w.h);
     if (st0) return st0;
-    gpu::launch_residual(ncol * nv, rhs, w.h, w.r, st_);
   } else {
     cudaMemsetAsync(x, 0, ncol * nv * sizeof(double), st_);
-    cudaMemcpyAsync(w.r, rhs, ncol * nv * sizeof(double), cudaMemcpyDeviceToDevice, st_);
   }
+  gpu::launch_refine(ncol, nb, nv, rhs, have_guess ? w.h : nullptr, nullptr, nullptr, d_.pol_alpha, w.r, w.partial,
+                     w.scal_h, st_);
   if (set0 >= 0)
     for (int k = 0; k < ncol && set0 + k < 2; ++k) stats_.hist[set0 + k].clear();
   std::vector<double> rms(ncol);
   int outer = 0;
   bool done = false;
   while (true) {
-    gpu::launch_scale_by_alpha(ncol, n, d_.pol_alpha, w.r, w.z, st_);
-    gpu::launch_dots(ncol, nv, w.r, w.z, w.partial, st_);
-    gpu::launch_reduce_partials(ncol, w.partial, w.dots, st_);
-    cudaMemcpyAsync(w.scal_h, w.dots, ncol * sizeof(double), cudaMemcpyDeviceToHost, st_);
     int st = check(cudaStreamSynchronize(st_), "refinement residual");
     if (st) return st;
     done = true;
@@ -445,11 +443,12 @@ int System::mixed_ir_ws(Workspace &w, int ncol, const double *rhs, double *x, in
       f32_product(w, ncol, shape);
       stats_.f32_matvecs += 1;
       stats_.updates += 1;
-      gpu::launch_residual_update(ncol, n, w.r, w.h32, w.dots + 2 * cap, st_);
+      gpu::launch_refine(ncol, nb, nv, rhs, nullptr, w.h32, w.dots + 2 * cap, d_.pol_alpha, w.r, w.partial, w.scal_h,
+                         st_);
     } else {
       st = matvec_residual(ncol, x, w.h);
       if (st) return st;
-      gpu::launch_residual(ncol * nv, rhs, w.h, w.r, st_);
+      gpu::launch_refine(ncol, nb, nv, rhs, w.h, nullptr, nullptr, d_.pol_alpha, w.r, w.partial, w.scal_h, st_);
     }
     ++outer;
   }

@@ -627,15 +627,6 @@ __global__ void __launch_bounds__(S32_TPB, G == 1 ? 4 : 3) k_tmu32_sym(const __g
   }
 }
 
-// fixed-point sums -> float (NaN when an accumulator overflowed)
-__global__ void k_fixed_to_float(size_t total, const unsigned long long *__restrict__ lo,
-                                 const unsigned long long *__restrict__ hi, const unsigned long long *bad,
-                                 float *__restrict__ out) {
-  const bool nan = *bad != 0ull;
-  for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += (size_t)gridDim.x * blockDim.x)
-    out[k] = nan ? __int_as_float(0x7fc00000) : (float)fixed_value(lo[k], hi[k]);
-}
-
 template <int G>
 struct S32Launch {
   int resident = 0;
@@ -668,12 +659,12 @@ void s32_schedule(int n, int g, double round_pairs, int &ntile, int &K, int &chu
 }
 
 template <int G>
-void launch_s32_table(const S32Table &tab, unsigned *next, cudaStream_t st) {
+void launch_s32_table(const S32Table &tab, unsigned *next, cudaStream_t st, bool zeroed) {
   const int total = tab.base[tab.njobs];
   if (total <= 0) return;
   const int ctas_max = s32_resident<G>() * sm_count();
   const int ctas = ctas_max < total ? ctas_max : total;
-  cudaMemsetAsync(next, 0, sizeof(unsigned), st);
+  if (!zeroed) cudaMemsetAsync(next, 0, sizeof(unsigned), st);
   k_tmu32_sym<G><<<ctas, S32_TPB, sizeof(S32Smem<G>), st>>>(tab, next);
 }
 
@@ -704,7 +695,7 @@ int tmu32_sym_items(const DevSites &s, int g, double round_pairs) {
   return ntile * nchunk;
 }
 
-void launch_tmu32_sym_multi(int g, const SymSlice *sl, int nsl, unsigned *next, cudaStream_t st) {
+void launch_tmu32_sym_multi(int g, const SymSlice *sl, int nsl, unsigned *next, cudaStream_t st, bool zeroed) {
   S32Table tab{};
   int total = 0;
   for (int k = 0; k < nsl && tab.njobs < kMaxSymSlices; ++k) {
@@ -719,27 +710,9 @@ void launch_tmu32_sym_multi(int g, const SymSlice *sl, int nsl, unsigned *next, 
   if (!total) return;
   add_launch_count(1);
   if (g == 2)
-    launch_s32_table<2>(tab, next, st);
+    launch_s32_table<2>(tab, next, st, zeroed);
   else
-    launch_s32_table<1>(tab, next, st);
-}
-
-void launch_fixed_to_float(size_t total, const unsigned long long *lo, const unsigned long long *hi,
-                           const unsigned long long *bad, float *out, cudaStream_t st) {
-  add_launch_count(1);
-  int blocks = (int)((total + 255) / 256);
-  if (blocks > 4 * 152 * 4) blocks = 4 * 152 * 4;
-  k_fixed_to_float<<<blocks < 1 ? 1 : blocks, 256, 0, st>>>(total, lo, hi, bad, out);
-}
-
-void launch_tmu32_sym_pairs(const DevSites &s, int g, const float *x, unsigned long long *lo, unsigned long long *hi,
-                            unsigned long long *bad, unsigned *next, float *out, cudaStream_t st) {
-  const size_t C = 3 * (size_t)g;
-  cudaMemsetAsync(lo, 0, 2 * C * s.n * sizeof(unsigned long long), st);
-  cudaMemsetAsync(bad, 0, sizeof(unsigned long long), st);
-  SymSlice one{&s, x, lo, hi, bad, 0, tmu32_sym_items(s, g)};
-  launch_tmu32_sym_multi(g, &one, 1, next, st);
-  launch_fixed_to_float(C * s.n, lo, hi, bad, out, st);
+    launch_s32_table<1>(tab, next, st, zeroed);
 }
 
 // one column group through the v2 pair kernel (g = 1, 2, 4 or 8)

@@ -358,45 +358,71 @@ __global__ void __launch_bounds__(256) k_sym_prepare(size_t total, const double 
 }
 
 // y = -(pair sums + scaled-pair corrections) (+ x / alpha): the fixed-point
-// sums read out (NaN when flagged) and scaled back
-template <bool AMOEBA>
-__global__ void __launch_bounds__(128) k_tmu_sym_finish(
+// sums read out (NaN when flagged) and scaled back; with part, the partial
+// sums of x.y of every block.  L lanes per site share its scaled pairs: four
+// below kFinishLanesSites (one thread per site left 5,001 sites on 40 CTAs,
+// bound by the latency of its pair list), one above.
+constexpr int FIN_TPB = 256;
+template <bool AMOEBA, int L>
+__global__ void __launch_bounds__(FIN_TPB) k_tmu_sym_finish(
     int n, const unsigned long long *__restrict__ lo, const unsigned long long *__restrict__ hi,
     const unsigned long long *__restrict__ bad, const Pos64 *__restrict__ pos, const double *__restrict__ damp,
-    const float2 *__restrict__ wa, const double *__restrict__ x, const double *__restrict__ alpha, bool dodiag,
+    const float2 *__restrict__ wa, const double *__restrict__ x, const double *__restrict__ ialpha, bool dodiag,
     const int *__restrict__ ri, const int *__restrict__ src, const double *__restrict__ scale, double thr, float thr2m,
-    double *__restrict__ y) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= n) return;
-  const size_t col = (size_t)blockIdx.y * n, o = (col + j) * 3;
+    double *__restrict__ y, double *__restrict__ part) {
+  __shared__ double s_dot[FIN_TPB / 32];
+  const size_t col = (size_t)blockIdx.y * n;
   const bool nan = *bad != 0ull;
   const int ex = dsp_exponent(*reinterpret_cast<const unsigned *>(bad + 1));
-  double e[3];
+  const int lane = threadIdx.x % L;
+  double dot = 0.0;
+  for (int j = (blockIdx.x * FIN_TPB + threadIdx.x) / L; j < n; j += gridDim.x * (FIN_TPB / L)) {
+    double e[3] = {0.0, 0.0, 0.0};
+    if (ri) {
+      const Pos64 pt = pos[j];
+      const double at = AMOEBA ? damp[j] : 0.0;
+      const float2 wat = wa[j];
+      for (int k = ri[j] + lane; k < ri[j + 1]; k += L) {
+        const int i = src[k];
+        const Pos64 ps = pos[i];
+        const double dx = pt.x - ps.x, dy = pt.y - ps.y, dz = pt.z - ps.z;
+        const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+        double k3, k5;
+        dd_pair_f64<AMOEBA, true>(r2, pt.w, ps.w, at, AMOEBA ? damp[i] : 0.0, wat, wa[i], thr, thr2m, k3, k5);
+        const double *mu = &x[(col + i) * 3];
+        const double f = 3.0 * k5 * fma(mu[0], dx, fma(mu[1], dy, mu[2] * dz));
+        const double cs = scale[k] - 1.0;
+        e[0] = fma(cs, fma(f, dx, -(k3 * mu[0])), e[0]);
+        e[1] = fma(cs, fma(f, dy, -(k3 * mu[1])), e[1]);
+        e[2] = fma(cs, fma(f, dz, -(k3 * mu[2])), e[2]);
+      }
+      if (L > 1) {
+        const unsigned group = ((1u << L) - 1u) << ((threadIdx.x & 31) / L * L);
 #pragma unroll
-  for (int c = 0; c < 3; ++c)
-    e[c] = nan ? __longlong_as_double(0x7ff8000000000000ll) : scale_up(fixed_value(lo[o + c], hi[o + c]), ex);
-  if (ri) {
-    const Pos64 pt = pos[j];
-    const double at = AMOEBA ? damp[j] : 0.0;
-    const float2 wat = wa[j];
-    for (int k = ri[j]; k < ri[j + 1]; ++k) {
-      const int i = src[k];
-      const Pos64 ps = pos[i];
-      const double dx = pt.x - ps.x, dy = pt.y - ps.y, dz = pt.z - ps.z;
-      const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-      double k3, k5;
-      dd_pair_f64<AMOEBA, true>(r2, pt.w, ps.w, at, AMOEBA ? damp[i] : 0.0, wat, wa[i], thr, thr2m, k3, k5);
-      const double *mu = &x[(col + i) * 3];
-      const double f = 3.0 * k5 * fma(mu[0], dx, fma(mu[1], dy, mu[2] * dz));
-      const double cs = scale[k] - 1.0;
-      e[0] = fma(cs, fma(f, dx, -(k3 * mu[0])), e[0]);
-      e[1] = fma(cs, fma(f, dy, -(k3 * mu[1])), e[1]);
-      e[2] = fma(cs, fma(f, dz, -(k3 * mu[2])), e[2]);
+        for (int c = 0; c < 3; ++c)
+          for (int o = L / 2; o > 0; o >>= 1) e[c] += __shfl_xor_sync(group, e[c], o);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      if (L > 1 && lane != c) continue;
+      const size_t o = (col + j) * 3 + c;
+      const double v =
+          e[c] + (nan ? __longlong_as_double(0x7ff8000000000000ll) : scale_up(fixed_value(lo[o], hi[o]), ex));
+      const double yv = dodiag ? fma(x[o], ialpha[j], -v) : -v;
+      y[o] = yv;
+      dot = fma(x[o], yv, dot);
     }
   }
-  const double ia = dodiag ? 1.0 / alpha[j] : 0.0;
-#pragma unroll
-  for (int c = 0; c < 3; ++c) y[o + c] = dodiag ? fma(x[o + c], ia, -e[c]) : -e[c];
+  if (!part) return;
+  for (int o = 16; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+  if ((threadIdx.x & 31) == 0) s_dot[threadIdx.x >> 5] = dot;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    dot = 0.0;
+    for (int w = 0; w < FIN_TPB / 32; ++w) dot += s_dot[w];
+    part[(size_t)blockIdx.y * gridDim.x + blockIdx.x] = dot;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -500,10 +526,10 @@ SymPlan sym_plan(int n, int ctas, double round_pairs) {
 }
 
 template <int G, bool AMOEBA>
-void launch_table(const SymTable &tab, unsigned *next, cudaStream_t st) {
+void launch_table(const SymTable &tab, unsigned *next, cudaStream_t st, bool zeroed) {
   const int total = tab.base[tab.njobs];
   const int ctas = std::min(sym_resident<G, AMOEBA>() * sm_count(), total);
-  cudaMemsetAsync(next, 0, sizeof(unsigned), st);
+  if (!zeroed) cudaMemsetAsync(next, 0, sizeof(unsigned), st);
   k_tmu_sym<G, AMOEBA><<<ctas, SYM_TILE, sizeof(SymSmem<G>), st>>>(tab, next);
 }
 
@@ -528,7 +554,8 @@ int tmu_f64_sym_items(const DevSites &s, int g, double round_pairs) {
   return sym_plan(s.n, sym_ctas(g, s.amoeba), round_pairs).items();
 }
 
-void launch_tmu_f64_sym_multi(int g, bool amoeba, const SymSlice *sl, int nsl, unsigned *next, cudaStream_t st) {
+void launch_tmu_f64_sym_multi(int g, bool amoeba, const SymSlice *sl, int nsl, unsigned *next, cudaStream_t st,
+                              bool zeroed) {
   SymTable tab{};
   int total = 0;
   for (int k = 0; k < nsl && tab.njobs < kMaxSymSlices; ++k) {
@@ -553,9 +580,9 @@ void launch_tmu_f64_sym_multi(int g, bool amoeba, const SymSlice *sl, int nsl, u
   if (!total) return;
   add_launch_count(1);
   if (g == 2)
-    amoeba ? launch_table<2, true>(tab, next, st) : launch_table<2, false>(tab, next, st);
+    amoeba ? launch_table<2, true>(tab, next, st, zeroed) : launch_table<2, false>(tab, next, st, zeroed);
   else
-    amoeba ? launch_table<1, true>(tab, next, st) : launch_table<1, false>(tab, next, st);
+    amoeba ? launch_table<1, true>(tab, next, st, zeroed) : launch_table<1, false>(tab, next, st, zeroed);
 }
 
 void launch_tmu_sym_prepare(const DevSites &s, int g, const double *x, unsigned long long *lo, unsigned long long *bad,
@@ -575,16 +602,23 @@ void launch_max_word(size_t total, const double *x, unsigned *word, cudaStream_t
 }
 
 void launch_tmu_sym_finish(const DevSites &s, int g, const unsigned long long *lo, const unsigned long long *hi,
-                           const unsigned long long *bad, const double *x, bool dodiag, double *y, cudaStream_t st) {
+                           const unsigned long long *bad, const double *x, bool dodiag, double *y, cudaStream_t st,
+                           double *part, int max_part, int *npart) {
   add_launch_count(1);
-  const dim3 grid((s.n + 127) / 128, g);
+  const int lanes = s.n < kFinishLanesSites ? 4 : 1;
+  int blocks = (int)(((size_t)s.n * lanes + FIN_TPB - 1) / FIN_TPB);
+  if (part) blocks = std::min(blocks, max_part);
+  if (npart) *npart = blocks;
+  const dim3 grid(blocks, g);
   const int *ri = s.d2d_nnz ? s.d2d_ri : nullptr;
-  if (s.amoeba)
-    k_tmu_sym_finish<true><<<grid, 128, 0, st>>>(s.n, lo, hi, bad, s.pol_pos, s.pol_a, s.pol_wa32, x, s.pol_alpha,
-                                                 dodiag, ri, s.d2d_src, s.d2d_s, s.damp_thr, thr2_margin(s), y);
+  auto go = [&](auto kernel) {
+    kernel<<<grid, FIN_TPB, 0, st>>>(s.n, lo, hi, bad, s.pol_pos, s.pol_a, s.pol_wa32, x, s.pol_ialpha, dodiag, ri,
+                                     s.d2d_src, s.d2d_s, s.damp_thr, thr2_margin(s), y, part);
+  };
+  if (lanes == 4)
+    s.amoeba ? go(k_tmu_sym_finish<true, 4>) : go(k_tmu_sym_finish<false, 4>);
   else
-    k_tmu_sym_finish<false><<<grid, 128, 0, st>>>(s.n, lo, hi, bad, s.pol_pos, s.pol_a, s.pol_wa32, x, s.pol_alpha,
-                                                  dodiag, ri, s.d2d_src, s.d2d_s, s.damp_thr, thr2_margin(s), y);
+    s.amoeba ? go(k_tmu_sym_finish<true, 1>) : go(k_tmu_sym_finish<false, 1>);
 }
 
 size_t tmu_sym_scratch_doubles(const DevSites &s, int nrhs) {
