@@ -681,10 +681,31 @@ void System::direct_product(int ncol, const double *x, double *y, bool dodiag, i
     sym = false;  // not enough memory for the accumulators: all-ordered-pairs kernel
     log_msg(kVerbHigh, nullptr, "symmetric T.mu scratch does not fit: using the all-ordered-pairs kernel");
   }
-  if (sym)
+  const size_t groups = sym ? gpu::tmu_sym_groups(d_, ncol) : 0;
+  if (groups > 1 && group_scratch(groups * gpu::tmu_sym_scratch_doubles(d_, 2)))
+    gpu::launch_tmu_f64_sym_groups(d_, ncol, x, y, dodiag, wsb_.sym, st_);
+  else if (sym)
     gpu::launch_tmu_f64_sym(d_, ncol, x, y, dodiag, sym_scratch_, st_);
   else
     gpu::launch_tmu_f64(d_, ncol, x, y, dodiag, st_);
+}
+
+// accumulators for the column groups of one launch, kept with the batch
+// workspace
+bool System::group_scratch(size_t doubles) {
+  if (wsb_.sym_len >= doubles) return true;
+  if (wsb_.sym) {
+    cudaStreamSynchronize(st_);
+    cudaFree(wsb_.sym);
+  }
+  wsb_.sym = nullptr, wsb_.sym_len = 0;
+  if (cudaMalloc((void **)&wsb_.sym, doubles * sizeof(double)) != cudaSuccess) {
+    cudaGetLastError();
+    wsb_.sym = nullptr;
+    return false;
+  }
+  wsb_.sym_len = doubles;
+  return true;
 }
 
 // matvec64 would take the symmetric direct product in one column group

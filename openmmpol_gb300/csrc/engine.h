@@ -45,6 +45,9 @@ struct Workspace {
   float *bcoef = nullptr;
   int *bidx = nullptr;
   double *bscal_h = nullptr;
+  // accumulators of the symmetric product for several column groups (grown on use)
+  double *sym = nullptr;
+  size_t sym_len = 0;
   gpu::CgCol *cols = nullptr;
   gpu::CgCol *cols_h = nullptr;  // pinned
   double *scal_h = nullptr;      // pinned 3 x cap (+ fcap)
@@ -237,6 +240,7 @@ class System {
                   int max_part = 0);
   gpu::CgJob<float> inner_job(Workspace &w, int ncol, bool prepared);
   bool direct_symmetric(int matv, int ncol);
+  bool group_scratch(size_t doubles);
   int ensure_batch_ws(int ncol, int nf);
   void free_ws(Workspace &w);
   int check(cudaError_t e, const char *what);

@@ -20,6 +20,7 @@
 #include <cmath>
 #include <cstdio>
 #include <type_traits>
+#include <vector>
 
 #include "kernels.h"
 #include "pair_math.cuh"
@@ -625,12 +626,14 @@ static void tmu_dispatch(const DevSites &s, int nrhs, const float *x, float *par
     int g = column_group(nrhs - done, gmax);
     size_t xo = (size_t)done * s.n * 3;
     float *pg = partial + (size_t)nsplit * done * s.n * 3;
-    done += g;
     if (kver == 2) {
+      const int groups = (nrhs - done) / g;
       add_launch_count(1);
-      launch_tmu32_pairs(s, g, x + xo, pg, nsplit, st);
+      launch_tmu32_pairs(s, g, groups, x + xo, pg, nsplit, st);
+      done += g * groups;
       continue;
     }
+    done += g;
     switch (g) {
       case 8: tmu_allpairs<8>(s, x + xo, pg, nsplit, st); break;
       case 4: tmu_allpairs<4>(s, x + xo, pg, nsplit, st); break;
@@ -660,6 +663,7 @@ int launch_tmu_f32(const DevSites &s, int nrhs, const float *x, float *y, float 
   const bool sym = kver == 3 && sym_scratch;
   if (!sym) tmu_dispatch(s, nrhs, x, scratch, nsplit, gmax, st, kver);
   int npart = 0;
+  std::vector<F32Finish> fins;
   for (int c = 0; c < nrhs;) {
     const int g = column_group(nrhs - c, sym ? std::min(gmax, 2) : gmax);
     F32Finish fin = f32_finish(s, g, x + c * nv, y + c * nv);
@@ -684,9 +688,13 @@ int launch_tmu_f32(const DevSites &s, int nrhs, const float *x, float *y, float 
       npart = fin.nblk = std::min(fin.nblk, max_part);
       fin.part = part + (size_t)c * npart;
     }
-    launch_f32_finish(&fin, 1, st);
+    if (sym)
+      launch_f32_finish(&fin, 1, st);
+    else
+      fins.push_back(fin);
     c += g;
   }
+  launch_f32_finish(fins.data(), (int)fins.size(), st);
   return npart;
 }
 

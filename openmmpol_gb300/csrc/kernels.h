@@ -97,6 +97,12 @@ constexpr float kSymNear2 = 36.f, kSymNear2Wang = 64.f;
 size_t tmu_sym_scratch_doubles(const DevSites &s, int nrhs);
 void launch_tmu_f64_sym(const DevSites &s, int nrhs, const double *x, double *y, bool dodiag, double *scratch,
                         cudaStream_t st);
+// the same for many columns: as many pairs of columns per launch as fill the
+// GPU (tmu_sym_groups; one for large systems), scratch of
+// tmu_sym_groups(s, nrhs) * tmu_sym_scratch_doubles(s, 2)
+int tmu_sym_groups(const DevSites &s, int nrhs);
+void launch_tmu_f64_sym_groups(const DevSites &s, int nrhs, const double *x, double *y, bool dodiag, double *scratch,
+                               cudaStream_t st);
 // its passes for callers that spread a product over launches: accumulators
 // [g][n][3] (lo, then hi) and the two words from bad zeroed and the scale of x
 // found (before the first share), and the sums read out into y = T x, with
@@ -105,7 +111,7 @@ void launch_tmu_sym_prepare(const DevSites &s, int g, const double *x, unsigned 
                             unsigned long long *bad, cudaStream_t st);
 void launch_tmu_sym_finish(const DevSites &s, int g, const unsigned long long *lo, const unsigned long long *hi,
                            const unsigned long long *bad, const double *x, bool dodiag, double *y, cudaStream_t st,
-                           double *part = nullptr, int max_part = 0, int *npart = nullptr);
+                           double *part = nullptr, int max_part = 0, int *npart = nullptr, size_t group_words = 0);
 // the largest high word of |x| (the scale of the double-single products)
 void launch_max_word(size_t total, const double *x, unsigned *word, cudaStream_t st);
 // near field of the FMM (fmm_near.cu): the dipoles x [col][n][3] of the 27
@@ -172,7 +178,8 @@ void launch_tmu32_sym_multi(int g, const SymSlice *sl, int nsl, unsigned *next, 
 int tmu_f64_sym_items(const DevSites &s, int g, double round_pairs = 0.0);
 void launch_tmu_f64_sym_multi(int g, bool amoeba, const SymSlice *sl, int nsl, unsigned *next, cudaStream_t st,
                               bool zeroed = false);
-void launch_tmu32_pairs(const DevSites &s, int g, const float *x, float *partial, int nsplit, cudaStream_t st);
+void launch_tmu32_pairs(const DevSites &s, int g, int groups, const float *x, float *partial, int nsplit,
+                        cudaStream_t st);
 // source splits an FP32 scratch must hold (per column) for every shape the
 // autotuner may pick
 int tmu32_max_split(const DevSites &s, int sm_count);

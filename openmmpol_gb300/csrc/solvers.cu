@@ -9,8 +9,8 @@
 //                once as a CUDA graph and replayed.
 //   mixed_ir_ws  iterative refinement: FP64 residual E - T mu, FP32 PCG on the
 //                normalised residual, FP64 accumulation, FP64 convergence test.
-//   tune_f32     picks the FP32 kernel's column-group width and source split
-//                by timing the candidates on this system (cached per width).
+//   tune_f32     picks the FP32 kernel, its column-group width and source split
+//                by the system's size (kept per width).
 //   solve_batch  nf fields at once (64 QM densities, say): one block of
 //                columns through the same solvers.
 #include <algorithm>
@@ -36,6 +36,8 @@ void System::free_ws(Workspace &w) {
   if (w.graph) cudaGraphExecDestroy(w.graph);
   w.graph = nullptr;
   w.graph_ncol = -1;
+  if (w.sym) cudaFree(w.sym);
+  w.sym = nullptr, w.sym_len = 0;
   if (!w.owned) return;
   void *b[] = {w.x, w.r, w.p, w.h, w.z, w.rhs, w.fields, w.out, w.x32, w.r32, w.p32, w.h32, w.z32,
                w.scratch32, w.partial, w.dots, w.hist, w.cols, w.t32, w.gram, w.bcoef, w.bidx};
@@ -200,64 +202,41 @@ int System::f32_product(Workspace &w, int ncol, const F32Shape &sh, bool prepare
                              part, max_part);
 }
 
+// The launch shape by size and columns (forced kernels keep their own shape).
+// Widest column groups.  Kernel by the measured time of one product with its
+// finishing pass, us (pairwise / tiled / symmetric):
+//   sites        999        2,001        3,003        4,200        6,000         9,003
+//   1 column   28/31/-    30/33/-    36/36/48    54/42/49    90/77/64   163/120/86
+//   2 columns  31/36/-    34/35/-    42/41/61    65/52/64   116/98/94  209/160/129
+//   4 columns  32/25/-    38/30/-    54/43/-     87/61/137  152/111/186 292/207/260
+//   8 columns  36/37/-    48/46/-    73/63/-    129/102/-   237/190/-   472/350/-
+// (15,000 sites, 8 columns: tiled 846, symmetric 1,088.)  Source splits: the
+// finer of the two candidates, as fine as the tiles allow, won everywhere.
 int System::tune_f32(Workspace &w, int ncol, F32Shape &shape) {
   auto it = f32_tune_.find(ncol);
   if (it != f32_tune_.end() && it->second.nsplit <= w.scratch32_nsplit) {
     shape = it->second;
     return kOk;
   }
-  const int sms = gpu::sm_count();
-  const int tiles = (d_.n + 127) / 128;
-  const int cap = std::min(w.scratch32_nsplit, tiles);
-  std::vector<F32Shape> cands;
-  std::vector<int> widths = {1};
-  for (int g : {2, 4, 8})
-    if (g <= ncol) widths.push_back(g);
-  // kernel 1: one target per thread; kernel 2: tile-classified, two
-  // targets per thread for one or two columns
-  const int s1 = gpu::tmu_pick_split(d_, ncol, sms, true), s2 = gpu::tmu32_pick_split(d_, sms);
-  for (int g : widths) {
-    if (fp32_kernel_ == 0 || fp32_kernel_ == 1)
-      for (int s : {s1, 2 * s1})
-        if (s <= cap) cands.push_back({g, s, 1});
-    if (fp32_kernel_ == 0 || fp32_kernel_ == 2)
-      for (int s : {std::max(1, s2 / 2), s2, 2 * s2})
-        if (s <= cap) cands.push_back({g, s, 2});
+  const int n = d_.n, sms = gpu::sm_count();
+  F32Shape pick{ncol >= 8 ? 8 : ncol >= 4 ? 4 : ncol >= 2 ? 2 : 1, 1, fp32_kernel_};
+  if (fp32_kernel_ == 0) {
+    pick.kver = pick.g >= 4 ? 2 : n < 3000 ? 1 : n < 5000 ? 2 : 3;
+    if (pick.kver == 3 && ensure_sym_scratch() != kOk) pick.kver = 2;
+  } else if (fp32_kernel_ == 3) {
+    const int st = ensure_sym_scratch();
+    if (st) return st;
   }
-  // kernel 3: each unordered pair once (tmu32.cu), column groups of 1 or 2,
-  // from 2048 sites (or when forced); its accumulators are allocated here,
-  // before any capture of the inner iteration
-  if ((fp32_kernel_ == 3 || (fp32_kernel_ == 0 && d_.n >= 2048)) && ensure_sym_scratch() == kOk)
-    for (int g : {1, 2})
-      if (g <= ncol) cands.push_back({g, 1, 3});
-  if (cands.empty()) cands.push_back({1, 1, fp32_kernel_ == 1 ? 1 : 2});
-  const size_t nv = 3 * (size_t)d_.n;
-  cudaMemsetAsync(w.p32, 0, ncol * nv * sizeof(float), st_);
-  cudaEvent_t a, b;
-  cudaEventCreate(&a);
-  cudaEventCreate(&b);
-  float best = 1e30f;
-  F32Shape pick = cands.front();
-  for (const F32Shape &c : cands) {
-    f32_product(w, ncol, c);  // warm-up
-    cudaEventRecord(a, st_);
-    f32_product(w, ncol, c);
-    f32_product(w, ncol, c);
-    cudaEventRecord(b, st_);
-    cudaEventSynchronize(b);
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, a, b);
-    if (ms < best) best = ms, pick = c;
+  if (pick.kver == 3) {
+    pick.g = std::min(pick.g, 2);
+  } else {
+    const int split = pick.kver == 1 ? gpu::tmu_pick_split(d_, ncol, sms, true) : gpu::tmu32_pick_split(d_, sms);
+    pick.nsplit = std::max(1, std::min({2 * split, w.scratch32_nsplit, (n + 127) / 128}));
   }
-  cudaEventDestroy(a);
-  cudaEventDestroy(b);
-  int st = check(cudaGetLastError(), "FP32 autotune");
-  if (st) return st;
   f32_tune_[ncol] = pick;
   shape = pick;
-  log_msg(kVerbHigh, nullptr,
-          "autotuned FP32 T.mu for %d columns: kernel %d, %d per launch, %d source splits (%.3f ms)", ncol,
-          pick.kver, pick.g, pick.nsplit, best / 2);
+  log_msg(kVerbHigh, nullptr, "FP32 T.mu for %d columns: kernel %d, %d per launch, %d source splits", ncol, pick.kver,
+          pick.g, pick.nsplit);
   return kOk;
 }
 

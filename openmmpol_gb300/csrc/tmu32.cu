@@ -74,6 +74,9 @@ __global__ void __launch_bounds__(T32_TPB) k_tmu32(int n, const float4 *__restri
   __shared__ float4 s_pos[T32_TILE];
   __shared__ float4 s_mu[G][T32_TILE];  // x, y, z of column c; w = damping a of the source
   const int jb = blockIdx.x * (T32_TPB * TPT);
+  // the column group: its own columns and block of partials
+  x += (size_t)blockIdx.z * G * n * 3;
+  partial += (size_t)blockIdx.z * gridDim.y * G * n * 3;
   float4 pt[TPT];
   float at[TPT];
   bool valid[TPT];
@@ -207,10 +210,10 @@ __global__ void __launch_bounds__(T32_TPB) k_tmu32(int n, const float4 *__restri
 }
 
 template <int G, int TPT>
-void launch_g(const DevSites &s, const float *x, float *partial, int nsplit, cudaStream_t st) {
+void launch_g(const DevSites &s, int groups, const float *x, float *partial, int nsplit, cudaStream_t st) {
   const int tiles = (s.n + T32_TILE - 1) / T32_TILE;
   const int per = ((tiles + nsplit - 1) / nsplit) * T32_TILE;
-  dim3 grid((s.n + T32_TPB * TPT - 1) / (T32_TPB * TPT), nsplit);
+  dim3 grid((s.n + T32_TPB * TPT - 1) / (T32_TPB * TPT), nsplit, groups);
   if (s.amoeba)
     k_tmu32<G, TPT, true><<<grid, T32_TPB, 0, st>>>(s.n, s.pol_pos32, s.pol_a32, s.tile_box32, x, partial, per,
                                                     (float)s.damp_thr, s.damp_r2max32);
@@ -715,13 +718,16 @@ void launch_tmu32_sym_multi(int g, const SymSlice *sl, int nsl, unsigned *next, 
     launch_s32_table<1>(tab, next, st, zeroed);
 }
 
-// one column group through the v2 pair kernel (g = 1, 2, 4 or 8)
-void launch_tmu32_pairs(const DevSites &s, int g, const float *x, float *partial, int nsplit, cudaStream_t st) {
+// groups of g columns (1, 2, 4 or 8) through the tiled pair kernel, side by
+// side in one launch: one group of 8 columns of 3,003 sites is 1.3 waves of
+// CTAs, three are 3.8
+void launch_tmu32_pairs(const DevSites &s, int g, int groups, const float *x, float *partial, int nsplit,
+                        cudaStream_t st) {
   switch (g) {
-    case 8: launch_g<8, 1>(s, x, partial, nsplit, st); break;
-    case 4: launch_g<4, 1>(s, x, partial, nsplit, st); break;
-    case 2: launch_g<2, 2>(s, x, partial, nsplit, st); break;
-    default: launch_g<1, 2>(s, x, partial, nsplit, st); break;
+    case 8: launch_g<8, 1>(s, groups, x, partial, nsplit, st); break;
+    case 4: launch_g<4, 1>(s, groups, x, partial, nsplit, st); break;
+    case 2: launch_g<2, 2>(s, groups, x, partial, nsplit, st); break;
+    default: launch_g<1, 2>(s, groups, x, partial, nsplit, st); break;
   }
 }
 

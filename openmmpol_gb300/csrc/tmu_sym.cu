@@ -344,7 +344,10 @@ __global__ void __launch_bounds__(SYM_TILE, G == 1 ? 5 : 3) k_tmu_sym(const __gr
 // accumulators (if any) to zero and the largest high word of |x| (ctl, zeroed
 // before)
 __global__ void __launch_bounds__(256) k_sym_prepare(size_t total, const double *__restrict__ x,
-                                                     unsigned long long *__restrict__ acc, unsigned *ctl) {
+                                                     unsigned long long *__restrict__ acc, unsigned *ctl,
+                                                     size_t group_words) {
+  x += (size_t)blockIdx.y * total;  // column groups
+  ctl += 2 * group_words * blockIdx.y;
   unsigned m = 0;
   for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += (size_t)gridDim.x * blockDim.x) {
     if (acc) {
@@ -369,9 +372,14 @@ __global__ void __launch_bounds__(FIN_TPB) k_tmu_sym_finish(
     const unsigned long long *__restrict__ bad, const Pos64 *__restrict__ pos, const double *__restrict__ damp,
     const float2 *__restrict__ wa, const double *__restrict__ x, const double *__restrict__ ialpha, bool dodiag,
     const int *__restrict__ ri, const int *__restrict__ src, const double *__restrict__ scale, double thr, float thr2m,
-    double *__restrict__ y, double *__restrict__ part) {
+    double *__restrict__ y, double *__restrict__ part, size_t group_words) {
   __shared__ double s_dot[FIN_TPB / 32];
   const size_t col = (size_t)blockIdx.y * n;
+  if (group_words) {  // groups of two columns, each with its own accumulators
+    const size_t shift = (blockIdx.y / 2) * group_words;
+    lo += shift, hi += shift, bad += shift;
+    lo -= (size_t)(blockIdx.y / 2) * 6 * n, hi -= (size_t)(blockIdx.y / 2) * 6 * n;
+  }
   const bool nan = *bad != 0ull;
   const int ex = dsp_exponent(*reinterpret_cast<const unsigned *>(bad + 1));
   const int lane = threadIdx.x % L;
@@ -591,19 +599,19 @@ void launch_tmu_sym_prepare(const DevSites &s, int g, const double *x, unsigned 
   add_launch_count(1);
   cudaMemsetAsync(bad, 0, 2 * sizeof(unsigned long long), st);
   const int blocks = (int)std::min<size_t>((total + 255) / 256, 1216);
-  k_sym_prepare<<<blocks, 256, 0, st>>>(total, x, lo, reinterpret_cast<unsigned *>(bad + 1));
+  k_sym_prepare<<<blocks, 256, 0, st>>>(total, x, lo, reinterpret_cast<unsigned *>(bad + 1), 0);
 }
 
 void launch_max_word(size_t total, const double *x, unsigned *word, cudaStream_t st) {
   add_launch_count(1);
   cudaMemsetAsync(word, 0, sizeof(unsigned), st);
   const int blocks = (int)std::min<size_t>((total + 255) / 256, 1216);
-  k_sym_prepare<<<blocks, 256, 0, st>>>(total, x, nullptr, word);
+  k_sym_prepare<<<blocks, 256, 0, st>>>(total, x, nullptr, word, 0);
 }
 
 void launch_tmu_sym_finish(const DevSites &s, int g, const unsigned long long *lo, const unsigned long long *hi,
                            const unsigned long long *bad, const double *x, bool dodiag, double *y, cudaStream_t st,
-                           double *part, int max_part, int *npart) {
+                           double *part, int max_part, int *npart, size_t group_words) {
   add_launch_count(1);
   const int lanes = s.n < kFinishLanesSites ? 4 : 1;
   int blocks = (int)(((size_t)s.n * lanes + FIN_TPB - 1) / FIN_TPB);
@@ -613,7 +621,7 @@ void launch_tmu_sym_finish(const DevSites &s, int g, const unsigned long long *l
   const int *ri = s.d2d_nnz ? s.d2d_ri : nullptr;
   auto go = [&](auto kernel) {
     kernel<<<grid, FIN_TPB, 0, st>>>(s.n, lo, hi, bad, s.pol_pos, s.pol_a, s.pol_wa32, x, s.pol_ialpha, dodiag, ri,
-                                     s.d2d_src, s.d2d_s, s.damp_thr, thr2_margin(s), y, part);
+                                     s.d2d_src, s.d2d_s, s.damp_thr, thr2_margin(s), y, part, group_words);
   };
   if (lanes == 4)
     s.amoeba ? go(k_tmu_sym_finish<true, 4>) : go(k_tmu_sym_finish<false, 4>);
@@ -648,6 +656,47 @@ void launch_tmu_f64_sym(const DevSites &s, int nrhs, const double *x, double *y,
     launch_tmu_sym_finish(s, g, lo, hi, bad, xg, dodiag, y + (size_t)done * s.n * 3, st);
     done += g;
   }
+}
+
+// Pairs of columns per launch: about 16 slots per resident CTA.  A product of
+// two columns of 3,003 sites has 312 slots for 456 CTAs:
+// 24 columns took 12 x 176 us one pair after another, 1,436 us in one launch.
+int tmu_sym_groups(const DevSites &s, int nrhs) {
+  const int pairs = nrhs / 2;
+  if (s.n == 0 || pairs < 2) return 1;
+  const SymPlan p = sym_plan(s.n, sym_ctas(2, s.amoeba), 0.0);
+  const long long units = (long long)p.ntile * (p.K + 1);
+  const long long want = (16LL * sym_ctas(2, s.amoeba) + units - 1) / units;
+  return (int)std::min<long long>(std::min<long long>(want, pairs), kMaxSymSlices);
+}
+
+void launch_tmu_f64_sym_groups(const DevSites &s, int nrhs, const double *x, double *y, bool dodiag, double *scratch,
+                               cudaStream_t st) {
+  if (s.n == 0) return;
+  const int most = tmu_sym_groups(s, nrhs);
+  const size_t nv = 3 * (size_t)s.n, words = tmu_sym_scratch_doubles(s, 2);
+  unsigned long long *base = reinterpret_cast<unsigned long long *>(scratch);
+  int done = 0;
+  while (most > 1 && nrhs - done >= 2) {
+    const int groups = std::min(most, (nrhs - done) / 2);
+    const double *xg = x + done * nv;
+    cudaMemsetAsync(scratch, 0, groups * words * sizeof(double), st);
+    add_launch_count(1);
+    const int blocks = (int)std::min<size_t>((2 * nv + 255) / 256, 1216);
+    k_sym_prepare<<<dim3(blocks, groups), 256, 0, st>>>(2 * nv, xg, nullptr,
+                                                        reinterpret_cast<unsigned *>(base + 6 * nv + 1), words);
+    SymSlice sl[kMaxSymSlices];
+    const int items = tmu_f64_sym_items(s, 2);
+    for (int g = 0; g < groups; ++g) {
+      unsigned long long *lo = base + g * words;
+      sl[g] = {&s, xg + 2 * g * nv, lo, lo + 2 * nv, lo + 6 * nv, 0, items};
+    }
+    launch_tmu_f64_sym_multi(2, s.amoeba, sl, groups, reinterpret_cast<unsigned *>(base + 6 * nv + 2), st, true);
+    launch_tmu_sym_finish(s, 2 * groups, base, base + 2 * nv, base + 6 * nv, xg, dodiag, y + done * nv, st, nullptr, 0,
+                          nullptr, words);
+    done += 2 * groups;
+  }
+  if (done < nrhs) launch_tmu_f64_sym(s, nrhs - done, x + done * nv, y + done * nv, dodiag, scratch, st);
 }
 
 // Below kSymMinSites a symmetric product is bound by the latency of its few

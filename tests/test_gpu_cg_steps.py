@@ -118,3 +118,17 @@ def test_systems_sharing_launches(tmp_path):
     og.solve_multi(systems, fields)
     for g, f in zip(systems, fields):
         assert residual(g, f) < 2 * TOL
+
+
+@pytest.mark.parametrize("kind,size", [("water", 340), ("water", 700), ("chain", 352)])
+@pytest.mark.parametrize("nf", [3, 9, 16])
+def test_column_groups(tmp_path, kind, size, nf):
+    """From 1,000 sites the products of several pairs of columns, and the
+    tiled FP32 products of several groups, share a launch (odd counts leave a
+    last column, 9 = 8 + 1)."""
+    g = load(tmp_path, kind, size)
+    g.set_precision("mixed")
+    fields = np.stack([field(g, 40 + k) for k in range(nf)])
+    ipd = np.asarray(g.set_external_fields_batch(fields)[0])
+    for k in range(nf):
+        assert residual(g, fields[k], ipd[k]) < 2 * TOL
