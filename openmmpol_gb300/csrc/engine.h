@@ -45,6 +45,7 @@ struct Workspace {
   float *bcoef = nullptr;
   int *bidx = nullptr;
   double *bscal_h = nullptr;
+  float *bcoef_h = nullptr;
   // accumulators of the symmetric product for several column groups (grown on use)
   double *sym = nullptr;
   size_t sym_len = 0;

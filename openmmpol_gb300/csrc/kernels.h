@@ -207,15 +207,18 @@ void launch_batch_rhs(int n, int nf, int nset, const double *e_m2d, const double
 void launch_batch_scatter(int n, int nf, int nipd, int nsolved, const double *x, double *out, cudaStream_t st);
 
 // ---- block CG (block_cg.cu) -----------------------------------------------
-// out[a][b] = sum_i U[ua[a]][i] V[vb[b]][i] (FP32 tiles, FP64 across tiles,
-// fixed order); partial of block_cg_gram_doubles(smax)
+// out[a][b] = sum_i U[ua[a]][i] V[vb[b]][i], b < sb, then V2[vb2[b]], b < sb2
+// (rows of sb + sb2; FP32 tiles, FP64 across tiles, fixed order); partial of
+// block_cg_gram_doubles(smax)
 size_t block_cg_gram_doubles(int smax);
 int block_cg_max_columns();
-void launch_gram(size_t nv, int sa, const float *U, const int *ua, int sb, const float *V, const int *vb,
-                 double *partial, double *out, cudaStream_t st);
-// out[oc[k]] = base[bc[k]] + sum_j in[ic[j]] C[j][k], C [nin][nout] (device)
+void launch_gram(size_t nv, int sa, const float *U, const int *ua, int sb, const float *V, const int *vb, int sb2,
+                 const float *V2, const int *vb2, double *partial, double *out, cudaStream_t st);
+// out[oc[k]] = base[bc[k]] + sum_j in[ic[j]] C[j][k], C [nin][nout] (device);
+// with in2 also out2[oc[k]] -= sum_j in2[ic[j]] C[j][k]
 void launch_combine(size_t nv, int nin, const float *in, const int *ic, int nout, float *out, const int *oc,
-                    const float *base, const int *bc, const float *C, cudaStream_t st);
+                    const float *base, const int *bc, const float *C, cudaStream_t st, const float *in2 = nullptr,
+                    float *out2 = nullptr);
 void launch_scale_alpha32(int ncol, int n, const float *alpha, const float *r, float *z, cudaStream_t st);
 
 // ---- dense T (incore matvec / inversion) ---------------------------------

@@ -47,6 +47,7 @@ void System::free_ws(Workspace &w) {
   pinned_free(w.cols_h);
   pinned_free(w.scal_h);
   pinned_free(w.bscal_h);
+  pinned_free(w.bcoef_h);
   w = Workspace();
 }
 
@@ -71,10 +72,11 @@ int System::ensure_batch_ws(int ncol, int nf) {
   // block CG buffers (sized for the widest block)
   const int smax = gpu::block_cg_max_columns();
   bad |= walloc(w.t32, ncol * nv) | walloc(w.gram, gpu::block_cg_gram_doubles(smax)) |
-         walloc(w.bcoef, 2 * (size_t)smax * smax) | walloc(w.bidx, 2 * (size_t)smax);
+         walloc(w.bcoef, (size_t)smax * smax) | walloc(w.bidx, 2 * (size_t)smax);
   if (bad || pinned_alloc((void **)&w.cols_h, ncol * sizeof(gpu::CgCol)) != cudaSuccess ||
       pinned_alloc((void **)&w.scal_h, (3 * (size_t)ncol + nf) * sizeof(double)) != cudaSuccess ||
-      pinned_alloc((void **)&w.bscal_h, (2 * (size_t)smax * smax + smax) * sizeof(double)) != cudaSuccess) {
+      pinned_alloc((void **)&w.bscal_h, (2 * (size_t)smax * smax + smax) * sizeof(double)) != cudaSuccess ||
+      pinned_alloc((void **)&w.bcoef_h, (size_t)smax * smax * sizeof(float)) != cudaSuccess) {
     w.owned = true;
     free_ws(w);
     set_last_error("out of device memory for the batch workspace");
