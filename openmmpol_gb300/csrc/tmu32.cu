@@ -371,19 +371,20 @@ struct S32Target {
   int idx;            // index in the super-tile
 };
 
-// one slot: the warp's 64 targets against the 256 staged sources.  The far
+// one slot (or, js0 to js1, some of its sub-tiles): the warp's 64 targets
+// against the staged sources.  The far
 // loop is unrolled by 8 and the near one not at all: fully unrolled, the two
 // loops overflowed the instruction cache (ncu: issue stalled on instruction
 // fetch, 44 % issue activity).
 template <bool NEAR, bool AMOEBA, int G>
-__device__ __forceinline__ void s32_slot(bool diag, S32Smem<G> &sm, int warp, int lane, const S32Target (&tg)[2],
+__device__ __forceinline__ void s32_slot(bool diag, int js0, int js1, S32Smem<G> &sm, int warp, int lane, const S32Target (&tg)[2],
                                          const float2 (&mt)[2][3 * G], float thr,
                                          float2 (&af)[2][3 * G], float2 (&ak)[2][3 * G]) {
   constexpr int C = 3 * G, R = s32_records<G>();
   const int src = (lane + 1) & 31;
   const bool source_side = !NEAR || !diag;
 #pragma unroll 1
-  for (int js = 0; js < S32_NSUB; ++js) {
+  for (int js = js0; js < js1; ++js) {
     float2 aj[C];
 #pragma unroll
     for (int c = 0; c < C; ++c) aj[c] = make_float2(0.f, 0.f);
@@ -480,7 +481,7 @@ struct S32Job {
   const float4 *boxes;
   const float *x;
   unsigned long long *lo, *hi, *bad;
-  int n, ntile, nbox, K, chunk, nchunk, item0, amoeba;
+  int n, ntile, nbox, K, chunk, nchunk, whole, item0, amoeba;
   float thr, r2max;
 };
 struct S32Table {
@@ -489,7 +490,9 @@ struct S32Table {
   S32Job job[kMaxSymSlices];
 };
 
-template <int G>
+// PARTS: some items are parts of a unit (run-time bounds of the sub-tile loop
+// cost 2 % of a 90,000-site product, so whole items keep their own code)
+template <int G, bool PARTS>
 __global__ void __launch_bounds__(S32_TPB, G == 1 ? 4 : 3) k_tmu32_sym(const __grid_constant__ S32Table tab,
                                                                        unsigned *__restrict__ next) {
   constexpr int C = 3 * G, R = s32_records<G>();
@@ -513,7 +516,13 @@ __global__ void __launch_bounds__(S32_TPB, G == 1 ? 4 : 3) k_tmu32_sym(const __g
     const float *__restrict__ x = jb.x;
     const bool amoeba = jb.amoeba != 0;
     const int local = jb.item0 + (item - tab.base[jx]);
-    const int I = local / nchunk;
+    // items from `whole` on are quarters of a unit
+    int unit = local, js0 = 0, js1 = S32_NSUB;
+    if (PARTS && local >= jb.whole) {
+      js0 = (local - jb.whole) % S32_NSUB, js1 = js0 + 1;
+      unit = jb.whole + (local - jb.whole) / S32_NSUB;
+    }
+    const int I = unit / nchunk;
     S32Target tg[2];
     float2 mt[2][C];
 #pragma unroll
@@ -534,7 +543,7 @@ __global__ void __launch_bounds__(S32_TPB, G == 1 ? 4 : 3) k_tmu32_sym(const __g
     }
     float4 ilo, ihi;
     box_of_supertile(jb.boxes, jb.nbox, I, ilo, ihi);
-    const int k0 = (local - I * nchunk) * jb.chunk;
+    const int k0 = (unit - I * nchunk) * jb.chunk;
     const int k1 = min(jb.K + 1, k0 + jb.chunk);
     for (int k = k0; k < k1; ++k) {
       int J = I + k;
@@ -542,7 +551,7 @@ __global__ void __launch_bounds__(S32_TPB, G == 1 ? 4 : 3) k_tmu32_sym(const __g
       if (k > 0 && 2 * k == ntile && I >= ntile / 2) continue;  // the other tile of the pair owns it
       const bool diag = (k == 0);
       __syncthreads();  // the previous slot's staging and sums are read
-      {
+      if (!PARTS || (warp >= js0 && warp < js1)) {
         // thread tid stages pair (tid mod 32) of sub-tile tid / 32
         const int sb = tid >> 5, p = tid & 31;
         const int sa = J * S32_TILE + sb * S32_SUB + p, sbb = sa + 32;
@@ -584,11 +593,11 @@ __global__ void __launch_bounds__(S32_TPB, G == 1 ? 4 : 3) k_tmu32_sym(const __g
 #pragma unroll
         for (int c = 0; c < C; ++c) af[u][c] = ak[u][c] = make_float2(0.f, 0.f);
       if (far)
-        s32_slot<false, false, G>(false, sm, warp, lane, tg, mt, jb.thr, af, ak);
+        s32_slot<false, false, G>(false, PARTS ? js0 : 0, PARTS ? js1 : S32_NSUB, sm, warp, lane, tg, mt, jb.thr, af, ak);
       else if (amoeba)
-        s32_slot<true, true, G>(diag, sm, warp, lane, tg, mt, jb.thr, af, ak);
+        s32_slot<true, true, G>(diag, PARTS ? js0 : 0, PARTS ? js1 : S32_NSUB, sm, warp, lane, tg, mt, jb.thr, af, ak);
       else
-        s32_slot<true, false, G>(diag, sm, warp, lane, tg, mt, jb.thr, af, ak);
+        s32_slot<true, false, G>(diag, PARTS ? js0 : 0, PARTS ? js1 : S32_NSUB, sm, warp, lane, tg, mt, jb.thr, af, ak);
       // the slot's target sums, compensated across slots
 #pragma unroll
       for (int u = 0; u < 2; ++u)
@@ -606,7 +615,7 @@ __global__ void __launch_bounds__(S32_TPB, G == 1 ? 4 : 3) k_tmu32_sym(const __g
         for (int h = 0; h < 2; ++h) {
           const int q = h * S32_TPB + tid;
           const int sj = J * S32_TILE + q;
-          if (sj < n) {
+          if (sj < n && (!PARTS || (q / S32_SUB >= js0 && q / S32_SUB < js1))) {
 #pragma unroll
             for (int c = 0; c < C; ++c) {
               const float v = ((sm.accj[0][c][q] + sm.accj[1][c][q]) + sm.accj[2][c][q]) + sm.accj[3][c][q];
@@ -635,8 +644,9 @@ struct S32Launch {
   int resident = 0;
   S32Launch() {
     const int smem = (int)sizeof(S32Smem<G>);
-    cudaFuncSetAttribute(k_tmu32_sym<G>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_tmu32_sym<G>, S32_TPB, smem);
+    cudaFuncSetAttribute(k_tmu32_sym<G, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaFuncSetAttribute(k_tmu32_sym<G, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, k_tmu32_sym<G, true>, S32_TPB, smem);
     if (resident < 1) resident = 1;
   }
 };
@@ -646,19 +656,32 @@ int s32_resident() {
   return cfg.resident;
 }
 
-// the item space of one system's product: super-tiles x chunks of slots,
-// about 16 items per resident CTA of the whole GPU
-void s32_schedule(int n, int g, double round_pairs, int &ntile, int &K, int &chunk, int &nchunk) {
-  ntile = (n + S32_TILE - 1) / S32_TILE;
-  K = ntile / 2;
-  const int ctas_max = (g == 2 ? s32_resident<2>() : s32_resident<1>()) * sm_count();
-  long long c = (long long)ntile * (K + 1) / (16LL * ctas_max);
+// the item space of one system's product: units of a super-tile and a chunk
+// of its slots, about 16 per resident CTA of the whole GPU.  With fewer than
+// 8 one-slot units per CTA, those beyond a whole number of rounds of all CTAs
+// are cut into their four sub-tiles, so that the last round is short (10,200
+// sites, 840 units for 608 CTAs: 95 to 86 us; 15,000 sites 5 % less; cutting
+// every unit instead was slower from 15,000 sites, by its target sums)
+struct S32Plan {
+  int ntile, K, chunk, nchunk, whole;
+  int items() const { return whole + S32_NSUB * (ntile * nchunk - whole); }
+};
+S32Plan s32_plan(int n, int g, double round_pairs) {
+  S32Plan p;
+  p.ntile = (n + S32_TILE - 1) / S32_TILE;
+  p.K = p.ntile / 2;
+  const int ctas = (g == 2 ? s32_resident<2>() : s32_resident<1>()) * sm_count();
+  long long c = (long long)p.ntile * (p.K + 1) / (16LL * ctas);
   // round_pairs > 0: at most a quarter of a CTA's share of round_pairs
-  if (round_pairs > 0.0) c = std::min(c, (long long)(round_pairs / (4.0 * ctas_max * S32_TILE * S32_TILE)));
+  if (round_pairs > 0.0) c = std::min(c, (long long)(round_pairs / (4.0 * ctas * S32_TILE * S32_TILE)));
   if (c < 1) c = 1;
-  if (c > K + 1) c = K + 1;
-  chunk = (int)c;
-  nchunk = (K + 1 + chunk - 1) / chunk;
+  if (c > p.K + 1) c = p.K + 1;
+  p.chunk = (int)c;
+  p.nchunk = (p.K + 1 + p.chunk - 1) / p.chunk;
+  const int units = p.ntile * p.nchunk;
+  p.whole = units;
+  if (p.chunk == 1 && units < 8 * ctas) p.whole = units / ctas * ctas;
+  return p;
 }
 
 template <int G>
@@ -668,7 +691,12 @@ void launch_s32_table(const S32Table &tab, unsigned *next, cudaStream_t st, bool
   const int ctas_max = s32_resident<G>() * sm_count();
   const int ctas = ctas_max < total ? ctas_max : total;
   if (!zeroed) cudaMemsetAsync(next, 0, sizeof(unsigned), st);
-  k_tmu32_sym<G><<<ctas, S32_TPB, sizeof(S32Smem<G>), st>>>(tab, next);
+  bool parts = false;
+  for (int k = 0; k < tab.njobs; ++k) parts = parts || tab.job[k].whole < tab.job[k].ntile * tab.job[k].nchunk;
+  if (parts)
+    k_tmu32_sym<G, true><<<ctas, S32_TPB, sizeof(S32Smem<G>), st>>>(tab, next);
+  else
+    k_tmu32_sym<G, false><<<ctas, S32_TPB, sizeof(S32Smem<G>), st>>>(tab, next);
 }
 
 void fill_s32_job(S32Job &j, const DevSites &s, int g, const float *x, unsigned long long *lo,
@@ -680,7 +708,8 @@ void fill_s32_job(S32Job &j, const DevSites &s, int g, const float *x, unsigned 
   j.lo = lo, j.hi = hi, j.bad = bad;
   j.n = s.n;
   j.nbox = s.ntile;
-  s32_schedule(s.n, g, round_pairs, j.ntile, j.K, j.chunk, j.nchunk);
+  const S32Plan p = s32_plan(s.n, g, round_pairs);
+  j.ntile = p.ntile, j.K = p.K, j.chunk = p.chunk, j.nchunk = p.nchunk, j.whole = p.whole;
   j.item0 = item0;
   j.amoeba = s.amoeba ? 1 : 0;
   j.thr = (float)s.damp_thr;
@@ -693,9 +722,7 @@ int tmu32_sym_resident(int g, bool) { return g == 2 ? s32_resident<2>() : s32_re
 
 int tmu32_sym_items(const DevSites &s, int g, double round_pairs) {
   if (s.n == 0) return 0;
-  int ntile, K, chunk, nchunk;
-  s32_schedule(s.n, g, round_pairs, ntile, K, chunk, nchunk);
-  return ntile * nchunk;
+  return s32_plan(s.n, g, round_pairs).items();
 }
 
 void launch_tmu32_sym_multi(int g, const SymSlice *sl, int nsl, unsigned *next, cudaStream_t st, bool zeroed) {
