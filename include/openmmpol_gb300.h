@@ -316,7 +316,7 @@ int32_t ommp_gpu_set_inner_preconditioner(OMMP_SYSTEM_PRT s, int32_t mode);
 int32_t ommp_gpu_set_inner_blocks(OMMP_SYSTEM_PRT s, int32_t max_sites, double link_bohr);
 /* forget the last dipoles as a starting guess */
 void ommp_gpu_clear_guess(OMMP_SYSTEM_PRT s);
-/* capture the inner FP32 iteration as a CUDA graph (default on) */
+/* run the CG loops on the device as captured CUDA graphs (default on) */
 void ommp_gpu_set_use_graphs(OMMP_SYSTEM_PRT s, int32_t on);
 /* FP32 inner solve of batches (mixed modes, at least 4 columns): 1 (default)
  * block CG, the columns sharing one Krylov space; 0 the scalar PCG per

@@ -271,12 +271,13 @@ int System::upload_static() {
          alloc(d_.sub_box32, 2 * (size_t)((n + 31) / 32));
   bad |= alloc(d_.mm_split, 3 * (size_t)mm) | alloc(d_.mm_sub_box32, 2 * (size_t)((mm + 31) / 32)) | alloc(d_.mm_tile_box32, 2 * (size_t)((mm + 127) / 128));
   bad |= alloc(partial_, (size_t)gpu::kRedBlocks * 32) | alloc(dots_, 64) | alloc(hist_, 2 * (size_t)maxhist_);
-  bad |= alloc(cols_, 2) | alloc(flag_, 1) | alloc(info_, 1);
+  bad |= alloc(cols_, 3) | alloc(flag_, 1) | alloc(info_, 1);
   if (bad || pinned_alloc((void **)&cols_h_, 2 * sizeof(gpu::CgCol)) != cudaSuccess ||
       pinned_alloc((void **)&scal_h_, 64 * sizeof(double)) != cudaSuccess) {
     set_last_error("out of device memory while allocating the system");
     return kErrMemory;
   }
+  cudaMemsetAsync(cols_, 0, 3 * sizeof(gpu::CgCol), st_);
   ws_.cap = 2;
   ws_.x = x_, ws_.r = r_, ws_.p = p_, ws_.h = h_, ws_.z = z_, ws_.rhs = rhs_;
   ws_.x32 = x32_, ws_.r32 = r32_, ws_.p32 = p32_, ws_.h32 = h32_, ws_.z32 = z32_;
@@ -426,11 +427,7 @@ int System::build_blocks() {
   cudaStreamSynchronize(st_);
   // a captured inner iteration holds the preconditioner's device pointers:
   // drop it before the buffers are replaced (it is captured again)
-  for (Workspace *w : {&ws_, &wsb_}) {
-    if (w->graph) cudaGraphExecDestroy(w->graph);
-    w->graph = nullptr;
-    w->graph_ncol = -1;
-  }
+  for (Workspace *w : {&ws_, &wsb_}) w->loop32.drop();
   release(blk_info_);
   release(blk_minv_);
   blk_info_ = nullptr;
@@ -470,11 +467,7 @@ int System::ensure_near() {
     return kErrMemory;
   }
   // a captured inner iteration was built without the Neumann step
-  for (Workspace *w : {&ws_, &wsb_}) {
-    if (w->graph) cudaGraphExecDestroy(w->graph);
-    w->graph = nullptr;
-    w->graph_ncol = -1;
-  }
+  for (Workspace *w : {&ws_, &wsb_}) w->loop32.drop();
   h2d(near_ri_, ri.data(), ri.size() * sizeof(int));
   h2d(near_ci_, ci.data(), ci.size() * sizeof(int));
   h2d(near_blk_, blk.data(), blk.size() * sizeof(float));
@@ -681,8 +674,7 @@ void System::direct_product(int ncol, const double *x, double *y, bool dodiag, i
     sym = false;  // not enough memory for the accumulators: all-ordered-pairs kernel
     log_msg(kVerbHigh, nullptr, "symmetric T.mu scratch does not fit: using the all-ordered-pairs kernel");
   }
-  const size_t groups = sym ? gpu::tmu_sym_groups(d_, ncol) : 0;
-  if (groups > 1 && group_scratch(groups * gpu::tmu_sym_scratch_doubles(d_, 2)))
+  if (sym && ready_groups(ncol))
     gpu::launch_tmu_f64_sym_groups(d_, ncol, x, y, dodiag, wsb_.sym, st_);
   else if (sym)
     gpu::launch_tmu_f64_sym(d_, ncol, x, y, dodiag, sym_scratch_, st_);
@@ -691,8 +683,11 @@ void System::direct_product(int ncol, const double *x, double *y, bool dodiag, i
 }
 
 // accumulators for the column groups of one launch, kept with the batch
-// workspace
-bool System::group_scratch(size_t doubles) {
+// workspace; false: one group per launch
+bool System::ready_groups(int ncol) {
+  const size_t groups = gpu::tmu_sym_groups(d_, ncol);
+  if (groups < 2) return false;
+  const size_t doubles = groups * gpu::tmu_sym_scratch_doubles(d_, 2);
   if (wsb_.sym_len >= doubles) return true;
   if (wsb_.sym) {
     cudaStreamSynchronize(st_);

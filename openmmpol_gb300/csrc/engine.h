@@ -2,6 +2,7 @@
 // inversion, and the FP32-inner / FP64-refinement solver).
 #pragma once
 
+#include <functional>
 #include <map>
 #include <string>
 #include <utility>
@@ -22,6 +23,19 @@ enum Status : int {
   kErrCuda = 5,
   kErrMemory = 6,
   kErrCancelled = 7,
+};
+
+// A CG iteration captured as the body of a conditional (while) CUDA graph, and
+// the bytes of everything that its kernel arguments were taken from
+struct CgLoop {
+  cudaGraphExec_t exec = nullptr;
+  std::vector<char> key;
+  long long kernels = 0;  // per iteration
+  void drop() {
+    if (exec) cudaGraphExecDestroy(exec);
+    exec = nullptr;
+    key.clear();
+  }
 };
 
 // Column buffers of one solve: a view of a system's default two-column
@@ -49,14 +63,13 @@ struct Workspace {
   // accumulators of the symmetric product for several column groups (grown on use)
   double *sym = nullptr;
   size_t sym_len = 0;
-  gpu::CgCol *cols = nullptr;
+  gpu::CgCol *cols = nullptr;  // cap, and one whose space the loops' meeting words use
   gpu::CgCol *cols_h = nullptr;  // pinned
   double *scal_h = nullptr;      // pinned 3 x cap (+ fcap)
   bool owned = false;
-  // captured inner FP32 iteration (CUDA graph) and what it was built for
-  cudaGraphExec_t graph = nullptr;
-  int graph_ncol = -1, graph_gmax = 0, graph_nsplit = 0, graph_kver = 0, graph_prec = -1;
-  long long graph_kernels = 0;
+  // captured CG loops: the FP32 inner one and two FP64 ones (two columns of
+  // the default workspace are solved one after the other)
+  CgLoop loop32, loop64[2];
 };
 
 // device data of the polarization gradient (grad.cu) and of the fast
@@ -241,7 +254,11 @@ class System {
                   int max_part = 0);
   gpu::CgJob<float> inner_job(Workspace &w, int ncol, bool prepared);
   bool direct_symmetric(int matv, int ncol);
-  bool group_scratch(size_t doubles);
+  bool ready_groups(int ncol);
+  // body(handle) enqueues one iteration on st_; false: not run (no graphs, or
+  // the capture failed), else the loop ran and the columns' states are back
+  bool run_loop(CgLoop &loop, const std::vector<char> &key, const std::function<void(cudaGraphConditionalHandle)> &body,
+                int &st);
   int ensure_batch_ws(int ncol, int nf);
   void free_ws(Workspace &w);
   int check(cudaError_t e, const char *what);

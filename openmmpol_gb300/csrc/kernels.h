@@ -270,6 +270,7 @@ struct CgCol {
   int quick;      // left through |p.Tp| < eps
   int converged;  // rms < tol
   int iters;
+  int passes, max_passes;  // iterations run on the column, active or not, and their limit
 };
 // cols[k] = {gold = dots[k], tol, active = dots[k] > 0} (inner PCG start)
 // mu[k] += scale[k] * dmu32[k]  (IR correction, FP64 accumulate)

@@ -209,6 +209,21 @@ __global__ void __launch_bounds__(TPB) k_cg_near_sub(const __grid_constant__ Tab
   if (threadIdx.x == 0) jb.pb[(size_t)k * jb.nb + blockIdx.x] = acc;
 }
 
+// another iteration of the captured loop while a column wants one; the last
+// column to arrive sets the condition
+template <typename T>
+__device__ void cg_continue(const CgJob<T> &jb, bool go) {
+  if (jb.loop == 0) return;
+  if (jb.ncol > 1) {
+    if (go) atomicOr(jb.meet + 1, 1u);
+    __threadfence();
+    if (atomicAdd(jb.meet, 1u) + 1 != (unsigned)jb.ncol) return;
+    go = atomicExch(jb.meet + 1, 0u) != 0;
+    atomicExch(jb.meet, 0u);
+  }
+  cudaGraphSetConditional(jb.loop, go ? 1u : 0u);
+}
+
 // the scalars of a column after its update: rho = r.z
 template <typename T>
 __device__ void cg_close(const CgJob<T> &jb, int k, double rho, double beta) {
@@ -217,6 +232,7 @@ __device__ void cg_close(const CgJob<T> &jb, int k, double rho, double beta) {
     CgCol c{};
     c.gnew = rho;
     c.tol = jb.tol;
+    c.max_passes = jb.max_passes;
     c.active = jb.init == kCgInitKeep || rho > 0.0 ? 1 : 0;
     col = c;
   } else if (col.active) {
@@ -237,7 +253,9 @@ __device__ void cg_close(const CgJob<T> &jb, int k, double rho, double beta) {
       }
     }
   }
+  if (!jb.init) ++col.passes;
   jb.cols_h[k] = col;  // page-locked host memory: read after the stream
+  if (!jb.init) cg_continue(jb, col.active && col.passes < col.max_passes);
 }
 
 template <typename T>
@@ -287,7 +305,11 @@ __global__ void __launch_bounds__(SMALL_TPB) k_cg_small(const __grid_constant__ 
   __shared__ double sh[SMALL_TPB / 32];
   const int k = blockIdx.x, nv = 3 * jb.n;
   CgCol &col = jb.cols[k];
-  if (!col.active) return;  // uniform; the host has its last state
+  if (!col.active) {  // uniform
+    __syncthreads();
+    if (threadIdx.x == 0) cg_close(jb, k, 0.0, 0.0);
+    return;
+  }
   const size_t off = (size_t)k * nv;
   double *x = jb.x + off, *r = jb.r + off, *p = jb.p + off;
   const double *h = jb.h + off;

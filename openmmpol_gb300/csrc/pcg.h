@@ -18,7 +18,8 @@ struct CgJob {
              // with x cleared (kCgInitZero) or kept (kCgInitKeep)
   int na, nb;  // partial sums per column of p.h and of r.z
   int nhist;
-  double eps, tol;  // |p.h| of the quick exit; threshold put into the columns at the start
+  int max_passes;   // iterations of the loop (put into the columns at the start, as tol)
+  double eps, tol;  // |p.h| of the quick exit; convergence threshold
   T *x, *r, *p, *h, *z, *w;  // [ncol][n][3]; z and w of modes 1 and 2
   const T *alpha;            // polarizability, mode 0
   const int4 *info;
@@ -31,6 +32,10 @@ struct CgJob {
   // the next product's accumulators and control words (or null)
   unsigned long long *acc, *words;
   size_t nacc;
+  // loop on the device: the condition of the captured loop (0: none), and two
+  // words, zero between iterations, where the columns meet to set it
+  cudaGraphConditionalHandle loop;
+  unsigned *meet;
 };
 
 struct F32Finish {

@@ -4,9 +4,8 @@
 //                for ncol independent columns sharing each T.mu product:
 //                zero-norm guess replaced by alpha*x, quick exit when
 //                |p.Tp| < 100 eps, convergence on sqrt(r.alpha r / n).
-//   pcg32_ws     the FP32 inner solver of the mixed-precision path; one
-//                iteration (FP32 T.mu, dots, updates, status copy) is captured
-//                once as a CUDA graph and replayed.
+//   pcg32_ws     the FP32 inner solver of the mixed-precision path.
+//   run_loop     either loop on the device, as a conditional CUDA graph.
 //   mixed_ir_ws  iterative refinement: FP64 residual E - T mu, FP32 PCG on the
 //                normalised residual, FP64 accumulation, FP64 convergence test.
 //   tune_f32     picks the FP32 kernel, its column-group width and source split
@@ -30,12 +29,17 @@ int walloc(T *&p, size_t count) {
   if (count == 0) count = 1;
   return cudaMalloc((void **)&p, count * sizeof(T)) == cudaSuccess ? 0 : 1;
 }
+
+template <typename T>
+void key_add(std::vector<char> &key, const T &v) {
+  const char *b = reinterpret_cast<const char *>(&v);
+  key.insert(key.end(), b, b + sizeof(T));
+}
 }  // namespace
 
 void System::free_ws(Workspace &w) {
-  if (w.graph) cudaGraphExecDestroy(w.graph);
-  w.graph = nullptr;
-  w.graph_ncol = -1;
+  w.loop32.drop();
+  for (CgLoop &l : w.loop64) l.drop();
   if (w.sym) cudaFree(w.sym);
   w.sym = nullptr, w.sym_len = 0;
   if (!w.owned) return;
@@ -68,7 +72,7 @@ int System::ensure_batch_ws(int ncol, int nf) {
   bad |= walloc(w.scratch32, (size_t)s0 * ncol * nv);
   w.partial_len = (size_t)gpu::kRedBlocks * std::max(ncol, nf);
   bad |= walloc(w.partial, w.partial_len) |
-         walloc(w.dots, 3 * (size_t)ncol + nf) | walloc(w.cols, ncol);
+         walloc(w.dots, 3 * (size_t)ncol + nf) | walloc(w.cols, ncol + 1);
   // block CG buffers (sized for the widest block)
   const int smax = gpu::block_cg_max_columns();
   bad |= walloc(w.t32, ncol * nv) | walloc(w.gram, gpu::block_cg_gram_doubles(smax)) |
@@ -82,11 +86,60 @@ int System::ensure_batch_ws(int ncol, int nf) {
     set_last_error("out of device memory for the batch workspace");
     return kErrMemory;
   }
+  cudaMemsetAsync(w.cols, 0, (ncol + 1) * sizeof(gpu::CgCol), st_);
   w.cap = ncol;
   w.fcap = nf;
   w.scratch32_nsplit = s0;
   w.owned = true;
   return kOk;
+}
+
+// ---------------------------------------------------------------------------
+// A CG loop on the device: one iteration captured as the body of a while node
+// whose condition the last step sets, so that the host waits once per solve
+// instead of once per iteration (about 10 us each).  The loop ends after
+// CgCol::max_passes iterations at the latest.
+// ---------------------------------------------------------------------------
+bool System::run_loop(CgLoop &loop, const std::vector<char> &key,
+                      const std::function<void(cudaGraphConditionalHandle)> &body, int &st) {
+  st = kOk;
+  if (!use_graphs_) return false;
+  if (!loop.exec || loop.key != key) {
+    loop.drop();
+    cudaGraph_t g = nullptr, captured = nullptr;
+    cudaGraphConditionalHandle handle = 0;
+    cudaGraphNodeParams par = {};
+    cudaGraphNode_t node;
+    bool ok = cudaGraphCreate(&g, 0) == cudaSuccess &&
+              cudaGraphConditionalHandleCreate(&handle, g, 1, cudaGraphCondAssignDefault) == cudaSuccess;
+    if (ok) {
+      par.type = cudaGraphNodeTypeConditional;
+      par.conditional.handle = handle;
+      par.conditional.type = cudaGraphCondTypeWhile;
+      par.conditional.size = 1;
+      ok = cudaGraphAddNode(&node, g, nullptr, nullptr, 0, &par) == cudaSuccess &&
+           cudaStreamBeginCaptureToGraph(st_, par.conditional.phGraph_out[0], nullptr, nullptr, 0,
+                                         cudaStreamCaptureModeThreadLocal) == cudaSuccess;
+    }
+    if (ok) {
+      const long long before = gpu::thread_launch_count();
+      body(handle);
+      loop.kernels = gpu::thread_launch_count() - before;
+      gpu::add_launch_count(-loop.kernels);  // captured, not launched
+      ok = cudaStreamEndCapture(st_, &captured) == cudaSuccess && cudaGraphInstantiate(&loop.exec, g, 0) == cudaSuccess;
+    }
+    if (g) cudaGraphDestroy(g);
+    if (!ok) {
+      loop.exec = nullptr;
+      cudaGetLastError();
+      log_msg(kVerbHigh, nullptr, "CUDA graph capture of the CG loop failed: launches from the host");
+      return false;
+    }
+    loop.key = key;
+  }
+  st = check(cudaGraphLaunch(loop.exec, st_), "CG loop");
+  if (!st) st = check(cudaStreamSynchronize(st_), "CG loop");
+  return true;
 }
 
 // ---------------------------------------------------------------------------
@@ -132,6 +185,7 @@ int System::cg64_ws(Workspace &w, int matv, int ncol, const double *rhs, double 
   job.x = x, job.r = w.r, job.p = w.p, job.h = w.h, job.alpha = d_.pol_alpha;
   job.pa = w.partial, job.pb = w.partial + share * ncol;
   job.cols = w.cols, job.cols_h = w.cols_h;
+  job.meet = reinterpret_cast<unsigned *>(w.cols + w.cap);
   job.hist = hist, job.nhist = maxhist_;
   // the direct symmetric product of one column group: its accumulators and
   // scale are prepared by the steps, its finishing pass sums p.h
@@ -140,10 +194,11 @@ int System::cg64_ws(Workspace &w, int matv, int ncol, const double *rhs, double 
   unsigned long long *lo = reinterpret_cast<unsigned long long *>(sym_scratch_);
   if (sym) job.acc = lo, job.nacc = 2 * C * n, job.words = lo + 3 * C * n;
   const bool small = !sym && n <= gpu::kCgSmallSites;
+  job.max_passes = maxiter_;
   job.init = gpu::kCgInitKeep;
   gpu::launch_cg_steps(&job, 1, st_);
   job.init = 0;
-  for (int it = 1; it <= maxiter_; ++it) {
+  auto enqueue = [&]() -> int {
     if (sym) {
       KEv e;
       if (ktime_on_) e = kt_begin(0, ncol);
@@ -153,14 +208,43 @@ int System::cg64_ws(Workspace &w, int matv, int ncol, const double *rhs, double 
       if (ktime_on_) kt_end(e);
       stats_.f64_matvecs += 1;
     } else {
-      st = matvec64(matv, ncol, w.p, w.h, true);
-      if (st) return st;
+      const int rc = matvec64(matv, ncol, w.p, w.h, true);
+      if (rc) return rc;
       if (!small) gpu::launch_cg_dot(ncol, job.na = job.nb, nv, w.h, w.p, job.pa, st_);
     }
     if (small)
       gpu::launch_cg_small(job, st_);
     else
       gpu::launch_cg_steps(&job, 1, st_);
+    return kOk;
+  };
+  // the loop of the direct products that are kernels alone (no memset) runs on
+  // the device; kernel timing, per-iteration messages, the FMM, the in-core T
+  // and symmetric products of more than two columns go from the host
+  bool looped = false;
+  const bool rows = !sym && !(fp64_kernel_ == 2 || (fp64_kernel_ == 0 && n >= gpu::kSymMinSites));
+  if (maxiter_ > 0 && !ktime_on_ && log_level() < kVerbHigh && !fmm_on_ && !(matv == kMatvIncore && tmat_ok_) &&
+      (sym || rows)) {
+    const long long products = stats_.f64_matvecs;
+    CgLoop &loop = w.loop64[x == w.x ? 0 : 1];
+    std::vector<char> key;
+    job.tol = 0.0, job.max_passes = 0;  // those of the start are in w.cols
+    key_add(key, d_), key_add(key, job), key_add(key, sym), key_add(key, small), key_add(key, fp64_kernel_);
+    key_add(key, sym_scratch_);
+    looped = run_loop(loop, key, [&](cudaGraphConditionalHandle hnd) {
+      job.loop = hnd;
+      enqueue();
+    }, st);
+    job.loop = 0;
+    if (st) return st;
+    int passes = 0;
+    for (int k = 0; k < ncol; ++k) passes = std::max(passes, w.cols_h[k].passes);
+    stats_.f64_matvecs = products + (looped ? passes : 0);
+    if (looped) gpu::add_launch_count(loop.kernels * passes);
+  }
+  for (int it = 1; !looped && it <= maxiter_; ++it) {
+    st = enqueue();
+    if (st) return st;
     st = check(cudaStreamSynchronize(st_), "CG iteration");
     if (st) return st;
     bool any = false;
@@ -259,6 +343,7 @@ gpu::CgJob<float> System::inner_job(Workspace &w, int ncol, bool prepared) {
   job.ri = near_ri_, job.ci = near_ci_, job.blk = near_blk_;
   job.pa = w.partial, job.pb = w.partial + w.partial_len / (2 * (size_t)ncol) * ncol;
   job.cols = w.cols, job.cols_h = w.cols_h;
+  job.meet = reinterpret_cast<unsigned *>(w.cols + w.cap);
   if (prepared) {
     unsigned long long *lo = reinterpret_cast<unsigned long long *>(sym_scratch_);
     job.acc = lo, job.nacc = 2 * 3 * (size_t)ncol * d_.n, job.words = lo + 3 * 3 * (size_t)ncol * d_.n;
@@ -280,6 +365,7 @@ int System::pcg32_ws(Workspace &w, int ncol, int max_it, double eta) {
   gpu::CgJob<float> job = inner_job(w, ncol, prepared);
   const int share = (int)(w.partial_len / (2 * (size_t)ncol));
   job.tol = eta;
+  job.max_passes = max_it;
   job.init = gpu::kCgInitZero;
   gpu::launch_cg_steps(&job, 1, st_);
   job.init = 0;
@@ -287,48 +373,31 @@ int System::pcg32_ws(Workspace &w, int ncol, int max_it, double eta) {
     job.na = f32_product(w, ncol, shape, prepared, job.pa, share);
     gpu::launch_cg_steps(&job, 1, st_);
   };
-  // capture one iteration as a graph (kernel arguments and buffers are fixed
-  // per workspace, width and launch shape; the tolerance lives in w.cols)
-  if (use_graphs_ && (w.graph_ncol != ncol || w.graph_gmax != shape.g || w.graph_nsplit != shape.nsplit ||
-                     w.graph_kver != shape.kver || w.graph_prec != job.mode)) {
-    if (w.graph) cudaGraphExecDestroy(w.graph);
-    w.graph = nullptr;
-    w.graph_ncol = -1;
-    cudaGraph_t g = nullptr;
-    long long before = gpu::thread_launch_count();
-    if (cudaStreamBeginCapture(st_, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+  int it = 0;
+  if (max_it > 0 && !ktime_on_ && (prepared || shape.kver != 3)) {
+    // the loop on the device (the tolerance lives in w.cols)
+    job.tol = 0.0, job.max_passes = 0;
+    std::vector<char> key;
+    key_add(key, d_), key_add(key, job), key_add(key, shape), key_add(key, prepared);
+    key_add(key, w.scratch32), key_add(key, sym_scratch_);
+    const bool looped = run_loop(w.loop32, key, [&](cudaGraphConditionalHandle hnd) {
+      job.loop = hnd;
       iteration();
-      cudaError_t e = cudaStreamEndCapture(st_, &g);
-      long long kernels = gpu::thread_launch_count() - before;
-      gpu::add_launch_count(-kernels);  // captured, not launched
-      if (e == cudaSuccess && g && cudaGraphInstantiate(&w.graph, g, 0) == cudaSuccess) {
-        w.graph_ncol = ncol;
-        w.graph_gmax = shape.g;
-        w.graph_nsplit = shape.nsplit;
-        w.graph_kver = shape.kver;
-        w.graph_prec = job.mode;
-        w.graph_kernels = kernels;
-      } else {
-        w.graph = nullptr;
-        cudaGetLastError();
-        log_msg(kVerbHigh, nullptr, "CUDA graph capture of the inner iteration failed: direct launches");
-      }
-      if (g) cudaGraphDestroy(g);
-    } else {
-      cudaGetLastError();
+    }, st);
+    job.loop = 0;
+    if (st) return st;
+    if (looped) {
+      for (int k = 0; k < ncol; ++k) it = std::max(it, w.cols_h[k].passes);
+      gpu::add_launch_count(w.loop32.kernels * it);
+      stats_.f32_matvecs += it;
+      stats_.inner_iters += it;
+      return kOk;
     }
   }
-  const bool graph = use_graphs_ && w.graph && w.graph_ncol == ncol;
-  int it = 0;
   for (it = 1; it <= max_it; ++it) {
     KEv ev;
     if (ktime_on_) ev = kt_begin(1, ncol);
-    if (graph) {
-      cudaGraphLaunch(w.graph, st_);
-      gpu::add_launch_count(w.graph_kernels);
-    } else {
-      iteration();
-    }
+    iteration();
     if (ktime_on_) kt_end(ev);
     stats_.f32_matvecs += 1;
     st = check(cudaStreamSynchronize(st_), "inner CG iteration");
