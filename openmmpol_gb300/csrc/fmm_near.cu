@@ -40,6 +40,9 @@ __global__ void __launch_bounds__(NT, 5) k_fmm_near(const __grid_constant__ FmmN
   for (int b0 = s0; b0 < s1; b0 += NT) {
     const int si = b0 + threadIdx.x;
     const bool valid = si < s1;
+    // a warp past the end of the leaf only stages: the last pass over a leaf of
+    // 140 sites has one warp of work, not four
+    const bool work = b0 + (int)(threadIdx.x & ~31) < s1;
     const int ti = valid ? si : s0;
     float tg[9];
     {
@@ -90,6 +93,7 @@ __global__ void __launch_bounds__(NT, 5) k_fmm_near(const __grid_constant__ FmmN
           s_wa[threadIdx.x] = a.swa[k];
         }
         __syncthreads();
+        if (!work) continue;
         const int cnt = min(NT, r1 - t0);
         float ah[3] = {0.f, 0.f, 0.f}, al[3] = {0.f, 0.f, 0.f};
 #pragma unroll 1
