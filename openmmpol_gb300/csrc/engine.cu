@@ -124,7 +124,7 @@ System::~System() {
   if (st_) cudaStreamSynchronize(st_);
   free_ws(ws_);
   free_ws(wsb_);
-  void *bufs[] = {inv32_, sqrt_alpha_, d_.pol_pos, d_.pol_a, d_.pol_alpha, d_.pol_ialpha, d_.polar_mm, d_.pol_pos32, d_.pol_a32,
+  void *bufs[] = {row_words_, inv32_, sqrt_alpha_, d_.pol_pos, d_.pol_a, d_.pol_alpha, d_.pol_ialpha, d_.polar_mm, d_.pol_pos32, d_.pol_a32,
                   d_.pol_wa32, d_.mm_split, d_.mm_sub_box32, d_.mm_tile_box32,
                   d_.mm_wa32, d_.mm_pos,
                   d_.mm_a, d_.mm_q, d_.m2d_ri, d_.m2d_src, d_.m2d_sP, d_.m2d_sD, d_.d2d_ri, d_.d2d_src,
@@ -271,7 +271,7 @@ int System::upload_static() {
          alloc(d_.sub_box32, 2 * (size_t)((n + 31) / 32));
   bad |= alloc(d_.mm_split, 3 * (size_t)mm) | alloc(d_.mm_sub_box32, 2 * (size_t)((mm + 31) / 32)) | alloc(d_.mm_tile_box32, 2 * (size_t)((mm + 127) / 128));
   bad |= alloc(partial_, (size_t)gpu::kRedBlocks * 32) | alloc(dots_, 64) | alloc(hist_, 2 * (size_t)maxhist_);
-  bad |= alloc(cols_, 3) | alloc(flag_, 1) | alloc(info_, 1);
+  bad |= alloc(row_words_, kRowWords) | alloc(cols_, 3) | alloc(flag_, 1) | alloc(info_, 1);
   if (bad || pinned_alloc((void **)&cols_h_, 2 * sizeof(gpu::CgCol)) != cudaSuccess ||
       pinned_alloc((void **)&scal_h_, 64 * sizeof(double)) != cudaSuccess) {
     set_last_error("out of device memory while allocating the system");
@@ -679,7 +679,12 @@ void System::direct_product(int ncol, const double *x, double *y, bool dodiag, i
   else if (sym)
     gpu::launch_tmu_f64_sym(d_, ncol, x, y, dodiag, sym_scratch_, st_);
   else
-    gpu::launch_tmu_f64(d_, ncol, x, y, dodiag, st_);
+    for (int c = 0; c < ncol; c += kRowWords) {
+      const int g = std::min(kRowWords, ncol - c);
+      const size_t nv = 3 * (size_t)d_.n, o = c * nv;
+      if (gpu::tmu_rows_parts(d_, g) > 0) gpu::launch_max_words(g, nv, x + o, row_words_, st_);
+      gpu::launch_tmu_rows(d_, g, x + o, y + o, dodiag, row_words_, nullptr, st_);
+    }
 }
 
 // accumulators for the column groups of one launch, kept with the batch
@@ -708,6 +713,12 @@ bool System::direct_symmetric(int matv, int ncol) {
   if ((matv == kMatvIncore && tmat_ok_) || fmm_on_ || ncol > 2) return false;
   if (fp64_kernel_ != 2 && !(fp64_kernel_ == 0 && d_.n >= gpu::kSymMinSites)) return false;
   return ensure_sym_scratch() == kOk;
+}
+
+// matvec64 would take the ordered direct product, its scales within row_words_
+bool System::direct_rows(int matv, int ncol) const {
+  if ((matv == kMatvIncore && tmat_ok_) || fmm_on_ || ncol > kRowWords) return false;
+  return fp64_kernel_ == 1 || (fp64_kernel_ == 0 && d_.n < gpu::kSymMinSites);
 }
 
 // fixed-point accumulators of the symmetric products (FP64, double-single

@@ -255,6 +255,7 @@ class System {
   gpu::CgJob<float> inner_job(Workspace &w, int ncol, bool prepared);
   bool direct_symmetric(int matv, int ncol);
   bool ready_groups(int ncol);
+  bool direct_rows(int matv, int ncol) const;
   // body(handle) enqueues one iteration on st_; false: not run (no graphs, or
   // the capture failed), else the loop ran and the columns' states are back
   bool run_loop(CgLoop &loop, const std::vector<char> &key, const std::function<void(cudaGraphConditionalHandle)> &body,
@@ -287,6 +288,7 @@ class System {
   double *scratch_ = nullptr;  // pair-kernel split partials
   size_t scratch_n_ = 0;
   double *sym_scratch_ = nullptr;  // symmetric-kernel partials (allocated on first use)
+  unsigned *row_words_ = nullptr;  // scales of the columns of an ordered product (kRowWords)
   int fp64_kernel_ = 0;
   int4 *blk_info_ = nullptr;   // block-Jacobi preconditioner (build_block_jacobi)
   float *blk_minv_ = nullptr;

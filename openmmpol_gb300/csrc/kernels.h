@@ -78,8 +78,12 @@ void launch_m2d_finish(const DevSites &s, double *out, const double *partial, in
 // y = T x (dodiag) or y = -E_dd(x) (no diagonal); x,y [nrhs][n][3], FP64.
 size_t tmu_scratch_doubles(const DevSites &s, int nrhs, int nsplit);
 int tmu_pick_split(const DevSites &s, int nrhs, int sm_count, bool fp32);
-// All ordered pairs in FP64, no scratch (tmu_sym.cu).
-void launch_tmu_f64(const DevSites &s, int nrhs, const double *x, double *y, bool dodiag, cudaStream_t st);
+// All ordered pairs to FP64 accuracy in one launch (tmu_rows.cu); words: the
+// largest high word of each column (launch_max_words).  part: partial sums of
+// x.y, tmu_rows_parts per column (0: this size gives none).
+int tmu_rows_parts(const DevSites &s, int ncol);
+void launch_tmu_rows(const DevSites &s, int nrhs, const double *x, double *y, bool dodiag, const unsigned *words,
+                     double *part, cudaStream_t st);
 // The finishing pass alone on a field partial [nrhs][n][3] (one split): the
 // u-scaled pair corrections, the sign and the 1/alpha diagonal
 void launch_tmu_finish64(const DevSites &s, int nrhs, const double *partial, const double *x, bool dodiag,
@@ -87,8 +91,8 @@ void launch_tmu_finish64(const DevSites &s, int nrhs, const double *partial, con
 // Same product with each unordered pair evaluated once (deterministic
 // half-shell schedule, tmu_sym.cu): near pairs in FP64, the others in
 // double-single; scratch of tmu_sym_scratch_doubles(s, nrhs_max).  The product
-// of every mode from kSymMinSites sites (launch_tmu_f64 below).
-constexpr int kSymMinSites = 1000;
+// of every mode from kSymMinSites sites (launch_tmu_rows below).
+constexpr int kSymMinSites = 2400;
 // the finishing passes give a site four lanes below this many sites, one above
 constexpr int kFinishLanesSites = 32768;
 // squared distances within which a pair always runs in FP64 (AMOEBA pairs
@@ -114,6 +118,7 @@ void launch_tmu_sym_finish(const DevSites &s, int g, const unsigned long long *l
                            double *part = nullptr, int max_part = 0, int *npart = nullptr, size_t group_words = 0);
 // the largest high word of |x| (the scale of the double-single products)
 void launch_max_word(size_t total, const double *x, unsigned *word, cudaStream_t st);
+void launch_max_words(int ncol, size_t nv, const double *x, unsigned *words, cudaStream_t st);
 // near field of the FMM (fmm_near.cu): the dipoles x [col][n][3] of the 27
 // neighbouring leaves at every site, sites sorted by leaf (split coordinates
 // [3][n], spos, sa, swa; perm the polarizable index); partial

@@ -9,8 +9,8 @@
 // and can fail at an arbitrary point of a long run.  The regular entry point
 // ommp_gpu_tmatvec stages through the system's own buffers; this variant
 // takes device pointers and keeps its only scratch (the fixed-point sums of
-// the symmetric product from 2048 sites, else the per-source-split partial
-// fields of the target-outer kernel) in a fixed, file-scope device array.
+// the symmetric product, else the scales of the ordered one) in a fixed,
+// file-scope device array.
 //
 // The product is always the direct FP64 sum over all pairs: the system's FMM
 // switch, its matrix-vector selector (in-core T) and its FP64 kernel choice
@@ -29,9 +29,7 @@
 // itself waits for its kernels, so calls issued one after another from one
 // thread never overlap.  What must start at zero is cleared on every call:
 // the symmetric branch clears its fixed-point accumulators with
-// cudaMemsetAsync before its pair kernel; in the target-outer branch every
-// partial the finishing kernel reads is first written by the pair kernel of
-// the same call.
+// cudaMemsetAsync before its pair kernel, the ordered one its scales.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -117,7 +115,7 @@ extern "C" int32_t ommp_gpu_tmatvec_noalloc(OMMP_SYSTEM_PRT sp, const double *x_
     ommp::set_last_error("ommp_gpu_tmatvec_noalloc: x and y overlap (an in-place product is not supported)");
     return ommp::kErrBadArg;
   }
-  // the pair kernel needs nsplit * nrhs * n * 3 doubles of partials
+  // the size limit of the entry point: nrhs * n * 3 doubles of scratch
   size_t per_split = (size_t)nrhs * (size_t)d.n * 3;
   size_t fit = kNoAllocScratchDoubles / per_split;
   if (fit < 1) {
@@ -133,7 +131,9 @@ extern "C" int32_t ommp_gpu_tmatvec_noalloc(OMMP_SYSTEM_PRT sp, const double *x_
     // each unordered pair once, fixed-point sums in the static scratch
     ommp::gpu::launch_tmu_f64_sym(d, nrhs, x_dev, y_dev, dodiag != 0, scratch, s->stream());
   } else {
-    ommp::gpu::launch_tmu_f64(d, nrhs, x_dev, y_dev, dodiag != 0, s->stream());
+    unsigned *words = reinterpret_cast<unsigned *>(scratch);
+    ommp::gpu::launch_max_words(nrhs, 3 * (size_t)d.n, x_dev, words, s->stream());
+    ommp::gpu::launch_tmu_rows(d, nrhs, x_dev, y_dev, dodiag != 0, words, nullptr, s->stream());
   }
   cudaError_t e = cudaStreamSynchronize(s->stream());
   if (e == cudaSuccess) e = cudaGetLastError();

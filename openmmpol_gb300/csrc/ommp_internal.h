@@ -90,6 +90,7 @@ void build_block_jacobi(const HostModel &m, const ScaledPairs &d2d, double damp_
 // build_block_jacobi) within rc, with the 3x3 block of T between them,
 // -s (3 k5 d d^T - k3 I) with the damping and the D2D scale of the product
 // (row-major, FP32): CSR ri [n + 1], ci [nnz], blk [nnz][9]
+constexpr int kRowWords = 256;  // columns of an ordered product per launch
 constexpr double kNearBohr = 6.5;
 void build_near_field(const HostModel &m, const ScaledPairs &d2d, double damp_thr, const std::vector<int> &info,
                       double rc, std::vector<int> &ri, std::vector<int> &ci, std::vector<float> &blk);

@@ -114,7 +114,10 @@ __global__ void __launch_bounds__(TPB) k_cg_step(const __grid_constant__ Table<C
     act = act && !quick;
   }
   const Scalar pal(al), mal(-al);
-  if (jb.words && k == 0 && blockIdx.x == 0 && threadIdx.x < 3) jb.words[threadIdx.x] = 0ull;
+  if (blockIdx.x == 0) {
+    if (jb.words && k == 0 && threadIdx.x < 3) jb.words[threadIdx.x] = 0ull;
+    if (jb.emax_stride && threadIdx.x == 0) jb.emax[k] = 0u;
+  }
   const size_t nv = 3 * (size_t)jb.n, off = (size_t)k * nv;
   T *x = jb.x + off, *r = jb.r + off;
   const T *p = jb.p + off, *h = jb.h + off;
@@ -285,12 +288,12 @@ __global__ void __launch_bounds__(TPB) k_cg_dir(const __grid_constant__ Table<Cg
     p[i] = z;
     if constexpr (sizeof(T) == 8) mx = max(mx, (unsigned)__double2hiint(z) & 0x7FFFFFFFu);
   }
-  if (jb.acc) {
-    if (k == 0)
-      for (size_t i = (size_t)blockIdx.x * TPB + threadIdx.x; i < jb.nacc; i += (size_t)jb.nb * TPB) jb.acc[i] = 0ull;
-    if constexpr (sizeof(T) == 8) {
+  if (jb.acc && k == 0)
+    for (size_t i = (size_t)blockIdx.x * TPB + threadIdx.x; i < jb.nacc; i += (size_t)jb.nb * TPB) jb.acc[i] = 0ull;
+  if constexpr (sizeof(T) == 8) {
+    if (jb.emax) {
       mx = __reduce_max_sync(0xffffffffu, mx);
-      if ((threadIdx.x & 31) == 0 && mx) atomicMax(reinterpret_cast<unsigned *>(jb.words + 1), mx);
+      if ((threadIdx.x & 31) == 0 && mx) atomicMax(jb.emax + k * jb.emax_stride, mx);
     }
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) cg_close(jb, k, rho, beta);
@@ -341,15 +344,26 @@ __global__ void __launch_bounds__(SMALL_TPB) k_cg_small(const __grid_constant__ 
   }
   const double rho = block_sum(acc, sh, blockDim.x / 32);
   const double beta = rho / gold;
+  __shared__ unsigned s_max;
+  unsigned mx = 0;
+  if (threadIdx.x == 0) s_max = 0;
   if (!quick) {
 #pragma unroll
     for (int u = 0; u < SMALL_PER; ++u) {
       const int i = u * blockDim.x + threadIdx.x;
-      if (i < nv) p[i] = fma(beta, pv[u], zv[u]);
+      if (i < nv) {
+        const double v = fma(beta, pv[u], zv[u]);
+        p[i] = v;
+        mx = max(mx, (unsigned)__double2hiint(v) & 0x7FFFFFFFu);
+      }
     }
   }
   __syncthreads();  // every thread has read the scalars
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if ((threadIdx.x & 31) == 0) atomicMax(&s_max, mx);
+  __syncthreads();
   if (threadIdx.x == 0) {
+    if (jb.emax) jb.emax[k * jb.emax_stride] = s_max;
     col.alpha = al;
     col.gold = gold;
     col.gama = ph;

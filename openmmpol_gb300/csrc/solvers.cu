@@ -192,7 +192,13 @@ int System::cg64_ws(Workspace &w, int matv, int ncol, const double *rhs, double 
   const bool sym = direct_symmetric(matv, ncol);
   const size_t C = 3 * (size_t)ncol;
   unsigned long long *lo = reinterpret_cast<unsigned long long *>(sym_scratch_);
-  if (sym) job.acc = lo, job.nacc = 2 * C * n, job.words = lo + 3 * C * n;
+  if (sym) {
+    job.acc = lo, job.nacc = 2 * C * n, job.words = lo + 3 * C * n;
+    job.emax = reinterpret_cast<unsigned *>(job.words + 1);
+  }
+  // the ordered one: the scale of every column
+  const bool rows = !sym && direct_rows(matv, ncol);
+  if (rows && gpu::tmu_rows_parts(d_, ncol) > 0) job.emax = row_words_, job.emax_stride = 1;
   const bool small = !sym && n <= gpu::kCgSmallSites;
   job.max_passes = maxiter_;
   job.init = gpu::kCgInitKeep;
@@ -205,6 +211,16 @@ int System::cg64_ws(Workspace &w, int matv, int ncol, const double *rhs, double 
       gpu::SymSlice one{&d_, w.p, lo, lo + C * n, job.words, 0, gpu::tmu_f64_sym_items(d_, ncol)};
       gpu::launch_tmu_f64_sym_multi(ncol, d_.amoeba, &one, 1, reinterpret_cast<unsigned *>(job.words + 2), st_, true);
       gpu::launch_tmu_sym_finish(d_, ncol, lo, lo + C * n, job.words, w.p, true, w.h, st_, job.pa, (int)share, &job.na);
+      if (ktime_on_) kt_end(e);
+      stats_.f64_matvecs += 1;
+    } else if (rows) {
+      KEv e;
+      if (ktime_on_) e = kt_begin(0, ncol);
+      const int parts = gpu::tmu_rows_parts(d_, ncol);
+      const bool dot = !small && parts > 0 && (size_t)parts <= share;
+      gpu::launch_tmu_rows(d_, ncol, w.p, w.h, true, row_words_, dot ? job.pa : nullptr, st_);
+      job.na = dot ? parts : job.nb;
+      if (!small && !dot) gpu::launch_cg_dot(ncol, job.nb, nv, w.h, w.p, job.pa, st_);
       if (ktime_on_) kt_end(e);
       stats_.f64_matvecs += 1;
     } else {
@@ -222,7 +238,6 @@ int System::cg64_ws(Workspace &w, int matv, int ncol, const double *rhs, double 
   // the device; kernel timing, per-iteration messages, the FMM, the in-core T
   // and symmetric products of more than two columns go from the host
   bool looped = false;
-  const bool rows = !sym && !(fp64_kernel_ == 2 || (fp64_kernel_ == 0 && n >= gpu::kSymMinSites));
   if (maxiter_ > 0 && !ktime_on_ && log_level() < kVerbHigh && !fmm_on_ && !(matv == kMatvIncore && tmat_ok_) &&
       (sym || rows)) {
     const long long products = stats_.f64_matvecs;

@@ -345,9 +345,9 @@ __global__ void __launch_bounds__(SYM_TILE, G == 1 ? 5 : 3) k_tmu_sym(const __gr
 // before)
 __global__ void __launch_bounds__(256) k_sym_prepare(size_t total, const double *__restrict__ x,
                                                      unsigned long long *__restrict__ acc, unsigned *ctl,
-                                                     size_t group_words) {
+                                                     size_t ctl_stride) {
   x += (size_t)blockIdx.y * total;  // column groups
-  ctl += 2 * group_words * blockIdx.y;
+  ctl += ctl_stride * blockIdx.y;
   unsigned m = 0;
   for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += (size_t)gridDim.x * blockDim.x) {
     if (acc) {
@@ -433,64 +433,6 @@ __global__ void __launch_bounds__(FIN_TPB) k_tmu_sym_finish(
   }
 }
 
-// ---------------------------------------------------------------------------
-// All ordered pairs in FP64, one target per CTA, its 128 threads striding over
-// the sources (and the scaled pairs), the sums reduced in a fixed order.
-// Bound by the FP64 pipe at every size: the work of even the smallest system
-// spreads over all SMs (one target per thread left a 192-site system on two
-// SMs, 250 us per product; see launch_tmu_f64 for the sizes it serves).
-// ---------------------------------------------------------------------------
-template <int G, bool AMOEBA>
-__global__ void __launch_bounds__(128) k_tmu_rows(int n, const Pos64 *__restrict__ pos,
-                                                  const double *__restrict__ damp, const float2 *__restrict__ wa,
-                                                  const double *__restrict__ x, const double *__restrict__ alpha,
-                                                  bool dodiag, const int *__restrict__ ri,
-                                                  const int *__restrict__ src, const double *__restrict__ scale,
-                                                  double thr, float thr2m, double *__restrict__ y) {
-  constexpr int C = 3 * G;
-  __shared__ double s_sum[4][C];
-  const int j = blockIdx.x;
-  const Pos64 pt = pos[j];
-  const double at = AMOEBA ? damp[j] : 0.0;
-  const float2 wat = wa[j];
-  double acc[C];
-#pragma unroll
-  for (int c = 0; c < C; ++c) acc[c] = 0.0;
-  auto pair = [&](int i, double w) {
-    const Pos64 ps = pos[i];
-    const double dx = pt.x - ps.x, dy = pt.y - ps.y, dz = pt.z - ps.z;
-    const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-    double k3, k5;
-    dd_pair_f64<AMOEBA, true>(r2, pt.w, ps.w, at, AMOEBA ? damp[i] : 0.0, wat, wa[i], thr, thr2m, k3, k5);
-    const double k3w = k3 * w, k5w = 3.0 * w * k5;
-#pragma unroll
-    for (int r = 0; r < G; ++r) {
-      const double *mu = &x[((size_t)r * n + i) * 3];
-      const double mx = mu[0], my = mu[1], mz = mu[2];
-      const double f = k5w * fma(mx, dx, fma(my, dy, mz * dz));
-      acc[3 * r] = fma(f, dx, fma(-k3w, mx, acc[3 * r]));
-      acc[3 * r + 1] = fma(f, dy, fma(-k3w, my, acc[3 * r + 1]));
-      acc[3 * r + 2] = fma(f, dz, fma(-k3w, mz, acc[3 * r + 2]));
-    }
-  };
-  for (int i = threadIdx.x; i < n; i += 128)
-    if (i != j) pair(i, 1.0);
-  if (ri)
-    for (int k = ri[j] + threadIdx.x; k < ri[j + 1]; k += 128) pair(src[k], scale[k] - 1.0);
-#pragma unroll
-  for (int c = 0; c < C; ++c) {
-    for (int o = 16; o > 0; o >>= 1) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
-    if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5][c] = acc[c];
-  }
-  __syncthreads();
-  if (threadIdx.x < C) {
-    const int c = threadIdx.x;
-    const double e = ((s_sum[0][c] + s_sum[1][c]) + s_sum[2][c]) + s_sum[3][c];
-    const size_t o = ((size_t)(c / 3) * n + j) * 3 + (c % 3);
-    y[o] = dodiag ? x[o] / alpha[j] - e : -e;
-  }
-}
-
 template <int G, bool AMOEBA>
 struct SymLaunch {
   int resident = 0;
@@ -543,17 +485,6 @@ void launch_table(const SymTable &tab, unsigned *next, cudaStream_t st, bool zer
 
 // thr^2 with the relative safety margin of the FP32 damping pre-test
 float thr2_margin(const DevSites &s) { return (float)(s.damp_thr * s.damp_thr * (1.0 + 1e-5)); }
-
-template <int G>
-void launch_rows(const DevSites &s, const double *x, double *y, bool dodiag, cudaStream_t st) {
-  const int *ri = s.d2d_nnz ? s.d2d_ri : nullptr;
-  if (s.amoeba)
-    k_tmu_rows<G, true><<<s.n, 128, 0, st>>>(s.n, s.pol_pos, s.pol_a, s.pol_wa32, x, s.pol_alpha, dodiag, ri,
-                                             s.d2d_src, s.d2d_s, s.damp_thr, thr2_margin(s), y);
-  else
-    k_tmu_rows<G, false><<<s.n, 128, 0, st>>>(s.n, s.pol_pos, s.pol_a, s.pol_wa32, x, s.pol_alpha, dodiag, ri,
-                                              s.d2d_src, s.d2d_s, s.damp_thr, thr2_margin(s), y);
-}
 
 }  // namespace
 
@@ -684,7 +615,7 @@ void launch_tmu_f64_sym_groups(const DevSites &s, int nrhs, const double *x, dou
     add_launch_count(1);
     const int blocks = (int)std::min<size_t>((2 * nv + 255) / 256, 1216);
     k_sym_prepare<<<dim3(blocks, groups), 256, 0, st>>>(2 * nv, xg, nullptr,
-                                                        reinterpret_cast<unsigned *>(base + 6 * nv + 1), words);
+                                                        reinterpret_cast<unsigned *>(base + 6 * nv + 1), 2 * words);
     SymSlice sl[kMaxSymSlices];
     const int items = tmu_f64_sym_items(s, 2);
     for (int g = 0; g < groups; ++g) {
@@ -699,22 +630,12 @@ void launch_tmu_f64_sym_groups(const DevSites &s, int nrhs, const double *x, dou
   if (done < nrhs) launch_tmu_f64_sym(s, nrhs - done, x + done * nv, y + done * nv, dodiag, scratch, st);
 }
 
-// Below kSymMinSites a symmetric product is bound by the latency of its few
-// items (67 us at 900 and at 1,200 sites, 92 us at 2,001) and all ordered
-// pairs in FP64 are faster: 12 us at 192 sites, 61 at 900, 92 at 1,200,
-// 233 at 2,001 (one target per thread: 250 us at 192).
-void launch_tmu_f64(const DevSites &s, int nrhs, const double *x, double *y, bool dodiag, cudaStream_t st) {
-  if (s.n == 0) return;
-  for (int c = 0; c < nrhs;) {
-    const int g = nrhs - c >= 2 ? 2 : 1;
-    const size_t o = (size_t)c * s.n * 3;
-    add_launch_count(1);
-    if (g == 2)
-      launch_rows<2>(s, x + o, y + o, dodiag, st);
-    else
-      launch_rows<1>(s, x + o, y + o, dodiag, st);
-    c += g;
-  }
+// the largest high word of |x| of each column, words zeroed here
+void launch_max_words(int ncol, size_t nv, const double *x, unsigned *words, cudaStream_t st) {
+  add_launch_count(1);
+  cudaMemsetAsync(words, 0, ncol * sizeof(unsigned), st);
+  const int blocks = (int)std::min<size_t>((nv + 255) / 256, 1216);
+  k_sym_prepare<<<dim3(blocks, ncol), 256, 0, st>>>(nv, x, nullptr, words, 1);
 }
 
 // x = h + m + l with h a multiple of g and m of g 2^-23 (g = 2^-23 of the

@@ -1,6 +1,6 @@
 """The fused conjugate-gradient steps (csrc/pcg.cu): solves at the sizes where
 a launch shape changes (one CTA for the whole FP64 iteration up to 682 sites,
-the symmetric product from 1,000, four lanes or one per site in the finishing
+the symmetric product from 2,400, four lanes or one per site in the finishing
 passes around 32,768), every inner preconditioner and FP32 product, one and
 two columns, blocks of columns, and systems of different sizes and
 preconditioners sharing the launches of the multi-system engine.
@@ -123,12 +123,14 @@ def test_systems_sharing_launches(tmp_path):
 @pytest.mark.parametrize("kind,size", [("water", 340), ("water", 700), ("chain", 352)])
 @pytest.mark.parametrize("nf", [3, 9, 16])
 def test_column_groups(tmp_path, kind, size, nf):
-    """From 1,000 sites the products of several pairs of columns, and the
-    tiled FP32 products of several groups, share a launch (odd counts leave a
-    last column, 9 = 8 + 1)."""
+    """The products of several pairs of columns (symmetric and ordered), and
+    the tiled FP32 products of several groups, share a launch (odd counts
+    leave a last column, 9 = 8 + 1)."""
     g = load(tmp_path, kind, size)
     g.set_precision("mixed")
     fields = np.stack([field(g, 40 + k) for k in range(nf)])
-    ipd = np.asarray(g.set_external_fields_batch(fields)[0])
-    for k in range(nf):
-        assert residual(g, fields[k], ipd[k]) < 2 * TOL
+    for kernel in ("auto", "symmetric", "ordered"):
+        g.set_fp64_kernel(kernel)
+        ipd = np.asarray(g.set_external_fields_batch(fields)[0])
+        for k in range(nf):
+            assert residual(g, fields[k], ipd[k]) < 2 * TOL
