@@ -19,12 +19,12 @@ CSRC = os.path.join(HERE, "csrc")
 OBJ = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libommp_gb300.so")
 
-CU_SOURCES = ["kernels.cu", "engine.cu", "solvers.cu", "noalloc.cu", "tmu32.cu", "tmu_sym.cu", "tmu_rows.cu", "m2d.cu", "m2m.cu", "external.cu", "grad.cu",
+CU_SOURCES = ["kernels.cu", "engine.cu", "solvers.cu", "noalloc.cu", "tmu32.cu", "tmu32_rows.cu", "tmu_sym.cu", "tmu_rows.cu", "m2d.cu", "m2m.cu", "external.cu", "grad.cu",
               "grad_sym.cu", "qm_helper.cu", "fmm.cu", "fmm_near.cu",
               "fixedelec.cu", "dense.cu", "pcg.cu", "block_cg.cu", "multisolve.cu"]
 # per-file nvcc flags: the FP32 operators flush subnormals (plain MUFU rsqrt);
 # the double-single kernel fuses nothing implicitly (its FMAs are explicit)
-CU_EXTRA = {"tmu32.cu": ["-ftz=true"], "m2d.cu": ["-ftz=true", "--fmad=false"], "m2m.cu": ["-ftz=true", "--fmad=false"],
+CU_EXTRA = {"tmu32.cu": ["-ftz=true"], "tmu32_rows.cu": ["-ftz=true"], "m2d.cu": ["-ftz=true", "--fmad=false"], "m2m.cu": ["-ftz=true", "--fmad=false"],
             "tmu_sym.cu": ["-ftz=true", "--fmad=false"], "tmu_rows.cu": ["-ftz=true", "--fmad=false"],
             "fmm_near.cu": ["-ftz=true", "--fmad=false"],
             "grad_sym.cu": ["-ftz=true", "--fmad=false"], "external.cu": ["-ftz=true", "--fmad=false"]}

@@ -283,7 +283,7 @@ int System::upload_static() {
   ws_.x32 = x32_, ws_.r32 = r32_, ws_.p32 = p32_, ws_.h32 = h32_, ws_.z32 = z32_;
   ws_.scratch32 = scratch32_;
   ws_.scratch32_nsplit = f32_splits;
-  ws_.partial = partial_, ws_.partial_len = (size_t)gpu::kRedBlocks * 8, ws_.dots = dots_, ws_.hist = hist_;
+  ws_.partial = partial_, ws_.partial_len = (size_t)gpu::kRedBlocks * 32, ws_.dots = dots_, ws_.hist = hist_;
   ws_.cols = cols_, ws_.cols_h = cols_h_, ws_.scal_h = scal_h_;
   ws_.owned = false;
   d_.m2d_nnz = (int)m2d_pairs_.src.size();
@@ -1267,8 +1267,7 @@ int System::tmatvec_f32(const double *xh, double *yh, int nrhs) {
   gpu::launch_to_f32(nrhs * nv, p_, nullptr, p32_, st_);
   int kver = fp32_kernel_ ? fp32_kernel_ : 2;
   if (kver == 3 && ensure_sym_scratch() != kOk) kver = 2;
-  const int split = kver == 2 ? nsplit_tmu32_ : gpu::tmu_pick_split(d_, nrhs, gpu::sm_count(), true);
-  gpu::launch_tmu_f32(d_, nrhs, p32_, h32_, scratch32_, split, st_, kver == 3 ? 2 : 4, kver, sym_scratch_);
+  gpu::launch_tmu_f32(d_, nrhs, p32_, h32_, scratch32_, nsplit_tmu32_, st_, kver == 3 ? 2 : 4, kver, sym_scratch_);
   std::vector<float> tmp(nrhs * nv);
   cudaMemcpyAsync(tmp.data(), h32_, tmp.size() * sizeof(float), cudaMemcpyDeviceToHost, st_);
   int st = check(cudaStreamSynchronize(st_), "tmatvec_f32");

@@ -6,10 +6,6 @@
 //                    the scaled-pair correction pass: for every listed pair
 //                    (s - 1) * f_ij is added, which equals the reference's
 //                    "skip when s == 0, multiply when s != 1" rule.
-//   k_tmu            FP32 dipole-dipole field T.mu, target-outer like
-//                    field_extD2D (src/mod_electrostatics.F90:2068-2109), with
-//                    compensated (Kahan) cross-tile sums; the products of FP64
-//                    accuracy are in tmu_sym.cu.
 //   k_tmu_finish     partial reduction, u-scale correction, sign and the
 //                    1/alpha diagonal of TMatVec_otf/TMatVec_diag
 //                    (src/mod_polarization.F90:459-504).
@@ -30,8 +26,7 @@ namespace ommp {
 namespace gpu {
 
 namespace {
-constexpr int TPB = 128;   // targets per CTA
-constexpr int TILE = 128;  // sources per shared-memory tile
+constexpr int TILE = 128;  // sources per tile of the FP32 operator
 
 // Reduce partials and apply the scaled-pair corrections; out [n_ipd][n][3]
 // with set 0 = D (direct field, d-scale) and set 1 = P (p-scale) for AMOEBA.
@@ -79,83 +74,6 @@ __global__ void k_m2d_finish(int n, int nsplit, const double *__restrict__ parti
     }
   } else {
     for (int c = 0; c < 3; ++c) out[(size_t)j * 3 + c] = eP[c];
-  }
-}
-
-// partial[split][rhs][j][3] = E_dd(x)_j over the split's source range.
-template <int NRHS, bool AMOEBA>
-__global__ void __launch_bounds__(TPB) k_tmu(int n, const float4 *__restrict__ pos,
-                                             const float *__restrict__ damp, const float *__restrict__ x,
-                                             float *__restrict__ partial, int per_split, float thr) {
-  __shared__ float4 s_pos[TILE];
-  __shared__ float s_a[TILE];
-  __shared__ float s_mu[NRHS * 3][TILE];
-  const int j = blockIdx.x * TPB + threadIdx.x;
-  const bool valid = j < n;
-  float4 pt;
-  if (valid) {
-    pt = pos[j];
-  } else {
-    pt.x = pt.y = pt.z = pt.w = 0.f;
-  }
-  const float at = (valid && AMOEBA) ? damp[j] : 0.f;
-  float acc[NRHS * 3], sum[NRHS * 3], comp[NRHS * 3];
-#pragma unroll
-  for (int c = 0; c < NRHS * 3; ++c) sum[c] = comp[c] = 0.f;
-  const int s0 = blockIdx.y * per_split;
-  const int s1 = min(n, s0 + per_split);
-  for (int t0 = s0; t0 < s1; t0 += TILE) {
-    __syncthreads();
-    {
-      int k = threadIdx.x;  // TILE == TPB
-      int i = t0 + k;
-      if (i < s1) {
-        s_pos[k] = pos[i];
-        s_a[k] = AMOEBA ? damp[i] : 0.f;
-#pragma unroll
-        for (int r = 0; r < NRHS; ++r)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) s_mu[r * 3 + c][k] = x[((size_t)r * n + i) * 3 + c];
-      }
-    }
-    __syncthreads();
-    const int cnt = min(TILE, s1 - t0);
-#pragma unroll
-    for (int c = 0; c < NRHS * 3; ++c) acc[c] = 0.f;
-    if (valid) {
-#pragma unroll 2
-      for (int k = 0; k < cnt; ++k) {
-        if (t0 + k == j) continue;
-        const float4 ps = s_pos[k];
-        float dx = pt.x - ps.x, dy = pt.y - ps.y, dz = pt.z - ps.z;
-        float r2 = dx * dx + dy * dy + dz * dz;
-        float k3, k5x3;
-        dd_kernel<float, AMOEBA>(r2, pt.w, ps.w, at, s_a[k], thr, k3, k5x3);
-#pragma unroll
-        for (int r = 0; r < NRHS; ++r) {
-          float mx = s_mu[r * 3 + 0][k], my = s_mu[r * 3 + 1][k], mz = s_mu[r * 3 + 2][k];
-          float f = k5x3 * (mx * dx + my * dy + mz * dz);
-          acc[r * 3 + 0] += f * dx - k3 * mx;
-          acc[r * 3 + 1] += f * dy - k3 * my;
-          acc[r * 3 + 2] += f * dz - k3 * mz;
-        }
-      }
-    }
-    // compensated (Kahan) cross-tile accumulation
-#pragma unroll
-    for (int c = 0; c < NRHS * 3; ++c) {
-      const float y = acc[c] - comp[c];
-      const float t = sum[c] + y;
-      comp[c] = (t - sum[c]) - y;
-      sum[c] = t;
-    }
-  }
-  if (valid) {
-#pragma unroll
-    for (int r = 0; r < NRHS; ++r)
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        partial[(((size_t)blockIdx.y * NRHS + r) * n + j) * 3 + c] = sum[r * 3 + c];
   }
 }
 
@@ -574,41 +492,13 @@ void launch_m2d_finish(const DevSites &s, double *out, const double *partial, in
 }
 
 // ---- T.mu -----------------------------------------------------------------
-int tmu_pick_split(const DevSites &s, int nrhs, int sms, bool fp32) {
-  (void)nrhs;
-  (void)fp32;
-  int tblocks = (s.n + TPB - 1) / TPB;
-  int want = 4 * sms;
-  int split = (want + tblocks - 1) / tblocks;
-  int maxsplit = (s.n + TILE - 1) / TILE;
-  if (split > maxsplit) split = maxsplit;
-  if (split < 1) split = 1;
-  return split;
-}
-
 int tmu32_max_split(const DevSites &s, int sms) {
-  int a = tmu_pick_split(s, 2, sms, true), b = tmu32_pick_split(s, sms);
-  int tiles = (s.n + TILE - 1) / TILE;
-  int m = 2 * (a > b ? a : b);
-  if (m > tiles) m = tiles;
-  return m < 1 ? 1 : m;
+  const int tiles = (s.n + TILE - 1) / TILE;
+  return std::max(1, std::min(2 * tmu32_pick_split(s, sms), tiles));
 }
 
 size_t tmu_scratch_doubles(const DevSites &s, int nrhs, int nsplit) {
   return (size_t)nsplit * nrhs * s.n * 3;
-}
-
-template <int NRHS>
-static void tmu_allpairs(const DevSites &s, const float *x, float *partial, int nsplit, cudaStream_t st) {
-  add_launch_count(1);
-  int tiles = (s.n + TILE - 1) / TILE;
-  int per = ((tiles + nsplit - 1) / nsplit) * TILE;
-  dim3 grid((s.n + TPB - 1) / TPB, nsplit);
-  const float thr = (float)s.damp_thr;
-  if (s.amoeba)
-    k_tmu<NRHS, true><<<grid, TPB, 0, st>>>(s.n, s.pol_pos32, s.pol_a32, x, partial, per, thr);
-  else
-    k_tmu<NRHS, false><<<grid, TPB, 0, st>>>(s.n, s.pol_pos32, s.pol_a32, x, partial, per, thr);
 }
 
 // Columns per launch: the widest of 8/4/2/1 not above what is left and gmax.
@@ -617,29 +507,16 @@ inline int column_group(int left, int gmax) {
   return g >= 8 ? 8 : (g >= 4 ? 4 : (g >= 2 ? 2 : 1));
 }
 
+// the tiled kernel on columns in groups sharing the pair geometry; every
+// group has its own [split][g][n][3] block of partials, one after the other
 static void tmu_dispatch(const DevSites &s, int nrhs, const float *x, float *partial, int nsplit, int gmax,
-                         cudaStream_t st, int kver) {
-  // process the columns in groups sharing the pair geometry; every group
-  // has its own [split][g][n][3] block of partials, one after the other
-  int done = 0;
-  while (done < nrhs) {
-    int g = column_group(nrhs - done, gmax);
-    size_t xo = (size_t)done * s.n * 3;
-    float *pg = partial + (size_t)nsplit * done * s.n * 3;
-    if (kver == 2) {
-      const int groups = (nrhs - done) / g;
-      add_launch_count(1);
-      launch_tmu32_pairs(s, g, groups, x + xo, pg, nsplit, st);
-      done += g * groups;
-      continue;
-    }
-    done += g;
-    switch (g) {
-      case 8: tmu_allpairs<8>(s, x + xo, pg, nsplit, st); break;
-      case 4: tmu_allpairs<4>(s, x + xo, pg, nsplit, st); break;
-      case 2: tmu_allpairs<2>(s, x + xo, pg, nsplit, st); break;
-      default: tmu_allpairs<1>(s, x + xo, pg, nsplit, st); break;
-    }
+                         cudaStream_t st) {
+  for (int done = 0; done < nrhs;) {
+    const int g = column_group(nrhs - done, gmax), groups = (nrhs - done) / g;
+    const size_t xo = (size_t)done * s.n * 3;
+    add_launch_count(1);
+    launch_tmu32_pairs(s, g, groups, x + xo, partial + nsplit * xo, nsplit, st);
+    done += g * groups;
   }
 }
 
@@ -660,8 +537,14 @@ int launch_tmu_f32(const DevSites &s, int nrhs, const float *x, float *y, float 
                    int gmax, int kver, double *sym_scratch, bool prepared, double *part, int max_part) {
   if (s.n == 0) return 0;
   const size_t nv = 3 * (size_t)s.n;
+  if (kver == 1) {
+    const int parts = tmu32_rows_parts(s.n);
+    if (parts > max_part) part = nullptr;
+    launch_tmu32_rows(s, nrhs, gmax, x, y, part, st);
+    return part ? parts : 0;
+  }
   const bool sym = kver == 3 && sym_scratch;
-  if (!sym) tmu_dispatch(s, nrhs, x, scratch, nsplit, gmax, st, kver);
+  if (!sym) tmu_dispatch(s, nrhs, x, scratch, nsplit, gmax, st);
   int npart = 0;
   std::vector<F32Finish> fins;
   for (int c = 0; c < nrhs;) {

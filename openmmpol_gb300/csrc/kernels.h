@@ -77,7 +77,6 @@ void launch_m2d_finish(const DevSites &s, double *out, const double *partial, in
 
 // y = T x (dodiag) or y = -E_dd(x) (no diagonal); x,y [nrhs][n][3], FP64.
 size_t tmu_scratch_doubles(const DevSites &s, int nrhs, int nsplit);
-int tmu_pick_split(const DevSites &s, int nrhs, int sm_count, bool fp32);
 // All ordered pairs to FP64 accuracy in one launch (tmu_rows.cu); words: the
 // largest high word of each column (launch_max_words).  part: partial sums of
 // x.y, tmu_rows_parts per column (0: this size gives none).
@@ -138,10 +137,14 @@ constexpr int kFmmNearSplit = 9;
 void launch_fmm_near(const FmmNearArgs &a, const double *x, const unsigned *word, double *partial, cudaStream_t st);
 // coordinates x [n][3] about a centre as three floats each, out [3][n]
 void split_coordinates(const double *x, int n, double centre[3], float4 *out);
+// The pairwise FP32 product (tmu32_rows.cu): columns in groups of up to gmax
+// (4); part: partial sums of x.y, tmu32_rows_parts per column
+int tmu32_rows_parts(int n);
+void launch_tmu32_rows(const DevSites &s, int ncol, int gmax, const float *x, float *y, double *part, cudaStream_t st);
 // FP32 inner operator with compensated cross-tile sums; x,y float.  Columns
 // go through the pair kernel in groups of up to gmax (8, 4, 2 or 1) sharing
 // the pair geometry; scratch holds nsplit * nrhs * n * 3 floats.
-// kver 1: one target per thread, per-pair damping test (kernels.cu);
+// kver 1: lanes over the sources, per-pair damping test (tmu32_rows.cu; scratch unused);
 // kver 2: the tile-classified kernel of tmu32.cu.
 // kver 3: the symmetric kernel of tmu32.cu (each unordered pair once),
 // columns in groups of gmax (1 or 2), sums in sym_scratch (laid out as for

@@ -562,6 +562,7 @@ void launch_cg_dot(int ncol, int nb, size_t nv, const T *a, const T *b, double *
   k_cg_dot<T><<<dim3(nb, ncol), TPB, 0, st>>>(nb, nv, a, b, part);
 }
 template void launch_cg_dot<double>(int, int, size_t, const double *, const double *, double *, cudaStream_t);
+template void launch_cg_dot<float>(int, int, size_t, const float *, const float *, double *, cudaStream_t);
 
 F32Finish f32_finish(const DevSites &s, int g, const float *x, float *y) {
   F32Finish j{};

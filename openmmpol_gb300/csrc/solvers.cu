@@ -70,7 +70,7 @@ int System::ensure_batch_ws(int ncol, int nf) {
   bad |= walloc(w.x32, ncol * nv) | walloc(w.r32, ncol * nv) | walloc(w.p32, ncol * nv) |
          walloc(w.h32, ncol * nv) | walloc(w.z32, ncol * nv);
   bad |= walloc(w.scratch32, (size_t)s0 * ncol * nv);
-  w.partial_len = (size_t)gpu::kRedBlocks * std::max(ncol, nf);
+  w.partial_len = 4 * (size_t)gpu::kRedBlocks * std::max(ncol, nf);
   bad |= walloc(w.partial, w.partial_len) |
          walloc(w.dots, 3 * (size_t)ncol + nf) | walloc(w.cols, ncol + 1);
   // block CG buffers (sized for the widest block)
@@ -303,26 +303,29 @@ int System::f32_product(Workspace &w, int ncol, const F32Shape &sh, bool prepare
                              part, max_part);
 }
 
-// The launch shape by size and columns (forced kernels keep their own shape).
-// Widest column groups.  Kernel by the measured time of one product with its
-// finishing pass, us (pairwise / tiled / symmetric):
-//   sites        999        2,001        3,003        4,200        6,000         9,003
-//   1 column   28/31/-    30/33/-    36/36/48    54/42/49    90/77/64   163/120/86
-//   2 columns  31/36/-    34/35/-    42/41/61    65/52/64   116/98/94  209/160/129
-//   4 columns  32/25/-    38/30/-    54/43/-     87/61/137  152/111/186 292/207/260
-//   8 columns  36/37/-    48/46/-    73/63/-    129/102/-   237/190/-   472/350/-
-// (15,000 sites, 8 columns: tiled 846, symmetric 1,088.)  Source splits: the
-// finer of the two candidates, as fine as the tiles allow, won everywhere.
+// The launch shape by size and columns (forced kernels keep their own shape):
+// widest column groups, kernel by the measured time of an inner iteration (all
+// its steps), us (pairwise / tiled / symmetric):
+//   sites       192       999      2,001      3,003      4,200      6,000        9,003
+//   1 column  31/53/48  39/59/53  45/61/56   54/65/60   67/73/65   94/95/82   166/159/119
+//   2         34/58/53  41/64/62  51/66/64   61/71/71   80/83/86  110/112/113 206/189/162
+//   4         34/48     45/56     58/63      74/74     128/94     164/138     318/247
+//   8         37/67     49/69     85/79     114/95     184/141    294/213     555/408
+//   24        40/68     72/79    152/130    251/199    415/310    747/537    1549/1095
+// (15,000 sites, 8 columns, the product alone: tiled 846, symmetric 1,088.)
+// The tiled kernel's source splits: the finer of two candidates, as fine as the
+// tiles allow, won everywhere.
 int System::tune_f32(Workspace &w, int ncol, F32Shape &shape) {
   auto it = f32_tune_.find(ncol);
   if (it != f32_tune_.end() && it->second.nsplit <= w.scratch32_nsplit) {
     shape = it->second;
     return kOk;
   }
-  const int n = d_.n, sms = gpu::sm_count();
+  const int n = d_.n;
   F32Shape pick{ncol >= 8 ? 8 : ncol >= 4 ? 4 : ncol >= 2 ? 2 : 1, 1, fp32_kernel_};
   if (fp32_kernel_ == 0) {
-    pick.kver = pick.g >= 4 ? 2 : n < 3000 ? 1 : n < 5000 ? 2 : 3;
+    const int rows = ncol == 1 ? 3600 : ncol < 4 ? 4500 : ncol < 8 ? 3000 : 1500;
+    pick.kver = n < rows ? 1 : pick.g >= 4 ? 2 : 3;
     if (pick.kver == 3 && ensure_sym_scratch() != kOk) pick.kver = 2;
   } else if (fp32_kernel_ == 3) {
     const int st = ensure_sym_scratch();
@@ -330,9 +333,10 @@ int System::tune_f32(Workspace &w, int ncol, F32Shape &shape) {
   }
   if (pick.kver == 3) {
     pick.g = std::min(pick.g, 2);
+  } else if (pick.kver == 1) {
+    pick.g = std::min(pick.g, 4);
   } else {
-    const int split = pick.kver == 1 ? gpu::tmu_pick_split(d_, ncol, sms, true) : gpu::tmu32_pick_split(d_, sms);
-    pick.nsplit = std::max(1, std::min({2 * split, w.scratch32_nsplit, (n + 127) / 128}));
+    pick.nsplit = std::max(1, std::min({2 * gpu::tmu32_pick_split(d_, gpu::sm_count()), w.scratch32_nsplit, (n + 127) / 128}));
   }
   f32_tune_[ncol] = pick;
   shape = pick;
@@ -386,6 +390,7 @@ int System::pcg32_ws(Workspace &w, int ncol, int max_it, double eta) {
   job.init = 0;
   auto iteration = [&]() {
     job.na = f32_product(w, ncol, shape, prepared, job.pa, share);
+    if (job.na == 0) gpu::launch_cg_dot(ncol, job.na = job.nb, 3 * (size_t)n, w.h32, w.p32, job.pa, st_);
     gpu::launch_cg_steps(&job, 1, st_);
   };
   int it = 0;

@@ -38,31 +38,6 @@ namespace {
 constexpr int T32_TPB = 128;   // threads per CTA
 constexpr int T32_TILE = 128;  // sources per shared-memory tile (= tile-box granularity)
 
-template <bool AMOEBA>
-__device__ __forceinline__ void damped_factors(float r2, float wt, float ws, float at, float as, float thr,
-                                               float &k3, float &k5) {
-  float rinv = rsqrtf(r2);
-  float ir2 = rinv * rinv;
-  k3 = rinv * ir2;
-  k5 = k3 * ir2;
-  float u = r2 * rinv * (wt * ws);
-  if (AMOEBA) {
-    float au3 = fminf(at, as) * u * u * u;
-    if (au3 < thr) {
-      float e = __expf(-au3);
-      k3 *= 1.f - e;
-      k5 *= 1.f - (1.f + au3) * e;
-    }
-  } else {
-    if (u < 1.f) {
-      float u3 = u * u * u;
-      float u4 = u3 * u;
-      k3 *= 4.f * u3 - 3.f * u4;
-      k5 *= u4;
-    }
-  }
-}
-
 // partial[split][g][j][3] over the split's sources.  TPT targets per thread:
 // target t of thread x is blockIdx.x * TPB * TPT + t * TPB + x.
 template <int G, int TPT, bool AMOEBA>

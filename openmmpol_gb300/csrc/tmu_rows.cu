@@ -122,6 +122,7 @@ __device__ __forceinline__ dsf add(dsf a, dsf b) {
 template <int G, bool AMOEBA, int T, int WT>
 __global__ void __launch_bounds__(TPB) k_rows_ds(const __grid_constant__ RowsArgs a) {
   constexpr int R = Rows<G>::R, C = 3 * G, WS = 4 / WT;
+  static_assert(WT * T * C <= TPB, "one thread per value of the CTA's targets");
   __shared__ float4 s_rec[R][TPB];
   __shared__ float2 s_wa[TPB];
   __shared__ int s_list[4][T][LIST];
