@@ -36,10 +36,16 @@
 // without a polarizable site are skipped.  The dipoles are scaled by a power
 // of two as in the products.
 //
-// 30,000 sites: 76 -> 37 ms in the mixed modes, 330 ms in FP64 before; 90,000:
-// 668 -> 332 ms (2.95 s in FP64).  Error against 64 bits 7e-15 to 8e-15 (before
-// 2.7e-14 in FP64, 3e-14 to 6e-14 in double-single).  255 registers without
-// spills at 2 CTAs per SM: bound by FP32 issue and its latency at 8 warps.
+// Products and sums keep their low parts unrenormalised, the accumulators are
+// renormalised per pair: renormalising every product cost 7 % for errors of
+// 7.5e-15.
+//
+// 30,000 sites: 76 -> 35 ms in the mixed modes, 330 ms in FP64 before; 90,000:
+// 668 -> 311 ms (2.95 s in FP64).  Error against 64 bits 0.95e-14 to 1.2e-14
+// (before 2.7e-14 in FP64, 3e-14 to 6e-14 in double-single).  255 registers
+// without spills at 2 CTAs per SM: bound by FP32 issue (54 % of the issue slots
+// at 6,000 sites) with 8 warps, a quarter of whose stalls is the fetch of the
+// 2,600-instruction step.
 //
 // Built with --fmad=false -ftz=true: every FMA is explicit.
 #include <algorithm>
@@ -76,18 +82,16 @@ __device__ __forceinline__ double neg(double a) { return -a; }
 __device__ __forceinline__ dsf neg(dsf a) { return {-a.h, -a.l}; }
 __device__ __forceinline__ double twice(double a) { return a + a; }
 __device__ __forceinline__ dsf twice(dsf a) { return {a.h + a.h, a.l + a.l}; }
-__device__ __forceinline__ double norm(double a) { return a; }
-__device__ __forceinline__ dsf norm(dsf a) { return dsp_norm(a); }
 __device__ __forceinline__ double sub(double a, double b) { return a - b; }
 __device__ __forceinline__ dsf sub(dsf a, dsf b) {
   const dsf s = two_sum(a.h, -b.h);
-  return dsp_norm({s.h, s.l + (a.l - b.l)});
+  return {s.h, s.l + (a.l - b.l)};
 }
 __device__ __forceinline__ double dot(const double *a, const double *b) {
   return fma(a[0], b[0], fma(a[1], b[1], a[2] * b[2]));
 }
 __device__ __forceinline__ dsf dot(const dsf *a, const dsf *b) {
-  return dsp_norm(dsp_dot(a[0], a[1], a[2], b[0], b[1], b[2]));
+  return dsp_dot(a[0], a[1], a[2], b[0], b[1], b[2]);
 }
 // Q v, Q = xx, xy, yy, xz, yz, zz
 template <typename T>
@@ -139,21 +143,18 @@ __device__ __forceinline__ void pair_force(const Site<T, true> &t, const Site<T,
   mad(x1, neg(k.D), st);
   mad(x2, k.C, bs);
   mad(x2, k.D, ss);
-  T X = mul(as, norm(x1));
-  mad(X, at, norm(x2));
+  T X = mul(as, x1);
+  mad(X, at, x2);
   mad(X, nF, dot(t.mp, s.p));
   mad(X, nF, dot(s.mp, t.p));
   mad(X, H2, dot(Tt, s.p));
   mad(X, neg(H2), dot(Ts, t.p));
-  X = norm(X);
   // p_s, p_t
   T ws = mul(k.K, t.q), wt = mul(neg(k.K), s.q);
   mad(ws, nF, bt);
   mad(ws, k.H, st);
   mad(wt, nF, bs);
   mad(wt, neg(k.H), ss);
-  ws = norm(ws);
-  wt = norm(wt);
   T Rt[3], Rs[3];
   apply(t.Q, s.p, Rt);
   apply(s.Q, t.p, Rs);
@@ -166,8 +167,8 @@ __device__ __forceinline__ void pair_force(const Site<T, true> &t, const Site<T,
     mad(f[c], X, n[c]);
     mad(f[c], ws, s.p[c]);
     mad(f[c], wt, t.p[c]);
-    mad(f[c], as, norm(u));
-    mad(f[c], at, norm(v));
+    mad(f[c], as, u);
+    mad(f[c], at, v);
     mad(f[c], F52, sub(Rs[c], Rt[c]));
   }
   T u[3], w[3];
@@ -175,12 +176,10 @@ __device__ __forceinline__ void pair_force(const Site<T, true> &t, const Site<T,
   for (int c = 0; c < 3; ++c) {
     T v = mul(C2, Tt[c]);
     mad(v, neg(k.G), t.m[c]);
-    u[c] = mul(as, norm(v));
+    u[c] = mul(as, v);
     mad(u[c], neg(F2), Rt[c]);
-    u[c] = norm(u[c]);
     w[c] = mul(k.K, t.m[c]);
     mad(w[c], neg(F2), Tt[c]);
-    w[c] = norm(w[c]);
   }
   add_cross(u, n, tau_t);
   add_cross(w, s.p, tau_t);
@@ -188,12 +187,10 @@ __device__ __forceinline__ void pair_force(const Site<T, true> &t, const Site<T,
   for (int c = 0; c < 3; ++c) {
     T v = mul(C2, Ts[c]);
     mad(v, k.G, s.m[c]);
-    u[c] = mul(neg(at), norm(v));
+    u[c] = mul(neg(at), v);
     mad(u[c], F2, Rs[c]);
-    u[c] = norm(u[c]);
     w[c] = mul(k.K, s.m[c]);
     mad(w[c], F2, Ts[c]);
-    w[c] = norm(w[c]);
   }
   add_cross(u, n, tau_s);
   add_cross(w, t.p, tau_s);
@@ -223,10 +220,8 @@ __device__ __forceinline__ void pair_force(const Site<T, false> &t, const T *p2,
   mad(X, mul(k.G, s.q), at);
   mad(X, neg(k.F), dot(p2, s.p));
   mad(X, mul(k.C, a2), as);
-  X = norm(X);
   T ws = mul(k.K, t.q);
   mad(ws, neg(k.F), a2);
-  ws = norm(ws);
   const T wt = mul(neg(k.K), s.q), w2 = mul(neg(k.F), as);
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
@@ -243,7 +238,6 @@ __device__ __forceinline__ void delta_force(const T *dt, const T *ds, const T *n
   const T at = dot(dt, n), as = dot(ds, n);
   T X = mul(k.F, dot(dt, ds));
   mad(X, mul(neg(k.C), at), as);
-  X = norm(X);
   const T ws = mul(k.F, at), wt = mul(k.F, as);
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
@@ -503,7 +497,7 @@ __global__ void __launch_bounds__(TILE, AMOEBA ? 2 : 4) k_grad_sym(const __grid_
             queued += __popc(mask);
           }
           const DspUnit u = dsp_unit(d, y);
-          const dsf n[3] = {dsp_norm(u.x), dsp_norm(u.y), dsp_norm(u.z)};
+          const dsf n[3] = {u.x, u.y, u.z};
           const float w3 = dsp_power<3>(u.eps), w5 = dsp_power<5>(u.eps), w7 = dsp_power<7>(u.eps),
                       w9 = dsp_power<9>(u.eps);
           const float y2 = y * y, y2l = fmaf(y, y, -y2);
