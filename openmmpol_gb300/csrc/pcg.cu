@@ -37,8 +37,9 @@ struct Table {
 };
 
 // The FP64 pipe issues a warp's instruction every 16 cycles per SM, so the
-// sums here are taken by as few warps as possible, FP32 vectors are updated
-// without it, and 1 / alpha comes from memory.
+// sums here are taken by as few warps as possible, one thread divides for its
+// block, FP32 vectors are updated without that pipe, and 1 / alpha comes from
+// memory.
 
 // sum over the block, the same value and order in every thread; nwarp <= 32
 __device__ __forceinline__ double block_sum(double v, double *sh, int nwarp) {
@@ -73,6 +74,16 @@ __device__ __forceinline__ double partial_sum(const double *part, int n, double 
   return s;
 }
 
+// a / b (0 when b is 0) by one thread, in every thread
+__device__ __forceinline__ double block_ratio(double a, double b, double *sh) {
+  __syncthreads();  // sh may still be read
+  if (threadIdx.x == 0) sh[0] = b != 0.0 ? a / b : 0.0;
+  __syncthreads();
+  const double q = sh[0];
+  __syncthreads();
+  return q;
+}
+
 // x + a p.  FP32 vectors: a as two floats, the products and the sum with
 // their rounding errors, one rounding of the result as from FP64 arithmetic
 struct Scalar {
@@ -102,7 +113,7 @@ __global__ void __launch_bounds__(TPB) k_cg_step(const __grid_constant__ Table<C
     const double ph = partial_sum(jb.pa + (size_t)k * jb.na, jb.na, sh);
     const bool quick = act && fabs(ph) < jb.eps;
     const double rho = col.gnew;
-    al = act && !quick ? rho / ph : 0.0;
+    al = block_ratio(act && !quick ? rho : 0.0, ph, sh);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       col.alpha = al;
       if (act) {
@@ -271,7 +282,9 @@ __global__ void __launch_bounds__(TPB) k_cg_dir(const __grid_constant__ Table<Cg
   const double rho = partial_sum(jb.pb + (size_t)k * jb.nb, jb.nb, sh);
   const double gold = jb.init ? 0.0 : col.gold;
   const Scalar mal(jb.init ? 0.0 : -col.alpha);
-  const double beta = gold != 0.0 ? rho / gold : 0.0;
+  const double beta = block_ratio(rho, gold, sh);
+  // one thread closes the column while the others go on
+  if (blockIdx.x == 0 && threadIdx.x == TPB - 32) cg_close(jb, k, rho, beta);
   const T bt = (T)beta;
   const size_t nv = 3 * (size_t)jb.n, off = (size_t)k * nv;
   T *p = jb.p + off, *r = jb.r + off;
@@ -296,13 +309,13 @@ __global__ void __launch_bounds__(TPB) k_cg_dir(const __grid_constant__ Table<Cg
       if ((threadIdx.x & 31) == 0 && mx) atomicMax(jb.emax + k * jb.emax_stride, mx);
     }
   }
-  if (blockIdx.x == 0 && threadIdx.x == 0) cg_close(jb, k, rho, beta);
 }
 
 // The whole FP64 iteration after the product in one CTA per column, up to
 // kCgSmallSites sites: up to 2 elements of each vector per thread, in
 // registers.  Bound by the FP64 pipe of its one SM
-// and the latency of its two sums: 12 us at 192 sites, seven launches before.
+// and the latency of its two sums: about 10 us at 192 sites (12 with the
+// divisions in every thread), seven launches before.
 constexpr int SMALL_TPB = 1024, SMALL_PER = 2;
 __global__ void __launch_bounds__(SMALL_TPB) k_cg_small(const __grid_constant__ CgJob<double> jb) {
   __shared__ double sh[SMALL_TPB / 32];
@@ -328,7 +341,7 @@ __global__ void __launch_bounds__(SMALL_TPB) k_cg_small(const __grid_constant__ 
   const double ph = block_sum(acc, sh, blockDim.x / 32);
   const double gold = col.gnew;
   const bool quick = fabs(ph) < jb.eps;
-  const double al = quick ? 0.0 : gold / ph;
+  const double al = block_ratio(quick ? 0.0 : gold, ph, sh);
   acc = 0.0;
   if (!quick) {
 #pragma unroll
@@ -343,7 +356,15 @@ __global__ void __launch_bounds__(SMALL_TPB) k_cg_small(const __grid_constant__ 
     }
   }
   const double rho = block_sum(acc, sh, blockDim.x / 32);
-  const double beta = rho / gold;
+  const double beta = block_ratio(rho, gold, sh);
+  // every thread has read the scalars
+  if (threadIdx.x == blockDim.x - 32) {
+    col.alpha = al;
+    col.gold = gold;
+    col.gama = ph;
+    if (quick) col.quick = 1;
+    cg_close(jb, k, rho, beta);
+  }
   __shared__ unsigned s_max;
   unsigned mx = 0;
   if (threadIdx.x == 0) s_max = 0;
@@ -358,18 +379,12 @@ __global__ void __launch_bounds__(SMALL_TPB) k_cg_small(const __grid_constant__ 
       }
     }
   }
-  __syncthreads();  // every thread has read the scalars
+  if (!jb.emax) return;
+  __syncthreads();
   mx = __reduce_max_sync(0xffffffffu, mx);
   if ((threadIdx.x & 31) == 0) atomicMax(&s_max, mx);
   __syncthreads();
-  if (threadIdx.x == 0) {
-    if (jb.emax) jb.emax[k * jb.emax_stride] = s_max;
-    col.alpha = al;
-    col.gold = gold;
-    col.gama = ph;
-    if (quick) col.quick = 1;
-    cg_close(jb, k, rho, beta);
-  }
+  if (threadIdx.x == 0) jb.emax[k * jb.emax_stride] = s_max;
 }
 
 // partial sums of a.b per column
