@@ -18,14 +18,14 @@ in the reference (src/mod_electrostatics.F90:1487-1596, M2D_done cache).
   and the permanent field from the fast multipole method (default order 10),
   with their error against it.
 * ``roofline``: the dominant pair kernel, its algorithmic operations over its
-  CUDA-event time against its pipe's peak measured in the same run: FP64
-  instructions of the symmetric FP64 product (32 per unordered pair and
-  right-hand side, both directions), FP32 instructions of the double-single
-  product; the conventional 45 flop per ordered pair is reported beside.
+  CUDA-event time against its pipe's peak measured in the same run: FP32
+  instructions of the product of FP64 accuracy (289 per unordered pair and
+  right-hand side, both directions, double-single) or of the FP32 product; the
+  conventional 45 flop per ordered pair is reported beside.
 * ``geomgrad``: the polarization-energy gradient (ommp_polelec_geomgrad) on
-  the solved system: calls/s with the double-single pair passes of the mixed
-  modes and with the FP64 pass, each against its pipe, their difference, and
-  the oracle's gradient on the host cores (3,000-molecule sample scaled).
+  the solved system: calls/s in a mixed and in the fp64 mode (the same
+  double-single pair pass) against the FP32 pipe, their difference, and the
+  oracle's gradient on the host cores (3,000-molecule sample scaled).
 * ``cpu_baseline``: the C/OpenMP oracle (restatement of the reference's
   OpenMP path) timed on two whole T.mu products of the box on all host cores,
   scaled to a solve by the oracle's own product count (20).
@@ -55,14 +55,12 @@ sys.path.insert(0, ROOT)
 
 METRIC = "induced-dipole solves/s (mixed FP32/FP64 at <=1e-7 rel. error vs FP64)"
 FLOP_PER_PAIR = 45.0  # per ordered T.mu pair and right-hand side (conventional count)
-# FP64 operations (an FMA counts once) per unordered pair and right-hand side
-# of the symmetric FP64 product (k_tmu_sym, openmmpol_gb300/csrc/kernels.cu,
-# both directions): 3 coordinate differences, r^2 (3), the Newton step of the
-# reciprocal square root (3), r^-2 / r^-3 / r^-5 (3) and per direction mu.d
-# (3), the field factor (1) and six accumulations (6); the FP32 seed, the
-# conversions and the damping pre-test run on other pipes
+# FP64 operations (an FMA counts once) that an unordered pair of T.mu takes on
+# the FP64 pipe, both directions: 3 coordinate differences, r^2 (3), the Newton
+# step of the reciprocal square root (3), r^-2 / r^-3 / r^-5 (3) and per
+# direction mu.d (3), the field factor (1) and six accumulations (6)
 FP64_SYM_OPS_PER_PAIR = 32.0
-SYM_MIN_SITES = 2048  # the engine's automatic choice of the symmetric product
+SYM_MIN_SITES = 2400  # the engine's automatic choice of the symmetric product
 # FP32 lane operations (an FMA counts once, a paired instruction twice) per
 # unordered pair and right-hand side of the symmetric FP32 product
 # (k_tmu32_sym, openmmpol_gb300/csrc/tmu32.cu): 3 coordinate differences, r^2
@@ -70,27 +68,16 @@ SYM_MIN_SITES = 2048  # the engine's automatic choice of the symmetric product
 # direction mu.d (3), the field factor (1) and six accumulations (6); the
 # reciprocal square root runs on the MUFU
 FP32_SYM_OPS_PER_PAIR = 30.0
-# FP32 operations (an FMA counts once) per undamped ordered pair of the
-# double-single kernel, counted in openmmpol_gb300/csrc/ds_kernels.cu: 3 coordinate differences
-# (33), r^2 (31), reciprocal square root (17 + 1 MUFU), r^-2 / r^-3 / 3 r^-5
-# (27), mu.d (31), the field factor (7), six accumulations (72) and three
-# renormalisations (9)
-DS_OPS_PER_PAIR = 227.0
-# the symmetric double-single product (k_tmu_ds_sym, from 2048 sites) forms
-# the geometry (coordinate differences, r^2, reciprocal square root, r^-2 /
-# r^-3 / 3 r^-5: 108 with the MUFU) once per unordered pair and the rest
-# (mu.d, field factor, accumulations, renormalisations: 119) per direction
-DS_SYM_OPS_PER_PAIR = 108.0 + 2 * 119.0
-# FP64 instructions per ordered (target, source) pair of the AMOEBA gradient
-# pair kernel (k_grad_pairs, openmmpol_gb300/csrc/grad.cu): 95 DFMA + 78 DMUL
-# + 34 DADD, from the ncu instruction counters of one launch on the
-# 30,000-site box (undamped pairs dominate); flop counts an FMA twice
-GRAD_F64_INST_PER_PAIR = 207.0
-GRAD_F64_FLOP_PER_PAIR = 302.0
-# FP32 arithmetic instructions (FADD + FMUL + FFMA) per ordered pair of the
-# double-single gradient passes (grad_ds.cu), same counters and box: 945 in
-# the static-multipole pass + 1,758 in the induced-dipole pass
-GRAD_DS_OPS_PER_PAIR = 2703.0
+# FP32 arithmetic instructions (FADD + FMUL + FFMA) per unordered pair of the
+# symmetric product of FP64 accuracy (k_tmu_sym, openmmpol_gb300/csrc/tmu_sym.cu:
+# double-single but for the close pairs), and per ordered pair of the product
+# over ordered pairs (k_rows_ds, tmu_rows.cu, counted in the source); the former
+# from the ncu instruction counters of one launch on the 30,000-site box
+DS_SYM_OPS_PER_PAIR = 289.0
+DS_OPS_PER_PAIR = 190.0
+# the same per unordered pair of the AMOEBA gradient pair kernel (k_grad_sym,
+# grad_sym.cu), same counters and box
+GRAD_OPS_PER_PAIR = 2076.0
 
 
 def parse():
@@ -338,9 +325,11 @@ def run_reference(args):
     print(json.dumps(line), flush=True)
 
 
-def kernel_table(kst, n, peak64, peak32, fp32_shape=None):
+def kernel_table(kst, n, peak64, peak32, fp32_shape=None, ds64=False):
     """Per pair kernel: launches, columns, time and the rate against its pipe.
-    fp32_shape: the autotuned FP32 launch shape of one column, if known."""
+    fp32_shape: the FP32 launch shape of one column, if known.  ds64: the
+    product of FP64 accuracy ran in double-single on the FP32 pipe (as this
+    library's does), not on the FP64 pipe."""
     pairs = float(n) * (n - 1)
     out = {}
     for name, (cnt, ms, cols), pk in (("tmu_fp64", kst[0], peak64), ("tmu_fp32", kst[1], peak32),
@@ -351,7 +340,10 @@ def kernel_table(kst, n, peak64, peak32, fp32_shape=None):
         ach = FLOP_PER_PAIR * pairs * cols / (ms * 1e-3) / 1e12
         out[name] = {"launches": cnt, "columns": cols, "total_ms": ms, "avg_ms": ms / cnt,
                      "achieved_tflops": ach, "peak_tflops": pk, "frac": ach / pk if pk else None}
-        if name == "tmu_fp64" and n >= SYM_MIN_SITES:
+        if name == "tmu_fp64" and ds64:
+            pk = peak32
+            out[name]["peak_tflops"] = pk
+        if name == "tmu_fp64" and not ds64 and n >= SYM_MIN_SITES:
             # FP64 pipe: operations of the symmetric product issued per second
             # against the FP64 instruction rate (peak flop / 2)
             ops = FP64_SYM_OPS_PER_PAIR * pairs / 2 * cols / (ms * 1e-3) / 1e12
@@ -366,12 +358,13 @@ def kernel_table(kst, n, peak64, peak32, fp32_shape=None):
                 out[name].update({"conventional_tflops": ach, "achieved_tops": ops, "peak_tops": pk / 2,
                                   "frac": ops / (pk / 2) if pk else None, "peak_nominal_tops": 40.3,
                                   "frac_nominal": ops / 40.3})
-        if name == "tmu_ds":
+        if name == "tmu_ds" or (name == "tmu_fp64" and ds64):
             # FP32 pipe: double-single operations issued per second against
             # the FMA-pipe instruction rate (peak flop / 2)
             ops = (DS_SYM_OPS_PER_PAIR * pairs / 2 if n >= SYM_MIN_SITES else DS_OPS_PER_PAIR * pairs) * cols / (
                 ms * 1e-3) / 1e12
-            out[name].update({"fp64_equivalent_tflops": ach, "achieved_tops": ops, "peak_tops": pk / 2,
+            out[name].update({"double_single": True, "fp64_equivalent_tflops": ach, "achieved_tops": ops,
+                              "peak_tops": pk / 2,
                               "frac": ops / (pk / 2) if pk else None})
     return out
 
@@ -380,7 +373,7 @@ def kernel_table(kst, n, peak64, peak32, fp32_shape=None):
 # captures (dram__bytes_read.sum + dram__bytes_write.sum) of one launch on the
 # 30,000-site box; the working set is O(N) and L2-resident, so the figure is
 # scaled by the site count
-TRAFFIC_30K = {"tmu_fp64": 3.6e6, "tmu_ds": 4.6e6}
+TRAFFIC_30K = {"tmu_fp64": 5.1e6, "tmu_ds": 5.1e6}
 
 
 def roofline_of(kstats, total_ms, n=30000):
@@ -388,10 +381,10 @@ def roofline_of(kstats, total_ms, n=30000):
         return None
     dom = max(kstats, key=lambda k: kstats[k]["total_ms"])
     d = kstats[dom]
-    ds = dom == "tmu_ds"
-    sym = dom == "tmu_fp64" and "achieved_tops" in d
+    ds = bool(d.get("double_single"))
+    sym = dom == "tmu_fp64" and "achieved_tops" in d and not ds
     traffic = TRAFFIC_30K[dom] * n / 30000.0 if dom in TRAFFIC_30K else None
-    return {"bound": "fp64" if dom == "tmu_fp64" else "fp32", "kernel": dom,
+    return {"bound": "fp64" if dom == "tmu_fp64" and not ds else "fp32", "kernel": dom,
             "achieved": d["achieved_tops"] if (ds or sym) else d["achieved_tflops"],
             "peak": d["peak_tops"] if (ds or sym) else d["peak_tflops"],
             "unit": ("Tops/s (FP32 instructions)" if ds else "Tops/s (FP64 instructions)" if sym else "TFLOP/s"),
@@ -401,7 +394,7 @@ def roofline_of(kstats, total_ms, n=30000):
             "peak_source": "FMA-chain kernel measured in this run (pipe peak; "
                            "MEASURED_PEAKS.json has no FP32/FP64 CUDA-core figure)",
             "algorithmic": ((f"{DS_SYM_OPS_PER_PAIR:.0f} FP32 operations per unordered pair x N(N-1)/2 pairs "
-                             "(symmetric double-single product)" if n >= SYM_MIN_SITES else
+                             "(double-single but for the close pairs)" if n >= SYM_MIN_SITES else
                              f"{DS_OPS_PER_PAIR:.0f} FP32 operations per ordered pair x N(N-1) pairs") if ds else
                             f"{FP64_SYM_OPS_PER_PAIR:.0f} FP64 operations per unordered pair x N(N-1)/2 pairs "
                             f"(symmetric product; {d.get('fp64_flop_equivalent_tflops', 0):.3f} TFLOP/s at the "
@@ -411,9 +404,9 @@ def roofline_of(kstats, total_ms, n=30000):
             "share_of_timed": d["total_ms"] / total_ms,
             # GB300 nominal pipe rates beside the measured ones: FP64 1.25 TFLOP/s (0.625 T FMA
             # instructions/s); FP32 152 SMs x 128 lanes x 2.07 GHz = 40.3 T instructions/s
-            "peak_nominal": 0.625 if dom == "tmu_fp64" else 40.3,
+            "peak_nominal": 0.625 if dom == "tmu_fp64" and not ds else 40.3,
             "frac_nominal": ((d["achieved_tops"] if (ds or sym) else d["achieved_tflops"] / 2.0) /
-                             (0.625 if dom == "tmu_fp64" else 40.3))}
+                             (0.625 if dom == "tmu_fp64" and not ds else 40.3))}
 
 
 def rel_err(a, b):
@@ -452,10 +445,9 @@ def grad_cpu_sample(cache, threads):
 
 def grad_pass(g, L, peak64, peak32, cache, restore, reps=2, cpu=True):
     """Polarization-energy gradient on the solved system through the public
-    call (ommp_gpu_polelec_geomgrad: gradient D2H included): the
-    double-single pair passes of the mixed modes and the FP64 pass of the
-    fp64 mode, each pair kernel against its pipe; the oracle's gradient on
-    the host cores."""
+    call (ommp_gpu_polelec_geomgrad: gradient D2H included) in a mixed and
+    in the fp64 mode, the pair kernel against the FP32 pipe; the oracle's
+    gradient on the host cores."""
     h = g._h
     mm = g.mm_atoms
     pairs = float(mm) * (mm - 1)
@@ -475,18 +467,14 @@ def grad_pass(g, L, peak64, peak32, cache, restore, reps=2, cpu=True):
         g.enable_kernel_timing(False)
         cnt, ms, _ = g.kernel_stats(3)
         kms = ms / max(cnt, 1)
-        if precision == "fp64":
-            inst, peak, unit = GRAD_F64_INST_PER_PAIR, peak64 / 2, "T FP64 instructions/s"
-            alg = (f"{GRAD_F64_INST_PER_PAIR:.0f} FP64 instructions ({GRAD_F64_FLOP_PER_PAIR:.0f} flop) "
-                   "per ordered pair x N(N-1)")
-        else:
-            inst, peak, unit = GRAD_DS_OPS_PER_PAIR, peak32 / 2, "T FP32 instructions/s"
-            alg = f"{GRAD_DS_OPS_PER_PAIR:.0f} FP32 operations per ordered pair (both passes) x N(N-1)"
+        # every unordered pair once, in double-single, in every mode
+        inst, peak, unit = GRAD_OPS_PER_PAIR / 2, peak32 / 2, "T FP32 instructions/s"
+        alg = f"{GRAD_OPS_PER_PAIR:.0f} FP32 operations per unordered pair x N(N-1)/2"
         ach = inst * pairs / (kms * 1e-3) / 1e12
         return grad, {"gradients_per_s": 1.0 / wall, "ms_per_gradient": wall * 1e3, "pair_kernels_ms": kms,
                       "pairs_per_s": pairs / (kms * 1e-3), "gpu_launches_per_gradient": launches / reps,
                       "net_force_rel": float(np.abs(grad.sum(0)).max() / np.abs(grad).max()),
-                      "roofline": {"bound": "fp64" if precision == "fp64" else "fp32", "achieved": ach,
+                      "roofline": {"bound": "fp32", "achieved": ach,
                                    "peak": peak, "unit": unit, "frac": ach / peak if peak else None,
                                    "algorithmic": alg,
                                    "peak_source": "FMA-chain kernel measured in this run (pipe instruction rate)"}}
@@ -494,7 +482,7 @@ def grad_pass(g, L, peak64, peak32, cache, restore, reps=2, cpu=True):
     g_ds, res = timed("mixed-ds")
     g_64, res64 = timed("fp64")
     g.set_precision(restore)
-    res["precision"] = "double-single pair sums (mixed modes)"
+    res["precision"] = "double-single pair sums, close pairs in FP64 (every mode)"
     res["fp64"] = res64
     res["max_rel_diff_vs_fp64"] = float(np.abs(g_ds - g_64).max() / np.abs(g_64).max())
     res["d2h_bytes_per_call"] = mm * 3 * 8
@@ -620,7 +608,7 @@ def run_gb300(args):
         sys_.enable_kernel_timing(False)
         kst = [sys_.kernel_stats(c) for c in range(3)]
         total_ms = replica_time_ms(sum(step_ms), dist)
-        kstats = kernel_table(kst, n, peak64.value, peak32.value, sys_.fp32_shape(1))
+        kstats = kernel_table(kst, n, peak64.value, peak32.value, sys_.fp32_shape(1), ds64=True)
         res = {"value": replica_value(ws, K, total_ms), "ms_per_step": total_ms / K, "steps_ms": step_ms,
                "solver_counters_per_step": counters,
                "solver_counters": "FP64 products, FP32 products, refinement steps, inner FP32 iterations, "

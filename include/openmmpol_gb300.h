@@ -55,8 +55,9 @@
 /* precision modes of ommp_gpu_set_precision */
 #define OMMP_GPU_PREC_FP64 0  /* plain FP64 solver (default) */
 #define OMMP_GPU_PREC_MIXED 1 /* FP32 inner CG + FP64 iterative refinement */
-#define OMMP_GPU_PREC_MIXED_DS 2 /* as MIXED, refinement residual products in  \
-                                    double-single arithmetic (~1e-13 relative) */
+#define OMMP_GPU_PREC_MIXED_DS 2 /* as MIXED (direct residual products whatever the \
+                                    FMM setting), later residuals updated by the    \
+                                    FP32 product of the correction */
 
 /* status codes of the ommp_gpu_* calls */
 #define OMMP_GPU_OK 0
@@ -282,7 +283,7 @@ const char *ommp_gpu_last_error(void);
 void ommp_gpu_set_solver_tol(OMMP_SYSTEM_PRT s, double tol);
 void ommp_gpu_set_solver_maxiter(OMMP_SYSTEM_PRT s, int32_t maxiter);
 void ommp_gpu_set_precision(OMMP_SYSTEM_PRT s, int32_t mode);
-/* FP64 direct T.mu kernel: 0 auto (symmetric from 2048 sites), 1 all ordered
+/* FP64 direct T.mu kernel: 0 auto (symmetric from 2400 sites), 1 all ordered
  * pairs, 2 symmetric (each unordered pair once, deterministic) */
 int32_t ommp_gpu_set_fp64_kernel(OMMP_SYSTEM_PRT s, int32_t mode);
 /* status-returning forms of ommp_{potential,field}_*2ext; which:
@@ -292,13 +293,13 @@ int32_t ommp_gpu_set_fp64_kernel(OMMP_SYSTEM_PRT s, int32_t mode);
 #define OMMP_GPU_EXT_POL 2
 int32_t ommp_gpu_potential_ext(OMMP_SYSTEM_PRT s, int32_t which, int32_t n, const double *cext, double *v);
 int32_t ommp_gpu_field_ext(OMMP_SYSTEM_PRT s, int32_t which, int32_t n, const double *cext, double *E);
-/* FP32 inner T.mu kernel: 0 autotuned (default), 1 one target per thread
- * with a per-pair damping test, 2 tile-classified (undamped inner loop for
+/* FP32 inner T.mu kernel: 0 by size and columns (default), 1 all ordered
+ * pairs with a per-pair damping test, 2 tile-classified (undamped inner loop for
  * tiles beyond the damping range, two targets per thread), 3 symmetric (each
  * unordered pair once for both directions, tile-classified, deterministic
  * fixed-point sums) */
 int32_t ommp_gpu_set_fp32_kernel(OMMP_SYSTEM_PRT s, int32_t mode);
-/* the FP32 launch shape the autotuner chose for ncol columns: shape[0] the
+/* the FP32 launch shape in use for ncol columns: shape[0] the
  * kernel (1, 2 or 3 as above), shape[1] the columns per launch, shape[2] the
  * source splits; zeros before the first mixed solve with ncol columns */
 int32_t ommp_gpu_get_fp32_shape(OMMP_SYSTEM_PRT s, int32_t ncol, int32_t *shape);

@@ -22,7 +22,7 @@ available_solvers = {"none": 0, "default": 1, "conjugate gradient": 1, "cg": 1,
 available_matrix_vector = {"none": 0, "default": 2, "incore": 1, "direct": 2}
 verbosity = {"none": 0, "low": 1, "high": 2, "debug": 3}
 PREC_FP64, PREC_MIXED, PREC_MIXED_DS = 0, 1, 2
-# 'mixed-ds': the refinement residual products in double-single arithmetic
+# 'mixed-ds': as 'mixed', later refinement residuals updated by an FP32 product
 PRECISIONS = {"fp64": PREC_FP64, "mixed": PREC_MIXED, "mixed-ds": PREC_MIXED_DS}
 ERR_CANCELLED = 7
 
@@ -365,13 +365,13 @@ class OMMPSystem:
         _check(self._L.ommp_gpu_set_inner_blocks(self._h, int(max_sites), float(link_bohr)))
 
     def set_fp32_kernel(self, mode) -> None:
-        """'auto' (autotuned) | 'pairwise' (kernel 1) | 'tiled' (kernel 2) |
+        """'auto' (by size and columns) | 'pairwise' (kernel 1) | 'tiled' (kernel 2) |
         'symmetric' (kernel 3: each unordered pair once)."""
         m = {"auto": 0, "pairwise": 1, "tiled": 2, "symmetric": 3}.get(mode, mode)
         _check(self._L.ommp_gpu_set_fp32_kernel(self._h, int(m)))
 
     def fp32_shape(self, ncol: int = 1):
-        """The autotuned FP32 launch shape for ncol columns: (kernel, columns
+        """The FP32 launch shape in use for ncol columns: (kernel, columns
         per launch, source splits) with kernel 'pairwise' | 'tiled' |
         'symmetric', or None before the first mixed solve with ncol columns."""
         out = (C.c_int32 * 3)()
@@ -415,7 +415,7 @@ class OMMPSystem:
         return self._tmatvec_alt(self._L.ommp_gpu_tmatvec_fp32, x)
 
     def tmatvec_ds(self, x) -> np.ndarray:
-        """y = T x with the double-single kernel of the 'mixed-ds' mode."""
+        """y = T x with the residual product of the 'mixed-ds' mode."""
         return self._tmatvec_alt(self._L.ommp_gpu_tmatvec_ds, x)
 
     def _tmatvec_alt(self, fn, x) -> np.ndarray:

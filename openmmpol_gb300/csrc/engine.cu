@@ -265,7 +265,7 @@ int System::upload_static() {
   bad |= alloc(x32_, nv * 2) | alloc(r32_, nv * 2) | alloc(p32_, nv * 2) | alloc(h32_, nv * 2) |
          alloc(z32_, nv * 2);
   scratch_n_ = gpu::m2d_scratch_doubles(d_, nsplit_m2d_);
-  // FP32 scratch for twice the default source split (the autotuner tries both)
+  // FP32 scratch for twice the default source split (the finer one is used)
   bad |= alloc(scratch_, scratch_n_) | alloc(scratch32_, gpu::tmu_scratch_doubles(d_, 2, f32_splits));
   bad |= alloc(d_.tile_box32, 2 * (size_t)d_.ntile) | alloc(d_.pol_split, 3 * (size_t)n) |
          alloc(d_.sub_box32, 2 * (size_t)((n + 31) / 32));
@@ -1176,7 +1176,7 @@ int System::set_inner_preconditioner(int mode) {
 
 int System::set_fp32_kernel(int mode) {
   if (mode < 0 || mode > 3) {
-    set_last_error("FP32 kernel mode must be 0 (autotuned), 1, 2 or 3");
+    set_last_error("FP32 kernel mode must be 0 (auto), 1, 2 or 3");
     return kErrBadArg;
   }
   if (mode != fp32_kernel_) f32_tune_.clear();

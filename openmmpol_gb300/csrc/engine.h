@@ -175,8 +175,8 @@ class System {
   void set_precision(int p) {
     if (p >= kPrecFP64 && p <= kPrecMixedDS) precision_ = p;
   }
-  // FP64 direct product: 0 auto (symmetric from 2048 sites), 1 all ordered
-  // pairs (target-outer), 2 symmetric (unordered pairs)
+  // FP64 direct product: 0 auto (symmetric from 2,400 sites), 1 all ordered
+  // pairs, 2 symmetric (unordered pairs)
   int set_fp64_kernel(int mode);
   int set_fp32_kernel(int mode);
   int fp32_shape(int ncol, int32_t *shape) const;
@@ -308,7 +308,7 @@ class System {
   // how the cached E_M2D was computed
   static constexpr int kM2dDirect = 0, kM2dFMM = 1;
   int m2d_method_ = kM2dDirect;
-  int fp32_kernel_ = 0;  // 0 autotuned, else the forced kernel version
+  int fp32_kernel_ = 0;  // 0 by size, else the forced kernel version
   float *scratch32_ = nullptr;
   double *partial_ = nullptr;  // reduction partials [kRedBlocks][8]
   double *dots_ = nullptr;     // [8]

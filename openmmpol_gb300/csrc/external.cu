@@ -55,7 +55,7 @@ __device__ __forceinline__ void split3(double v, double g1, float *o) {
 }
 
 struct ExtArgs {
-  int n, m, nv;        // points, sources, polarizable sites (dipole sets)
+  int n, m;            // points, sources
   const double *cext;
   const Pos64 *pos;    // sources
   const double *q;     // [m][ld] multipoles, or null (induced dipoles alone)
@@ -318,7 +318,7 @@ int System::ext_props(int which, bool field, int n, const double *cext_h, double
   double *out = partial + (size_t)nsplit * n * C;
   unsigned *word = reinterpret_cast<unsigned *>(out + (size_t)n * C);
   int *polar = reinterpret_cast<int *>(word + 2);
-  a.n = n, a.m = m, a.nv = d_.n;
+  a.n = n, a.m = m;
   a.cext = cext;
   a.pos = do_mm ? d_.mm_pos : d_.pol_pos;
   a.q = do_mm ? d_.mm_q : nullptr;

@@ -65,7 +65,6 @@ struct GradArgs {
   int mm, n;
   const Pos64 *mm_pos;
   const double *mm_a, *mm_q;
-  const float2 *mm_wa;
   const int *mm_polar, *polar_mm;
   const double *ipd;  // [n_ipd][n][3]
   const int *m2d_ri, *m2d_src;
@@ -81,7 +80,6 @@ struct GradArgs {
   // the pair pass's fixed-point sums [mm][6 or 3], flag and scale
   const unsigned long long *lo, *hi, *bad;
   double thr;
-  float thr2m;
   int *err;
 };
 
@@ -358,7 +356,6 @@ int System::polelec_geomgrad(double *grad_h) {
   a.mm_pos = d_.mm_pos;
   a.mm_a = d_.mm_a;
   a.mm_q = d_.mm_q;
-  a.mm_wa = d_.mm_wa32;
   a.mm_polar = gs.mm_polar;
   a.polar_mm = d_.polar_mm;
   a.ipd = ipd_;
@@ -384,7 +381,6 @@ int System::polelec_geomgrad(double *grad_h) {
   a.rot = gs.rot;
   a.grad = gs.grad;
   a.thr = d_.damp_thr;
-  a.thr2m = (float)(d_.damp_thr * d_.damp_thr * (1.0 + 1e-5));
   a.err = flag_;
   cudaMemsetAsync(flag_, 0, sizeof(int), st_);
   const int tb = (mm + gpu::GTPB - 1) / gpu::GTPB;

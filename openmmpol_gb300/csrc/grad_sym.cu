@@ -13,7 +13,7 @@
 // ordered passes that formed the field gradients of either dipole set, the
 // field, its gradient and its contracted Hessian at every site took 2 x 2,703
 // FP32 operations per pair in double-single, or 2 x 207 on the FP64 pipe; the
-// pair form takes about 1,900.  p_t p_s is covered by adding p / 2 to m.
+// pair form takes about 2,080 (ncu).  p_t p_s is covered by adding p / 2 to m.
 //
 // Notation (n the unit vector from s to t, a = p.n, b = m.n, T = Q n,
 // s = n.T, R = Q p'; K = y^3, G = 3 y^3, F = 3 y^4, C = 15 y^4, F5 = 3 y^5,
@@ -43,9 +43,10 @@
 // 30,000 sites: 76 -> 35 ms in the mixed modes, 330 ms in FP64 before; 90,000:
 // 668 -> 311 ms (2.95 s in FP64).  Error against 64 bits 0.95e-14 to 1.2e-14
 // (before 2.7e-14 in FP64, 3e-14 to 6e-14 in double-single).  255 registers
-// without spills at 2 CTAs per SM: bound by FP32 issue (54 % of the issue slots
-// at 6,000 sites) with 8 warps, a quarter of whose stalls is the fetch of the
-// 2,600-instruction step.
+// without spills at 2 CTAs per SM: bound by FP32 issue at 8 warps (71 % of the
+// issue slots, 2,076 operations per pair; at 6,000 sites 54 %, a quarter of the
+// stalls the fetch of the 2,600-instruction step, which far and near
+// sub-tiles' warps pass through at different places).
 //
 // Built with --fmad=false -ftz=true: every FMA is explicit.
 #include <algorithm>

@@ -1,16 +1,14 @@
 // GB300 (sm_103a) kernels of the induced-point-dipole path.
 //
-// Pair kernels (all-pairs, CUDA cores; the pair tensor math is not a dense
-// contraction, so no tensor cores):
+// Finishing passes of the pair kernels (whose pair tensor math is not a dense
+// contraction, so no tensor cores), dense T, LU and BLAS-1:
 //   k_m2d_finish     fixed-order reduction of the source-split partials plus
 //                    the scaled-pair correction pass: for every listed pair
 //                    (s - 1) * f_ij is added, which equals the reference's
 //                    "skip when s == 0, multiply when s != 1" rule.
-//   k_tmu_finish     partial reduction, u-scale correction, sign and the
+//   k_tmu_finish     the FMM's finishing pass: u-scale correction, sign and the
 //                    1/alpha diagonal of TMatVec_otf/TMatVec_diag
 //                    (src/mod_polarization.F90:459-504).
-// Source tiles are staged in shared memory by the whole CTA with coalesced
-// loads and broadcast to all threads; each thread owns one target site.
 #include <algorithm>
 #include <atomic>
 #include <cmath>

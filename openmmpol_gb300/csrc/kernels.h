@@ -155,7 +155,6 @@ void launch_tmu32_rows(const DevSites &s, int ncol, int gmax, const float *x, fl
 int launch_tmu_f32(const DevSites &s, int nrhs, const float *x, float *y, float *scratch, int nsplit, cudaStream_t st,
                    int gmax = 4, int kver = 2, double *sym_scratch = nullptr, bool prepared = false,
                    double *part = nullptr, int max_part = 0);
-int tmu32_sym_resident(int g, bool amoeba);
 
 // ---- multi-system symmetric products --------------------------------------
 // One system's share of a launch that serves several systems (the products
@@ -188,8 +187,7 @@ void launch_tmu_f64_sym_multi(int g, bool amoeba, const SymSlice *sl, int nsl, u
                               bool zeroed = false);
 void launch_tmu32_pairs(const DevSites &s, int g, int groups, const float *x, float *partial, int nsplit,
                         cudaStream_t st);
-// source splits an FP32 scratch must hold (per column) for every shape the
-// autotuner may pick
+// source splits an FP32 scratch must hold (per column)
 int tmu32_max_split(const DevSites &s, int sm_count);
 // Split of the source range for the FP32 operator (tmu32.cu) and its tile
 // boxes / undamped distance, computed on the host from the FP32 positions.

@@ -7,13 +7,13 @@
 // that fill the whole GPU, would run one system's product after another.
 // Here one engine stream advances every queued solve in rounds:
 //
-//   * every solve is the iterative refinement of System::mixed_ir_ws (FP64 or
-//     double-single residual E - T mu, convergence test on the reference's
+//   * every solve is the iterative refinement of System::mixed_ir_ws (residual
+//     E - T mu of FP64 accuracy, convergence test on the reference's
 //     rms of alpha r, FP32 inner PCG on the normalised residual, FP64
 //     accumulation), written as a state machine;
 //   * in each round, all systems that need a pair product share one launch
-//     per product kind (FP32 inner product, FP64 or double-single residual
-//     product) and column width: a persistent kernel whose work items are
+//     per product kind (FP32 inner product, residual product) and column
+//     width: a persistent kernel whose work items are
 //     (system, super-tile, chunk of slots), taken in order from one counter
 //     (the launch_*_sym_multi kernels);
 //   * a product gets a bounded share of each round (about 1.5 ms of work per
@@ -24,14 +24,14 @@
 //     work items are cut to a quarter of a resident CTA's share of a round
 //     (SymSlice::round_pairs), so that every CTA stays busy for the whole
 //     round whatever the systems' sizes;
-//   * after the launches, every system whose product completed runs its CG
-//     bookkeeping (finishing pass, dots, updates, convergence flags) on the
-//     same stream, and one synchronisation per round brings the flags to
+//   * after the launches, the systems whose product completed share the
+//     launches of the finishing pass and the CG steps (pcg.cu) on the same
+//     stream, and one synchronisation per round brings the flags to
 //     the host, where each solve takes its next step.
 //
 // Results equal those of the single-system solve to rounding: the products
-// are the same symmetric kernels (the FP64 one also below 2048 sites, where
-// the single-system path uses the target-outer kernel).
+// are the same symmetric kernels (also below the sizes where the single-system
+// path takes ordered pairs).
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -59,9 +59,9 @@ enum Kind { kNone, kF32, kF64, kDS };
 constexpr int kMaxOuter = 30;
 constexpr int kMaxInner = 200;
 // pairs per millisecond of the symmetric kernels on GB300 per product kind
-// (measured: FP32 8.6e11, FP64 1.76e10, double-single 8.6e10 pairs/s); a
-// round's budget is round_ms_ of work per kind
-constexpr double kPairsPerMs[4] = {0.0, 8.6e8, 1.76e7, 8.6e7};
+// (measured: FP32 9.5e11, either residual product 1.0e11 pairs/s); a round's
+// budget is round_ms_ of work per kind
+constexpr double kPairsPerMs[4] = {0.0, 9.5e8, 1.0e8, 1.0e8};
 }  // namespace
 
 struct MultiSolver::Job {

@@ -1,5 +1,4 @@
-// Pair arithmetic shared by the FP64/FP32 pair kernels (kernels.cu) and
-// the double-single kernels (ds_kernels.cu): FP64 reciprocal square root from an
+// Pair arithmetic shared by the FP64, FP32 and double-single pair kernels: FP64 reciprocal square root from an
 // FP32 seed, the FP32 damping pre-tests, and the damped dipole-field factors
 // (Thole damping of the reference, src/mod_electrostatics.F90:978-1095).
 #pragma once
@@ -184,20 +183,6 @@ __device__ __forceinline__ void damped_factors(float r2, float wt, float ws, flo
   }
 }
 
-// The pair factors k3 and 3 k5 in the precision of the kernel (FP64:
-// dd_pair_f64; FP32: the plain formulas).
-template <typename T, bool AMOEBA>
-__device__ __forceinline__ void dd_pair(T r2, T wt, T ws, T at, T as, float2 wat, float2 was, T thr,
-                                        float thr2m, T &k3, T &k5x3) {
-  if constexpr (std::is_same<T, double>::value) {
-    double k5;
-    dd_pair_f64<AMOEBA>(r2, wt, ws, at, as, wat, was, thr, thr2m, k3, k5);
-    k5x3 = 3.0 * k5;
-  } else {
-    dd_kernel<T, AMOEBA>(r2, wt, ws, at, as, thr, k3, k5x3);
-  }
-}
-
 // Field of a static multipole (charge; + dipole and quadrupole for AMOEBA,
 // q[0..9]) at a polarizable target, d = target - source, Thole-damped
 // (elec_prop_M2D pair term, src/mod_electrostatics.F90:2579-2731).
@@ -337,7 +322,7 @@ __device__ __forceinline__ void m2d_field(const double *acc, double &ex, double 
 __device__ __forceinline__ bool coincident(double r2) { return __double2hiint(r2) < 0x3a436930; }
 
 // Per-site 128-bit fixed-point accumulators of the symmetric products
-// (kernels.cu, ds_kernels.cu): integer addition is exact and associative,
+// (tmu_sym.cu, tmu32.cu, grad_sym.cu): integer addition is exact and associative,
 // so the sums do not depend on the order of the CTAs.
 // v added exactly into the two-word fixed-point value hi * 2^-16 + lo * 2^-80
 // (hi two's complement, lo unsigned), with integer operations instead of FP64

@@ -693,8 +693,6 @@ void fill_s32_job(S32Job &j, const DevSites &s, int g, const float *x, unsigned 
 
 }  // namespace
 
-int tmu32_sym_resident(int g, bool) { return g == 2 ? s32_resident<2>() : s32_resident<1>(); }
-
 int tmu32_sym_items(const DevSites &s, int g, double round_pairs) {
   if (s.n == 0) return 0;
   return s32_plan(s.n, g, round_pairs).items();
