@@ -305,6 +305,8 @@ class System {
   int build_blocks();
   double *ext_buf_ = nullptr;  // external points: coordinates, partials, output, dipoles
   size_t ext_cap_ = 0;
+  double *fe_buf_ = nullptr;  // static-static sums: partials, results, pair lists
+  size_t fe_cap_ = 0;
   // how the cached E_M2D was computed
   static constexpr int kM2dDirect = 0, kM2dFMM = 1;
   int m2d_method_ = kM2dDirect;
@@ -350,7 +352,7 @@ class System {
   double fixedelec_ = 0.0;
   bool fixedelec_grad_done_ = false;
   std::vector<double> fixedelec_grad_;
-  int m2m_launch(bool grad, double **buf, double **site, double **E, double **G, double **base);
+  int m2m_launch(bool grad, double **site, double **E, double **G, double **base);
   GradState *grad_ = nullptr;
   int ensure_grad_state();
   int frame_forces(const double *E_dev, const double *G_dev, const double *base_dev, double *grad_host);

@@ -352,7 +352,8 @@ int System::ext_props(int which, bool field, int n, const double *cext_h, double
     gpu::launch_ext<true>(field, a, partial, nsplit, flag_, st_);
   else
     gpu::launch_ext<false>(field, a, partial, nsplit, flag_, st_);
-  gpu::k_ext_sum<<<gpu::blocks_for_ext((size_t)n * C), 256, 0, st_>>>((size_t)n * C, nsplit, partial, a.word, out);
+  const int left = gpu::launch_sum_splits((size_t)n * C, nsplit, partial, st_);
+  gpu::k_ext_sum<<<gpu::blocks_for_ext((size_t)n * C), 256, 0, st_>>>((size_t)n * C, left, partial, a.word, out);
   gpu::add_launch_count(1);
   std::vector<double> h((size_t)n * C);
   int flag = 0;

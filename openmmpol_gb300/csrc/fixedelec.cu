@@ -124,9 +124,9 @@ void build_ss(const HostModel &m, int mm, std::vector<int> &ri, std::vector<int>
 }  // namespace
 
 // The pair and finish passes of the energy (grad false) or of the gradient
-// (grad true: E, G and the site terms into e_out, g_out, base_out).  buf
-// receives the device block to free after the stream is synchronised.
-int System::m2m_launch(bool grad, double **buf_out, double **site_out, double **e_out, double **g_out,
+// (grad true: E, G and the site terms into e_out, g_out, base_out, in the kept
+// buffer).
+int System::m2m_launch(bool grad, double **site_out, double **e_out, double **g_out,
                        double **base_out) {
   const int mm = d_.m;
   const bool amoeba = m_.amoeba;
@@ -137,12 +137,19 @@ int System::m2m_launch(bool grad, double **buf_out, double **site_out, double **
   const int nsplit = gpu::m2m_pick_split(d_, grad, gpu::sm_count());
   const size_t out = grad ? 12 * (size_t)mm : (size_t)mm;  // E, G, base | site
   const size_t need = (size_t)nsplit * nv * mm + out + ri.size() + 2 * src.size() + 1;
-  double *buf = nullptr;
-  if (cudaMalloc((void **)&buf, need * sizeof(double)) != cudaSuccess) {
-    cudaGetLastError();
-    set_last_error("out of device memory for the static multipole field");
-    return kErrMemory;
+  if (need > fe_cap_) {  // kept for the next geometry
+    if (fe_buf_) cudaFree(fe_buf_);
+    fe_buf_ = nullptr;
+    fe_cap_ = 0;
+    if (cudaMalloc((void **)&fe_buf_, need * sizeof(double)) != cudaSuccess) {
+      cudaGetLastError();
+      fe_buf_ = nullptr;
+      set_last_error("out of device memory for the static multipole field");
+      return kErrMemory;
+    }
+    fe_cap_ = need;
   }
+  double *buf = fe_buf_;
   gpu::M2mArgs a{};
   a.mm = mm;
   a.nsplit = nsplit;
@@ -169,6 +176,7 @@ int System::m2m_launch(bool grad, double **buf_out, double **site_out, double **
   cudaMemsetAsync(flag_, 0, sizeof(int), st_);
   const int fb = (mm + 127) / 128;
   gpu::launch_m2m(d_, grad, buf, nsplit, flag_, st_);
+  a.nsplit = gpu::launch_sum_splits((size_t)nv * mm, nsplit, buf, st_);
   if (amoeba && grad)
     gpu::k_m2m_finish<true, true><<<fb, 128, 0, st_>>>(a);
   else if (amoeba)
@@ -182,18 +190,13 @@ int System::m2m_launch(bool grad, double **buf_out, double **site_out, double **
   int flag = 0;
   cudaMemcpyAsync(&flag, flag_, sizeof(int), cudaMemcpyDeviceToHost, st_);
   int st = check(cudaStreamSynchronize(st_), "static multipole field");
-  if (st) {
-    cudaFree(buf);
-    return st;
-  }
+  if (st) return st;
   if (flag) {
-    cudaFree(buf);
     set_last_error(
         "Requesting Coulomb kernel for two atoms placed in the same point, this could be an internal bug or "
         "a problem in your input file, please check.");
     return kErrNumeric;
   }
-  *buf_out = buf;
   if (site_out) *site_out = a.site;
   if (e_out) *e_out = a.E;
   if (g_out) *g_out = a.G;
@@ -209,13 +212,12 @@ int System::fixedelec_energy(double &energy) {
     energy = fixedelec_;
     return kOk;
   }
-  double *buf = nullptr, *site_d = nullptr;
-  int st = m2m_launch(false, &buf, &site_d, nullptr, nullptr, nullptr);
+  double *site_d = nullptr;
+  int st = m2m_launch(false, &site_d, nullptr, nullptr, nullptr);
   if (st) return st;
   std::vector<double> site(mm);
   cudaMemcpyAsync(site.data(), site_d, mm * sizeof(double), cudaMemcpyDeviceToHost, st_);
   st = check(cudaStreamSynchronize(st_), "static multipole energy");
-  cudaFree(buf);
   if (st) return st;
   double e = 0.0;
   for (int t = 0; t < mm; ++t) e += site[t];
@@ -233,11 +235,10 @@ int System::fixedelec_geomgrad(double *grad_h) {
     std::copy(fixedelec_grad_.begin(), fixedelec_grad_.end(), grad_h);
     return kOk;
   }
-  double *buf = nullptr, *E = nullptr, *G = nullptr, *base = nullptr;
-  int st = m2m_launch(true, &buf, nullptr, &E, &G, &base);
+  double *E = nullptr, *G = nullptr, *base = nullptr;
+  int st = m2m_launch(true, nullptr, &E, &G, &base);
   if (st) return st;
   st = frame_forces(E, G, base, grad_h);  // synchronises the stream
-  cudaFree(buf);
   if (st) return st;
   fixedelec_grad_.assign(grad_h, grad_h + 3 * (size_t)mm);
   fixedelec_grad_done_ = true;

@@ -73,7 +73,10 @@ void launch_m2d(const DevSites &s, double *out, double *scratch, int nsplit, int
                 cudaStream_t st);
 // the finishing pass alone: split partials [nsplit][n][3] summed, the
 // scaled-pair corrections, out [n_ipd][n][3]
-void launch_m2d_finish(const DevSites &s, double *out, const double *partial, int nsplit, cudaStream_t st);
+void launch_m2d_finish(const DevSites &s, double *out, double *partial, int nsplit, cudaStream_t st);
+// split partials [nsplit][total] summed into the first block (few splits are
+// left to the reader); returns the splits left
+int launch_sum_splits(size_t total, int nsplit, double *partial, cudaStream_t st);
 
 // y = T x (dodiag) or y = -E_dd(x) (no diagonal); x,y [nrhs][n][3], FP64.
 size_t tmu_scratch_doubles(const DevSites &s, int nrhs, int nsplit);

@@ -30,7 +30,7 @@ namespace ommp {
 namespace gpu {
 namespace {
 
-constexpr int QTPB = 128;
+constexpr int QTPB = 64;  // sites per CTA (FP64 pipe: 9,003 sites on 141 SMs, 71 with 128)
 
 // E (and G, H when GRAD) of nq point charges (x, y, z, q) at the sites
 // pos[idx ? idx[j] : j], j < nt
