@@ -5,7 +5,8 @@
 // GB300 design: a uniform octree over the polarizable sites whose leaf side
 // is at least the Thole damping range (every damped pair is a near pair), of
 // the depth that minimises near-field pairs plus M2L work; Cartesian Taylor
-// expansions of order p (fmm_math.cuh); all passes in FP64:
+// expansions of order p (fmm_math.cuh); FP64 but for the FP32 M2L of orders
+// <= 10 (k_fmm_m2l_reg) and the near field:
 //   k_fmm_p2m     leaf multipoles of the dipoles (one CTA per leaf)
 //   k_fmm_m2m     parent multipoles from the 8 children, level by level
 //   k_fmm_m2l     local expansions from the well-separated cells of each
@@ -57,17 +58,18 @@ struct FmmTree {
   double *sq = nullptr;                                // sorted multipoles [n][ld] (M2D sources)
   int *tmm = nullptr;                                  // targets' static index (M2D self pair)
   double *M = nullptr, *Lc = nullptr;                  // [2][ncell][K]
-  float *M32 = nullptr;  // M scaled to the cell size, FP32 (the M2L input), after M in its block
+  float *M32 = nullptr;  // the M2L input [2][ncell][row32(K)] (k_fmm_m32)
   bool shared = false;                                 // targets are the sources
 };
 
 struct FmmState {
-  int p = 0, K = 0, KD = 0, npairs = 0;
+  int p = 0, K = 0, KD = 0, npairs = 0, nquads = 0;
   short4 *terms = nullptr;     // exponents (a, b, c) and order of each term
   int4 *pairs = nullptr;       // M2L pairs: g, index of g + h in the derivative table, h, (-1)^|g|
   int *hoff = nullptr;         // [K + 1] first pair of each target term h
+  int2 *quads = nullptr;       // the pairs by four target terms (build_tables)
   double *dunit = nullptr;     // [343][KD] derivatives of 1/r to order p at unit cell offsets
-  float *dunit32 = nullptr;    // the same in FP32 (the FP32 M2L)
+  float *dunit32 = nullptr;    // the same in FP32, [343][row32(K)] (the FP32 M2L)
   // translation lists (M2M, L2L), grouped by target term: source term and
   // packed |m| (bits 0-7) with the parities of m (bits 8-10), coefficient
   int2 *mm_e = nullptr, *ll_e = nullptr;
@@ -85,7 +87,7 @@ struct FmmState {
 };
 
 void free_tree(FmmTree &t) {
-  void *b[] = {t.cnt, t.leaf_start, t.perm, t.spos, t.sa, t.swa, t.sq, t.M, t.Lc, t.split};
+  void *b[] = {t.cnt, t.leaf_start, t.perm, t.spos, t.sa, t.swa, t.sq, t.M, t.M32, t.Lc, t.split};
   for (void *p : b)
     if (p) cudaFree(p);
   if (!t.shared) {
@@ -100,8 +102,8 @@ void free_tree(FmmTree &t) {
 
 void free_fmm_state(FmmState *f) {
   if (!f) return;
-  void *b[] = {f->terms, f->pairs, f->hoff, f->dunit, f->dunit32, f->field, f->mm_e, f->ll_e, f->mm_c, f->ll_c, f->mm_off,
-               f->ll_off};
+  void *b[] = {f->terms, f->pairs, f->hoff, f->quads, f->dunit, f->dunit32, f->field, f->mm_e, f->ll_e, f->mm_c,
+               f->ll_c, f->mm_off, f->ll_off};
   for (void *p : b)
     if (p) cudaFree(p);
   free_tree(f->d2d);
@@ -116,6 +118,10 @@ namespace gpu {
 namespace {
 
 constexpr int FT = 128;  // threads per CTA
+
+// floats of a row of the FP32 M2L's inputs: whole 16-byte copies
+__host__ __device__ constexpr int row32(int K) { return (K + 3) & ~3; }
+
 constexpr int FCH = 32;  // sites staged per chunk in the P2M
 constexpr int kMaxTermsPerThread = (fmm::nterms(fmm::kMaxOrder) + FT - 1) / FT;
 
@@ -130,6 +136,8 @@ struct FmmArgs {
   const short4 *terms;
   const int4 *pairs;
   const int *hoff;
+  const int2 *quads;
+  int nquads;
   const double *dunit;
   const float *dunit32;
   double *M, *Lc;
@@ -301,53 +309,65 @@ __global__ void __launch_bounds__(FT) k_fmm_m2l(FmmArgs a, int l) {
 }
 
 // The FP32 M2L input: the multipoles of the cells of levels 2..L scaled to
-// the cell size, M_g h^-|g| (h the level's cell side), in FP32; one thread
-// per (column, cell, term)
+// the cell size, (-1)^|g| M_g h^-|g| (h the level's cell side), in FP32; one
+// thread per (column, cell, term of the padded row)
 __global__ void k_fmm_m32(FmmArgs a, int first_cell, int ncells) {
-  const size_t total = (size_t)a.ncol * ncells * a.K;
+  const int row = row32(a.K);
+  const size_t total = (size_t)a.ncol * ncells * row;
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
-    const int g = (int)(i % a.K);
-    const size_t cc = i / a.K;
+    const int g = (int)(i % row);
+    const size_t cc = i / row;
     const int col = (int)(cc / ncells);
     const int c = first_cell + (int)(cc % ncells);
     int l = 0;
     while (l < a.L && level_off(l + 1) <= c) ++l;
-    const double hinv = (1 << l) / a.h0;
-    double f = 1.0;
-    for (int r = 0; r < a.terms[g].w; ++r) f *= hinv;
-    const size_t o = ((size_t)col * a.ncell + c) * a.K + g;
-    a.M32[o] = (float)(a.M[o] * f);
+    const size_t o = (size_t)col * a.ncell + c;
+    float v = 0.f;
+    if (g < a.K) {
+      const int ng = a.terms[g].w;
+      const double hinv = (1 << l) / a.h0;
+      double f = (ng & 1) ? -1.0 : 1.0;
+      for (int r = 0; r < ng; ++r) f *= hinv;
+      v = (float)(a.M[o * a.K + g] * f);
+    }
+    a.M32[o * row + g] = v;
   }
 }
 
-// The same M2L in FP32 for the cells of all levels in one launch, the (target
-// term, source term) pairs of each thread held in registers (PJ pairs per
-// thread of NT; 256 x 12 serve orders <= 8, 512 x 16 orders <= 10): the
-// multipoles (scaled to the cell size), the unit-offset derivatives and the
-// pair sums in FP32, the sum over source terms of each local term and the
-// local expansion in FP64.  The FP32 rounding (~1e-6 of a local coefficient)
-// is far below the expansion's own truncation error (~1e-4 at order 10), and
-// GB300 issues FP32 at 64x its FP64 rate.
-// A step (one source cell) is 16 multiply-adds per thread and column, less
-// than the latency of fetching the next cell's multipoles and derivatives, so
-// the sources are listed first and M2L_NB of them are fetched ahead with
-// asynchronous copies while the previous ones are used (both levels of a
-// 60,000-site box at order 10: 1.03 -> 0.74 ms).
+// The same M2L in FP32 for the cells of all levels in one launch, the sums of
+// the (target term, source term) pairs held in registers: the multipoles
+// (scaled to the cell size, with the sign of their order), the unit-offset
+// derivatives and the pair sums in FP32, the sum over source terms of each
+// local term and the local expansion in FP64.  The FP32 rounding (~1e-6 of a
+// local coefficient) is far below the expansion's own truncation error (~1e-4
+// at order 10), and GB300 issues FP32 at 64x its FP64 rate.
+// A pair is one multiply-add of a multipole and a derivative, both from shared
+// memory, so the loads bound the kernel, not the multiply-adds: a thread holds
+// QJ quads of pairs, four target terms against one source term, whose
+// multipole it loads once (5 loads for 4 multiply-adds instead of 8).  Threads
+// of a warp take consecutive source terms of the same target terms: no bank
+// conflicts in the multipoles, few in the derivatives.  288 x 3 quads serve
+// orders <= 8, 544 x 4 orders <= 10.
+// The source cells are listed first and M2L_NB of them are fetched ahead with
+// asynchronous 16-byte copies while the previous ones are used.
+// 60,000 sites, order 10, one column (both levels, 512 + 64 target cells): 738
+// us with a thread's pairs unrelated and 4-byte copies, 299 us now, the same
+// sums bit for bit.
 constexpr int M2L_NB = 4;
 
-__device__ __forceinline__ void copy_async4(float *dst, const float *src) {
+__device__ __forceinline__ void copy_async16(float *dst, const float *src) {
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
 }
 
-template <int NT, int PJ, int NCOL>
+template <int NT, int QJ, int NCOL>
 __global__ void __launch_bounds__(NT) k_fmm_m2l_reg(FmmArgs a) {
   extern __shared__ __align__(16) float sh32[];
   __shared__ int s_src[192], s_off[192], s_n;
-  const int rec = (NCOL + 1) * a.K;  // K == KD: multipoles of the columns, derivatives
+  const int row = row32(a.K);        // K == KD
+  const int rec = (NCOL + 1) * row;  // multipoles of the columns, derivatives
   float *s_buf = sh32;               // [2][M2L_NB][rec]
   float *s_acc = sh32;               // [npairs], after the last step
-  const int npairs = a.hoff[a.K];
   int l = 2;
   while (level_off(l + 1) - level_off(2) <= (int)blockIdx.x) ++l;
   const int tc = blockIdx.x - (level_off(l) - level_off(2));
@@ -382,29 +402,27 @@ __global__ void __launch_bounds__(NT) k_fmm_m2l_reg(FmmArgs a) {
     }
     if (threadIdx.x == 0) s_n = cnt;
   }
-  int pk[PJ];
-  float acc[NCOL][PJ];
+  int2 qd[QJ];
+  float acc[NCOL][QJ][4];
 #pragma unroll
-  for (int j = 0; j < PJ; ++j) {
+  for (int j = 0; j < QJ; ++j) {
     const int q = threadIdx.x + j * NT;
-    pk[j] = -1;
-    if (q < npairs) {
-      const int4 pr = a.pairs[q];
-      pk[j] = pr.x | (pr.y << 10) | (pr.w << 20);
-    }
+    qd[j] = q < a.nquads ? a.quads[q] : make_int2(-1, -1);
 #pragma unroll
-    for (int c = 0; c < NCOL; ++c) acc[c][j] = 0.f;
+    for (int c = 0; c < NCOL; ++c)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) acc[c][j][k] = 0.f;
   }
   __syncthreads();
   const int ns = s_n;
   auto fetch = [&](int b0, int buf) {
-    for (int i = threadIdx.x; i < M2L_NB * rec; i += NT) {
-      const int k = i / rec, r = i - k * rec;
-      if (b0 + k >= ns) break;
-      const int col = r / a.K, g = r - col * a.K;
-      const float *src = col < NCOL ? a.M32 + ((size_t)col * a.ncell + level_off(l) + s_src[b0 + k]) * a.K + g
-                                    : a.dunit32 + (size_t)s_off[b0 + k] * a.KD + g;
-      copy_async4(&s_buf[(buf * M2L_NB + k) * rec + r], src);
+    const int chunks = row / 4, total = min(M2L_NB, ns - b0) * (NCOL + 1) * chunks;
+    for (int i = threadIdx.x; i < total; i += NT) {
+      const int r = i / chunks, ch = i - r * chunks;
+      const int k = r / (NCOL + 1), col = r - k * (NCOL + 1);
+      const float *src = col < NCOL ? a.M32 + ((size_t)col * a.ncell + level_off(l) + s_src[b0 + k]) * row
+                                    : a.dunit32 + (size_t)s_off[b0 + k] * row;
+      copy_async16(&s_buf[buf * M2L_NB * rec + r * row + 4 * ch], src + 4 * ch);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
@@ -415,14 +433,21 @@ __global__ void __launch_bounds__(NT) k_fmm_m2l_reg(FmmArgs a) {
     __syncthreads();
     const int kn = min(M2L_NB, ns - b0);
     for (int k = 0; k < kn; ++k) {
-      const float *s_m = &s_buf[(buf * M2L_NB + k) * rec], *s_d = s_m + NCOL * a.K;
+      const float *s_m = &s_buf[(buf * M2L_NB + k) * rec], *s_d = s_m + NCOL * row;
 #pragma unroll
-      for (int j = 0; j < PJ; ++j) {
-        if (pk[j] < 0) continue;
-        const int g = pk[j] & 1023;
-        const float d = (pk[j] >> 20) ? -s_d[(pk[j] >> 10) & 1023] : s_d[(pk[j] >> 10) & 1023];
+      for (int j = 0; j < QJ; ++j) {
+        if (qd[j].x < 0) continue;
+        const int g = (qd[j].y >> 10) & 1023;
+        const float d0 = s_d[qd[j].x & 1023], d1 = s_d[(qd[j].x >> 10) & 1023], d2 = s_d[qd[j].x >> 20],
+                    d3 = s_d[qd[j].y & 1023];
 #pragma unroll
-        for (int c = 0; c < NCOL; ++c) acc[c][j] += s_m[c * a.K + g] * d;
+        for (int c = 0; c < NCOL; ++c) {
+          const float m = s_m[c * row + g];
+          acc[c][j][0] += m * d0;
+          acc[c][j][1] += m * d1;
+          acc[c][j][2] += m * d2;
+          acc[c][j][3] += m * d3;
+        }
       }
     }
     __syncthreads();  // the buffer is filled again by the next fetch
@@ -432,9 +457,12 @@ __global__ void __launch_bounds__(NT) k_fmm_m2l_reg(FmmArgs a) {
   for (int col = 0; col < NCOL; ++col) {
     __syncthreads();
 #pragma unroll
-    for (int j = 0; j < PJ; ++j) {
-      const int q = threadIdx.x + j * NT;
-      if (q < npairs) s_acc[q] = acc[col][j];
+    for (int j = 0; j < QJ; ++j) {
+      if (qd[j].x < 0) continue;
+      const int g = (qd[j].y >> 10) & 1023, h = qd[j].y >> 20;
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (h + k < a.K && g < a.hoff[h + k + 1] - a.hoff[h + k]) s_acc[a.hoff[h + k] + g] = acc[col][j][k];
     }
     __syncthreads();
     double *Lt = a.Lc + ((size_t)col * a.ncell + level_off(l) + tc) * a.K;
@@ -789,7 +817,16 @@ namespace {
 
 // shared memory of k_fmm_m2l_reg: two batches of sources, or the pair sums
 size_t m2l_smem(const FmmState &f, int ncol) {
-  return sizeof(float) * std::max<size_t>(2 * gpu::M2L_NB * (size_t)(ncol + 1) * f.K, f.npairs);
+  return sizeof(float) * std::max<size_t>(2 * gpu::M2L_NB * (size_t)(ncol + 1) * gpu::row32(f.K), f.npairs);
+}
+
+constexpr int kQuadsSmall = 288 * 3, kQuadsLarge = 544 * 4;  // of the two shapes of k_fmm_m2l_reg
+
+int alloc_m32(const FmmState &f, FmmTree &t, int ncol) {
+  if (t.M32) cudaFree(t.M32);
+  t.M32 = nullptr;
+  if (f.nquads > kQuadsLarge) return 0;
+  return cudaMalloc((void **)&t.M32, ncol * (size_t)t.ncell * gpu::row32(f.K) * sizeof(float)) != cudaSuccess;
 }
 
 // per-order tables: terms, M2L pairs sorted by target term, unit-offset
@@ -815,6 +852,18 @@ int build_tables(FmmState &f, int p, cudaStream_t st) {
   }
   hoff[f.K] = (int)pairs.size();
   f.npairs = (int)pairs.size();
+  // Target terms h..h+3 against source term g: x the indexes of g + h, + 1, + 2
+  // (10 bits each), y that of g + h + 3, g and h.  Where a quad straddles two
+  // orders its later terms may have no pair with g: index 0, sum not used.
+  std::vector<int2> quads;
+  if (f.npairs <= 4 * kQuadsLarge)
+    for (int h = 0; h < f.K; h += 4)
+      for (int g = 0; g < hoff[h + 1] - hoff[h]; ++g) {
+        int d[4];
+        for (int k = 0; k < 4; ++k) d[k] = h + k < f.K && g < hoff[h + k + 1] - hoff[h + k] ? pairs[hoff[h + k] + g].y : 0;
+        quads.push_back(make_int2(d[0] | d[1] << 10 | d[2] << 20, d[3] | g << 10 | h << 20));
+      }
+  f.nquads = quads.empty() ? kQuadsLarge + 1 : (int)quads.size();
   std::vector<double> dunit((size_t)343 * f.KD, 0.0);
   for (int i = -3; i <= 3; ++i)
     for (int j = -3; j <= 3; ++j)
@@ -857,9 +906,11 @@ int build_tables(FmmState &f, int p, cudaStream_t st) {
     cudaMemcpyAsync(dst, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, st);
     return 0;
   };
-  std::vector<float> dunit32(dunit.begin(), dunit.end());
-  int bad = up(f.terms, terms) | up(f.pairs, pairs) | up(f.hoff, hoff) | up(f.dunit, dunit) |
-            up(f.dunit32, dunit32) | up(f.mm_e, mm_e) |
+  std::vector<float> dunit32((size_t)343 * gpu::row32(f.K), 0.f);
+  for (int o = 0; o < 343; ++o)
+    for (int k = 0; k < f.KD; ++k) dunit32[(size_t)o * gpu::row32(f.K) + k] = (float)dunit[(size_t)o * f.KD + k];
+  int bad = up(f.terms, terms) | up(f.pairs, pairs) | up(f.hoff, hoff) | up(f.quads, quads) |
+            up(f.dunit, dunit) | up(f.dunit32, dunit32) | up(f.mm_e, mm_e) |
             up(f.ll_e, ll_e) | up(f.mm_c, mm_c) | up(f.ll_c, ll_c) | up(f.mm_off, mm_off) | up(f.ll_off, ll_off);
   if (bad) {
     cudaGetLastError();
@@ -870,8 +921,8 @@ int build_tables(FmmState &f, int p, cudaStream_t st) {
   if (smem > 48 * 1024) cudaFuncSetAttribute(gpu::k_fmm_m2l, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   for (int ncol = 1; ncol <= 2; ++ncol) {
     const int b = (int)m2l_smem(f, ncol);
-    const void *k[2] = {ncol == 2 ? (const void *)gpu::k_fmm_m2l_reg<256, 12, 2> : (const void *)gpu::k_fmm_m2l_reg<256, 12, 1>,
-                        ncol == 2 ? (const void *)gpu::k_fmm_m2l_reg<512, 16, 2> : (const void *)gpu::k_fmm_m2l_reg<512, 16, 1>};
+    const void *k[2] = {ncol == 2 ? (const void *)gpu::k_fmm_m2l_reg<288, 3, 2> : (const void *)gpu::k_fmm_m2l_reg<288, 3, 1>,
+                        ncol == 2 ? (const void *)gpu::k_fmm_m2l_reg<544, 4, 2> : (const void *)gpu::k_fmm_m2l_reg<544, 4, 1>};
     if (b > 48 * 1024)
       for (const void *fn : k) cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, b);
   }
@@ -1001,6 +1052,8 @@ void tree_args(const FmmState &f, const FmmTree &t, int ncol, gpu::FmmArgs &a) {
   a.terms = f.terms;
   a.pairs = f.pairs;
   a.hoff = f.hoff;
+  a.quads = f.quads;
+  a.nquads = f.nquads;
   a.dunit = f.dunit;
   a.dunit32 = f.dunit32;
   a.M = t.M;
@@ -1021,23 +1074,23 @@ void run_tree(const FmmState &f, const FmmTree &t, const gpu::FmmArgs &a, int nc
   for (int l = t.L; l >= 3; --l)
     gpu::k_fmm_m2m<<<dim3(1 << (3 * (l - 1)), ncol), 8 * gpu::FT, 8 * (size_t)f.K * sizeof(double), st>>>(a, l);
   const size_t smem_reg = m2l_smem(f, ncol);
-  const bool reg = f.npairs <= 16 * 512;
+  const bool reg = f.nquads <= kQuadsLarge;
   const int c0 = ((1 << 6) - 1) / 7, nc = t.ncell - c0;  // the cells of levels 2..L
   if (reg && t.L >= 2) {
     gpu::k_fmm_m32<<<gpu::sm_count() * 8, 256, 0, st>>>(a, c0, nc);
     gpu::add_launch_count(1);
   }
   int launches = 1;
-  if (f.npairs <= 12 * 256) {
+  if (f.nquads <= kQuadsSmall) {
     if (ncol == 2)
-      gpu::k_fmm_m2l_reg<256, 12, 2><<<nc, 256, smem_reg, st>>>(a);
+      gpu::k_fmm_m2l_reg<288, 3, 2><<<nc, 288, smem_reg, st>>>(a);
     else
-      gpu::k_fmm_m2l_reg<256, 12, 1><<<nc, 256, smem_reg, st>>>(a);
+      gpu::k_fmm_m2l_reg<288, 3, 1><<<nc, 288, smem_reg, st>>>(a);
   } else if (reg) {
     if (ncol == 2)
-      gpu::k_fmm_m2l_reg<512, 16, 2><<<nc, 512, smem_reg, st>>>(a);
+      gpu::k_fmm_m2l_reg<544, 4, 2><<<nc, 544, smem_reg, st>>>(a);
     else
-      gpu::k_fmm_m2l_reg<512, 16, 1><<<nc, 512, smem_reg, st>>>(a);
+      gpu::k_fmm_m2l_reg<544, 4, 1><<<nc, 544, smem_reg, st>>>(a);
   } else {
     for (int l = 2; l <= t.L; ++l) gpu::k_fmm_m2l<<<dim3(1 << (3 * l), ncol), gpu::FT, smem, st>>>(a, l);
     launches = t.L - 1;
@@ -1106,9 +1159,9 @@ int System::fmm_prepare() {
     if (t.M) cudaFree(t.M);
     if (t.Lc) cudaFree(t.Lc);
     t.M = t.Lc = nullptr;
-    bad |= cudaMalloc((void **)&t.M, 2 * (size_t)t.ncell * f.K * (sizeof(double) + sizeof(float))) != cudaSuccess;
+    bad |= cudaMalloc((void **)&t.M, 2 * (size_t)t.ncell * f.K * sizeof(double)) != cudaSuccess;
     bad |= cudaMalloc((void **)&t.Lc, 2 * (size_t)t.ncell * f.K * sizeof(double)) != cudaSuccess;
-    t.M32 = t.M ? reinterpret_cast<float *>(t.M + 2 * (size_t)t.ncell * f.K) : nullptr;
+    bad |= alloc_m32(f, t, 2);
     t.nalloc_cell = t.ncell;
   }
   if (f.field_n < 6 * (size_t)n) {
@@ -1139,8 +1192,8 @@ int System::fmm_prepare() {
 // The expansions (P2M to L2L: FP64 and latency bound) and the near field (FP32
 // bound) need each other only in L2P.  They run on two streams, the expansions
 // at the highest priority so that their short kernels get in between the
-// near field's CTAs: 60,000 sites, a product 3.33 to 3.02 ms (near field alone
-// 1.80, M2L, also FP32 bound, 0.74).
+// near field's CTAs: 60,000 sites, a product 3.33 to 3.02 ms when that was
+// measured (near field alone 1.80, M2L 0.74), 2.35 with their present kernels.
 int System::fmm_tmu(int ncol, const double *x, double *y, bool dodiag) {
   int st = fmm_prepare();
   if (st) return st;
@@ -1263,9 +1316,9 @@ int System::fmm_m2d(double *out, bool &done) {
       if (t.M) cudaFree(t.M);
       if (t.Lc) cudaFree(t.Lc);
       t.M = t.Lc = nullptr;
-      bad |= cudaMalloc((void **)&t.M, (size_t)t.ncell * f.K * (sizeof(double) + sizeof(float))) != cudaSuccess;
+      bad |= cudaMalloc((void **)&t.M, (size_t)t.ncell * f.K * sizeof(double)) != cudaSuccess;
       bad |= cudaMalloc((void **)&t.Lc, (size_t)t.ncell * f.K * sizeof(double)) != cudaSuccess;
-      t.M32 = t.M ? reinterpret_cast<float *>(t.M + (size_t)t.ncell * f.K) : nullptr;
+      bad |= alloc_m32(f, t, 1);
       t.nalloc_cell = t.ncell;
     }
     if (bad) {

@@ -21,3 +21,21 @@ def test_fmm_columns_do_not_mix(order, tmp_path):
     for k in range(2):
         assert np.array_equal(y[k], g.tmatvec(x[k]))
     assert 0 < np.linalg.norm(y - d) / np.linalg.norm(d) < 0.02
+
+
+# relative errors of the products of the same cluster by the M2L kernel that
+# gave each (target term, source term) pair its own loads
+_ERR = {2: 3.10e-3, 3: 1.75e-3, 4: 9.61e-4, 6: 3.26e-4, 7: 1.96e-4, 8: 1.26e-4, 9: 8.32e-5, 10: 5.24e-5}
+
+
+@pytest.mark.parametrize("order", sorted(_ERR))
+def test_fmm_truncation_by_order(order, tmp_path):
+    """The FP32 M2L at each order (rows of 10 to 286 terms padded to 16 bytes,
+    quads of target terms that straddle two orders, both launch shapes) keeps
+    the truncation error that the order has: the same sums, so 1 % above."""
+    w = synth.water_cluster(1500, seed=5)
+    g = OMMPSystem(synth.write_mmp(str(tmp_path / "w.mmp"), w))
+    x = np.random.default_rng(order).standard_normal((2, g.pol_atoms, 3))
+    d = g.tmatvec(x)
+    g.set_fmm(True, order=order)
+    assert np.linalg.norm(g.tmatvec(x) - d) / np.linalg.norm(d) < 1.01 * _ERR[order]
