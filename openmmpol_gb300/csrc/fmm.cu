@@ -70,11 +70,6 @@ struct FmmState {
   int2 *quads = nullptr;       // the pairs by four target terms (build_tables)
   double *dunit = nullptr;     // [343][KD] derivatives of 1/r to order p at unit cell offsets
   float *dunit32 = nullptr;    // the same in FP32, [343][row32(K)] (the FP32 M2L)
-  // translation lists (M2M, L2L), grouped by target term: source term and
-  // packed |m| (bits 0-7) with the parities of m (bits 8-10), coefficient
-  int2 *mm_e = nullptr, *ll_e = nullptr;
-  double *mm_c = nullptr, *ll_c = nullptr;
-  int *mm_off = nullptr, *ll_off = nullptr;
   FmmTree d2d, m2d;            // polarizable sites; static sources with polarizable targets
   double *field = nullptr;     // [2][n][3]
   double *near = nullptr;      // T.mu near-field partials [kFmmNearSplit][2][n][3], after field
@@ -102,8 +97,7 @@ void free_tree(FmmTree &t) {
 
 void free_fmm_state(FmmState *f) {
   if (!f) return;
-  void *b[] = {f->terms, f->pairs, f->hoff, f->quads, f->dunit, f->dunit32, f->field, f->mm_e, f->ll_e, f->mm_c,
-               f->ll_c, f->mm_off, f->ll_off};
+  void *b[] = {f->terms, f->pairs, f->hoff, f->quads, f->dunit, f->dunit32, f->field};
   for (void *p : b)
     if (p) cudaFree(p);
   free_tree(f->d2d);
@@ -143,18 +137,10 @@ struct FmmArgs {
   double *M, *Lc;
   float *M32;
   int KD;
-  const int2 *mm_e, *ll_e;
-  const double *mm_c, *ll_c;
-  const int *mm_off, *ll_off;
 };
 
 // sign of s^m for the child offset s = (b - 1/2) h_c per axis (bit b = 0:
 // negative component) and the parities packed in e.y bits 8-10
-__device__ __forceinline__ double child_sign(int packed, int bx, int by, int bz) {
-  const int neg = (((packed >> 8) & 1) & (bx ^ 1)) ^ (((packed >> 9) & 1) & (by ^ 1)) ^ (((packed >> 10) & 1) & (bz ^ 1));
-  return neg ? -1.0 : 1.0;
-}
-
 __device__ __forceinline__ void cell_xyz(int idx, int l, int &x, int &y, int &z) {
   const int n = 1 << l;
   z = idx % n;
@@ -216,41 +202,61 @@ __global__ void __launch_bounds__(512) k_fmm_p2m(FmmArgs a, const double *__rest
   if (t < a.K) a.M[((size_t)col * a.ncell + level_off(a.L) + c) * a.K + t] = acc;
 }
 
+// index of the term (a, b, c); first: that of each order's first term
+__device__ __forceinline__ int term_at(const int *first, int a, int b, int c) {
+  const int u = b + c;
+  return first[a + u] + u * (u + 1) / 2 + c;
+}
+
+constexpr int TT = 256;  // threads of the translations
+
 // parents at level l - 1 from their children at level l:
 // M_g(parent) = sum_children sum_(k <= g) M_k(child) s^(g - k) / (g - k)!
-// The eight children are worked on side by side (FT threads each) and added
-// in order: one after another they were a chain of 8 K loads (256 -> 167 us at
-// order 10, 64 parents; latency of the longest term's list).
-__global__ void __launch_bounds__(8 * FT) k_fmm_m2m(FmmArgs a, int l) {
-  extern __shared__ double s_w[];  // [8][K]
+// One direction after the other (z, y, x), the two children that differ in it
+// added on the way: sums of up to p + 1 terms over 4, 2 and 1 sets instead of
+// 28 products of three directions on average for each child, their lists read
+// from global memory (64 parents at order 10: 166 -> 23 us).
+__global__ void __launch_bounds__(TT) k_fmm_m2m(FmmArgs a, int l) {
+  extern __shared__ double s_w[];  // [8][K] and [4][K]
+  __shared__ int s_first[fmm::kMaxOrder + 1];
+  __shared__ double s_c[fmm::kMaxOrder + 1];  // (h_c / 2)^j / j!
   const int pc = blockIdx.x, col = blockIdx.y;
   if (a.cnt[level_off(l - 1) + pc] == 0) return;
   int px, py, pz;
   cell_xyz(pc, l - 1, px, py, pz);
-  double hp[fmm::kMaxOrder + 1];  // (h_c / 2)^k
-  hp[0] = 1.0;
-  for (int k = 1; k <= a.p; ++k) hp[k] = hp[k - 1] * 0.5 * a.h0 / (1 << l);
-  const int ch = threadIdx.x / FT, lane = threadIdx.x % FT;
-  const int bx = ch >> 2, by = (ch >> 1) & 1, bz = ch & 1;
-  const int cc = cell_idx(l, 2 * px + bx, 2 * py + by, 2 * pz + bz);
-  const bool any = a.cnt[level_off(l) + cc] != 0;
-  const double *Mc = a.M + ((size_t)col * a.ncell + level_off(l) + cc) * a.K;
-  for (int t = lane; t < a.K; t += FT) {
-    double w = 0.0;
-    if (any)
-      for (int e = a.mm_off[t]; e < a.mm_off[t + 1]; ++e) {
-        const int2 ent = a.mm_e[e];
-        w += Mc[ent.x] * a.mm_c[e] * hp[ent.y & 255] * child_sign(ent.y, bx, by, bz);
-      }
-    s_w[ch * a.K + t] = w;
+  if ((int)threadIdx.x <= a.p) {
+    s_first[threadIdx.x] = fmm::nterms((int)threadIdx.x - 1);
+    const double hh = 0.5 * a.h0 / (1 << l);
+    double f = 1.0;
+    for (int j = 1; j <= (int)threadIdx.x; ++j) f *= hh / j;
+    s_c[threadIdx.x] = f;
+  }
+  for (int i = threadIdx.x; i < 8 * a.K; i += TT) {
+    const int ch = i / a.K;
+    const int cc = cell_idx(l, 2 * px + (ch >> 2), 2 * py + ((ch >> 1) & 1), 2 * pz + (ch & 1));
+    s_w[i] = a.M[((size_t)col * a.ncell + level_off(l) + cc) * a.K + (i - ch * a.K)];  // zero without sources
   }
   __syncthreads();
-  double *Mp = a.M + ((size_t)col * a.ncell + level_off(l - 1) + pc) * a.K;
-  for (int t = threadIdx.x; t < a.K; t += 8 * FT) {
-    double s = 0.0;
-    for (int k = 0; k < 8; ++k) s += s_w[k * a.K + t];
-    Mp[t] = s;
-  }
+  // out[o] from in[2 o] (shifted by -h_c / 2 in the direction) and in[2 o + 1]
+  auto pass = [&](const double *in, int nout, double *out, int dx, int dy, int dz) {
+    for (int i = threadIdx.x; i < nout * a.K; i += TT) {
+      const int o = i / a.K, t = i - o * a.K;
+      const short4 e = a.terms[t];
+      const double *lo = in + 2 * o * a.K, *hi = lo + a.K;
+      const int m = dx ? e.x : dy ? e.y : e.z;
+      double w = 0.0;
+      for (int j = 0; j <= m; ++j) {
+        const int k = term_at(s_first, e.x - dx * j, e.y - dy * j, e.z - dz * j);
+        w = fma(s_c[j], (j & 1) ? hi[k] - lo[k] : hi[k] + lo[k], w);
+      }
+      out[i] = w;
+    }
+    __syncthreads();
+  };
+  double *s_v = s_w + 8 * a.K;
+  pass(s_w, 4, s_v, 0, 0, 1);
+  pass(s_v, 2, s_w, 0, 1, 0);
+  pass(s_w, 1, a.M + ((size_t)col * a.ncell + level_off(l - 1) + pc) * a.K, 1, 0, 0);
 }
 
 // local expansions at level l from the well-separated cells of the level
@@ -482,24 +488,62 @@ __global__ void __launch_bounds__(NT) k_fmm_m2l_reg(FmmArgs a) {
 
 // children at level l + 1 from their parent at level l:
 // L_k(child) += sum_(h >= k) L_h(parent) h! / (k! (h - k)!) t^(h - k)
-__global__ void __launch_bounds__(FT) k_fmm_l2l(FmmArgs a, int l) {
-  const int cc = blockIdx.x, col = blockIdx.y;
-  if (a.cnt_t[level_off(l + 1) + cc] == 0) return;
-  int cx, cy, cz;
-  cell_xyz(cc, l + 1, cx, cy, cz);
-  double hp[fmm::kMaxOrder + 1];  // (h_c / 2)^k
-  hp[0] = 1.0;
-  for (int k = 1; k <= a.p; ++k) hp[k] = hp[k - 1] * 0.5 * a.h0 / (1 << (l + 1));
-  const int bx = cx & 1, by = cy & 1, bz = cz & 1;
-  const double *Lp = a.Lc + ((size_t)col * a.ncell + level_off(l) + cell_idx(l, cx >> 1, cy >> 1, cz >> 1)) * a.K;
-  double *Lch = a.Lc + ((size_t)col * a.ncell + level_off(l + 1) + cc) * a.K;
-  for (int k = threadIdx.x; k < a.K; k += FT) {
-    double w = 0.0;
-    for (int e = a.ll_off[k]; e < a.ll_off[k + 1]; ++e) {
-      const int2 ent = a.ll_e[e];
-      w += Lp[ent.x] * a.ll_c[e] * hp[ent.y & 255] * child_sign(ent.y, bx, by, bz);
+// One direction after the other, the even and odd powers of t apart, so that
+// the two children that differ in it share one sum (512 children at order 10,
+// as lists of products per child 128 us, now 23).
+__global__ void __launch_bounds__(TT) k_fmm_l2l(FmmArgs a, int l) {
+  extern __shared__ double s_w[];  // [1][K], [2][K] and [4][K]
+  __shared__ int s_first[fmm::kMaxOrder + 1];
+  __shared__ double s_c[(fmm::kMaxOrder + 1) * (fmm::kMaxOrder + 1)];  // [k][j] (k + j over k) (h_c / 2)^j
+  const int pc = blockIdx.x, col = blockIdx.y;
+  if (a.cnt_t[level_off(l) + pc] == 0) return;
+  int px, py, pz;
+  cell_xyz(pc, l, px, py, pz);
+  const int p1 = a.p + 1;
+  if ((int)threadIdx.x < p1) s_first[threadIdx.x] = fmm::nterms((int)threadIdx.x - 1);
+  if ((int)threadIdx.x < p1 * p1) {
+    const int k = threadIdx.x / p1, m = threadIdx.x % p1;
+    const double hh = 0.5 * a.h0 / (1 << (l + 1));
+    double b = 1.0, f = 1.0;
+    for (int j = 1; j <= m; ++j) {
+      b = b * (k + j) / j;
+      f *= hh;
     }
-    Lch[k] += w;
+    s_c[threadIdx.x] = b * f;
+  }
+  for (int i = threadIdx.x; i < a.K; i += TT) s_w[i] = a.Lc[((size_t)col * a.ncell + level_off(l) + pc) * a.K + i];
+  __syncthreads();
+  // term t of the sets 2 o (shifted by -h_c / 2 in the direction) and 2 o + 1 from in[o]
+  auto shift = [&](const double *in, int t, int dx, int dy, int dz, double &lo, double &hi) {
+    const short4 e = a.terms[t];
+    const double *c = s_c + (dx ? e.x : dy ? e.y : e.z) * p1;
+    double even = 0.0, odd = 0.0;
+    for (int j = 0; j <= a.p - e.w; ++j) {
+      const double v = in[term_at(s_first, e.x + dx * j, e.y + dy * j, e.z + dz * j)];
+      if (j & 1)
+        odd = fma(c[j], v, odd);
+      else
+        even = fma(c[j], v, even);
+    }
+    lo = even - odd;
+    hi = even + odd;
+  };
+  double *s_x = s_w + a.K, *s_y = s_x + 2 * a.K;
+  for (int t = threadIdx.x; t < a.K; t += TT) shift(s_w, t, 1, 0, 0, s_x[t], s_x[a.K + t]);
+  __syncthreads();
+  for (int i = threadIdx.x; i < 2 * a.K; i += TT) {
+    const int o = i / a.K, t = i - o * a.K;
+    shift(s_x + o * a.K, t, 0, 1, 0, s_y[2 * o * a.K + t], s_y[(2 * o + 1) * a.K + t]);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < 4 * a.K; i += TT) {
+    const int o = i / a.K, t = i - o * a.K;
+    double w[2];
+    shift(s_y + o * a.K, t, 0, 0, 1, w[0], w[1]);
+    for (int bz = 0; bz < 2; ++bz) {
+      const int cc = cell_idx(l + 1, 2 * px + (o >> 1), 2 * py + (o & 1), 2 * pz + bz);
+      if (a.cnt_t[level_off(l + 1) + cc]) a.Lc[((size_t)col * a.ncell + level_off(l + 1) + cc) * a.K + t] += w[bz];
+    }
   }
 }
 
@@ -830,7 +874,7 @@ int alloc_m32(const FmmState &f, FmmTree &t, int ncol) {
 }
 
 // per-order tables: terms, M2L pairs sorted by target term, unit-offset
-// derivative tensors, M2M / L2L translation lists
+// derivative tensors
 int build_tables(FmmState &f, int p, cudaStream_t st) {
   f.p = p;
   f.K = fmm::nterms(p);
@@ -871,36 +915,6 @@ int build_tables(FmmState &f, int p, cudaStream_t st) {
         if (std::abs(i) <= 1 && std::abs(j) <= 1 && std::abs(k) <= 1) continue;
         fmm::derivatives(i, j, k, p, &dunit[(size_t)(((i + 3) * 7 + (j + 3)) * 7 + (k + 3)) * f.KD]);
       }
-  std::vector<int2> mm_e, ll_e;
-  std::vector<double> mm_c, ll_c;
-  std::vector<int> mm_off(f.K + 1, 0), ll_off(f.K + 1, 0);
-  auto fact = [](int k) {
-    double r = 1.0;
-    for (int i = 2; i <= k; ++i) r *= i;
-    return r;
-  };
-  auto pack = [](int mx, int my, int mz) { return (mx + my + mz) | ((mx & 1) << 8) | ((my & 1) << 9) | ((mz & 1) << 10); };
-  for (int t = 0; t < f.K; ++t) {
-    const short4 e = terms[t];
-    mm_off[t] = (int)mm_e.size();
-    for (int k = 0; k < f.K; ++k) {
-      const short4 q = terms[k];
-      if (q.x > e.x || q.y > e.y || q.z > e.z) continue;
-      const int mx = e.x - q.x, my = e.y - q.y, mz = e.z - q.z;
-      mm_e.push_back(make_int2(k, pack(mx, my, mz)));
-      mm_c.push_back(1.0 / (fact(mx) * fact(my) * fact(mz)));
-    }
-    ll_off[t] = (int)ll_e.size();
-    for (int h = 0; h < f.K; ++h) {
-      const short4 q = terms[h];
-      if (q.x < e.x || q.y < e.y || q.z < e.z) continue;
-      const int mx = q.x - e.x, my = q.y - e.y, mz = q.z - e.z;
-      ll_e.push_back(make_int2(h, pack(mx, my, mz)));
-      ll_c.push_back(fact(q.x) * fact(q.y) * fact(q.z) / (fact(e.x) * fact(e.y) * fact(e.z) * fact(mx) * fact(my) * fact(mz)));
-    }
-  }
-  mm_off[f.K] = (int)mm_e.size();
-  ll_off[f.K] = (int)ll_e.size();
   auto up = [&](auto *&dst, const auto &v) {
     if (cudaMalloc((void **)&dst, std::max<size_t>(v.size(), 1) * sizeof(v[0])) != cudaSuccess) return 1;
     cudaMemcpyAsync(dst, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice, st);
@@ -910,8 +924,7 @@ int build_tables(FmmState &f, int p, cudaStream_t st) {
   for (int o = 0; o < 343; ++o)
     for (int k = 0; k < f.KD; ++k) dunit32[(size_t)o * gpu::row32(f.K) + k] = (float)dunit[(size_t)o * f.KD + k];
   int bad = up(f.terms, terms) | up(f.pairs, pairs) | up(f.hoff, hoff) | up(f.quads, quads) |
-            up(f.dunit, dunit) | up(f.dunit32, dunit32) | up(f.mm_e, mm_e) |
-            up(f.ll_e, ll_e) | up(f.mm_c, mm_c) | up(f.ll_c, ll_c) | up(f.mm_off, mm_off) | up(f.ll_off, ll_off);
+            up(f.dunit, dunit) | up(f.dunit32, dunit32);
   if (bad) {
     cudaGetLastError();
     set_last_error("out of device memory for the FMM tables");
@@ -1059,12 +1072,6 @@ void tree_args(const FmmState &f, const FmmTree &t, int ncol, gpu::FmmArgs &a) {
   a.M = t.M;
   a.M32 = t.M32;
   a.Lc = t.Lc;
-  a.mm_e = f.mm_e;
-  a.ll_e = f.ll_e;
-  a.mm_c = f.mm_c;
-  a.ll_c = f.ll_c;
-  a.mm_off = f.mm_off;
-  a.ll_off = f.ll_off;
 }
 
 // upward pass from the leaf multipoles, M2L, downward pass (columns of a)
@@ -1072,7 +1079,7 @@ void run_tree(const FmmState &f, const FmmTree &t, const gpu::FmmArgs &a, int nc
   const size_t smem = (f.K + (size_t)f.npairs) * sizeof(double);
   // no cell above level 2 has well-separated neighbours: their multipoles are not needed
   for (int l = t.L; l >= 3; --l)
-    gpu::k_fmm_m2m<<<dim3(1 << (3 * (l - 1)), ncol), 8 * gpu::FT, 8 * (size_t)f.K * sizeof(double), st>>>(a, l);
+    gpu::k_fmm_m2m<<<dim3(1 << (3 * (l - 1)), ncol), gpu::TT, 12 * (size_t)f.K * sizeof(double), st>>>(a, l);
   const size_t smem_reg = m2l_smem(f, ncol);
   const bool reg = f.nquads <= kQuadsLarge;
   const int c0 = ((1 << 6) - 1) / 7, nc = t.ncell - c0;  // the cells of levels 2..L
@@ -1095,7 +1102,7 @@ void run_tree(const FmmState &f, const FmmTree &t, const gpu::FmmArgs &a, int nc
     for (int l = 2; l <= t.L; ++l) gpu::k_fmm_m2l<<<dim3(1 << (3 * l), ncol), gpu::FT, smem, st>>>(a, l);
     launches = t.L - 1;
   }
-  for (int l = 2; l < t.L; ++l) gpu::k_fmm_l2l<<<dim3(1 << (3 * (l + 1)), ncol), gpu::FT, 0, st>>>(a, l);
+  for (int l = 2; l < t.L; ++l) gpu::k_fmm_l2l<<<dim3(1 << (3 * l), ncol), gpu::TT, 7 * (size_t)f.K * sizeof(double), st>>>(a, l);
   gpu::add_launch_count(std::max(0, t.L - 2) + launches + std::max(0, t.L - 2));
 }
 
@@ -1193,7 +1200,7 @@ int System::fmm_prepare() {
 // bound) need each other only in L2P.  They run on two streams, the expansions
 // at the highest priority so that their short kernels get in between the
 // near field's CTAs: 60,000 sites, a product 3.33 to 3.02 ms when that was
-// measured (near field alone 1.80, M2L 0.74), 2.35 with their present kernels.
+// measured (near field alone 1.80, M2L 0.74), 2.25 with their present kernels.
 int System::fmm_tmu(int ncol, const double *x, double *y, bool dodiag) {
   int st = fmm_prepare();
   if (st) return st;
