@@ -116,7 +116,7 @@ constexpr int FT = 128;  // threads per CTA
 // floats of a row of the FP32 M2L's inputs: whole 16-byte copies
 __host__ __device__ constexpr int row32(int K) { return (K + 3) & ~3; }
 
-constexpr int FCH = 32;  // sites staged per chunk in the P2M
+constexpr int FCH = 32;  // sites staged per chunk in the P2M of the static multipoles
 constexpr int kMaxTermsPerThread = (fmm::nterms(fmm::kMaxOrder) + FT - 1) / FT;
 
 struct FmmArgs {
@@ -154,13 +154,19 @@ __device__ __forceinline__ int cell_idx(int l, int x, int y, int z) {
 __device__ __forceinline__ int level_off(int l) { return ((1 << (3 * l)) - 1) / 7; }
 
 // leaf multipoles of the dipoles x [col][n][3], one term per thread (blockDim
-// covers K): with the powers v^m / m! of a site and the same shifted by one
-// and times the dipole (A), a term's share is
-//   Ax[a] Y[b] Z[c] + X[a] (Ay[b] Z[c] + Y[b] Az[c]),
-// five FP64 operations (the three products formed apart: 12; 502 -> 283 us
-// at 60,000 sites, order 10).  FP64 pipe.
+// covers K): with the powers v^m / m! of a site (X, Y, Z) and the same shifted
+// by one and times the dipole (A), a term's share is
+//   U[ab] Z[c] + V[ab] Az[c],  U = Ax[a] Y[b] + X[a] Ay[b],  V = X[a] Y[b],
+// U and V once per site and pair (a, b): about 2.7 FP64 operations a term
+// (five with the sum formed per term, and a division for each power: 283 us at
+// 60,000 sites, order 10; now 157, 69 of them the FP64 pipe's).
+constexpr int PCH = 16;                                                     // sites per chunk
+constexpr int kMaxAB = (fmm::kMaxOrder + 1) * (fmm::kMaxOrder + 2) / 2;  // pairs (a, b), a + b <= p
+
 __global__ void __launch_bounds__(512) k_fmm_p2m(FmmArgs a, const double *__restrict__ x, int n) {
-  __shared__ double s_p[3][fmm::kMaxOrder + 1][FCH + 1], s_a[3][fmm::kMaxOrder + 1][FCH + 1];
+  __shared__ double s_p[3][fmm::kMaxOrder + 1][PCH + 1], s_a[3][fmm::kMaxOrder + 1][PCH + 1];
+  __shared__ double s_u[kMaxAB][PCH + 1], s_v[kMaxAB][PCH + 1], s_r[fmm::kMaxOrder + 1];
+  __shared__ short2 s_ab[kMaxAB];
   const int c = blockIdx.x, col = blockIdx.y;
   const int s0 = a.leaf_start[c], s1 = a.leaf_start[c + 1];
   if (s0 == s1) return;
@@ -169,12 +175,16 @@ __global__ void __launch_bounds__(512) k_fmm_p2m(FmmArgs a, const double *__rest
   const double h = a.h0 / (1 << a.L);
   const int t = threadIdx.x;
   const short4 e = t < a.K ? a.terms[t] : make_short4(0, 0, 0, 0);
+  const int nab = (a.p + 1) * (a.p + 2) / 2, ab = (e.x + e.y) * (e.x + e.y + 1) / 2 + e.y;
+  if (t < a.K && e.z == 0) s_ab[ab] = make_short2(e.x, e.y);
+  if (t > 0 && t <= a.p) s_r[t] = 1.0 / t;
   double acc = 0.0;
-  for (int b0 = s0; b0 < s1; b0 += FCH) {
+  for (int b0 = s0; b0 < s1; b0 += PCH) {
+    const int cnt = min(PCH, s1 - b0);
     __syncthreads();
-    for (int i = threadIdx.x; i < 3 * FCH; i += blockDim.x) {
-      const int d = i / FCH, k = i % FCH;
-      if (b0 + k >= s1) continue;
+    for (int i = threadIdx.x; i < 3 * PCH; i += blockDim.x) {
+      const int d = i / PCH, k = i % PCH;
+      if (k >= cnt) continue;
       const Pos64 ps = a.spos[b0 + k];
       const double v = d == 0 ? ps.x - (a.ox + (cx + 0.5) * h) : d == 1 ? ps.y - (a.oy + (cy + 0.5) * h)
                                                                         : ps.z - (a.oz + (cz + 0.5) * h);
@@ -184,19 +194,23 @@ __global__ void __launch_bounds__(512) k_fmm_p2m(FmmArgs a, const double *__rest
       s_a[d][0][k] = 0.0;
       for (int m = 1; m <= a.p; ++m) {
         s_a[d][m][k] = mu * pw;
-        pw = pw * v * (1.0 / m);
+        pw = pw * v * s_r[m];
         s_p[d][m][k] = pw;
       }
     }
     __syncthreads();
-    const int cnt = min(FCH, s1 - b0);
+    for (int i = threadIdx.x; i < nab * PCH; i += blockDim.x) {
+      const int j = i / PCH, k = i % PCH;
+      if (k >= cnt) continue;
+      const short2 w = s_ab[j];
+      const double X = s_p[0][w.x][k], Y = s_p[1][w.y][k];
+      s_u[j][k] = fma(s_a[0][w.x][k], Y, X * s_a[1][w.y][k]);
+      s_v[j][k] = X * Y;
+    }
+    __syncthreads();
     if (t >= a.K) continue;
     double w = 0.0;
-    for (int q = 0; q < cnt; ++q) {
-      const double Y = s_p[1][e.y][q], Z = s_p[2][e.z][q];
-      w = fma(s_a[0][e.x][q], Y * Z, w);
-      w = fma(s_p[0][e.x][q], fma(s_a[1][e.y][q], Z, Y * s_a[2][e.z][q]), w);
-    }
+    for (int q = 0; q < cnt; ++q) w = fma(s_u[ab][q], s_p[2][e.z][q], fma(s_v[ab][q], s_a[2][e.z][q], w));
     acc += w;
   }
   if (t < a.K) a.M[((size_t)col * a.ncell + level_off(a.L) + c) * a.K + t] = acc;
@@ -1200,7 +1214,7 @@ int System::fmm_prepare() {
 // bound) need each other only in L2P.  They run on two streams, the expansions
 // at the highest priority so that their short kernels get in between the
 // near field's CTAs: 60,000 sites, a product 3.33 to 3.02 ms when that was
-// measured (near field alone 1.80, M2L 0.74), 2.25 with their present kernels.
+// measured (near field alone 1.80, M2L 0.74), 2.13 with their present kernels.
 int System::fmm_tmu(int ncol, const double *x, double *y, bool dodiag) {
   int st = fmm_prepare();
   if (st) return st;
