@@ -22,8 +22,8 @@
 //   k_fmm_l2l     children's local expansions from the parent's
 //   k_fmm_near    (fmm_near.cu) the near field of the 27 neighbouring leaves,
 //                 direct, with the Thole damping of the direct kernels
-//   k_fmm_l2p     far field of the leaf's local expansion at each site plus
-//                 the near field's partial sums
+//   k_fmm_l2p     far field of the leaf's local expansion at each site
+//   k_fmm_add_near  the near field's partial sums added to it
 // then the finishing pass of the direct product (scaled-pair corrections
 // with exact pair terms, sign, 1/alpha diagonal).  Sites are kept in leaf
 // order on the device (a counting sort per geometry).
@@ -595,11 +595,9 @@ __device__ __forceinline__ void horner_field(int p, const double *s_H, double X,
   e[2] -= wz;
 }
 
-// far field of the leaf's local expansion at each site of the leaf plus the
-// near field's partial sums (near [kFmmNearSplit][ncol][n][3], fmm_near.cu);
-// field [col][n][3]
-__global__ void __launch_bounds__(FT) k_fmm_l2p(FmmArgs a, int n, const double *__restrict__ near,
-                                                 double *__restrict__ field) {
+// far field of the leaf's local expansion at each site of the leaf; field
+// [col][n][3]
+__global__ void __launch_bounds__(FT) k_fmm_l2p(FmmArgs a, int n, double *__restrict__ field) {
   __shared__ double s_H[fmm::nterms(fmm::kMaxOrder)];
   const int c = blockIdx.x, col = blockIdx.y;
   const int s0 = a.leaf_start[c], s1 = a.leaf_start[c + 1];
@@ -619,12 +617,19 @@ __global__ void __launch_bounds__(FT) k_fmm_l2p(FmmArgs a, int n, const double *
     horner_field(a.p, s_H, pt.x - (a.ox + (cx + 0.5) * h), pt.y - (a.oy + (cy + 0.5) * h),
                  pt.z - (a.oz + (cz + 0.5) * h), e);
     const size_t o = ((size_t)col * n + a.perm[si]) * 3;
-    for (int d = 0; d < 3; ++d) {
-      double s = 0.0;
-      for (int k = 0; k < kFmmNearSplit; ++k) s += near[(size_t)k * a.ncol * n * 3 + o + d];
-      field[o + d] = e[d] + s;
-    }
+    for (int d = 0; d < 3; ++d) field[o + d] = e[d];
   }
+}
+
+// the near field's partial sums (near [kFmmNearSplit][nv], fmm_near.cu) added
+// to the far field
+__global__ void k_fmm_add_near(size_t nv, const double *__restrict__ near, double *__restrict__ field) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nv) return;
+  double s = 0.0;
+#pragma unroll
+  for (int k = 0; k < kFmmNearSplit; ++k) s += near[k * nv + i];
+  field[i] += s;
 }
 
 // leaf multipoles of the static multipoles (charge; dipole and quadrupole
@@ -1210,11 +1215,11 @@ int System::fmm_prepare() {
   return kOk;
 }
 
-// The expansions (P2M to L2L: FP64 and latency bound) and the near field (FP32
-// bound) need each other only in L2P.  They run on two streams, the expansions
+// The expansions (P2M to L2P: FP64 and latency bound) and the near field (FP32
+// bound) meet only in the sum of the two fields.  They run on two streams, the expansions
 // at the highest priority so that their short kernels get in between the
 // near field's CTAs: 60,000 sites, a product 3.33 to 3.02 ms when that was
-// measured (near field alone 1.80, M2L 0.74), 2.13 with their present kernels.
+// measured (near field alone 1.80, M2L 0.74), 2.05 with their present kernels and L2P beside it too.
 int System::fmm_tmu(int ncol, const double *x, double *y, bool dodiag) {
   int st = fmm_prepare();
   if (st) return st;
@@ -1247,13 +1252,14 @@ int System::fmm_tmu(int ncol, const double *x, double *y, bool dodiag) {
     const int nleaf = 1 << (3 * t.L);
     gpu::k_fmm_p2m<<<dim3(nleaf, g), (f.K + 31) / 32 * 32, 0, f.far>>>(a, xg, n);
     run_tree(f, t, a, g, f.far);
+    gpu::k_fmm_l2p<<<dim3(nleaf, g), gpu::FT, 0, f.far>>>(a, n, f.field);
     cudaEventRecord(f.join, f.far);
     gpu::launch_max_word(g * nv, xg, f.word, st_);
     gpu::launch_fmm_near({n, t.L, g, m_.amoeba, t.leaf_start, t.perm, t.split, t.spos, t.sa, t.swa, d_.damp_thr, thr2m},
                          xg, f.word, f.near, st_);
     cudaStreamWaitEvent(st_, f.join, 0);
-    gpu::k_fmm_l2p<<<dim3(nleaf, g), gpu::FT, 0, st_>>>(a, n, f.near, f.field);
-    gpu::add_launch_count(2);
+    gpu::k_fmm_add_near<<<(unsigned)((g * nv + 255) / 256), 256, 0, st_>>>(g * nv, f.near, f.field);
+    gpu::add_launch_count(3);
     gpu::launch_tmu_finish64(d_, g, f.field, xg, dodiag, y + c0 * nv, st_);
   }
   return check(cudaGetLastError(), "FMM T.mu launch");
