@@ -1216,10 +1216,10 @@ int System::fmm_prepare() {
 }
 
 // The expansions (P2M to L2P: FP64 and latency bound) and the near field (FP32
-// bound) meet only in the sum of the two fields.  They run on two streams, the expansions
-// at the highest priority so that their short kernels get in between the
-// near field's CTAs: 60,000 sites, a product 3.33 to 3.02 ms when that was
-// measured (near field alone 1.80, M2L 0.74), 2.05 with their present kernels and L2P beside it too.
+// bound) meet only in the sum of the two fields.  They run on two streams, the
+// expansions at the highest priority so that their short kernels get in between
+// the near field's CTAs: 60,000 sites, a product 2.05 ms (near field alone 1.60;
+// the kernels one after the other 2.3).
 int System::fmm_tmu(int ncol, const double *x, double *y, bool dodiag) {
   int st = fmm_prepare();
   if (st) return st;

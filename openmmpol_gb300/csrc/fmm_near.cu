@@ -4,8 +4,8 @@
 //
 // All pairs of neighbouring leaves (about 3,300 sources per site on a
 // 60,000-site box) in FP64 took 13.1 ms of a 15.5 ms product, the FP64 pipe
-// busy; this kernel takes 1.78 ms (2.1 ms with a third of the CTAs).  Here they run in double-single on the FP32 pipes (ds_pair.cuh), one
-// target per thread; the pairs that are close or strongly damped are masked
+// busy; this kernel takes 1.60 ms.  Here they run in double-single on the FP32
+// pipes (ds_pair.cuh), one target per thread; the pairs that are close or strongly damped are masked
 // and noted in a list of the target's own, which its thread then forms in
 // FP64 (about 18 sources per site in water).  A CTA takes one leaf and one
 // column of three neighbours, so that uneven leaves do not hold up the GPU (512
