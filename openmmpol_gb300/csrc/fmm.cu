@@ -20,8 +20,9 @@
 //                 shared-memory accumulator summed per target term in a
 //                 fixed order (deterministic)
 //   k_fmm_l2l     children's local expansions from the parent's
-//   k_fmm_near    (fmm_near.cu) the near field of the 27 neighbouring leaves,
-//                 direct, with the Thole damping of the direct kernels
+//   k_fmm_near    (fmm_near.cu; k_m2d_leaf of m2d.cu for the static multipoles)
+//                 the near field of the 27 neighbouring leaves, direct, with
+//                 the Thole damping of the direct kernels
 //   k_fmm_l2p     far field of the leaf's local expansion at each site
 //   k_fmm_add_near  the near field's partial sums added to it
 // then the finishing pass of the direct product (scaled-pair corrections
@@ -52,11 +53,10 @@ struct FmmTree {
   int *leaf_start = nullptr, *leaf_start_t = nullptr;  // [nleaf + 1]
   int *perm = nullptr, *perm_t = nullptr;              // sorted -> site index
   gpu::Pos64 *spos = nullptr, *spos_t = nullptr;       // w = 1/thole (inf without Thole factor)
-  double *sa = nullptr, *sa_t = nullptr;               // Thole damping a
-  float2 *swa = nullptr, *swa_t = nullptr;             // FP32 damping pre-test data
+  double *sa = nullptr;                                // T.mu: Thole damping a
+  float2 *swa = nullptr;                               // T.mu: FP32 damping pre-test data
   float4 *split = nullptr;                             // T.mu: split coordinates [3][n] (fmm_near.cu)
   double *sq = nullptr;                                // sorted multipoles [n][ld] (M2D sources)
-  int *tmm = nullptr;                                  // targets' static index (M2D self pair)
   double *M = nullptr, *Lc = nullptr;                  // [2][ncell][K]
   float *M32 = nullptr;  // the M2L input [2][ncell][row32(K)] (k_fmm_m32)
   bool shared = false;                                 // targets are the sources
@@ -86,11 +86,9 @@ void free_tree(FmmTree &t) {
   for (void *p : b)
     if (p) cudaFree(p);
   if (!t.shared) {
-    void *c[] = {t.cnt_t, t.leaf_start_t, t.perm_t, t.spos_t, t.sa_t, t.swa_t, t.tmm};
+    void *c[] = {t.cnt_t, t.leaf_start_t, t.perm_t, t.spos_t};
     for (void *p : c)
       if (p) cudaFree(p);
-  } else if (t.tmm) {
-    cudaFree(t.tmm);
   }
   t = FmmTree();
 }
@@ -125,8 +123,6 @@ struct FmmArgs {
   const int *cnt, *leaf_start, *perm;
   const int *cnt_t;  // targets per cell (M2L / L2L skip cells without targets)
   const Pos64 *spos;
-  const double *sa;
-  const float2 *swa;
   const short4 *terms;
   const int4 *pairs;
   const int *hoff;
@@ -704,85 +700,30 @@ __global__ void __launch_bounds__(FT) k_fmm_p2m_mp(FmmArgs a, const double *__re
   }
 }
 
-// far field of the leaf's local expansion plus the direct damped near field
-// of the static multipoles in the 27 neighbouring leaves at each polarizable
-// target of the leaf; field [n][3] at the targets' polarizable index
-template <bool AMOEBA>
+// the same at targets that are not the sources; field [n][3]
 __global__ void __launch_bounds__(FT) k_fmm_l2p_m2d(FmmArgs a, const int *__restrict__ leaf_start_t,
                                                      const int *__restrict__ perm_t, const Pos64 *__restrict__ spos_t,
-                                                     const double *__restrict__ sa_t, const float2 *__restrict__ swa_t,
-                                                     const int *__restrict__ tmm, const double *__restrict__ sq,
-                                                     double thr, float thr2m, double *__restrict__ field, int *err) {
-  constexpr int LD = AMOEBA ? 10 : 1;
-  __shared__ Pos64 s_pos[FT];
-  __shared__ double s_a[FT];
-  __shared__ float2 s_wa[FT];
-  __shared__ int s_mm[FT];
-  __shared__ double s_q[FT * LD];
+                                                     double *__restrict__ field) {
   __shared__ double s_H[fmm::nterms(fmm::kMaxOrder)];
   const int c = blockIdx.x;
   const int s0 = leaf_start_t[c], s1 = leaf_start_t[c + 1];
   if (s0 == s1) return;
   int cx, cy, cz;
   cell_xyz(c, a.L, cx, cy, cz);
-  const int nl = 1 << a.L;
-  const double h = a.h0 / nl;
-  const double ctr[3] = {a.ox + (cx + 0.5) * h, a.oy + (cy + 0.5) * h, a.oz + (cz + 0.5) * h};
+  const double h = a.h0 / (1 << a.L);
   const double *Lt = a.Lc + ((size_t)level_off(a.L) + c) * a.K;
   for (int t = threadIdx.x; t < a.K; t += FT) {
-    const short4 ex = a.terms[t];
-    s_H[horner_pos(a.p, ex.x, ex.y, ex.z)] = Lt[t];
+    const short4 e = a.terms[t];
+    s_H[horner_pos(a.p, e.x, e.y, e.z)] = Lt[t];
   }
-  int bad = 0;
-  for (int b0 = s0; b0 < s1; b0 += FT) {
-    const int si = b0 + threadIdx.x;
-    const bool valid = si < s1;
-    const Pos64 pt = valid ? spos_t[si] : Pos64{0, 0, 0, 0};
-    const double at = valid && AMOEBA ? sa_t[si] : 0.0;
-    const float2 wat = valid ? swa_t[si] : make_float2(0.f, 0.f);
-    const int self = valid ? tmm[si] : -1;
+  __syncthreads();
+  for (int si = s0 + threadIdx.x; si < s1; si += FT) {
+    const Pos64 pt = spos_t[si];
     double e[3] = {0.0, 0.0, 0.0};
-    __syncthreads();
-    if (valid) horner_field(a.p, s_H, pt.x - ctr[0], pt.y - ctr[1], pt.z - ctr[2], e);
-    for (int ox = -1; ox <= 1; ++ox)
-      for (int oy = -1; oy <= 1; ++oy)
-        for (int oz = -1; oz <= 1; ++oz) {
-          const int X = cx + ox, Y = cy + oy, Z = cz + oz;
-          if (X < 0 || Y < 0 || Z < 0 || X >= nl || Y >= nl || Z >= nl) continue;
-          const int nc = cell_idx(a.L, X, Y, Z);
-          const int r0 = a.leaf_start[nc], r1 = a.leaf_start[nc + 1];
-          for (int t0 = r0; t0 < r1; t0 += FT) {
-            __syncthreads();
-            const int k = t0 + threadIdx.x;
-            if (k < r1) {
-              s_pos[threadIdx.x] = a.spos[k];
-              s_a[threadIdx.x] = AMOEBA ? a.sa[k] : 0.0;
-              s_wa[threadIdx.x] = a.swa[k];
-              s_mm[threadIdx.x] = a.perm[k];
-              for (int d = 0; d < LD; ++d) s_q[threadIdx.x * LD + d] = sq[(size_t)k * LD + d];
-            }
-            __syncthreads();
-            if (!valid) continue;
-            const int cnt = min(FT, r1 - t0);
-            for (int q = 0; q < cnt; ++q) {
-              if (s_mm[q] == self) continue;
-              const Pos64 ps = s_pos[q];
-              const double dx = pt.x - ps.x, dy = pt.y - ps.y, dz = pt.z - ps.z;
-              if (coincident(dx * dx + dy * dy + dz * dz)) {
-                bad = 1;
-                continue;
-              }
-              m2d_pair_f64<AMOEBA, true>(dx, dy, dz, pt.w, ps.w, at, s_a[q], wat, s_wa[q], &s_q[q * LD], thr, thr2m, e[0],
-                                   e[1], e[2]);
-            }
-          }
-        }
-    if (valid) {
-      const int pi = perm_t[si];
-      for (int d = 0; d < 3; ++d) field[(size_t)pi * 3 + d] = e[d];
-    }
+    horner_field(a.p, s_H, pt.x - (a.ox + (cx + 0.5) * h), pt.y - (a.oy + (cy + 0.5) * h),
+                 pt.z - (a.oz + (cz + 0.5) * h), e);
+    for (int d = 0; d < 3; ++d) field[3 * (size_t)perm_t[si] + d] = e[d];
   }
-  if (bad) atomicOr(err, 1);
 }
 
 }  // namespace
@@ -1079,8 +1020,6 @@ void tree_args(const FmmState &f, const FmmTree &t, int ncol, gpu::FmmArgs &a) {
   a.leaf_start = t.leaf_start;
   a.perm = t.perm;
   a.spos = t.spos;
-  a.sa = t.sa;
-  a.swa = t.swa;
   a.terms = f.terms;
   a.pairs = f.pairs;
   a.hoff = f.hoff;
@@ -1180,7 +1119,7 @@ int System::fmm_prepare() {
   t.shared = true;
   int bad = upload(t.cnt, o.cnt_s, st_) | upload(t.leaf_start, o.start_s, st_) | upload(t.perm, o.perm_s, st_) |
             upload(t.spos, spos, st_) | upload(t.sa, sa, st_) | upload(t.swa, swa, st_) | upload(t.split, split, st_);
-  t.cnt_t = t.cnt, t.leaf_start_t = t.leaf_start, t.perm_t = t.perm, t.spos_t = t.spos, t.sa_t = t.sa, t.swa_t = t.swa;
+  t.cnt_t = t.cnt, t.leaf_start_t = t.leaf_start, t.perm_t = t.perm, t.spos_t = t.spos;
   if (t.nalloc_cell < t.ncell) {
     if (t.M) cudaFree(t.M);
     if (t.Lc) cudaFree(t.Lc);
@@ -1282,10 +1221,10 @@ int System::fmm_m2d(double *out, bool &done) {
   FmmState &f = *fmms_;
   FmmTree &t = f.m2d;
   const int n = d_.n, mm = d_.m, ld = m_.ld_cart;
-  if (f.field_n < 3 * (size_t)n) {
+  if (f.field_n < 3 * (size_t)n) {  // far field, parts of the near field
     if (f.field) cudaFree(f.field);
     f.field = nullptr;
-    if (cudaMalloc((void **)&f.field, 3 * (size_t)n * sizeof(double)) != cudaSuccess) {
+    if (cudaMalloc((void **)&f.field, (1 + gpu::kFmmNearSplit) * 3 * (size_t)n * sizeof(double)) != cudaSuccess) {
       cudaGetLastError();
       f.field_n = 0;
       set_last_error("out of device memory for the FMM field");
@@ -1304,29 +1243,16 @@ int System::fmm_m2d(double *out, bool &done) {
       t.built = true;
       return kOk;
     }
-    const double inf = std::numeric_limits<double>::infinity();
     std::vector<gpu::Pos64> spos(mm), spos_t(n);
-    std::vector<double> sa(mm), sa_t(n), sq((size_t)mm * ld);
-    std::vector<float2> swa(mm), swa_t(n);
-    std::vector<int> tmm(n);
+    std::vector<double> sq((size_t)mm * ld);
     for (int s = 0; s < mm; ++s) {
       const int i = o.perm_s[s];
-      const double th = m_.thole[i];
-      const double w = th > 0.0 ? 1.0 / th : inf;
-      const int pi = m_.mm_polar[i];
-      const double a = pi >= 0 ? m_.damping[pi] : 0.0;
-      spos[s] = gpu::Pos64{m_.cmm[3 * (size_t)i], m_.cmm[3 * (size_t)i + 1], m_.cmm[3 * (size_t)i + 2], w};
-      sa[s] = a;
-      swa[s] = make_float2((float)(w * w), (float)(a * a));
+      spos[s] = gpu::Pos64{m_.cmm[3 * (size_t)i], m_.cmm[3 * (size_t)i + 1], m_.cmm[3 * (size_t)i + 2], 0.0};
       for (int c = 0; c < ld; ++c) sq[(size_t)s * ld + c] = m_.q[(size_t)i * ld + c];
     }
     for (int s = 0; s < n; ++s) {
       const int j = o.perm_t[s];
-      const double w = 1.0 / m_.thole[m_.polar_mm[j]];
-      spos_t[s] = gpu::Pos64{xp[3 * (size_t)j], xp[3 * (size_t)j + 1], xp[3 * (size_t)j + 2], w};
-      sa_t[s] = m_.damping[j];
-      swa_t[s] = make_float2((float)(w * w), (float)(m_.damping[j] * m_.damping[j]));
-      tmm[s] = m_.polar_mm[j];
+      spos_t[s] = gpu::Pos64{xp[3 * (size_t)j], xp[3 * (size_t)j + 1], xp[3 * (size_t)j + 2], 0.0};
     }
     t.L = o.L;
     t.h0 = o.side;
@@ -1335,10 +1261,9 @@ int System::fmm_m2d(double *out, bool &done) {
     t.ncell = o.ncell;
     t.shared = false;
     int bad = upload(t.cnt, o.cnt_s, st_) | upload(t.leaf_start, o.start_s, st_) | upload(t.perm, o.perm_s, st_) |
-              upload(t.spos, spos, st_) | upload(t.sa, sa, st_) | upload(t.swa, swa, st_) | upload(t.sq, sq, st_) |
-              upload(t.cnt_t, o.cnt_t, st_) | upload(t.leaf_start_t, o.start_t, st_) |
-              upload(t.perm_t, o.perm_t, st_) | upload(t.spos_t, spos_t, st_) | upload(t.sa_t, sa_t, st_) |
-              upload(t.swa_t, swa_t, st_) | upload(t.tmm, tmm, st_);
+              upload(t.spos, spos, st_) | upload(t.sq, sq, st_) | upload(t.cnt_t, o.cnt_t, st_) |
+              upload(t.leaf_start_t, o.start_t, st_) | upload(t.perm_t, o.perm_t, st_) |
+              upload(t.spos_t, spos_t, st_);
     if (t.nalloc_cell < t.ncell) {
       if (t.M) cudaFree(t.M);
       if (t.Lc) cudaFree(t.Lc);
@@ -1369,15 +1294,11 @@ int System::fmm_m2d(double *out, bool &done) {
   else
     gpu::k_fmm_p2m_mp<false><<<nleaf, gpu::FT, 0, st_>>>(a, t.sq);
   run_tree(f, t, a, 1, st_);
-  const float thr2m = (float)(d_.damp_thr * d_.damp_thr * (1.0 + 1e-5));
-  if (m_.amoeba)
-    gpu::k_fmm_l2p_m2d<true><<<nleaf, gpu::FT, 0, st_>>>(a, t.leaf_start_t, t.perm_t, t.spos_t, t.sa_t, t.swa_t, t.tmm,
-                                                         t.sq, d_.damp_thr, thr2m, f.field, flag_);
-  else
-    gpu::k_fmm_l2p_m2d<false><<<nleaf, gpu::FT, 0, st_>>>(a, t.leaf_start_t, t.perm_t, t.spos_t, t.sa_t, t.swa_t,
-                                                          t.tmm, t.sq, d_.damp_thr, thr2m, f.field, flag_);
+  // the finishing pass sums the far field and the near field's parts in order
+  gpu::k_fmm_l2p_m2d<<<nleaf, gpu::FT, 0, st_>>>(a, t.leaf_start_t, t.perm_t, t.spos_t, f.field);
+  gpu::launch_m2d_leaf(d_, t.L, t.leaf_start, t.perm, t.leaf_start_t, t.perm_t, f.field + 3 * (size_t)n, flag_, st_);
   gpu::add_launch_count(2);
-  gpu::launch_m2d_finish(d_, out, f.field, 1, st_);
+  gpu::launch_m2d_finish(d_, out, f.field, 1 + gpu::kFmmNearSplit, st_);
   done = true;
   return check(cudaGetLastError(), "FMM M2D launch");
 }

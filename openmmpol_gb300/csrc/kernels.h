@@ -138,6 +138,11 @@ struct FmmNearArgs {
 };
 constexpr int kFmmNearSplit = 9;
 void launch_fmm_near(const FmmNearArgs &a, const double *x, const unsigned *word, double *partial, cudaStream_t st);
+// the same for the field of the static multipoles (m2d.cu): sources and targets
+// sorted by leaf (perm: static site, perm_t: polarizable site); partial
+// [kFmmNearSplit][n][3] in polarizable order
+void launch_m2d_leaf(const DevSites &s, int L, const int *leaf_start, const int *perm, const int *leaf_start_t,
+                     const int *perm_t, double *partial, int *err_flag, cudaStream_t st);
 // coordinates x [n][3] about a centre as three floats each, out [3][n]
 void split_coordinates(const double *x, int n, double centre[3], float4 *out);
 // The pairwise FP32 product (tmu32_rows.cu): columns in groups of up to gmax
