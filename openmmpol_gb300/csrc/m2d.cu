@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(NT, 4) k_m2d(const __grid_constant__ DevSites 
 // static multipoles), every pair tested; partial [kFmmNearSplit][n][3].  In FP64
 // (40 operations a pair, one CTA for a leaf and all its neighbours) it was most
 // of the FMM's field: 60,000 sites, order 10, with the coordinate update
-// 31.4 -> 8.1 ms, 24,000 sites 6.5 -> 3.0.  FP32 issue.
+// 31.4 -> 8.1 ms, 24,000 sites 6.5 -> 3.0 (this kernel 3.2 ms).  FP32 issue.
 template <bool AMOEBA>
 __global__ void __launch_bounds__(NT, 4) k_m2d_leaf(const __grid_constant__ DevSites s, int L,
                                                     const int *__restrict__ leaf_start, const int *__restrict__ perm,
