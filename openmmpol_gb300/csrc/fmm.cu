@@ -1140,7 +1140,7 @@ int System::fmm_prepare() {
     t.nalloc_cell = t.ncell;
   }
   if (f.field_n < 6 * (size_t)n) {
-    // field, near-field partials and the scale of their dipoles
+    // field, near-field partials and the scales of their two columns of dipoles
     if (f.field) cudaFree(f.field);
     f.field = nullptr;
     const size_t v = 6 * (size_t)n;
@@ -1203,7 +1203,7 @@ int System::fmm_tmu(int ncol, const double *x, double *y, bool dodiag) {
     run_tree(f, t, a, g, f.far);
     gpu::k_fmm_l2p<<<dim3(nleaf, g), gpu::FT, 0, f.far>>>(a, n, f.field);
     cudaEventRecord(f.join, f.far);
-    gpu::launch_max_word(g * nv, xg, f.word, st_);
+    gpu::launch_max_words(g, nv, xg, f.word, st_);
     gpu::launch_fmm_near({n, t.L, g, m_.amoeba, t.leaf_start, t.perm, t.split, t.spos, t.sa, t.swa, d_.damp_thr, thr2m},
                          xg, f.word, f.near, st_);
     cudaStreamWaitEvent(st_, f.join, 0);

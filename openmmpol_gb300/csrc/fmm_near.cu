@@ -34,7 +34,7 @@ __global__ void __launch_bounds__(NT, 5) k_fmm_near(const __grid_constant__ FmmN
   const int nl = 1 << a.L;
   const int cz = c % nl, cy = (c / nl) % nl, cx = c / (nl * nl);
   const int X = cx + (int)blockIdx.z / 3 - 1, Y = cy + (int)blockIdx.z % 3 - 1;
-  const int ex = dsp_exponent(*word);
+  const int ex = dsp_exponent(word[col]);  // the column's own scale
   const double *xc = x + (size_t)col * n * 3;
   double *out = partial + ((size_t)blockIdx.z * a.ncol + col) * n * 3;
   for (int b0 = s0; b0 < s1; b0 += NT) {

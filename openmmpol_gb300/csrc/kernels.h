@@ -110,8 +110,8 @@ int tmu_sym_groups(const DevSites &s, int nrhs);
 void launch_tmu_f64_sym_groups(const DevSites &s, int nrhs, const double *x, double *y, bool dodiag, double *scratch,
                                cudaStream_t st);
 // its passes for callers that spread a product over launches: accumulators
-// [g][n][3] (lo, then hi) and the two words from bad zeroed and the scale of x
-// found (before the first share), and the sums read out into y = T x, with
+// [g][n][3] (lo, then hi) and the two words from bad zeroed and the scales of
+// the columns of x found (before the first share), and the sums read out into y = T x, with
 // at most max_part partial sums of x.y per column (part [g][*npart])
 void launch_tmu_sym_prepare(const DevSites &s, int g, const double *x, unsigned long long *lo,
                             unsigned long long *bad, cudaStream_t st);
@@ -124,7 +124,7 @@ void launch_max_words(int ncol, size_t nv, const double *x, unsigned *words, cud
 // near field of the FMM (fmm_near.cu): the dipoles x [col][n][3] of the 27
 // neighbouring leaves at every site, sites sorted by leaf (split coordinates
 // [3][n], spos, sa, swa; perm the polarizable index); partial
-// [kFmmNearSplit][col][n][3] in polarizable order, word from launch_max_word
+// [kFmmNearSplit][col][n][3] in polarizable order, word from launch_max_words
 struct FmmNearArgs {
   int n, L, ncol;
   bool amoeba;

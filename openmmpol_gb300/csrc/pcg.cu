@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(TPB) k_cg_step(const __grid_constant__ Table<C
   const Scalar pal(al), mal(-al);
   if (blockIdx.x == 0) {
     if (jb.words && k == 0 && threadIdx.x < 3) jb.words[threadIdx.x] = 0ull;
-    if (jb.emax_stride && threadIdx.x == 0) jb.emax[k] = 0u;
+    if (jb.emax && threadIdx.x == 0) jb.emax[k] = 0u;
   }
   const size_t nv = 3 * (size_t)jb.n, off = (size_t)k * nv;
   T *x = jb.x + off, *r = jb.r + off;
@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(TPB) k_cg_dir(const __grid_constant__ Table<Cg
   if constexpr (sizeof(T) == 8) {
     if (jb.emax) {
       mx = __reduce_max_sync(0xffffffffu, mx);
-      if ((threadIdx.x & 31) == 0 && mx) atomicMax(jb.emax + k * jb.emax_stride, mx);
+      if ((threadIdx.x & 31) == 0 && mx) atomicMax(jb.emax + k, mx);
     }
   }
 }
@@ -384,7 +384,7 @@ __global__ void __launch_bounds__(SMALL_TPB) k_cg_small(const __grid_constant__ 
   mx = __reduce_max_sync(0xffffffffu, mx);
   if ((threadIdx.x & 31) == 0) atomicMax(&s_max, mx);
   __syncthreads();
-  if (threadIdx.x == 0) jb.emax[k * jb.emax_stride] = s_max;
+  if (threadIdx.x == 0) jb.emax[k] = s_max;
 }
 
 // partial sums of a.b per column

@@ -32,10 +32,8 @@ struct CgJob {
   // the next product's accumulators and control words (or null)
   unsigned long long *acc, *words;
   size_t nacc;
-  // largest high word of |p| for the next FP64 product: one word of all columns
-  // (within words) or one per column (or null)
+  // largest high word of |p| of each column for the next FP64 product (or null)
   unsigned *emax;
-  int emax_stride;
   // loop on the device: the condition of the captured loop (0: none), and two
   // words, zero between iterations, where the columns meet to set it
   cudaGraphConditionalHandle loop;

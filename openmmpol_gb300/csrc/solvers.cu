@@ -188,7 +188,7 @@ int System::cg64_ws(Workspace &w, int matv, int ncol, const double *rhs, double 
   job.meet = reinterpret_cast<unsigned *>(w.cols + w.cap);
   job.hist = hist, job.nhist = maxhist_;
   // the direct symmetric product of one column group: its accumulators and
-  // scale are prepared by the steps, its finishing pass sums p.h
+  // scales are prepared by the steps, its finishing pass sums p.h
   const bool sym = direct_symmetric(matv, ncol);
   const size_t C = 3 * (size_t)ncol;
   unsigned long long *lo = reinterpret_cast<unsigned long long *>(sym_scratch_);
@@ -198,7 +198,7 @@ int System::cg64_ws(Workspace &w, int matv, int ncol, const double *rhs, double 
   }
   // the ordered one: the scale of every column
   const bool rows = !sym && direct_rows(matv, ncol);
-  if (rows && gpu::tmu_rows_parts(d_, ncol) > 0) job.emax = row_words_, job.emax_stride = 1;
+  if (rows && gpu::tmu_rows_parts(d_, ncol) > 0) job.emax = row_words_;
   const bool small = !sym && n <= gpu::kCgSmallSites;
   job.max_passes = maxiter_;
   job.init = gpu::kCgInitKeep;

@@ -45,9 +45,10 @@
 // 128-bit fixed-point accumulators (2^-80 resolution) with integer atomics:
 // the sums do not depend on the order of the CTAs.
 //
-// The dipoles are scaled by a power of two per product (sym_prepare: largest
-// magnitude in [2^-12, 2^-11)), so that neither the FP32 range nor the
-// fixed-point resolution depends on their size; k_tmu_sym_finish scales back.
+// The dipoles of each column are scaled by a power of two (sym_prepare: largest
+// magnitude of the column in [2^-12, 2^-11)), so that neither the FP32 range nor
+// the fixed-point resolution depends on their size or on the other column of
+// the group; k_tmu_sym_finish scales back.
 //
 // Built with --fmad=false -ftz=true: every FMA is explicit.
 #include <algorithm>
@@ -178,7 +179,7 @@ __device__ __forceinline__ int sym_pairs(SymSmem<G> &sm, int js, int warp, int l
 // one per lane, both sides straight into the fixed-point sums
 template <int G, bool AMOEBA>
 __device__ __noinline__ void sym_queued(const unsigned short *queue, int count, int lane, int i0, int j0,
-                                        const SymJob &jb, int ex) {
+                                        const SymJob &jb, int ex0, int ex1) {
   const int n = jb.n;
   for (int e = lane; e < count; e += 32) {
     const int q = queue[e], i = i0 + (q >> 5), j = j0 + (q & 31);
@@ -192,6 +193,7 @@ __device__ __noinline__ void sym_queued(const unsigned short *queue, int count, 
     k5 *= 3.0;
 #pragma unroll
     for (int r = 0; r < G; ++r) {
+      const int ex = r ? ex1 : ex0;
       for (int side = 0; side < 2; ++side) {
         const size_t o = ((size_t)r * n + (side ? i : j)) * 3, d = ((size_t)r * n + (side ? j : i)) * 3;
         const double mx = scale_down(jb.x[o], ex), my = scale_down(jb.x[o + 1], ex), mz = scale_down(jb.x[o + 2], ex);
@@ -231,7 +233,9 @@ __global__ void __launch_bounds__(SYM_TILE, G == 1 ? 5 : 3) k_tmu_sym(const __gr
     const int I = unit / jb.nchunk;
     const int ti = I * SYM_TILE + tid;
     const bool vi = ti < n;
-    const int ex = dsp_exponent(*reinterpret_cast<const unsigned *>(jb.bad + 1));
+    int ex[G];
+#pragma unroll
+    for (int c = 0; c < G; ++c) ex[c] = dsp_exponent(reinterpret_cast<const unsigned *>(jb.bad + 1)[c]);
     float tg[9], mih[G][3], mil[G][3];
     {
       const float4 h = vi ? gc[ti] : make_float4(SYM_FAR, SYM_FAR, SYM_FAR, 0.f);
@@ -242,7 +246,7 @@ __global__ void __launch_bounds__(SYM_TILE, G == 1 ? 5 : 3) k_tmu_sym(const __gr
     }
 #pragma unroll
     for (int c = 0; c < C; ++c) {
-      const double m = vi ? scale_down(x[((size_t)(c / 3) * n + ti) * 3 + (c % 3)], ex) : 0.0;
+      const double m = vi ? scale_down(x[((size_t)(c / 3) * n + ti) * 3 + (c % 3)], ex[c / 3]) : 0.0;
       const dsf d = to_ds(m);
       mih[c / 3][c % 3] = d.h;
       mil[c / 3][c % 3] = d.l;
@@ -270,7 +274,7 @@ __global__ void __launch_bounds__(SYM_TILE, G == 1 ? 5 : 3) k_tmu_sym(const __gr
         float f[4 * R] = {h.x, h.y, h.z, m.x, m.y, m.z, l.x, l.y, l.z};
 #pragma unroll
         for (int c = 0; c < C; ++c) {
-          const double mu = v ? scale_down(x[((size_t)(c / 3) * n + sj) * 3 + (c % 3)], ex) : 0.0;
+          const double mu = v ? scale_down(x[((size_t)(c / 3) * n + sj) * 3 + (c % 3)], ex[c / 3]) : 0.0;
           const dsf d = to_ds(mu);
           f[9 + 6 * (c / 3) + c % 3] = d.h;
           f[12 + 6 * (c / 3) + c % 3] = d.l;
@@ -305,7 +309,8 @@ __global__ void __launch_bounds__(SYM_TILE, G == 1 ? 5 : 3) k_tmu_sym(const __gr
             const int queued =
                 sym_pairs<G, true, AMOEBA>(sm, js, warp, lane, self, tg, wai, mih, mil, aih, ail, ajh, ajl);
             __syncwarp();
-            sym_queued<G, AMOEBA>(sm.queue[warp], queued, lane, I * SYM_TILE + warp * 32, J * SYM_TILE + js * 32, jb, ex);
+            sym_queued<G, AMOEBA>(sm.queue[warp], queued, lane, I * SYM_TILE + warp * 32, J * SYM_TILE + js * 32, jb,
+                                  ex[0], ex[G - 1]);
             __syncwarp();
           } else {
             sym_pairs<G, false, AMOEBA>(sm, js, warp, lane, false, tg, make_float2(0.f, 0.f), mih, mil, aih, ail, ajh,
@@ -341,18 +346,20 @@ __global__ void __launch_bounds__(SYM_TILE, G == 1 ? 5 : 3) k_tmu_sym(const __gr
   }
 }
 
-// accumulators (if any) to zero and the largest high word of |x| (ctl, zeroed
-// before)
+// column blockIdx.y: its accumulators (if any; the columns' low words, then
+// their high words) to zero and its largest high word of |x| (ctl, zeroed
+// before: one word per column, or two per group of group_words unsigneds)
 __global__ void __launch_bounds__(256) k_sym_prepare(size_t total, const double *__restrict__ x,
                                                      unsigned long long *__restrict__ acc, unsigned *ctl,
-                                                     size_t ctl_stride) {
-  x += (size_t)blockIdx.y * total;  // column groups
-  ctl += ctl_stride * blockIdx.y;
+                                                     size_t group_words) {
+  const size_t col = (size_t)blockIdx.y * total;
+  x += col;
+  ctl += group_words ? (blockIdx.y / 2) * group_words + blockIdx.y % 2 : blockIdx.y;
   unsigned m = 0;
   for (size_t k = (size_t)blockIdx.x * blockDim.x + threadIdx.x; k < total; k += (size_t)gridDim.x * blockDim.x) {
     if (acc) {
-      acc[k] = 0ull;
-      acc[total + k] = 0ull;
+      acc[col + k] = 0ull;
+      acc[gridDim.y * total + col + k] = 0ull;
     }
     m = max(m, (unsigned)__double2hiint(x[k]) & 0x7FFFFFFFu);
   }
@@ -381,7 +388,7 @@ __global__ void __launch_bounds__(FIN_TPB) k_tmu_sym_finish(
     lo -= (size_t)(blockIdx.y / 2) * 6 * n, hi -= (size_t)(blockIdx.y / 2) * 6 * n;
   }
   const bool nan = *bad != 0ull;
-  const int ex = dsp_exponent(*reinterpret_cast<const unsigned *>(bad + 1));
+  const int ex = dsp_exponent(reinterpret_cast<const unsigned *>(bad + 1)[blockIdx.y % 2]);
   const int lane = threadIdx.x % L;
   double dot = 0.0;
   for (int j = (blockIdx.x * FIN_TPB + threadIdx.x) / L; j < n; j += gridDim.x * (FIN_TPB / L)) {
@@ -526,11 +533,11 @@ void launch_tmu_f64_sym_multi(int g, bool amoeba, const SymSlice *sl, int nsl, u
 
 void launch_tmu_sym_prepare(const DevSites &s, int g, const double *x, unsigned long long *lo, unsigned long long *bad,
                             cudaStream_t st) {
-  const size_t total = 3 * (size_t)g * s.n;
+  const size_t nv = 3 * (size_t)s.n;
   add_launch_count(1);
   cudaMemsetAsync(bad, 0, 2 * sizeof(unsigned long long), st);
-  const int blocks = (int)std::min<size_t>((total + 255) / 256, 1216);
-  k_sym_prepare<<<blocks, 256, 0, st>>>(total, x, lo, reinterpret_cast<unsigned *>(bad + 1), 0);
+  const int blocks = (int)std::min<size_t>((nv + 255) / 256, 1216);
+  k_sym_prepare<<<dim3(blocks, g), 256, 0, st>>>(nv, x, lo, reinterpret_cast<unsigned *>(bad + 1), 0);
 }
 
 void launch_max_word(size_t total, const double *x, unsigned *word, cudaStream_t st) {
@@ -563,8 +570,8 @@ void launch_tmu_sym_finish(const DevSites &s, int g, const unsigned long long *l
 size_t tmu_sym_scratch_doubles(const DevSites &s, int nrhs) {
   if (s.n == 0) return 0;
   // two 64-bit accumulator words and one value read out (FP32 product) per
-  // value of a column group (at most two columns), the error flag, the scale
-  // and the work counter
+  // value of a column group (at most two columns), the error flag, the scales
+  // (a 32-bit word per column) and the work counter
   const size_t C = 3 * (size_t)(nrhs < 2 ? nrhs : 2);
   return 3 * C * (size_t)s.n + 3;
 }
@@ -613,9 +620,9 @@ void launch_tmu_f64_sym_groups(const DevSites &s, int nrhs, const double *x, dou
     const double *xg = x + done * nv;
     cudaMemsetAsync(scratch, 0, groups * words * sizeof(double), st);
     add_launch_count(1);
-    const int blocks = (int)std::min<size_t>((2 * nv + 255) / 256, 1216);
-    k_sym_prepare<<<dim3(blocks, groups), 256, 0, st>>>(2 * nv, xg, nullptr,
-                                                        reinterpret_cast<unsigned *>(base + 6 * nv + 1), 2 * words);
+    const int blocks = (int)std::min<size_t>((nv + 255) / 256, 1216);
+    k_sym_prepare<<<dim3(blocks, 2 * groups), 256, 0, st>>>(nv, xg, nullptr,
+                                                            reinterpret_cast<unsigned *>(base + 6 * nv + 1), 2 * words);
     SymSlice sl[kMaxSymSlices];
     const int items = tmu_f64_sym_items(s, 2);
     for (int g = 0; g < groups; ++g) {
@@ -635,7 +642,7 @@ void launch_max_words(int ncol, size_t nv, const double *x, unsigned *words, cud
   add_launch_count(1);
   cudaMemsetAsync(words, 0, ncol * sizeof(unsigned), st);
   const int blocks = (int)std::min<size_t>((nv + 255) / 256, 1216);
-  k_sym_prepare<<<dim3(blocks, ncol), 256, 0, st>>>(nv, x, nullptr, words, 1);
+  k_sym_prepare<<<dim3(blocks, ncol), 256, 0, st>>>(nv, x, nullptr, words, 0);
 }
 
 // x = h + m + l with h a multiple of g and m of g 2^-23 (g = 2^-23 of the
