@@ -77,7 +77,7 @@ struct GradArgs {
   const int4 *frame;
   const int *r_ri, *r_src;
   double *base, *rot, *grad;
-  // the pair pass's fixed-point sums [mm][6 or 3], flag and scale
+  // the pair pass's fixed-point sums [mm][6 or 3], flag and scales
   const unsigned long long *lo, *hi, *bad;
   double thr;
   int *err;
@@ -105,10 +105,13 @@ __global__ void k_grad_finish(GradArgs g) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= g.mm) return;
   double sums[NO];
-  const int ex = dsp_exponent(reinterpret_cast<const unsigned *>(g.bad + 1)[1]);
+  const unsigned word = reinterpret_cast<const unsigned *>(g.bad + 1)[1];
+  const int ex = dsp_exponent(word);
+  const int es = dsp_exponent_of(*reinterpret_cast<const unsigned *>(g.bad + 3), word);
   for (int c = 0; c < NO; ++c) {
     const size_t o = (size_t)t * NO + c;
-    sums[c] = *g.bad ? __longlong_as_double(0x7ff8000000000000ll) : scale_up(fixed_value(g.lo[o], g.hi[o]), ex);
+    const double v = scale_up(scale_up(fixed_value(g.lo[o], g.hi[o]), ex), es);
+    sums[c] = *g.bad ? __longlong_as_double(0x7ff8000000000000ll) : v;
   }
   // corrections of the scaled pairs
   double hd[6] = {0, 0, 0, 0, 0, 0}, hp[6] = {0, 0, 0, 0, 0, 0}, e[3] = {0, 0, 0}, h[3] = {0, 0, 0};

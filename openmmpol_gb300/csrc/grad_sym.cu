@@ -34,7 +34,10 @@
 // 32 x 32 sub-tile pair, close and strongly damped pairs (x < 28: the r^-9
 // damping reaches farther) queued for FP64, fixed-point sums.  Sub-tile pairs
 // without a polarizable site are skipped.  The dipoles are scaled by a power
-// of two as in the products.
+// of two as in the products, and so is the other factor of every term, the
+// static multipoles and unscaled dipoles (largest magnitude in [1, 2)): with
+// charges of 1e-8 and dipoles of 1e-5 the terms of the fixed-point sums would
+// else lose 1e-11 of their value, with dipoles of 1e-8 8e-9.
 //
 // Products and sums keep their low parts unrenormalised, the accumulators are
 // renormalised per pair: renormalising every product cost 7 % for errors of
@@ -67,6 +70,7 @@ struct GradSymJob {
   const double *p, *d;    // [m][3] scaled mean dipole and half difference
   const int *any;         // [0] some d is not zero, [1] some quadrupole has a trace
   const unsigned *word;   // largest high word of the dipoles
+  const unsigned *qword;  // and of the static multipoles
   const unsigned *polar;  // [ceil(m / 32)] sites of the sub-tile that are polarizable
   unsigned long long *lo, *hi, *bad;
   int ntile, K, chunk, nchunk, quarters, items;
@@ -256,22 +260,27 @@ struct Rec {
   static constexpr int R = (9 + 2 * NV + 3) / 4;
 };
 
+// es: 2^-es scales the static multipoles, eu = ex - es takes a scaled dipole
+// to that scale
 template <bool AMOEBA>
-__device__ __forceinline__ void site_values(const GradSymJob &jb, int i, int ex, double *v) {
-  const double *q = jb.s.mm_q + (size_t)i * (AMOEBA ? 10 : 1), *p = jb.p + 3 * (size_t)i;
+__device__ __forceinline__ void site_values(const GradSymJob &jb, int i, int es, int eu, double *v) {
+  constexpr int LD = AMOEBA ? 10 : 1;
+  const double *p = jb.p + 3 * (size_t)i;
+  double q[LD];
+  for (int c = 0; c < LD; ++c) q[c] = scale_down(jb.s.mm_q[(size_t)i * LD + c], es);
   v[0] = q[0];
-  if (!AMOEBA) {
+  if constexpr (!AMOEBA) {
     for (int c = 0; c < 3; ++c) v[1 + c] = p[c];
-    return;
+  } else {
+    for (int c = 0; c < 3; ++c) {
+      v[1 + c] = fma(0.5, scale_up(p[c], eu), q[1 + c]);
+      v[4 + c] = q[1 + c];
+      v[14 + c] = p[c];
+      v[17 + c] = jb.d[3 * (size_t)i + c];
+    }
+    for (int c = 0; c < 6; ++c) v[7 + c] = q[4 + c];
+    v[13] = (q[4] + q[6]) + q[9];
   }
-  for (int c = 0; c < 3; ++c) {
-    v[1 + c] = fma(0.5, scale_up(p[c], ex), q[1 + c]);
-    v[4 + c] = q[1 + c];
-    v[14 + c] = p[c];
-    v[17 + c] = jb.d[3 * (size_t)i + c];
-  }
-  for (int c = 0; c < 6; ++c) v[7 + c] = q[4 + c];
-  v[13] = (q[4] + q[6]) + q[9];
 }
 
 template <typename T>
@@ -306,7 +315,7 @@ __device__ __forceinline__ void fixed_add_to(const GradSymJob &jb, size_t o, dou
 // the queued pairs in FP64, one per lane
 template <bool AMOEBA>
 __device__ __noinline__ void grad_queued(const GradSymJob &jb, const unsigned short *queue, int count, int lane,
-                                         int i0, int j0, int ex, bool delta, bool trace) {
+                                         int i0, int j0, int es, int eu, bool delta, bool trace) {
   constexpr int NO = GradSmem<AMOEBA>::NO;
   const DevSites &s = jb.s;
   for (int e = lane; e < count; e += 32) {
@@ -337,8 +346,8 @@ __device__ __noinline__ void grad_queued(const GradSymJob &jb, const unsigned sh
     k.D = 105.0 * k9 * r2 * r2;
     constexpr int NV = Rec<AMOEBA>::NV;
     double vi[NV], vj[NV];
-    site_values<AMOEBA>(jb, i, ex, vi);
-    site_values<AMOEBA>(jb, j, ex, vj);
+    site_values<AMOEBA>(jb, i, es, eu, vi);
+    site_values<AMOEBA>(jb, j, es, eu, vj);
     double f[3] = {0.0, 0.0, 0.0}, gi[3] = {0.0, 0.0, 0.0}, gj[3] = {0.0, 0.0, 0.0}, tt[3] = {0.0, 0.0, 0.0}, ts[3] = {0.0, 0.0, 0.0};
     Site<double, AMOEBA> a, b;
     fill(a, vi);
@@ -350,11 +359,11 @@ __device__ __noinline__ void grad_queued(const GradSymJob &jb, const unsigned sh
         trace_force(b.tr, a.p, n, k, gj);
       }
       if (delta) {
-        const double du[3] = {scale_up(vi[17], ex), scale_up(vi[18], ex), scale_up(vi[19], ex)};
+        const double du[3] = {scale_up(vi[17], eu), scale_up(vi[18], eu), scale_up(vi[19], eu)};
         delta_force(du, vj + 17, n, k, f);
       }
     } else {
-      const double pu[3] = {scale_up(vi[1], ex), scale_up(vi[2], ex), scale_up(vi[3], ex)};
+      const double pu[3] = {scale_up(vi[1], eu), scale_up(vi[2], eu), scale_up(vi[3], eu)};
       pair_force(a, pu, b, n, k, f);
     }
 #pragma unroll
@@ -386,7 +395,7 @@ __global__ void __launch_bounds__(TILE, AMOEBA ? 2 : 4) k_grad_sym(const __grid_
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const DevSites &s = jb.s;
   const int m = s.m, nsub = (m + SUB - 1) / SUB;
-  const int ex = dsp_exponent(*jb.word);
+  const int es = dsp_exponent_of(*jb.qword, *jb.word), eu = dsp_exponent(*jb.word) - es;
   const bool delta = AMOEBA && jb.any[0] != 0, trace = AMOEBA && jb.any[1] != 0;
   for (;;) {
     __syncthreads();
@@ -408,19 +417,19 @@ __global__ void __launch_bounds__(TILE, AMOEBA ? 2 : 4) k_grad_sym(const __grid_
       tg[0] = h.x, tg[1] = h.y, tg[2] = h.z, tg[3] = c.x, tg[4] = c.y, tg[5] = c.z, tg[6] = l.x, tg[7] = l.y,
       tg[8] = l.z;
       double v[NV];
-      if (vi) site_values<AMOEBA>(jb, ti, ex, v);
+      if (vi) site_values<AMOEBA>(jb, ti, es, eu, v);
 #pragma unroll
       for (int c2 = 0; c2 < NV; ++c2) {
         // the difference dipoles (and, without multipoles, the second copy of
         // the dipole) enter the target's side unscaled
-        const double w = !vi ? 0.0 : (AMOEBA && c2 >= 17) ? scale_up(v[c2], ex) : v[c2];
+        const double w = !vi ? 0.0 : (AMOEBA && c2 >= 17) ? scale_up(v[c2], eu) : v[c2];
         tv[c2] = to_ds(w);
       }
     }
     dsf p2[3];
     if (!AMOEBA)
 #pragma unroll
-      for (int c = 0; c < 3; ++c) p2[c] = to_ds(vi ? scale_up(jb.p[3 * (size_t)ti + c], ex) : 0.0);
+      for (int c = 0; c < 3; ++c) p2[c] = to_ds(vi ? scale_up(jb.p[3 * (size_t)ti + c], eu) : 0.0);
     const float2 wai = vi ? s.mm_wa32[ti] : make_float2(0.f, 0.f);
     double sumi[NO];
 #pragma unroll
@@ -443,7 +452,7 @@ __global__ void __launch_bounds__(TILE, AMOEBA ? 2 : 4) k_grad_sym(const __grid_
         const float4 l = v ? s.mm_split[2 * (size_t)m + sj] : make_float4(0.f, 0.f, 0.f, 0.f);
         float f[4 * R] = {h.x, h.y, h.z, c.x, c.y, c.z, l.x, l.y, l.z};
         double w[NV];
-        if (v) site_values<AMOEBA>(jb, sj, ex, w);
+        if (v) site_values<AMOEBA>(jb, sj, es, eu, w);
 #pragma unroll
         for (int c2 = 0; c2 < NV; ++c2) {
           const dsf d = to_ds(v ? w[c2] : 0.0);
@@ -559,8 +568,8 @@ __global__ void __launch_bounds__(TILE, AMOEBA ? 2 : 4) k_grad_sym(const __grid_
         }
         if (near) {
           __syncwarp();
-          grad_queued<AMOEBA>(jb, sm.queue[warp], queued, lane, I * TILE + warp * SUB, J * TILE + js * SUB, ex, delta,
-                              trace);
+          grad_queued<AMOEBA>(jb, sm.queue[warp], queued, lane, I * TILE + warp * SUB, J * TILE + js * SUB, es, eu,
+                              delta, trace);
           __syncwarp();
         }
 #pragma unroll
@@ -586,11 +595,17 @@ __global__ void __launch_bounds__(TILE, AMOEBA ? 2 : 4) k_grad_sym(const __grid_
 }
 
 // scaled mean dipoles and half differences in static-site order, whether any
-// difference is not zero and whether any quadrupole has a trace beyond rounding
+// difference is not zero and whether any quadrupole has a trace beyond
+// rounding, and the largest high word of the static multipoles
 __global__ void k_grad_dipoles(int m, int n, int nset, const int *__restrict__ mm_polar, const double *__restrict__ ipd,
                                const unsigned *__restrict__ word, double *__restrict__ p, double *__restrict__ d,
-                               const double *__restrict__ q, int *any) {
+                               const double *__restrict__ q, int *any, unsigned *qword) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int ld = nset == 2 ? 10 : 1;
+  unsigned big = 0;
+  for (int c = 0; i < m && c < ld; ++c) big = max(big, (unsigned)__double2hiint(q[(size_t)i * ld + c]) & 0x7FFFFFFFu);
+  big = __reduce_max_sync(0xffffffffu, big);
+  if ((threadIdx.x & 31) == 0 && big) atomicMax(qword, big);
   if (i >= m) return;
   const int j = mm_polar[i], ex = dsp_exponent(*word);
   bool diff = false;
@@ -604,8 +619,8 @@ __global__ void k_grad_dipoles(int m, int n, int nset, const int *__restrict__ m
   if (diff) any[0] = 1;
   if (nset == 2) {
     const double *Q = q + (size_t)i * 10 + 4;
-    const double big = fmax(fmax(fabs(Q[0]), fabs(Q[2])), fabs(Q[5]));
-    if (fabs((Q[0] + Q[2]) + Q[5]) > 2e-15 * big) any[1] = 1;
+    const double diag = fmax(fmax(fabs(Q[0]), fabs(Q[2])), fabs(Q[5]));
+    if (fabs((Q[0] + Q[2]) + Q[5]) > 2e-15 * diag) any[1] = 1;
   }
 }
 
@@ -624,7 +639,8 @@ int resident() {
 }  // namespace
 
 // the buffer of launch_grad_sym: fixed-point words (lo, hi) of the outputs,
-// flag, counter, scale, difference flag, dipoles and differences
+// flag, counter and scale of the dipoles, two flags, scale of the multipoles,
+// dipoles and differences
 size_t grad_sym_doubles(const DevSites &s) {
   const size_t no = s.amoeba ? 6 : 3;
   return (2 * no + 6) * (size_t)s.m + 4;
@@ -641,11 +657,13 @@ void launch_grad_sym(const DevSites &s, const double *ipd, const int *mm_polar, 
   j.bad = j.hi + no * s.m;
   unsigned *next = reinterpret_cast<unsigned *>(j.bad + 1), *word = next + 1;
   int *any = reinterpret_cast<int *>(j.bad + 2);
+  unsigned *qword = reinterpret_cast<unsigned *>(j.bad + 3);
   double *p = reinterpret_cast<double *>(j.bad + 4);
   j.p = p;
   j.d = p + 3 * (size_t)s.m;
   j.any = any;
   j.word = word;
+  j.qword = qword;
   j.polar = polar;
   j.err = err;
   j.thr2m = (float)(s.damp_thr * s.damp_thr * (1.0 + 1e-5));
@@ -663,7 +681,7 @@ void launch_grad_sym(const DevSites &s, const double *ipd, const int *mm_polar, 
   launch_max_word(nset * 3 * (size_t)s.n, ipd, word, st);
   add_launch_count(2);
   k_grad_dipoles<<<(s.m + 255) / 256, 256, 0, st>>>(s.m, s.n, (int)nset, mm_polar, ipd, word, p,
-                                                    p + 3 * (size_t)s.m, s.mm_q, any);
+                                                    p + 3 * (size_t)s.m, s.mm_q, any, qword);
   const int grid = std::min(ctas, j.items);
   if (s.amoeba)
     k_grad_sym<true><<<grid, TILE, sizeof(GradSmem<true>), st>>>(j, next);
