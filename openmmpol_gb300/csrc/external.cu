@@ -14,8 +14,10 @@
 // static multipoles and 6.3 ms for the induced dipoles.  They run in
 // double-single on the FP32 pipes (ds_pair.cuh; about 350 FP32 operations per
 // point and AMOEBA site), static and induced dipole of a site added first so
-// that one pass serves both.  Points and sites are split on one grid per call;
-// one thread owns a point, sources stream through shared memory in tiles of
+// that one pass serves both.  Points and sites are split on one grid per call,
+// which covers the sites and the points within kExtReach of the first one;
+// points beyond (or not finite) take FP64 for all their sources and leave the
+// resolution to the others.  One thread owns a point, sources stream through shared memory in tiles of
 // 128; pairs closer than 5 bohr go to a list of the point's own and are formed
 // in FP64 by its thread.  The source range is split over blockIdx.y (quarters
 // of a tile: a few QM nuclei alone fill the GPU) and the partials are summed in
@@ -37,6 +39,10 @@ namespace {
 constexpr int NT = 128;
 constexpr int NLIST = 24;       // listed sources per point before they are formed
 constexpr float CLOSE2 = 25.f;  // bohr^2
+// The three floats of a coordinate on a grid as wide as 2^e resolve 2^(e - 71):
+// up to 2^22 bohr that is 2^-49, below the rounding of a coordinate of 8 bohr
+// (one point at 1e10 bohr on the common grid left the others with 1e-10).
+constexpr double kExtReach = 4194304.0;
 
 // values of a source: q, dipole (3), with QUAD the quadrupole (6)
 template <bool QUAD>
@@ -62,7 +68,7 @@ struct ExtArgs {
   int ld;
   const int *polar;    // [m] polarizable index of a source or -1; null: the source itself
   const double *mu, *mu2;  // induced dipoles added (null: none) and a second set averaged with them
-  double c[3], g1;
+  double c[3], g1, reach;  // the grid: origin, step, width
   const unsigned *word;  // scale of the dipoles, or null
   double *val;         // [m][NV] FP64 values
   float4 *rec;         // [R][m]
@@ -110,9 +116,11 @@ __global__ void __launch_bounds__(NT, 4) k_ext(const __grid_constant__ ExtArgs a
   const int tj = valid ? j : a.n - 1;
   const double px = a.cext[3 * (size_t)tj], py = a.cext[3 * (size_t)tj + 1], pz = a.cext[3 * (size_t)tj + 2];
   float tg[9];
-  split3(px - a.c[0], a.g1, tg);
-  split3(py - a.c[1], a.g1, tg + 1);
-  split3(pz - a.c[2], a.g1, tg + 2);
+  const bool outside = !(fmax(fabs(px - a.c[0]), fmax(fabs(py - a.c[1]), fabs(pz - a.c[2]))) <= a.reach) ||
+                       isnan(px) || isnan(py) || isnan(pz);
+  split3(outside ? 0.0 : px - a.c[0], a.g1, tg);
+  split3(outside ? 0.0 : py - a.c[1], a.g1, tg + 1);
+  split3(outside ? 0.0 : pz - a.c[2], a.g1, tg + 2);
   double sum[C];
 #pragma unroll
   for (int c = 0; c < C; ++c) sum[c] = 0.0;
@@ -174,7 +182,7 @@ __global__ void __launch_bounds__(NT, 4) k_ext(const __grid_constant__ ExtArgs a
       for (int c = 0; c < 9; ++c) sc[c] = f[c];
       const DspDelta d = dsp_delta(tg, sc);
       float y = d.ri;
-      if (!(d.r2 >= CLOSE2)) {
+      if (outside || !(d.r2 >= CLOSE2)) {
         y = 0.f;
         if (listed == NLIST) form();
         s_list[listed++][threadIdx.x] = t0 + k;
@@ -333,15 +341,24 @@ int System::ext_props(int which, bool field, int n, const double *cext_h, double
     }
   }
   // one grid for the points and the sites: about the first site, rounded to
-  // whole bohr (an exact shift), as wide as the farthest of them
+  // whole bohr (an exact shift), as wide as the farthest site or point within
+  // kExtReach
   double big = 1.0;
   for (int c = 0; c < 3; ++c) a.c[c] = std::nearbyint(m_.cmm[c]);
   for (int i = 0; i < d_.m; ++i)
-    for (int c = 0; c < 3; ++c) big = std::max(big, std::fabs(m_.cmm[3 * (size_t)i + c] - a.c[c]));
-  for (size_t k = 0; k < 3 * (size_t)n; ++k) big = std::max(big, std::fabs(cext_h[k] - a.c[k % 3]));
+    for (int c = 0; c < 3; ++c) {
+      const double v = std::fabs(m_.cmm[3 * (size_t)i + c] - a.c[c]);
+      if (v > big && std::isfinite(v)) big = v;
+    }
+  const double reach = std::max(big, gpu::kExtReach);
+  for (size_t k = 0; k < 3 * (size_t)n; ++k) {
+    const double v = std::fabs(cext_h[k] - a.c[k % 3]);
+    if (v > big && v <= reach) big = v;
+  }
   int e = 0;
-  std::frexp(std::isfinite(big) ? big : 1.0, &e);
+  std::frexp(big, &e);
   a.g1 = std::ldexp(1.0, e - 23);
+  a.reach = big;
   cudaMemcpyAsync(cext, cext_h, 3 * (size_t)n * sizeof(double), cudaMemcpyHostToDevice, st_);
   cudaMemsetAsync(flag_, 0, sizeof(int), st_);
   if (!do_mm) {
