@@ -932,8 +932,16 @@ int System::refine_inverse(const double *rhs, double *x, bool &done) {
     if (it == 0) {
       first = rms;
       if (rms == 0.0) {
-        cudaMemsetAsync(x, 0, bytes, st_);
-        done = true;
+        // all zero, or the squares underflow (the LU factors serve such a field)
+        unsigned word = 0;
+        gpu::launch_max_word(nn, rhs, reinterpret_cast<unsigned *>(info_), st_);
+        cudaMemcpyAsync(&word, info_, sizeof(unsigned), cudaMemcpyDeviceToHost, st_);
+        const int zst = check(cudaStreamSynchronize(st_), "refinement of the inverse");
+        if (zst) return zst;
+        if (word == 0) {
+          cudaMemsetAsync(x, 0, bytes, st_);
+          done = true;
+        }
         return kOk;
       }
     }
