@@ -270,6 +270,8 @@ int System::cg64_ws(Workspace &w, int matv, int ncol, const double *rhs, double 
     }
     if (!any) break;
   }
+  // without an iteration nothing has waited for the start's columns
+  if (maxiter_ < 1 && (st = check(cudaStreamSynchronize(st_), "CG start"))) return st;
   std::vector<double> h(maxhist_);
   int rc = kOk;
   for (int k = 0; k < ncol; ++k) {
