@@ -323,6 +323,7 @@ int32_t ommp_gpu_device_alloc(int64_t bytes, void **ptr) {
   *ptr = nullptr;
   cudaError_t e = cudaMalloc(ptr, (size_t)(bytes > 0 ? bytes : 1));
   if (e != cudaSuccess) {
+    cudaGetLastError();
     ommp::set_last_error(std::string("cudaMalloc: ") + cudaGetErrorString(e));
     return ommp::kErrMemory;
   }
@@ -361,7 +362,7 @@ int32_t ommp_gpu_device_mem_info(int64_t *free_bytes, int64_t *total_bytes) {
 int32_t ommp_gpu_measure_pipe_peak(int32_t fp64, double *tflops) {
   *tflops = 0.0;
   void *out = nullptr;
-  if (cudaMalloc(&out, 1 << 20) != cudaSuccess) return ommp::kErrMemory;
+  if (ommp::device_alloc(&out, 1 << 20)) return ommp::kErrMemory;
   cudaEvent_t a, b;
   cudaEventCreate(&a);
   cudaEventCreate(&b);

@@ -29,9 +29,7 @@ constexpr size_t kMaxDenseBytes = size_t(24) << 30;  // incore T / inversion bud
 
 template <typename T>
 int dalloc(T *&p, size_t count) {
-  p = nullptr;
-  if (count == 0) count = 1;
-  return cudaMalloc((void **)&p, count * sizeof(T)) == cudaSuccess ? 0 : 1;
+  return device_alloc((void **)&p, std::max<size_t>(count, 1) * sizeof(T));
 }
 }  // namespace
 
@@ -64,8 +62,17 @@ cudaError_t pinned_alloc(void **p, size_t bytes) {
   if (e == cudaSuccess) {
     std::lock_guard<std::mutex> lk(g_pin_mu);
     g_pin_class[*p] = c;
+  } else {
+    cudaGetLastError();
   }
   return e;
+}
+
+int device_alloc(void **p, size_t bytes) {
+  if (cudaMalloc(p, bytes) == cudaSuccess) return 0;
+  cudaGetLastError();
+  *p = nullptr;
+  return 1;
 }
 
 void pinned_free(void *p) {
@@ -106,7 +113,7 @@ int System::alloc(T *&p, size_t count) {
     async_bufs_.push_back((void *)p);
     return 0;
   }
-  return cudaMalloc((void **)&p, count * sizeof(T)) == cudaSuccess ? 0 : 1;
+  return device_alloc((void **)&p, count * sizeof(T));
 }
 
 void System::release(void *p) {
@@ -569,7 +576,7 @@ int System::flush_l2(size_t bytes) {
     if (flush_buf_) cudaFree(flush_buf_);
     flush_buf_ = nullptr;
     flush_bytes_ = 0;
-    if (cudaMalloc(&flush_buf_, bytes) != cudaSuccess) {
+    if (device_alloc(&flush_buf_, bytes)) {
       set_last_error("out of device memory for the L2 flush buffer");
       return kErrMemory;
     }

@@ -401,6 +401,8 @@ const char *last_error();
 // evicted system would stall every solve in flight).  The caller must have
 // completed all copies into or out of a buffer before returning it.
 cudaError_t pinned_alloc(void **p, size_t bytes);
+// cudaMalloc: 0, or 1 with p null and no error left for a later call's check to find
+int device_alloc(void **p, size_t bytes);
 void pinned_free(void *p);
 
 }  // namespace ommp

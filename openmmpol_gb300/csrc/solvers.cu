@@ -25,9 +25,7 @@ namespace ommp {
 namespace {
 template <typename T>
 int walloc(T *&p, size_t count) {
-  p = nullptr;
-  if (count == 0) count = 1;
-  return cudaMalloc((void **)&p, count * sizeof(T)) == cudaSuccess ? 0 : 1;
+  return device_alloc((void **)&p, std::max<size_t>(count, 1) * sizeof(T));
 }
 
 template <typename T>

@@ -1,0 +1,84 @@
+"""Device allocations that fail, without a GPU: the library's own objects linked
+with a stand-in for the CUDA runtime (tests/host/fake_cuda.cpp) whose memory is
+the host's and whose kernels do nothing.
+
+Every size that a call allocates is made to fail in turn.  As long as it fails
+the call either does without (each time) or reports an error (each time, never
+going on with the buffer that it did not get), and once there is memory again
+the same call succeeds."""
+import ctypes as C
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import ROOT
+from openmmpol_gb300 import OMMPError, OMMPSystem, _lib, build, synth
+
+
+@pytest.fixture(scope="module")
+def fake(tmp_path_factory):
+    build.build()
+    d = tmp_path_factory.mktemp("fake")
+    obj, so = str(d / "fake.o"), str(d / "libommp_fake.so")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-I", build._cuda_include(), "-c",
+                    os.path.join(ROOT, "tests", "host", "fake_cuda.cpp"), "-o", obj], check=True)
+    objs = [os.path.join(build.OBJ, s + ".o") for s in build.CU_SOURCES + build.CXX_SOURCES]
+    subprocess.run(["g++", "-shared", "-Wl,-Bsymbolic", "-o", so, *objs, obj, "-lpthread", "-ldl", "-lrt"], check=True)
+    saved, _lib._lib = _lib._lib, None
+    try:
+        L = _lib.load(so)
+        for name in ("fake_launches", "fake_instantiations", "fake_live"):
+            getattr(L, name).restype = C.c_longlong
+        for name in ("fake_fail_bytes",):
+            getattr(L, name).argtypes = [C.c_longlong]
+        yield L
+    finally:
+        _lib._lib = saved
+
+
+@pytest.fixture(scope="module")
+def path(tmp_path_factory):
+    return synth.write_mmp(str(tmp_path_factory.mktemp("sys") / "w.mmp"), synth.water_cluster(1000, seed=3))
+
+
+CALLS = {
+    "tmatvec": lambda g: g.tmatvec(np.ones((2, g.pol_atoms, 3))),
+    "solve": lambda g: g.set_external_field(np.ones((g.pol_atoms, 3))),
+    "batch": lambda g: g.set_external_fields_batch(np.ones((3, g.pol_atoms, 3))),
+    "points": lambda g: g.potential_mm2ext(np.ones((300, 3))),
+    "static_energy": lambda g: g.get_fixedelec_energy(),
+    "static_gradient": lambda g: g.fixedelec_geomgrad(),
+    "gradient": lambda g: g.polelec_geomgrad(),
+}
+
+
+@pytest.mark.parametrize("name", sorted(CALLS))
+def test_call_survives_failed_allocations(fake, path, name):
+    call = CALLS[name]
+    g = OMMPSystem(path)
+    fake.fake_forget_sizes()
+    call(g)
+    sizes = (C.c_longlong * 256)()
+    n = fake.fake_sizes(sizes, 256)
+    g.close()
+    live = fake.fake_live()
+    for size in sorted({s for s in sizes[:n] if s > 8}):
+        g = OMMPSystem(path)
+        fake.fake_fail_bytes(size)
+        try:
+            outcome = []
+            for _ in range(3):
+                try:
+                    call(g)
+                    outcome.append("ok")
+                except OMMPError as e:
+                    outcome.append(e.status)
+        finally:
+            fake.fake_fail_bytes(0)
+        assert len(set(outcome)) == 1, (size, outcome)
+        assert fake.fake_last_error() == 0, size  # nothing left for the next call to find
+        call(g)
+        g.close()
+        assert fake.fake_live() == live, size
