@@ -441,6 +441,8 @@ int System::build_blocks() {
   blk_minv_ = nullptr;
   if (n > 0) {
     if (alloc(blk_info_, (size_t)n) || alloc(blk_minv_, minv.size())) {
+      release(blk_info_);
+      blk_info_ = nullptr;
       set_last_error("out of device memory for the block preconditioner");
       return kErrMemory;
     }
@@ -470,6 +472,9 @@ int System::ensure_near() {
   std::vector<float> blk;
   build_near_field(m_, d2d_pairs_, d_.damp_thr, blk_runs_, kNearBohr, ri, ci, blk);
   if (alloc(near_ri_, ri.size()) || alloc(near_ci_, ci.size()) || alloc(near_blk_, blk.size())) {
+    release(near_ri_);
+    release(near_ci_);
+    near_ri_ = near_ci_ = nullptr;
     set_last_error("out of device memory for the near-field preconditioner");
     return kErrMemory;
   }
@@ -635,6 +640,8 @@ int System::ensure_tmat() {
   }
   if (!tmat_) {
     if (dalloc(tmat_, nn * nn) || dalloc(piv_, nn)) {
+      if (tmat_) cudaFree(tmat_);
+      tmat_ = nullptr;
       set_last_error("out of device memory for the dense T matrix");
       return kErrMemory;
     }
@@ -794,6 +801,8 @@ int System::diis64(int matv, const double *rhs, double *x, int set) {
   log_msg(kVerbLow, nullptr, "Tolerance: %8.1E", tol_);
   log_msg(kVerbLow, nullptr, "DIIS is enabled with n = %4d", nd);
   if (!diis_x_ && (dalloc(diis_x_, nv * nd) || dalloc(diis_e_, nv * nd))) {
+    if (diis_x_) cudaFree(diis_x_);
+    diis_x_ = nullptr;
     set_last_error("out of device memory for the DIIS history");
     return kErrMemory;
   }

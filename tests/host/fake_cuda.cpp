@@ -16,7 +16,7 @@ std::mutex mu;
 std::map<void *, size_t> live;
 std::vector<long long> sizes;
 std::set<void *> events;
-long long fail_bytes = 0, launches = 0, instantiations = 0;
+long long fail_bytes = 0, fail_skip = 0, launches = 0, instantiations = 0;
 bool fail_events = false, capturing = false, memset_node = false;
 int captured_nodes = 0;
 cudaError_t last = cudaSuccess;
@@ -30,7 +30,7 @@ cudaError_t take(void **p, size_t n) {
   std::lock_guard<std::mutex> lk(mu);
   sizes.push_back((long long)n);
   *p = nullptr;
-  if (fail_bytes && (long long)n == fail_bytes) return fail(cudaErrorMemoryAllocation);
+  if (fail_bytes && (long long)n == fail_bytes && fail_skip-- <= 0) return fail(cudaErrorMemoryAllocation);
   *p = std::calloc(n ? n : 1, 1);
   live[*p] = n;
   return cudaSuccess;
@@ -52,7 +52,8 @@ thread_local Config config;
 
 extern "C" {
 // ---- controls -----------------------------------------------------------------
-void fake_fail_bytes(long long n) { fail_bytes = n; }  // allocations of this size fail (0: none)
+// allocations of this size fail but for the first few (0: none fails)
+void fake_fail_bytes(long long n, long long skip) { fail_bytes = n, fail_skip = skip; }
 void fake_fail_events(int on) { fail_events = on != 0; }
 void fake_memset_node(int on) { memset_node = on != 0; }  // captured bodies hold a memset
 long long fake_launches() { return launches; }

@@ -31,8 +31,7 @@ def fake(tmp_path_factory):
         L = _lib.load(so)
         for name in ("fake_launches", "fake_instantiations", "fake_live"):
             getattr(L, name).restype = C.c_longlong
-        for name in ("fake_fail_bytes",):
-            getattr(L, name).argtypes = [C.c_longlong]
+        L.fake_fail_bytes.argtypes = [C.c_longlong, C.c_longlong]
         yield L
     finally:
         _lib._lib = saved
@@ -43,7 +42,31 @@ def path(tmp_path_factory):
     return synth.write_mmp(str(tmp_path_factory.mktemp("sys") / "w.mmp"), synth.water_cluster(1000, seed=3))
 
 
+def other(**options):
+    """A solve with another solver, product or precision."""
+    def call(g):
+        g.set_precision(options.get("precision", "fp64"))
+        g.set_default_matv(options.get("matv", "direct"))
+        f = np.ones((g.pol_atoms, 3))
+        if "columns" in options:
+            g.set_external_fields_batch(np.ones((options["columns"], *f.shape)))
+        else:
+            g.set_external_field(f, solver=options.get("solver", "cg"))
+    return call
+
+
+def geometry(g):
+    g.update_coordinates(g.cmm)
+    other(precision="mixed")(g)
+
+
 CALLS = {
+    "geometry": geometry,
+    "incore": other(matv="incore"),
+    "inversion": other(solver="inversion"),
+    "diis": other(solver="diis"),
+    "mixed": other(precision="mixed"),
+    "mixed_batch": other(precision="mixed-ds", columns=5),
     "tmatvec": lambda g: g.tmatvec(np.ones((2, g.pol_atoms, 3))),
     "solve": lambda g: g.set_external_field(np.ones((g.pol_atoms, 3))),
     "batch": lambda g: g.set_external_fields_batch(np.ones((3, g.pol_atoms, 3))),
@@ -64,9 +87,11 @@ def test_call_survives_failed_allocations(fake, path, name):
     n = fake.fake_sizes(sizes, 256)
     g.close()
     live = fake.fake_live()
-    for size in sorted({s for s in sizes[:n] if s > 8}):
+    wanted = [s for s in sizes[:n] if s > 8]
+    # every allocation, by its size and the number of the same size before it
+    for size, skip in sorted({(s, wanted[:k].count(s)) for k, s in enumerate(wanted)}):
         g = OMMPSystem(path)
-        fake.fake_fail_bytes(size)
+        fake.fake_fail_bytes(size, skip)
         try:
             outcome = []
             for _ in range(3):
@@ -76,8 +101,8 @@ def test_call_survives_failed_allocations(fake, path, name):
                 except OMMPError as e:
                     outcome.append(e.status)
         finally:
-            fake.fake_fail_bytes(0)
-        assert len(set(outcome)) == 1, (size, outcome)
+            fake.fake_fail_bytes(0, 0)
+        assert len(set(outcome)) == 1, (size, skip, outcome)
         assert fake.fake_last_error() == 0, size  # nothing left for the next call to find
         call(g)
         g.close()
