@@ -1147,7 +1147,7 @@ int System::fmm_prepare() {
     bad |= cudaMalloc((void **)&f.field, ((1 + gpu::kFmmNearSplit) * v + 1) * sizeof(double)) != cudaSuccess;
     f.near = f.field ? f.field + v : nullptr;
     f.word = f.field ? reinterpret_cast<unsigned *>(f.field + (1 + gpu::kFmmNearSplit) * v) : nullptr;
-    f.field_n = 6 * (size_t)n;
+    f.field_n = f.field ? v : 0;
   }
   if (bad) {
     cudaGetLastError();

@@ -42,6 +42,21 @@ def path(tmp_path_factory):
     return synth.write_mmp(str(tmp_path_factory.mktemp("sys") / "w.mmp"), synth.water_cluster(1000, seed=3))
 
 
+def fmm(g):
+    g.set_fmm(True, order=8)
+    g.set_fmm_lmax(8)
+
+
+def tmatvec_fmm(g):
+    fmm(g)
+    g.tmatvec(np.ones((2, g.pol_atoms, 3)))
+
+
+def e_m2d_fmm(g):
+    fmm(g)
+    g.e_m2d()
+
+
 def other(**options):
     """A solve with another solver, product or precision."""
     def call(g):
@@ -61,6 +76,8 @@ def geometry(g):
 
 
 CALLS = {
+    "tmatvec_fmm": tmatvec_fmm,
+    "e_m2d_fmm": e_m2d_fmm,
     "geometry": geometry,
     "incore": other(matv="incore"),
     "inversion": other(solver="inversion"),
