@@ -1186,8 +1186,14 @@ int System::fmm_tmu(int ncol, const double *x, double *y, bool dodiag) {
     cudaDeviceGetStreamPriorityRange(&least, &greatest);
     if (cudaStreamCreateWithPriority(&f.far, cudaStreamNonBlocking, greatest) != cudaSuccess ||
         cudaEventCreateWithFlags(&f.fork, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&f.join, cudaEventDisableTiming) != cudaSuccess)
-      return check(cudaGetLastError(), "FMM streams");
+        cudaEventCreateWithFlags(&f.join, cudaEventDisableTiming) != cudaSuccess) {
+      st = check(cudaGetLastError(), "FMM streams");
+      if (f.fork) cudaEventDestroy(f.fork);
+      if (f.far) cudaStreamDestroy(f.far);
+      f.far = nullptr;
+      f.fork = f.join = nullptr;
+      return st;
+    }
   }
   for (int c0 = 0; c0 < ncol; c0 += 2) {
     const int g = std::min(2, ncol - c0);

@@ -124,3 +124,22 @@ def test_call_survives_failed_allocations(fake, path, name):
         call(g)
         g.close()
         assert fake.fake_live() == live, size
+
+
+def test_fmm_streams_that_cannot_be_made(fake, path):
+    """The FMM product's second stream and its two events are one set: while an
+    event cannot be made the product reports it, and then it works."""
+    g = OMMPSystem(path)
+    live = fake.fake_live()
+    fake.fake_fail_events(1)
+    try:
+        for _ in range(2):
+            launches = fake.fake_launches()
+            with pytest.raises(OMMPError, match="streams"):
+                tmatvec_fmm(g)
+            assert fake.fake_launches() == launches
+    finally:
+        fake.fake_fail_events(0)
+    tmatvec_fmm(g)
+    g.close()
+    assert fake.fake_live() < live
