@@ -96,8 +96,24 @@ int System::ensure_batch_ws(int ncol, int nf) {
 // A CG loop on the device: one iteration captured as the body of a while node
 // whose condition the last step sets, so that the host waits once per solve
 // instead of once per iteration (about 10 us each).  The loop ends after
-// CgCol::max_passes iterations at the latest.
+// CgCol::max_passes iterations at the latest.  The body holds kernels alone: one
+// with memset nodes crashed the host process (the GPU kept answering), so that
+// anything else is refused here, whoever captures it.
 // ---------------------------------------------------------------------------
+namespace {
+bool kernels_only(cudaGraph_t g) {
+  size_t n = 0;
+  if (cudaGraphGetNodes(g, nullptr, &n) != cudaSuccess) return false;
+  std::vector<cudaGraphNode_t> nodes(n);
+  if (n && cudaGraphGetNodes(g, nodes.data(), &n) != cudaSuccess) return false;
+  for (cudaGraphNode_t node : nodes) {
+    cudaGraphNodeType type;
+    if (cudaGraphNodeGetType(node, &type) != cudaSuccess || type != cudaGraphNodeTypeKernel) return false;
+  }
+  return n > 0;
+}
+}  // namespace
+
 bool System::run_loop(CgLoop &loop, const std::vector<char> &key,
                       const std::function<void(cudaGraphConditionalHandle)> &body, int &st) {
   st = kOk;
@@ -124,7 +140,8 @@ bool System::run_loop(CgLoop &loop, const std::vector<char> &key,
       body(handle);
       loop.kernels = gpu::thread_launch_count() - before;
       gpu::add_launch_count(-loop.kernels);  // captured, not launched
-      ok = cudaStreamEndCapture(st_, &captured) == cudaSuccess && cudaGraphInstantiate(&loop.exec, g, 0) == cudaSuccess;
+      ok = cudaStreamEndCapture(st_, &captured) == cudaSuccess && kernels_only(par.conditional.phGraph_out[0]) &&
+           cudaGraphInstantiate(&loop.exec, g, 0) == cudaSuccess;
     }
     if (g) cudaGraphDestroy(g);
     if (!ok) {

@@ -143,3 +143,21 @@ def test_fmm_streams_that_cannot_be_made(fake, path):
     tmatvec_fmm(g)
     g.close()
     assert fake.fake_live() < live
+
+
+def test_captured_loop_of_kernels_only(fake, path):
+    """A CG loop whose captured body holds anything but kernels is not made into
+    a graph: the solve goes from the host."""
+    g = OMMPSystem(path)
+    fake.fake_memset_node(1)
+    try:
+        made, launches = fake.fake_instantiations(), fake.fake_launches()
+        for precision in ("fp64", "mixed"):
+            other(precision=precision)(g)
+        assert fake.fake_instantiations() == made and fake.fake_launches() > launches
+    finally:
+        fake.fake_memset_node(0)
+    g.clear_guess()
+    other()(g)
+    assert fake.fake_instantiations() > made
+    g.close()
