@@ -35,7 +35,7 @@
 // damping reaches farther) queued for FP64, fixed-point sums.  Sub-tile pairs
 // without a polarizable site are skipped.  The dipoles are scaled by a power
 // of two as in the products, and so is the other factor of every term, the
-// static multipoles and unscaled dipoles (largest magnitude in [1, 2)): with
+// static multipoles and unscaled dipoles, unless it is near one: with
 // charges of 1e-8 and dipoles of 1e-5 the terms of the fixed-point sums would
 // else lose 1e-11 of their value, with dipoles of 1e-8 8e-9.
 //
@@ -69,8 +69,8 @@ struct GradSymJob {
   DevSites s;
   const double *p, *d;    // [m][3] scaled mean dipole and half difference
   const int *any;         // [0] some d is not zero, [1] some quadrupole has a trace
-  const unsigned *word;   // largest high word of the dipoles
-  const unsigned *qword;  // and of the static multipoles
+  const double *q;        // [m][10 or 1] scaled static multipoles
+  const int *eu;          // 2^eu takes a scaled dipole to their scale
   const unsigned *polar;  // [ceil(m / 32)] sites of the sub-tile that are polarizable
   unsigned long long *lo, *hi, *bad;
   int ntile, K, chunk, nchunk, quarters, items;
@@ -260,27 +260,22 @@ struct Rec {
   static constexpr int R = (9 + 2 * NV + 3) / 4;
 };
 
-// es: 2^-es scales the static multipoles, eu = ex - es takes a scaled dipole
-// to that scale
 template <bool AMOEBA>
-__device__ __forceinline__ void site_values(const GradSymJob &jb, int i, int es, int eu, double *v) {
-  constexpr int LD = AMOEBA ? 10 : 1;
-  const double *p = jb.p + 3 * (size_t)i;
-  double q[LD];
-  for (int c = 0; c < LD; ++c) q[c] = scale_down(jb.s.mm_q[(size_t)i * LD + c], es);
+__device__ __forceinline__ void site_values(const GradSymJob &jb, int i, int eu, double *v) {
+  const double *q = jb.q + (size_t)i * (AMOEBA ? 10 : 1), *p = jb.p + 3 * (size_t)i;
   v[0] = q[0];
-  if constexpr (!AMOEBA) {
+  if (!AMOEBA) {
     for (int c = 0; c < 3; ++c) v[1 + c] = p[c];
-  } else {
-    for (int c = 0; c < 3; ++c) {
-      v[1 + c] = fma(0.5, scale_up(p[c], eu), q[1 + c]);
-      v[4 + c] = q[1 + c];
-      v[14 + c] = p[c];
-      v[17 + c] = jb.d[3 * (size_t)i + c];
-    }
-    for (int c = 0; c < 6; ++c) v[7 + c] = q[4 + c];
-    v[13] = (q[4] + q[6]) + q[9];
+    return;
   }
+  for (int c = 0; c < 3; ++c) {
+    v[1 + c] = fma(0.5, scale_up(p[c], eu), q[1 + c]);
+    v[4 + c] = q[1 + c];
+    v[14 + c] = p[c];
+    v[17 + c] = jb.d[3 * (size_t)i + c];
+  }
+  for (int c = 0; c < 6; ++c) v[7 + c] = q[4 + c];
+  v[13] = (q[4] + q[6]) + q[9];
 }
 
 template <typename T>
@@ -315,7 +310,7 @@ __device__ __forceinline__ void fixed_add_to(const GradSymJob &jb, size_t o, dou
 // the queued pairs in FP64, one per lane
 template <bool AMOEBA>
 __device__ __noinline__ void grad_queued(const GradSymJob &jb, const unsigned short *queue, int count, int lane,
-                                         int i0, int j0, int es, int eu, bool delta, bool trace) {
+                                         int i0, int j0, int eu, bool delta, bool trace) {
   constexpr int NO = GradSmem<AMOEBA>::NO;
   const DevSites &s = jb.s;
   for (int e = lane; e < count; e += 32) {
@@ -346,8 +341,8 @@ __device__ __noinline__ void grad_queued(const GradSymJob &jb, const unsigned sh
     k.D = 105.0 * k9 * r2 * r2;
     constexpr int NV = Rec<AMOEBA>::NV;
     double vi[NV], vj[NV];
-    site_values<AMOEBA>(jb, i, es, eu, vi);
-    site_values<AMOEBA>(jb, j, es, eu, vj);
+    site_values<AMOEBA>(jb, i, eu, vi);
+    site_values<AMOEBA>(jb, j, eu, vj);
     double f[3] = {0.0, 0.0, 0.0}, gi[3] = {0.0, 0.0, 0.0}, gj[3] = {0.0, 0.0, 0.0}, tt[3] = {0.0, 0.0, 0.0}, ts[3] = {0.0, 0.0, 0.0};
     Site<double, AMOEBA> a, b;
     fill(a, vi);
@@ -395,7 +390,7 @@ __global__ void __launch_bounds__(TILE, AMOEBA ? 2 : 4) k_grad_sym(const __grid_
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const DevSites &s = jb.s;
   const int m = s.m, nsub = (m + SUB - 1) / SUB;
-  const int es = dsp_exponent_of(*jb.qword, *jb.word), eu = dsp_exponent(*jb.word) - es;
+  const int eu = *jb.eu;
   const bool delta = AMOEBA && jb.any[0] != 0, trace = AMOEBA && jb.any[1] != 0;
   for (;;) {
     __syncthreads();
@@ -417,7 +412,7 @@ __global__ void __launch_bounds__(TILE, AMOEBA ? 2 : 4) k_grad_sym(const __grid_
       tg[0] = h.x, tg[1] = h.y, tg[2] = h.z, tg[3] = c.x, tg[4] = c.y, tg[5] = c.z, tg[6] = l.x, tg[7] = l.y,
       tg[8] = l.z;
       double v[NV];
-      if (vi) site_values<AMOEBA>(jb, ti, es, eu, v);
+      if (vi) site_values<AMOEBA>(jb, ti, eu, v);
 #pragma unroll
       for (int c2 = 0; c2 < NV; ++c2) {
         // the difference dipoles (and, without multipoles, the second copy of
@@ -452,7 +447,7 @@ __global__ void __launch_bounds__(TILE, AMOEBA ? 2 : 4) k_grad_sym(const __grid_
         const float4 l = v ? s.mm_split[2 * (size_t)m + sj] : make_float4(0.f, 0.f, 0.f, 0.f);
         float f[4 * R] = {h.x, h.y, h.z, c.x, c.y, c.z, l.x, l.y, l.z};
         double w[NV];
-        if (v) site_values<AMOEBA>(jb, sj, es, eu, w);
+        if (v) site_values<AMOEBA>(jb, sj, eu, w);
 #pragma unroll
         for (int c2 = 0; c2 < NV; ++c2) {
           const dsf d = to_ds(v ? w[c2] : 0.0);
@@ -568,8 +563,8 @@ __global__ void __launch_bounds__(TILE, AMOEBA ? 2 : 4) k_grad_sym(const __grid_
         }
         if (near) {
           __syncwarp();
-          grad_queued<AMOEBA>(jb, sm.queue[warp], queued, lane, I * TILE + warp * SUB, J * TILE + js * SUB, es, eu,
-                              delta, trace);
+          grad_queued<AMOEBA>(jb, sm.queue[warp], queued, lane, I * TILE + warp * SUB, J * TILE + js * SUB, eu, delta,
+                              trace);
           __syncwarp();
         }
 #pragma unroll
@@ -624,6 +619,14 @@ __global__ void k_grad_dipoles(int m, int n, int nset, const int *__restrict__ m
   }
 }
 
+// the static multipoles scaled by 2^-es (dsp_exponent_of), and eu = ex - es
+__global__ void k_grad_scale(int total, const double *__restrict__ q, const unsigned *__restrict__ word,
+                             const unsigned *__restrict__ qword, double *__restrict__ out, int *eu) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, es = dsp_exponent_of(*qword, *word);
+  if (i == 0) *eu = dsp_exponent(*word) - es;
+  if (i < total) out[i] = scale_down(q[i], es);
+}
+
 template <bool AMOEBA>
 int resident() {
   static const int r = [] {
@@ -639,11 +642,11 @@ int resident() {
 }  // namespace
 
 // the buffer of launch_grad_sym: fixed-point words (lo, hi) of the outputs,
-// flag, counter and scale of the dipoles, two flags, scale of the multipoles,
-// dipoles and differences
+// flag, counter and scale of the dipoles, two flags, scales of the multipoles,
+// dipoles and differences, scaled multipoles
 size_t grad_sym_doubles(const DevSites &s) {
   const size_t no = s.amoeba ? 6 : 3;
-  return (2 * no + 6) * (size_t)s.m + 4;
+  return (2 * no + 6 + (s.amoeba ? 10 : 1)) * (size_t)s.m + 4;
 }
 
 void launch_grad_sym(const DevSites &s, const double *ipd, const int *mm_polar, const unsigned *polar, double *buf,
@@ -662,8 +665,9 @@ void launch_grad_sym(const DevSites &s, const double *ipd, const int *mm_polar, 
   j.p = p;
   j.d = p + 3 * (size_t)s.m;
   j.any = any;
-  j.word = word;
-  j.qword = qword;
+  double *q = p + 6 * (size_t)s.m;
+  j.q = q;
+  j.eu = reinterpret_cast<int *>(qword + 1);
   j.polar = polar;
   j.err = err;
   j.thr2m = (float)(s.damp_thr * s.damp_thr * (1.0 + 1e-5));
@@ -679,9 +683,11 @@ void launch_grad_sym(const DevSites &s, const double *ipd, const int *mm_polar, 
   j.items = j.ntile * j.nchunk * j.quarters;
   cudaMemsetAsync(buf, 0, (2 * no * s.m + 4) * sizeof(double), st);
   launch_max_word(nset * 3 * (size_t)s.n, ipd, word, st);
-  add_launch_count(2);
+  add_launch_count(3);
   k_grad_dipoles<<<(s.m + 255) / 256, 256, 0, st>>>(s.m, s.n, (int)nset, mm_polar, ipd, word, p,
                                                     p + 3 * (size_t)s.m, s.mm_q, any, qword);
+  const int values = (s.amoeba ? 10 : 1) * s.m;
+  k_grad_scale<<<(values + 255) / 256, 256, 0, st>>>(values, s.mm_q, word, qword, q, reinterpret_cast<int *>(qword + 1));
   const int grid = std::min(ctas, j.items);
   if (s.amoeba)
     k_grad_sym<true><<<grid, TILE, sizeof(GradSmem<true>), st>>>(j, next);
