@@ -316,19 +316,7 @@ int System::upload_static() {
   up(alpha32_, alpha32.data(), n * sizeof(float));
   up(d_.pol_a32, a32.data(), n * sizeof(float));
   up(d_.polar_mm, m.polar_mm.data(), n * sizeof(int));
-  // FP32 damping pre-test data: (1/thole)^2 and a^2 (inf / 0 for static sites)
-  std::vector<float2> pwa(n), mwa(mm);
-  for (int j = 0; j < n; ++j) {
-    double w = 1.0 / m.thole[m.polar_mm[j]];
-    pwa[j] = make_float2((float)(w * w), (float)(m.damping[j] * m.damping[j]));
-  }
-  for (int i = 0; i < mm; ++i) {
-    int p = m.mm_polar[i];
-    double w = m.thole[i] > 0.0 ? 1.0 / m.thole[i] : std::numeric_limits<double>::infinity();
-    double a = p >= 0 ? m.damping[p] : 0.0;
-    mwa[i] = make_float2((float)(w * w), (float)(a * a));
-  }
-  up(d_.pol_wa32, pwa.data(), n * sizeof(float2));
+  upload_damping_test();
   {
     std::vector<double> w(n);
     for (int j = 0; j < n; ++j) w[j] = 1.0 / m.thole[m.polar_mm[j]];
@@ -340,7 +328,6 @@ int System::upload_static() {
     }
     d_.m2d_r2max32 = gpu::m2d_r2max32(m.amoeba, d_.damp_thr, w.data(), m.damping.data(), n, mw.data(), ma.data(), mm);
   }
-  up(d_.mm_wa32, mwa.data(), mm * sizeof(float2));
   cudaMemsetAsync(ipd_, 0, nv * nipd * sizeof(double), st_);
   cudaMemsetAsync(e_m2d_, 0, nv * nipd * sizeof(double), st_);
   ipd_h_.assign(nv * nipd, 0.0);
@@ -353,6 +340,26 @@ int System::upload_static() {
   st = check(cudaStreamSynchronize(st_), "upload");
   h2d_release();
   return st;
+}
+
+// FP32 damping pre-test data: (1/thole)^2 and a^2 (inf / 0 for static sites; 0
+// in a wide system: every pair goes to FP64 and is tested there)
+void System::upload_damping_test() {
+  const HostModel &m = m_;
+  const int n = m.npol, mm = m.mm;
+  std::vector<float2> pwa(n), mwa(mm);
+  for (int j = 0; j < n; ++j) {
+    double w = d_.wide ? 0.0 : 1.0 / m.thole[m.polar_mm[j]];
+    pwa[j] = make_float2((float)(w * w), (float)(m.damping[j] * m.damping[j]));
+  }
+  for (int i = 0; i < mm; ++i) {
+    int p = m.mm_polar[i];
+    double w = d_.wide ? 0.0 : m.thole[i] > 0.0 ? 1.0 / m.thole[i] : std::numeric_limits<double>::infinity();
+    double a = p >= 0 ? m.damping[p] : 0.0;
+    mwa[i] = make_float2((float)(w * w), (float)(a * a));
+  }
+  h2d(d_.pol_wa32, pwa.data(), n * sizeof(float2));
+  h2d(d_.mm_wa32, mwa.data(), mm * sizeof(float2));
 }
 
 int System::upload_geometry() {
@@ -391,6 +398,13 @@ int System::upload_geometry() {
   std::vector<float4> subs(2 * (size_t)((n + 31) / 32)), msplit(3 * (size_t)mm), split(3 * (size_t)n);
   gpu::tile_boxes32(pp32.data(), n, subs.data(), 32);
   double whole[3] = {std::nearbyint(c[0]), std::nearbyint(c[1]), std::nearbyint(c[2])};
+  bool wide = false;
+  for (int i = 0; i < mm; ++i)
+    for (int k = 0; k < 3; ++k) wide = wide || std::fabs(m.cmm[3 * (size_t)i + k] - whole[k]) > gpu::kGridReach;
+  if (wide != d_.wide) {
+    d_.wide = wide;
+    upload_damping_test();
+  }
   gpu::split_coordinates(m.cmm.data(), mm, whole, msplit.data());
   for (int p = 0; p < 3; ++p)
     for (int j = 0; j < n; ++j) split[(size_t)p * n + j] = msplit[(size_t)p * mm + m.polar_mm[j]];
@@ -683,7 +697,7 @@ int System::matvec64(int matv, int ncol, const double *x, double *y, bool dodiag
 // The direct T.mu of FP64 accuracy: each unordered pair once, or for small
 // systems (and when forced) all ordered pairs.
 void System::direct_product(int ncol, const double *x, double *y, bool dodiag, int kernel) {
-  bool sym = kernel == 2 || (kernel == 0 && d_.n >= gpu::kSymMinSites);
+  bool sym = kernel == 2 || (kernel == 0 && d_.n >= gpu::kSymMinSites && !d_.wide);
   if (sym && ensure_sym_scratch() != kOk) {
     sym = false;  // not enough memory for the accumulators: all-ordered-pairs kernel
     log_msg(kVerbHigh, nullptr, "symmetric T.mu scratch does not fit: using the all-ordered-pairs kernel");
@@ -725,14 +739,14 @@ bool System::ready_groups(int ncol) {
 // matvec64 would take the symmetric direct product in one column group
 bool System::direct_symmetric(int matv, int ncol) {
   if ((matv == kMatvIncore && tmat_ok_) || fmm_on_ || ncol > 2) return false;
-  if (fp64_kernel_ != 2 && !(fp64_kernel_ == 0 && d_.n >= gpu::kSymMinSites)) return false;
+  if (fp64_kernel_ != 2 && !(fp64_kernel_ == 0 && d_.n >= gpu::kSymMinSites && !d_.wide)) return false;
   return ensure_sym_scratch() == kOk;
 }
 
 // matvec64 would take the ordered direct product, its scales within row_words_
 bool System::direct_rows(int matv, int ncol) const {
   if ((matv == kMatvIncore && tmat_ok_) || fmm_on_ || ncol > kRowWords) return false;
-  return fp64_kernel_ == 1 || (fp64_kernel_ == 0 && d_.n < gpu::kSymMinSites);
+  return fp64_kernel_ == 1 || (fp64_kernel_ == 0 && (d_.n < gpu::kSymMinSites || d_.wide));
 }
 
 // fixed-point accumulators of the symmetric products (FP64, double-single

@@ -228,6 +228,7 @@ class System {
   std::vector<void *> async_bufs_;
   int upload_static();
   int upload_geometry();
+  void upload_damping_test();
   int ensure_m2d();
   int ensure_tmat();
   int polarization(const double *e_dev, int solver, int matv, const bool *mask);

@@ -15,9 +15,9 @@
 // double-single on the FP32 pipes (ds_pair.cuh; about 350 FP32 operations per
 // point and AMOEBA site), static and induced dipole of a site added first so
 // that one pass serves both.  Points and sites are split on one grid per call,
-// which covers the sites and the points within kExtReach of the first one;
+// which covers the sites and the points within kGridReach of the first one;
 // points beyond (or not finite) take FP64 for all their sources and leave the
-// resolution to the others.  One thread owns a point, sources stream through shared memory in tiles of
+// resolution to the others (so do all points of a system as wide as that).  One thread owns a point, sources stream through shared memory in tiles of
 // 128; pairs closer than 5 bohr go to a list of the point's own and are formed
 // in FP64 by its thread.  The source range is split over blockIdx.y (quarters
 // of a tile: a few QM nuclei alone fill the GPU) and the partials are summed in
@@ -39,10 +39,6 @@ namespace {
 constexpr int NT = 128;
 constexpr int NLIST = 24;       // listed sources per point before they are formed
 constexpr float CLOSE2 = 25.f;  // bohr^2
-// The three floats of a coordinate on a grid as wide as 2^e resolve 2^(e - 71):
-// up to 2^22 bohr that is 2^-49, below the rounding of a coordinate of 8 bohr
-// (one point at 1e10 bohr on the common grid left the others with 1e-10).
-constexpr double kExtReach = 4194304.0;
 
 // values of a source: q, dipole (3), with QUAD the quadrupole (6)
 template <bool QUAD>
@@ -342,7 +338,7 @@ int System::ext_props(int which, bool field, int n, const double *cext_h, double
   }
   // one grid for the points and the sites: about the first site, rounded to
   // whole bohr (an exact shift), as wide as the farthest site or point within
-  // kExtReach
+  // kGridReach
   double big = 1.0;
   for (int c = 0; c < 3; ++c) a.c[c] = std::nearbyint(m_.cmm[c]);
   for (int i = 0; i < d_.m; ++i)
@@ -350,7 +346,7 @@ int System::ext_props(int which, bool field, int n, const double *cext_h, double
       const double v = std::fabs(m_.cmm[3 * (size_t)i + c] - a.c[c]);
       if (v > big && std::isfinite(v)) big = v;
     }
-  const double reach = std::max(big, gpu::kExtReach);
+  const double reach = std::max(big, gpu::kGridReach);
   for (size_t k = 0; k < 3 * (size_t)n; ++k) {
     const double v = std::fabs(cext_h[k] - a.c[k % 3]);
     if (v > big && v <= reach) big = v;
@@ -358,7 +354,7 @@ int System::ext_props(int which, bool field, int n, const double *cext_h, double
   int e = 0;
   std::frexp(big, &e);
   a.g1 = std::ldexp(1.0, e - 23);
-  a.reach = big;
+  a.reach = big > gpu::kGridReach ? -1.0 : big;
   cudaMemcpyAsync(cext, cext_h, 3 * (size_t)n * sizeof(double), cudaMemcpyHostToDevice, st_);
   cudaMemsetAsync(flag_, 0, sizeof(int), st_);
   if (!do_mm) {

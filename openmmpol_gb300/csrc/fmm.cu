@@ -1111,7 +1111,7 @@ int System::fmm_prepare() {
     const double w = 1.0 / m_.thole[m_.polar_mm[j]];
     spos[s] = gpu::Pos64{xp[3 * (size_t)j], xp[3 * (size_t)j + 1], xp[3 * (size_t)j + 2], w};
     sa[s] = m_.damping[j];
-    swa[s] = make_float2((float)(w * w), (float)(m_.damping[j] * m_.damping[j]));
+    swa[s] = make_float2(d_.wide ? 0.f : (float)(w * w), (float)(m_.damping[j] * m_.damping[j]));
   }
   std::vector<float4> split(3 * (size_t)n);
   {

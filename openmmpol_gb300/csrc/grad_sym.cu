@@ -74,7 +74,7 @@ struct GradSymJob {
   const unsigned *polar;  // [ceil(m / 32)] sites of the sub-tile that are polarizable
   unsigned long long *lo, *hi, *bad;
   int ntile, K, chunk, nchunk, quarters, items;
-  float thr2m, r2near;
+  float r2near;
   int *err;
 };
 
@@ -670,8 +670,7 @@ void launch_grad_sym(const DevSites &s, const double *ipd, const int *mm_polar, 
   j.eu = reinterpret_cast<int *>(qword + 1);
   j.polar = polar;
   j.err = err;
-  j.thr2m = (float)(s.damp_thr * s.damp_thr * (1.0 + 1e-5));
-  j.r2near = std::max(s.m2d_r2max32, s.amoeba ? kSymNear2 : kSymNear2Wang);
+  j.r2near = near_range2(s, s.m2d_r2max32);
   j.ntile = (s.m + TILE - 1) / TILE;
   j.K = j.ntile / 2;
   const int ctas = (s.amoeba ? resident<true>() : resident<false>()) * sm_count();

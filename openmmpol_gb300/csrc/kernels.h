@@ -6,6 +6,7 @@
 //   as the reference's Fortran (3, n, n_ipd) arrays seen from C.
 #pragma once
 
+#include <cmath>
 #include <cstddef>
 #include <cstdint>
 
@@ -57,6 +58,9 @@ struct DevSites {
   float4 *pol_split = nullptr, *sub_box32 = nullptr;
   // the same split of the static sites [3][m] (one grid for both)
   float4 *mm_split = nullptr, *mm_sub_box32 = nullptr;  // and their 32-site boxes
+  // a site is farther than kGridReach from the grid's origin: every pair in FP64
+  // (the damping pre-test data have (1/thole)^2 = 0, so that no pair passes it)
+  bool wide = false;
   float damp_r2max32 = 0.f;
   // tile boxes of the static sites and the squared distance beyond which no
   // M2D pair is damped
@@ -100,6 +104,16 @@ constexpr int kFinishLanesSites = 32768;
 // squared distances within which a pair always runs in FP64 (AMOEBA pairs
 // also while the damping is strong, a u^3 < 20)
 constexpr float kSymNear2 = 36.f, kSymNear2Wang = 64.f;
+// The three floats of a coordinate on a grid as wide as 2^e resolve 2^(e - 71)
+// bohr: up to 2^22 that is 2^-49, below the rounding of a coordinate of 8 bohr.
+// Wider grids lose it (one external point at 1e10 bohr left the others with
+// 1e-10, a water molecule at 1e12 the solve of 300 others with 4e-7).
+constexpr double kGridReach = 4194304.0;
+// squared distance of boxes within which their pairs are tested one by one
+inline float near_range2(const DevSites &s, float damped) {
+  const float close = s.amoeba ? kSymNear2 : kSymNear2Wang;
+  return s.wide ? INFINITY : damped > close ? damped : close;
+}
 size_t tmu_sym_scratch_doubles(const DevSites &s, int nrhs);
 void launch_tmu_f64_sym(const DevSites &s, int nrhs, const double *x, double *y, bool dodiag, double *scratch,
                         cudaStream_t st);

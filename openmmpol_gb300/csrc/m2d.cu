@@ -320,7 +320,7 @@ void launch_m2d(const DevSites &s, double *out, double *scratch, int nsplit, int
   const int per = per_split(s, nsplit);
   const dim3 grid((s.n + NT - 1) / NT, nsplit);
   const float thr2m = (float)(s.damp_thr * s.damp_thr * (1.0 + 1e-5));
-  const float r2near = std::max(s.m2d_r2max32, s.amoeba ? kSymNear2 : kSymNear2Wang);
+  const float r2near = near_range2(s, s.m2d_r2max32);
   if (s.amoeba)
     k_m2d<true><<<grid, NT, 0, st>>>(s, scratch, per, thr2m, r2near, err_flag);
   else

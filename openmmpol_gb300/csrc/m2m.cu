@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(NT) k_m2m(const __grid_constant__ DevSites s, 
       const dsf dx = ds_delta(th.x, td.x, tl.x, ph.x, pm.x, pl.x);
       const dsf dy = ds_delta(th.y, td.y, tl.y, ph.y, pm.y, pl.y);
       const dsf dz = ds_delta(th.z, td.z, tl.z, ph.z, pm.z, pl.z);
-      if (!(fmaf(dx.h, dx.h, fmaf(dy.h, dy.h, dz.h * dz.h)) >= CLOSE2)) {
+      if (s.wide || !(fmaf(dx.h, dx.h, fmaf(dy.h, dy.h, dz.h * dz.h)) >= CLOSE2)) {
         if (t0 + k != tc) {
           if (listed == NLIST) form();
           s_list[listed++][threadIdx.x] = t0 + k;

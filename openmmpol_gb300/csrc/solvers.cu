@@ -456,9 +456,10 @@ int System::pcg32_ws(Workspace &w, int ncol, int max_it, double eta) {
 // (relative, the tested bound), so the updated residual is within 1e-5 rms
 // of the recomputed one, which must stay below a tenth of the tolerance for
 // every unconverged column (a converged column's correction is zero).  The
-// first step (r = E) never qualifies: its correction is the whole solution.
+// first step (r = E) never qualifies: its correction is the whole solution, nor
+// does a wide system, whose FP32 positions are farther off.
 bool System::update_allowed(const std::vector<double> &rms) const {
-  if (!residual_update()) return false;
+  if (!residual_update() || d_.wide) return false;
   for (double r : rms)
     if (r >= tol_ && !(kResidualUpdateRel * r <= 0.1 * tol_)) return false;
   return true;

@@ -351,15 +351,16 @@ void launch_f64(const RowsArgs &a, bool amoeba, const double *alpha, cudaStream_
 }
 
 // The kernel by size and columns (times above): FP64 for up to three columns
-// of fewer than 300 sites, one target per CTA for one column of fewer than
-// 800, else 8 targets per CTA.
+// of fewer than 300 sites (and for systems wider than the split coordinates
+// resolve), one target per CTA for one column of fewer than 800, else 8 targets
+// per CTA.
 constexpr int kF64Sites = 300, kOneSites = 800;
-bool use_f64(int n, int ncol) { return n < kF64Sites && ncol < 4; }
+bool use_f64(const DevSites &s, int ncol) { return s.wide || (s.n < kF64Sites && ncol < 4); }
 
 }  // namespace
 
 int tmu_rows_parts(const DevSites &s, int ncol) {
-  if (use_f64(s.n, ncol)) return 0;
+  if (use_f64(s, ncol)) return 0;
   return ncol == 1 && s.n < kOneSites ? s.n : (s.n + 7) / 8;
 }
 
@@ -373,7 +374,7 @@ void launch_tmu_rows(const DevSites &s, int nrhs, const double *x, double *y, bo
   a.ri = s.d2d_nnz ? s.d2d_ri : nullptr, a.src = s.d2d_src, a.scale = s.d2d_s;
   a.thr = s.damp_thr;
   a.thr2m = (float)(s.damp_thr * s.damp_thr * (1.0 + 1e-5));
-  const bool f64 = use_f64(s.n, nrhs), one = nrhs == 1 && s.n < kOneSites;
+  const bool f64 = use_f64(s, nrhs), one = nrhs == 1 && s.n < kOneSites;
   const int npart = tmu_rows_parts(s, nrhs);
   for (int c = 0; c < nrhs;) {
     const int g = nrhs - c >= 2 ? 2 : 1, groups = g == 2 && !f64 ? (nrhs - c) / 2 : 1;

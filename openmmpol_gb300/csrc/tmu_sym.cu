@@ -517,7 +517,7 @@ void launch_tmu_f64_sym_multi(int g, bool amoeba, const SymSlice *sl, int nsl, u
     j.item0 = sl[k].item0;
     j.thr = s.damp_thr;
     j.thr2m = thr2_margin(s);
-    j.r2near = std::max(s.damp_r2max32, s.amoeba ? kSymNear2 : kSymNear2Wang);
+    j.r2near = near_range2(s, s.damp_r2max32);
     tab.base[tab.njobs] = total;
     total += sl[k].count;
     ++tab.njobs;
