@@ -40,6 +40,7 @@ struct DevSites {
   Pos64 *mm_pos = nullptr;    // x, y, z, thole (0 when not polarizable)
   double *mm_a = nullptr;       // damping a of the source (AMOEBA)
   double *mm_q = nullptr;       // [m][ld] lab-frame multipoles
+  int q_ex = 0;                 // 2^q_ex is their size (0 where that is near one)
   int ld = 1;
   // scaled pairs, target-major
   int *m2d_ri = nullptr, *m2d_src = nullptr;
