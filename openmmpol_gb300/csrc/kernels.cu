@@ -94,16 +94,18 @@ __global__ void k_tmu_finish(int n, const double *__restrict__ field, const Pos6
     for (int k = ri[j]; k < ri[j + 1]; ++k) {
       int i = src[k];
       const Pos64 ps = pos[i];
-      double dx = pt.x - ps.x, dy = pt.y - ps.y, dz = pt.z - ps.z;
-      double r2 = dx * dx + dy * dy + dz * dz;
+      const double dx = pt.x - ps.x, dy = pt.y - ps.y, dz = pt.z - ps.z;
+      const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
       double k3, k5;
-      dd_pair_f64<AMOEBA>(r2, pt.w, ps.w, at, AMOEBA ? damp[i] : 0.0, wat, wa[i], thr, thr2m, k3, k5);
+      // every operation as in the near field (fmm_near.cu): the excluded pairs
+      // are the largest terms and have to cancel
+      dd_pair_f64<AMOEBA, true>(r2, pt.w, ps.w, at, AMOEBA ? damp[i] : 0.0, wat, wa[i], thr, thr2m, k3, k5);
       const double *mu = &x[((size_t)r * n + i) * 3];
-      double f = 3.0 * k5 * (mu[0] * dx + mu[1] * dy + mu[2] * dz);
-      double cs = scale[k] - 1.0;
-      e[0] += cs * (f * dx - k3 * mu[0]);
-      e[1] += cs * (f * dy - k3 * mu[1]);
-      e[2] += cs * (f * dz - k3 * mu[2]);
+      const double f = 3.0 * k5 * fma(mu[0], dx, fma(mu[1], dy, mu[2] * dz));
+      const double cs = scale[k] - 1.0;
+      e[0] = fma(cs, fma(f, dx, -(k3 * mu[0])), e[0]);
+      e[1] = fma(cs, fma(f, dy, -(k3 * mu[1])), e[1]);
+      e[2] = fma(cs, fma(f, dz, -(k3 * mu[2])), e[2]);
     }
   }
   const double *xj = &x[((size_t)r * n + j) * 3];
