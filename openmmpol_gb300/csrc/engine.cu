@@ -924,6 +924,13 @@ int System::inversion64(const double *rhs, double *x) {
   bool done = false;
   st = refine_inverse(rhs, x, done);
   if (st || done) return st;
+  // the LU factors serve this geometry, beside T for a while: they may need
+  // the room, and nothing reads the inverse any more
+  cudaStreamSynchronize(st_);
+  release(inv32_);
+  inv32_ = nullptr;
+  inv_ok_ = false;
+  inv_failed_ = true;
   return lu64(rhs, x);
 }
 
@@ -934,8 +941,7 @@ int System::refine_inverse(const double *rhs, double *x, bool &done) {
   const int nn = 3 * d_.n;
   if (!inv_ok_) {
     if (inv_failed_) return kOk;
-    if (!inv32_ && (alloc(inv32_, gpu::inverse32_floats(nn)) || alloc(sqrt_alpha_, (size_t)nn))) {
-      cudaGetLastError();
+    if ((!inv32_ && alloc(inv32_, gpu::inverse32_floats(nn))) || (!sqrt_alpha_ && alloc(sqrt_alpha_, (size_t)nn))) {
       release(inv32_);
       inv32_ = nullptr;
       inv_failed_ = true;  // the LU factorisation reports its own memory
