@@ -31,7 +31,7 @@ __device__ __forceinline__ dsf fast_two_sum(float a, float b) {
   float e = b - (s - a);
   return {s, e};
 }
-// t - s of two coordinates split on a common grid (split_coordinates): the two
+// t - s of two coordinates split on a common grid (launch_split): the two
 // leading differences are exact and |th - sh| is 0 or at least |tm - sm|, so
 // the fast sum is exact too
 __device__ __forceinline__ dsf ds_delta(float th, float tm, float tl, float sh, float sm, float sl) {

@@ -4,7 +4,7 @@
 // Tensors of a pair are written with the unit-length vector n = d y, y the FP32
 // reciprocal distance; for the dipole field
 //   E = 3 r^-5 (mu.d) d - r^-3 mu = K (mu.n) n - k3 mu.
-// Coordinates come split on a grid into three floats (split_coordinates), so
+// Coordinates come split on a grid into three floats (launch_split), so
 // differences are exact; |n|^2 is within 2^-22 of 1 and its deviation eps is
 // collected exactly by adding the squares to 2; the damped inverse powers
 // follow from powers of y by first- and second-order factors in eps:

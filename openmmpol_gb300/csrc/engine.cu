@@ -401,24 +401,30 @@ int System::upload_geometry() {
   if (n) h2d(d_.tile_box32, boxes.data(), boxes.size() * sizeof(float4));
   // double-single kernels: 32-site boxes, and the coordinates about the
   // centroid rounded to whole bohr (so that the shift is exact) in three floats
-  std::vector<float4> subs(2 * (size_t)((n + 31) / 32)), msplit(3 * (size_t)mm), split(3 * (size_t)n);
+  std::vector<float4> subs(2 * (size_t)((n + 31) / 32));
   gpu::tile_boxes32(pp32.data(), n, subs.data(), 32);
   double whole[3] = {std::nearbyint(c[0]), std::nearbyint(c[1]), std::nearbyint(c[2])};
-  bool wide = false;
+  double extent = 0.0;
   for (int i = 0; i < mm; ++i)
-    for (int k = 0; k < 3; ++k) wide = wide || std::fabs(m.cmm[3 * (size_t)i + k] - whole[k]) > gpu::kGridReach;
-  if (wide != d_.wide) {
-    d_.wide = wide;
+    for (int k = 0; k < 3; ++k) extent = std::max(extent, std::fabs(m.cmm[3 * (size_t)i + k] - whole[k]));
+  const double step = gpu::split_step(extent);
+  // up to here the host splits them in less than two launches take (a
+  // coordinate update of 36 sites 78 us, 90 with the launches); beyond, the
+  // loop and the copies were half of an update (18,331 static sites 0.50 ms,
+  // now 0.31)
+  const bool host_split = mm <= 4096;
+  auto split = [&](int count, const std::vector<gpu::Pos64> &x, const gpu::Pos64 *dev, float4 *out) {
+    if (!host_split) return gpu::launch_split(count, dev, whole, step, out, st_);
+    std::vector<float4> parts(3 * (size_t)count);
+    gpu::split_coordinates(count, x.data(), whole, step, parts.data());
+    h2d(out, parts.data(), parts.size() * sizeof(float4));
+  };
+  split(n, pp, d_.pol_pos, d_.pol_split);
+  if (d_.wide != (extent > gpu::kGridReach)) {
+    d_.wide = !d_.wide;
     upload_damping_test();
   }
-  gpu::split_coordinates(m.cmm.data(), mm, whole, msplit.data());
-  for (int p = 0; p < 3; ++p)
-    for (int j = 0; j < n; ++j) split[(size_t)p * n + j] = msplit[(size_t)p * mm + m.polar_mm[j]];
-  if (mm) h2d(d_.mm_split, msplit.data(), msplit.size() * sizeof(float4));
-  if (n) {
-    h2d(d_.sub_box32, subs.data(), subs.size() * sizeof(float4));
-    h2d(d_.pol_split, split.data(), split.size() * sizeof(float4));
-  }
+  if (n) h2d(d_.sub_box32, subs.data(), subs.size() * sizeof(float4));
   // tile boxes of the static sites
   std::vector<float4> mp32(mm);
   for (int i = 0; i < mm; ++i) {
@@ -434,6 +440,7 @@ int System::upload_geometry() {
     h2d(d_.mm_sub_box32, msubs.data(), msubs.size() * sizeof(float4));
   }
   h2d(d_.mm_pos, mp.data(), mm * sizeof(gpu::Pos64));
+  split(mm, mp, d_.mm_pos, d_.mm_split);
   h2d(d_.mm_a, ma.data(), mm * sizeof(double));
   h2d(d_.mm_q, m.q.data(), m.q.size() * sizeof(double));
   // the host vectors above die at return: wait for the copies

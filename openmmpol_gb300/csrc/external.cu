@@ -47,7 +47,7 @@ struct ExtRec {
   static constexpr int R = (9 + 2 * NV + 3) / 4;
 };
 
-// x - c as three floats on the grid g1, g1 2^-23 (split_coordinates)
+// x - c as three floats on the grid g1, g1 2^-23 (launch_split)
 __device__ __forceinline__ void split3(double v, double g1, float *o) {
   const double g2 = g1 * 1.1920928955078125e-7;
   const double h = rint(v / g1) * g1, m = rint((v - h) / g2) * g2;

@@ -1113,14 +1113,10 @@ int System::fmm_prepare() {
     sa[s] = m_.damping[j];
     swa[s] = make_float2(d_.wide ? 0.f : (float)(w * w), (float)(m_.damping[j] * m_.damping[j]));
   }
-  std::vector<float4> split(3 * (size_t)n);
-  {
-    std::vector<double> xs(3 * (size_t)n);
-    for (int s = 0; s < n; ++s) std::copy_n(&xp[3 * (size_t)o.perm_s[s]], 3, &xs[3 * (size_t)s]);
-    double whole[3];
-    for (int d = 0; d < 3; ++d) whole[d] = std::nearbyint(o.lo[d] + 0.5 * o.side);
-    gpu::split_coordinates(xs.data(), n, whole, split.data());
-  }
+  double whole[3], extent = 0.0;
+  for (int d = 0; d < 3; ++d) whole[d] = std::nearbyint(o.lo[d] + 0.5 * o.side);
+  for (int j = 0; j < n; ++j)
+    for (int d = 0; d < 3; ++d) extent = std::max(extent, std::fabs(xp[3 * (size_t)j + d] - whole[d]));
   t.L = o.L;
   t.h0 = o.side;
   t.ox = o.lo[0], t.oy = o.lo[1], t.oz = o.lo[2];
@@ -1128,7 +1124,10 @@ int System::fmm_prepare() {
   t.ncell = o.ncell;
   t.shared = true;
   int bad = upload(t.cnt, o.cnt_s, st_) | upload(t.leaf_start, o.start_s, st_) | upload(t.perm, o.perm_s, st_) |
-            upload(t.spos, spos, st_) | upload(t.sa, sa, st_) | upload(t.swa, swa, st_) | upload(t.split, split, st_);
+            upload(t.spos, spos, st_) | upload(t.sa, sa, st_) | upload(t.swa, swa, st_);
+  if (t.split) cudaFree(t.split);
+  t.split = nullptr;
+  bad |= cudaMalloc((void **)&t.split, 3 * (size_t)n * sizeof(float4)) != cudaSuccess;
   t.cnt_t = t.cnt, t.leaf_start_t = t.leaf_start, t.perm_t = t.perm, t.spos_t = t.spos;
   if (t.nalloc_cell < t.ncell) {
     if (t.M) cudaFree(t.M);
@@ -1155,6 +1154,7 @@ int System::fmm_prepare() {
     set_last_error("out of device memory for the FMM tree");
     return kErrMemory;
   }
+  gpu::launch_split(n, t.spos, whole, gpu::split_step(extent), t.split, st_);
   int st = check(cudaStreamSynchronize(st_), "FMM tree upload");  // host vectors die here
   if (st) return st;
   log_msg(kVerbHigh, nullptr, "FMM: order %d, %d levels, leaf side %.2f bohr, %d sites", f.p, t.L, t.h0 / (1 << t.L),

@@ -55,7 +55,7 @@ struct DevSites {
   float4 *tile_box32 = nullptr;
   int ntile = 0;
   // symmetric FP64 product: coordinates split into three floats [3][n]
-  // (split_coordinates) and the bounding boxes of 32 sites
+  // (launch_split) and the bounding boxes of 32 sites
   float4 *pol_split = nullptr, *sub_box32 = nullptr;
   // the same split of the static sites [3][m] (one grid for both)
   float4 *mm_split = nullptr, *mm_sub_box32 = nullptr;  // and their 32-site boxes
@@ -158,8 +158,11 @@ void launch_fmm_near(const FmmNearArgs &a, const double *x, const unsigned *word
 // [kFmmNearSplit][n][3] in polarizable order
 void launch_m2d_leaf(const DevSites &s, int L, const int *leaf_start, const int *perm, const int *leaf_start_t,
                      const int *perm_t, double *partial, int *err_flag, cudaStream_t st);
-// coordinates x [n][3] about a centre as three floats each, out [3][n]
-void split_coordinates(const double *x, int n, double centre[3], float4 *out);
+// coordinates of the sites pos about a centre as three floats each, out [3][n],
+// on the grid of a step for the largest of them
+double split_step(double extent);
+void launch_split(int n, const Pos64 *pos, const double centre[3], double g1, float4 *out, cudaStream_t st);
+void split_coordinates(int n, const Pos64 *pos, const double centre[3], double g1, float4 *out);  // on the host
 // The pairwise FP32 product (tmu32_rows.cu): columns in groups of up to gmax
 // (4); part: partial sums of x.y, tmu32_rows_parts per column
 int tmu32_rows_parts(int n);

@@ -11,7 +11,7 @@
 // r) or that are close.  All others are formed on the FP32 pipes in
 // double-single arithmetic (ds_math.cuh), ~285 FP32 operations per unordered
 // pair, with
-//   * coordinates split on a grid into three floats (split_coordinates), so
+//   * coordinates split on a grid into three floats (launch_split), so
 //     that the difference of two sites is exact and costs 7 operations;
 //   * the unit-length form E = K (mu.n) n - k3 mu of the dipole field
 //     (n = d y, y the FP32 reciprocal distance): |n|^2 is within 2^-22 of 1,
@@ -62,6 +62,22 @@ namespace ommp {
 namespace gpu {
 
 namespace {
+
+// x = h + m + l with h a multiple of g1 and m of g1 2^-23 (g1 = 2^-23 of the
+// power of two that bounds every coordinate), so that differences of h and of
+// m are exact in FP32; the parts a stride apart
+__host__ __device__ inline void split_site(const Pos64 &p, double c0, double c1, double c2, double g1, float4 *out,
+                                           size_t stride) {
+  const double v[3] = {p.x - c0, p.y - c1, p.z - c2}, g2 = g1 * 1.1920928955078125e-7;
+  float h[3], m[3], l[3];
+  for (int k = 0; k < 3; ++k) {
+    const double hk = rint(v[k] / g1) * g1, mk = rint((v[k] - hk) / g2) * g2;
+    h[k] = (float)hk, m[k] = (float)mk, l[k] = (float)((v[k] - hk) - mk);
+  }
+  out[0] = make_float4(h[0], h[1], h[2], 0.f);
+  out[stride] = make_float4(m[0], m[1], m[2], 0.f);
+  out[2 * stride] = make_float4(l[0], l[1], l[2], 0.f);
+}
 
 constexpr int SYM_TILE = 128;
 constexpr int SYM_SUB = 32;
@@ -440,6 +456,12 @@ __global__ void __launch_bounds__(FIN_TPB) k_tmu_sym_finish(
   }
 }
 
+__global__ void __launch_bounds__(256) k_split(int n, const Pos64 *__restrict__ pos, double c0, double c1, double c2,
+                                               double g1, float4 *__restrict__ out) {
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i < n) split_site(pos[i], c0, c1, c2, g1, out + i, n);
+}
+
 template <int G, bool AMOEBA>
 struct SymLaunch {
   int resident = 0;
@@ -645,28 +667,20 @@ void launch_max_words(int ncol, size_t nv, const double *x, unsigned *words, cud
   k_sym_prepare<<<dim3(blocks, ncol), 256, 0, st>>>(nv, x, nullptr, words, 0);
 }
 
-// x = h + m + l with h a multiple of g and m of g 2^-23 (g = 2^-23 of the
-// power of two that bounds every coordinate), so that differences of h and of
-// m are exact in FP32
-void split_coordinates(const double *x, int n, double centre[3], float4 *out) {
-  double big = 1.0;
-  for (int i = 0; i < n; ++i)
-    for (int k = 0; k < 3; ++k) big = std::max(big, std::fabs(x[3 * (size_t)i + k] - centre[k]));
+double split_step(double extent) {
   int e = 0;
-  std::frexp(big, &e);  // big < 2^e
-  const double g1 = std::ldexp(1.0, e - 23), g2 = std::ldexp(g1, -23);
-  for (int i = 0; i < n; ++i) {
-    float h[3], m[3], l[3];
-    for (int k = 0; k < 3; ++k) {
-      const double v = x[3 * (size_t)i + k] - centre[k];
-      const double hk = std::nearbyint(v / g1) * g1;
-      const double mk = std::nearbyint((v - hk) / g2) * g2;
-      h[k] = (float)hk, m[k] = (float)mk, l[k] = (float)((v - hk) - mk);
-    }
-    out[i] = make_float4(h[0], h[1], h[2], 0.f);
-    out[(size_t)n + i] = make_float4(m[0], m[1], m[2], 0.f);
-    out[2 * (size_t)n + i] = make_float4(l[0], l[1], l[2], 0.f);
-  }
+  std::frexp(std::max(1.0, extent), &e);  // extent < 2^e
+  return std::ldexp(1.0, e - 23);
+}
+
+void split_coordinates(int n, const Pos64 *pos, const double centre[3], double g1, float4 *out) {
+  for (int i = 0; i < n; ++i) split_site(pos[i], centre[0], centre[1], centre[2], g1, out + i, n);
+}
+
+void launch_split(int n, const Pos64 *pos, const double centre[3], double g1, float4 *out, cudaStream_t st) {
+  if (n == 0) return;
+  add_launch_count(1);
+  k_split<<<(n + 255) / 256, 256, 0, st>>>(n, pos, centre[0], centre[1], centre[2], g1, out);
 }
 
 }  // namespace gpu

@@ -133,11 +133,12 @@ def test_fmm_streams_that_cannot_be_made(fake, path):
     live = fake.fake_live()
     fake.fake_fail_events(1)
     try:
-        for _ in range(2):
-            launches = fake.fake_launches()
+        for k in range(2):
             with pytest.raises(OMMPError, match="streams"):
                 tmatvec_fmm(g)
-            assert fake.fake_launches() == launches
+            if k == 0:  # the tree is there
+                launches = fake.fake_launches()
+        assert fake.fake_launches() == launches
     finally:
         fake.fake_fail_events(0)
     tmatvec_fmm(g)
