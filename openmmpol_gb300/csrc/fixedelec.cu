@@ -27,6 +27,7 @@
 #include <cmath>
 #include <vector>
 
+#include "ds_pair.cuh"
 #include "engine.h"
 #include "grad_math.cuh"
 #include "m2m_math.cuh"
@@ -38,6 +39,7 @@ namespace {
 
 struct M2mArgs {
   int mm, nsplit;
+  int ex;  // the multipoles are scaled by 2^-ex
   const Pos64 *pos;
   const double *q;
   const int *ri, *src;
@@ -47,6 +49,15 @@ struct M2mArgs {
   double *E, *G;    // [mm][3], [mm][6] field and field gradient (gradient pass)
   double *base;     // [mm][3] site gradient terms (gradient pass)
 };
+
+// Multipoles far from one, scaled by a power of two for the passes: products of
+// two quadrupoles and r^-11 would leave the range of the FP32 pair pass (3e-10 of
+// the gradient at 1e-12, 1e-3 at 1e-18).  The finishing pass scales back.  (Scaling
+// in the pair kernel cost it 4 % at 30,000 sites for every system.)
+__global__ void k_m2m_scale(int total, const double *__restrict__ q, int ex, double *__restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < total) out[i] = scale_down(q[i], ex);
+}
 
 template <bool AMOEBA, bool GRAD>
 __global__ void k_m2m_finish(M2mArgs a) {
@@ -74,19 +85,20 @@ __global__ void k_m2m_finish(M2mArgs a) {
     m2m_any<AMOEBA, GRAD>(&a.q[(size_t)i * LD], dx, dy, dz, 1.0 / sqrt(r2), a.sc[k] - 1.0, Qt, trq, acc);
   }
   const double *q = &a.q[(size_t)t * LD];
+  auto back = [&](double v) { return scale_up(v, a.ex); };
   if (GRAD) {
     double g[3];
     for (int c = 0; c < 3; ++c) {
-      a.E[3 * (size_t)t + c] = acc[c];
+      a.E[3 * (size_t)t + c] = back(acc[c]);
       g[c] = -q[0] * acc[c];
     }
     if (AMOEBA) {
       double mg[3];
       gradmath::sym_apply(acc + 3, q + 1, mg);
-      for (int c = 0; c < 6; ++c) a.G[6 * (size_t)t + c] = acc[3 + c];
+      for (int c = 0; c < 6; ++c) a.G[6 * (size_t)t + c] = back(acc[3 + c]);
       for (int c = 0; c < 3; ++c) g[c] += mg[c] - acc[9 + c];
     }
-    for (int c = 0; c < 3; ++c) a.base[3 * (size_t)t + c] = g[c];
+    for (int c = 0; c < 3; ++c) a.base[3 * (size_t)t + c] = back(back(g[c]));
     return;
   }
   double e = q[0] * acc[0];
@@ -95,7 +107,7 @@ __global__ void k_m2m_finish(M2mArgs a) {
     const double *g = acc + (GRAD ? 3 : 4);
     e += q[4] * g[0] + q[6] * g[2] + q[9] * g[5] + 2.0 * (q[5] * g[1] + q[7] * g[3] + q[8] * g[4]);
   }
-  a.site[t] = e;
+  a.site[t] = back(back(e));
 }
 
 }  // namespace
@@ -136,7 +148,8 @@ int System::m2m_launch(bool grad, double **site_out, double **e_out, double **g_
   build_ss(m_, mm, ri, src, sc);
   const int nsplit = gpu::m2m_pick_split(d_, grad, gpu::sm_count());
   const size_t out = grad ? 12 * (size_t)mm : (size_t)mm;  // E, G, base | site
-  const size_t need = (size_t)nsplit * nv * mm + out + ri.size() + 2 * src.size() + 1;
+  const size_t scaled = d_.q_ex ? (size_t)d_.ld * mm : 0;
+  const size_t need = (size_t)nsplit * nv * mm + out + ri.size() + 2 * src.size() + 1 + scaled;
   if (need > fe_cap_) {  // kept for the next geometry
     if (fe_buf_) cudaFree(fe_buf_);
     fe_buf_ = nullptr;
@@ -170,12 +183,21 @@ int System::m2m_launch(bool grad, double **site_out, double **e_out, double **g_
   a.ri = ri_d;
   a.src = src_d;
   a.sc = sc_d;
+  gpu::DevSites d = d_;
+  if (scaled) {
+    double *q = fe_buf_ + need - scaled;
+    gpu::k_m2m_scale<<<(unsigned)((scaled + 255) / 256), 256, 0, st_>>>((int)scaled, d_.mm_q, d_.q_ex, q);
+    gpu::add_launch_count(1);
+    d.mm_q = q;
+    a.q = q;
+    a.ex = d_.q_ex;
+  }
   cudaMemcpyAsync(sc_d, sc.data(), sc.size() * sizeof(double), cudaMemcpyHostToDevice, st_);
   cudaMemcpyAsync(ri_d, ri.data(), ri.size() * sizeof(int), cudaMemcpyHostToDevice, st_);
   cudaMemcpyAsync(src_d, src.data(), src.size() * sizeof(int), cudaMemcpyHostToDevice, st_);
   cudaMemsetAsync(flag_, 0, sizeof(int), st_);
   const int fb = (mm + 127) / 128;
-  gpu::launch_m2m(d_, grad, buf, nsplit, flag_, st_);
+  gpu::launch_m2m(d, grad, buf, nsplit, flag_, st_);
   a.nsplit = gpu::launch_sum_splits((size_t)nv * mm, nsplit, buf, st_);
   if (amoeba && grad)
     gpu::k_m2m_finish<true, true><<<fb, 128, 0, st_>>>(a);

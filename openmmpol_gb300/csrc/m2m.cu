@@ -11,14 +11,12 @@
 // are added to FP64 ones; partial [split][component][site].  6,000 sites:
 // 1.09 and 2.27 ms (1.52 and 3.36 with every product and sum renormalised, for
 // gradient errors of 2e-14 instead of 3.4e-14; 1.7e-13 in FP64 before).  80 % of
-// the FP32 issue slots.  Multipoles far from one are scaled by a power of two:
-// products of two quadrupoles and r^-11 would leave the range of FP32 (1e-11 of
-// the gradient at 1e-12, 1e-3 at 1e-18).
+// the FP32 issue slots.
 //
 // Built with --fmad=false -ftz=true like the other double-single kernels.
 #include <algorithm>
 
-#include "ds_pair.cuh"
+#include "ds_math.cuh"
 #include "kernels.h"
 #include "m2m_math.cuh"
 #include "pair_math.cuh"
@@ -64,7 +62,7 @@ __global__ void __launch_bounds__(NT) k_m2m(const __grid_constant__ DevSites s, 
   dsf Q[6], trq{0.f, 0.f};
   if (GRAD && AMOEBA) {
 #pragma unroll
-    for (int c = 0; c < 6; ++c) Q[c] = to_ds(scale_down(s.mm_q[(size_t)tc * LD + 4 + c], s.q_ex));
+    for (int c = 0; c < 6; ++c) Q[c] = to_ds(s.mm_q[(size_t)tc * LD + 4 + c]);
     trq = Q[0] + Q[2] + Q[5];
   }
   double sum[NV];
@@ -85,8 +83,7 @@ __global__ void __launch_bounds__(NT) k_m2m(const __grid_constant__ DevSites s, 
       s_pl[threadIdx.x] = s.mm_split[2 * (size_t)s.m + i];
 #pragma unroll
       for (int c = 0; c < LD; ++c) {
-        const double v = s.mm_q[(size_t)i * LD + c];
-        const dsf q = to_ds(s.q_ex ? scale_down(v, s.q_ex) : v);
+        const dsf q = to_ds(s.mm_q[(size_t)i * LD + c]);
         s_qh[threadIdx.x * LD + c] = q.h;
         s_ql[threadIdx.x * LD + c] = q.l;
       }
@@ -116,14 +113,7 @@ __global__ void __launch_bounds__(NT) k_m2m(const __grid_constant__ DevSites s, 
       m2m_any<AMOEBA, GRAD>(q, dx, dy, dz, rinv, gradmath::One{}, Q, trq, acc);
     }
 #pragma unroll
-    for (int c = 0; c < NV; ++c) {
-      double v = (double)acc[c].h + (double)acc[c].l;
-      if (s.q_ex) {  // the contracted Hessian has two multipoles
-        v = scale_up(v, s.q_ex);
-        if (GRAD && AMOEBA && c >= 9) v = scale_up(v, s.q_ex);
-      }
-      sum[c] += v;
-    }
+    for (int c = 0; c < NV; ++c) sum[c] += (double)acc[c].h + (double)acc[c].l;
   }
   form();
   if (!valid) return;
