@@ -26,14 +26,6 @@ __device__ __forceinline__ int dsp_exponent(unsigned emax) {
   const int e = (int)(emax >> 20);
   return e == 0 ? 0 : e - 1023 + 12;
 }
-// 2^e of a scaling of two sets of values together, from their largest high
-// words: e with the largest magnitude in [2^e, 2^(e + 1)), or 0, no scaling,
-// when all are zero or the magnitude is within 2^-4 to 2^4 (a few bits more or
-// less are not missed)
-__device__ __forceinline__ int dsp_exponent_of(unsigned a, unsigned b) {
-  const int e = (int)(max(a, b) >> 20);
-  return e == 0 || (e >= 1023 - 4 && e < 1023 + 4) ? 0 : e - 1023;
-}
 __device__ __forceinline__ double pow2(int e) {  // |e| <= 1022
   return __hiloint2double((1023 + e) << 20, 0);
 }

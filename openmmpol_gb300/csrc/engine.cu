@@ -317,12 +317,9 @@ int System::upload_static() {
   up(d_.pol_a32, a32.data(), n * sizeof(float));
   up(d_.polar_mm, m.polar_mm.data(), n * sizeof(int));
   upload_damping_test();
-  // the size of the multipoles (a rotation changes a value at most threefold)
   double big = 0.0;
   for (double q : m.q) big = std::max(big, std::fabs(q));
-  int e = 0;
-  if (big > 0.0 && std::isfinite(big)) std::frexp(big, &e);
-  d_.q_ex = std::abs(e) > 4 ? e : 0;
+  if (big > 0.0 && std::isfinite(big)) d_.q_e = std::ilogb(big);
   {
     std::vector<double> w(n);
     for (int j = 0; j < n; ++j) w[j] = 1.0 / m.thole[m.polar_mm[j]];

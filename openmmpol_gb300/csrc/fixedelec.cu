@@ -148,7 +148,8 @@ int System::m2m_launch(bool grad, double **site_out, double **e_out, double **g_
   build_ss(m_, mm, ri, src, sc);
   const int nsplit = gpu::m2m_pick_split(d_, grad, gpu::sm_count());
   const size_t out = grad ? 12 * (size_t)mm : (size_t)mm;  // E, G, base | site
-  const size_t scaled = d_.q_ex ? (size_t)d_.ld * mm : 0;
+  const int ex = gpu::scaling_exponent(d_.q_e);
+  const size_t scaled = ex ? (size_t)d_.ld * mm : 0;
   const size_t need = (size_t)nsplit * nv * mm + out + ri.size() + 2 * src.size() + 1 + scaled;
   if (need > fe_cap_) {  // kept for the next geometry
     if (fe_buf_) cudaFree(fe_buf_);
@@ -186,11 +187,11 @@ int System::m2m_launch(bool grad, double **site_out, double **e_out, double **g_
   gpu::DevSites d = d_;
   if (scaled) {
     double *q = fe_buf_ + need - scaled;
-    gpu::k_m2m_scale<<<(unsigned)((scaled + 255) / 256), 256, 0, st_>>>((int)scaled, d_.mm_q, d_.q_ex, q);
+    gpu::k_m2m_scale<<<(unsigned)((scaled + 255) / 256), 256, 0, st_>>>((int)scaled, d_.mm_q, ex, q);
     gpu::add_launch_count(1);
     d.mm_q = q;
     a.q = q;
-    a.ex = d_.q_ex;
+    a.ex = ex;
   }
   cudaMemcpyAsync(sc_d, sc.data(), sc.size() * sizeof(double), cudaMemcpyHostToDevice, st_);
   cudaMemcpyAsync(ri_d, ri.data(), ri.size() * sizeof(int), cudaMemcpyHostToDevice, st_);

@@ -105,9 +105,8 @@ __global__ void k_grad_finish(GradArgs g) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= g.mm) return;
   double sums[NO];
-  const unsigned word = reinterpret_cast<const unsigned *>(g.bad + 1)[1];
-  const int ex = dsp_exponent(word);
-  const int es = dsp_exponent_of(*reinterpret_cast<const unsigned *>(g.bad + 3), word);
+  const int ex = dsp_exponent(reinterpret_cast<const unsigned *>(g.bad + 1)[1]);
+  const int es = ex - *reinterpret_cast<const int *>(g.bad + 3);
   for (int c = 0; c < NO; ++c) {
     const size_t o = (size_t)t * NO + c;
     const double v = scale_up(scale_up(fixed_value(g.lo[o], g.hi[o]), ex), es);

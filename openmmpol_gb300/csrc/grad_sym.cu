@@ -591,18 +591,18 @@ __global__ void __launch_bounds__(TILE, AMOEBA ? 2 : 4) k_grad_sym(const __grid_
 
 // scaled mean dipoles and half differences in static-site order, whether any
 // difference is not zero and whether any quadrupole has a trace beyond
-// rounding, and the largest high word of the static multipoles
+// rounding; the static multipoles scaled by 2^-es, es from their exponent and
+// that of the dipoles, and eu = ex - es
 __global__ void k_grad_dipoles(int m, int n, int nset, const int *__restrict__ mm_polar, const double *__restrict__ ipd,
                                const unsigned *__restrict__ word, double *__restrict__ p, double *__restrict__ d,
-                               const double *__restrict__ q, int *any, unsigned *qword) {
+                               const double *__restrict__ q, int q_e, double *__restrict__ qs, int *any, int *eu) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int ld = nset == 2 ? 10 : 1;
-  unsigned big = 0;
-  for (int c = 0; i < m && c < ld; ++c) big = max(big, (unsigned)__double2hiint(q[(size_t)i * ld + c]) & 0x7FFFFFFFu);
-  big = __reduce_max_sync(0xffffffffu, big);
-  if ((threadIdx.x & 31) == 0 && big) atomicMax(qword, big);
   if (i >= m) return;
   const int j = mm_polar[i], ex = dsp_exponent(*word);
+  const int es = scaling_exponent(max(q_e, *word >> 20 ? (int)(*word >> 20) - 1023 : kNoExponent));
+  if (i == 0) *eu = ex - es;
+  const int ld = nset == 2 ? 10 : 1;
+  for (int c = 0; c < ld; ++c) qs[(size_t)i * ld + c] = scale_down(q[(size_t)i * ld + c], es);
   bool diff = false;
   for (int c = 0; c < 3; ++c) {
     const double a = j >= 0 ? scale_down(ipd[3 * (size_t)j + c], ex) : 0.0;
@@ -617,14 +617,6 @@ __global__ void k_grad_dipoles(int m, int n, int nset, const int *__restrict__ m
     const double diag = fmax(fmax(fabs(Q[0]), fabs(Q[2])), fabs(Q[5]));
     if (fabs((Q[0] + Q[2]) + Q[5]) > 2e-15 * diag) any[1] = 1;
   }
-}
-
-// the static multipoles scaled by 2^-es (dsp_exponent_of), and eu = ex - es
-__global__ void k_grad_scale(int total, const double *__restrict__ q, const unsigned *__restrict__ word,
-                             const unsigned *__restrict__ qword, double *__restrict__ out, int *eu) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x, es = dsp_exponent_of(*qword, *word);
-  if (i == 0) *eu = dsp_exponent(*word) - es;
-  if (i < total) out[i] = scale_down(q[i], es);
 }
 
 template <bool AMOEBA>
@@ -642,7 +634,7 @@ int resident() {
 }  // namespace
 
 // the buffer of launch_grad_sym: fixed-point words (lo, hi) of the outputs,
-// flag, counter and scale of the dipoles, two flags, scales of the multipoles,
+// flag, counter and scale of the dipoles, two flags, scale of the multipoles,
 // dipoles and differences, scaled multipoles
 size_t grad_sym_doubles(const DevSites &s) {
   const size_t no = s.amoeba ? 6 : 3;
@@ -660,14 +652,14 @@ void launch_grad_sym(const DevSites &s, const double *ipd, const int *mm_polar, 
   j.bad = j.hi + no * s.m;
   unsigned *next = reinterpret_cast<unsigned *>(j.bad + 1), *word = next + 1;
   int *any = reinterpret_cast<int *>(j.bad + 2);
-  unsigned *qword = reinterpret_cast<unsigned *>(j.bad + 3);
   double *p = reinterpret_cast<double *>(j.bad + 4);
   j.p = p;
   j.d = p + 3 * (size_t)s.m;
   j.any = any;
   double *q = p + 6 * (size_t)s.m;
   j.q = q;
-  j.eu = reinterpret_cast<int *>(qword + 1);
+  int *eu = reinterpret_cast<int *>(j.bad + 3);
+  j.eu = eu;
   j.polar = polar;
   j.err = err;
   j.r2near = near_range2(s, s.m2d_r2max32);
@@ -681,12 +673,10 @@ void launch_grad_sym(const DevSites &s, const double *ipd, const int *mm_polar, 
   j.quarters = units < 8LL * ctas ? 4 : 1;
   j.items = j.ntile * j.nchunk * j.quarters;
   cudaMemsetAsync(buf, 0, (2 * no * s.m + 4) * sizeof(double), st);
-  launch_max_word(nset * 3 * (size_t)s.n, ipd, word, st);
-  add_launch_count(3);
+  launch_max_word(nset * 3 * (size_t)s.n, ipd, word, st, true);
+  add_launch_count(2);
   k_grad_dipoles<<<(s.m + 255) / 256, 256, 0, st>>>(s.m, s.n, (int)nset, mm_polar, ipd, word, p,
-                                                    p + 3 * (size_t)s.m, s.mm_q, any, qword);
-  const int values = (s.amoeba ? 10 : 1) * s.m;
-  k_grad_scale<<<(values + 255) / 256, 256, 0, st>>>(values, s.mm_q, word, qword, q, reinterpret_cast<int *>(qword + 1));
+                                                    p + 3 * (size_t)s.m, s.mm_q, s.q_e, q, any, eu);
   const int grid = std::min(ctas, j.items);
   if (s.amoeba)
     k_grad_sym<true><<<grid, TILE, sizeof(GradSmem<true>), st>>>(j, next);

@@ -22,6 +22,11 @@ struct __align__(32) Pos64 {
 };
 
 // Immutable per-geometry device data of one system.
+constexpr int kNoExponent = -4096;
+// 2^e of a scaling of values of the exponent e: nothing to scale when there are
+// none or they are within 2^-4 to 2^4 (a few bits more or less are not missed)
+__host__ __device__ inline int scaling_exponent(int e) { return e == kNoExponent || (e >= -4 && e < 4) ? 0 : e; }
+
 struct DevSites {
   int n = 0;      // polarizable sites
   int m = 0;      // MM (static) sites
@@ -40,7 +45,9 @@ struct DevSites {
   Pos64 *mm_pos = nullptr;    // x, y, z, thole (0 when not polarizable)
   double *mm_a = nullptr;       // damping a of the source (AMOEBA)
   double *mm_q = nullptr;       // [m][ld] lab-frame multipoles
-  int q_ex = 0;                 // 2^q_ex is their size (0 where that is near one)
+  // their largest magnitude is in [2^q_e, 2^(q_e + 1)) (before the rotation of
+  // the frames, which changes a value at most threefold); kNoExponent: all zero
+  int q_e = kNoExponent;
   int ld = 1;
   // scaled pairs, target-major
   int *m2d_ri = nullptr, *m2d_src = nullptr;
@@ -134,7 +141,7 @@ void launch_tmu_sym_finish(const DevSites &s, int g, const unsigned long long *l
                            const unsigned long long *bad, const double *x, bool dodiag, double *y, cudaStream_t st,
                            double *part = nullptr, int max_part = 0, int *npart = nullptr, size_t group_words = 0);
 // the largest high word of |x| (the scale of the double-single products)
-void launch_max_word(size_t total, const double *x, unsigned *word, cudaStream_t st);
+void launch_max_word(size_t total, const double *x, unsigned *word, cudaStream_t st, bool zeroed = false);
 void launch_max_words(int ncol, size_t nv, const double *x, unsigned *words, cudaStream_t st);
 // near field of the FMM (fmm_near.cu): the dipoles x [col][n][3] of the 27
 // neighbouring leaves at every site, sites sorted by leaf (split coordinates

@@ -562,9 +562,9 @@ void launch_tmu_sym_prepare(const DevSites &s, int g, const double *x, unsigned 
   k_sym_prepare<<<dim3(blocks, g), 256, 0, st>>>(nv, x, lo, reinterpret_cast<unsigned *>(bad + 1), 0);
 }
 
-void launch_max_word(size_t total, const double *x, unsigned *word, cudaStream_t st) {
+void launch_max_word(size_t total, const double *x, unsigned *word, cudaStream_t st, bool zeroed) {
   add_launch_count(1);
-  cudaMemsetAsync(word, 0, sizeof(unsigned), st);
+  if (!zeroed) cudaMemsetAsync(word, 0, sizeof(unsigned), st);
   const int blocks = (int)std::min<size_t>((total + 255) / 256, 1216);
   k_sym_prepare<<<blocks, 256, 0, st>>>(total, x, nullptr, word, 0);
 }
