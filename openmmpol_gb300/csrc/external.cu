@@ -133,7 +133,7 @@ __global__ void __launch_bounds__(NT, 4) k_ext(const __grid_constant__ ExtArgs a
         continue;
       }
       const double *q = a.val + (size_t)i * NV;
-      const double k1 = rinv_f64_full(r2, r2_f32(r2)), ir2 = k1 * k1, k3 = k1 * ir2, k5 = k3 * ir2;
+      const double k1 = rinv_f64(r2, r2_f32(r2)), ir2 = k1 * k1, k3 = k1 * ir2, k5 = k3 * ir2;
       const double md = fma(q[1], dx, fma(q[2], dy, q[3] * dz));
       double tx = 0.0, ty = 0.0, tz = 0.0, s = 0.0;
       if (QUAD) {

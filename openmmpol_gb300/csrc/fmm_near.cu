@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(NT, 5) k_fmm_near(const __grid_constant__ FmmN
         const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
         if (coincident(r2)) continue;
         double k3, k5;
-        dd_pair_f64<AMOEBA, true>(r2, pt.w, ps.w, at, AMOEBA ? a.sa[k] : 0.0, wat, a.swa[k], a.thr, a.thr2m, k3, k5);
+        dd_pair_f64<AMOEBA>(r2, pt.w, ps.w, at, AMOEBA ? a.sa[k] : 0.0, wat, a.swa[k], a.thr, a.thr2m, k3, k5);
         const double *mu = xc + 3 * (size_t)a.perm[k];
         const double mx = scale_down(mu[0], ex), my = scale_down(mu[1], ex), mz = scale_down(mu[2], ex);
         const double f = 3.0 * k5 * fma(mx, dx, fma(my, dy, mz * dz));

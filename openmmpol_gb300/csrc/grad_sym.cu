@@ -325,7 +325,7 @@ __device__ __noinline__ void grad_queued(const GradSymJob &jb, const unsigned sh
       atomicOr(jb.err, 1);
       continue;
     }
-    const double y = rinv_f64_full(r2, r2_f32(r2));
+    const double y = rinv_f64(r2, r2_f32(r2));
     double k3, k5, k7, k9;
     gradmath::damped_k<AMOEBA>(r2, y, pi.w * pj.w, AMOEBA ? fmin(s.mm_a[i], s.mm_a[j]) : 0.0, s.damp_thr, true, k3, k5,
                                k7, k9);

@@ -55,7 +55,7 @@ __global__ void k_m2d_finish(int n, int nsplit, const double *__restrict__ parti
     double fx = 0, fy = 0, fz = 0;
     // the same reciprocal distance as the pair pass: the excluded pairs are
     // the largest terms and have to cancel
-    m2d_pair_f64<AMOEBA, true>(pt.x - ps.x, pt.y - ps.y, pt.z - ps.z, pt.w, ps.w, at,
+    m2d_pair_f64<AMOEBA>(pt.x - ps.x, pt.y - ps.y, pt.z - ps.z, pt.w, ps.w, at,
                          AMOEBA ? mm_a[i] : 0.0, wat, mm_wa[i], q, thr, thr2m, fx, fy, fz);
     double cp = sP[k] - 1.0, cd = sD[k] - 1.0;
     eP[0] += cp * fx;
@@ -99,7 +99,7 @@ __global__ void k_tmu_finish(int n, const double *__restrict__ field, const Pos6
       double k3, k5;
       // every operation as in the near field (fmm_near.cu): the excluded pairs
       // are the largest terms and have to cancel
-      dd_pair_f64<AMOEBA, true>(r2, pt.w, ps.w, at, AMOEBA ? damp[i] : 0.0, wat, wa[i], thr, thr2m, k3, k5);
+      dd_pair_f64<AMOEBA>(r2, pt.w, ps.w, at, AMOEBA ? damp[i] : 0.0, wat, wa[i], thr, thr2m, k3, k5);
       const double *mu = &x[((size_t)r * n + i) * 3];
       const double f = 3.0 * k5 * fma(mu[0], dx, fma(mu[1], dy, mu[2] * dz));
       const double cs = scale[k] - 1.0;
@@ -412,14 +412,6 @@ __global__ void k_any_diff(size_t n, const double *a, const double *b, int *flag
   const unsigned long long *ub = reinterpret_cast<const unsigned long long *>(b);
   for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
     if (ua[i] != ub[i]) {
-      *flag = 1;
-      return;
-    }
-}
-
-__global__ void k_check_finite(size_t n, const double *x, int *flag) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    if (!isfinite(x[i])) {
       *flag = 1;
       return;
     }
@@ -740,10 +732,6 @@ void launch_reduce_norms(const double *partial, double *out, cudaStream_t st) {
 void launch_any_diff(size_t n, const double *a, const double *b, int *flag, cudaStream_t st) {
   add_launch_count(1);
   k_any_diff<<<blocks_for(n, 256), 256, 0, st>>>(n, a, b, flag);
-}
-void launch_check_finite(size_t n, const double *x, int *flag, cudaStream_t st) {
-  add_launch_count(1);
-  k_check_finite<<<blocks_for(n, 256), 256, 0, st>>>(n, x, flag);
 }
 
 }  // namespace gpu

@@ -326,7 +326,6 @@ void launch_diff_norms(size_t n, const double *a, const double *b, double *parti
                        cudaStream_t st);
 void launch_reduce_norms(const double *partial, double *out, cudaStream_t st);
 // NaN / Inf check: flag set to 1 when any entry is not finite
-void launch_check_finite(size_t n, const double *x, int *flag, cudaStream_t st);
 // flag set to 1 when a and b differ in any bit of any entry
 void launch_any_diff(size_t n, const double *a, const double *b, int *flag, cudaStream_t st);
 

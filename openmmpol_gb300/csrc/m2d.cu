@@ -66,7 +66,7 @@ __device__ __forceinline__ bool m2d_close(const DevSites &s, int i, const Pos64 
   if (coincident(fma(dx, dx, fma(dy, dy, dz * dz)))) return true;
   double o[M2D_SLD], acc[9] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0}, e[3];
   m2d_stage<AMOEBA>(&s.mm_q[(size_t)i * LD], o);
-  m2d_pair_acc<AMOEBA, true>(dx, dy, dz, pt.w, ps.w, at, AMOEBA ? s.mm_a[i] : 0.0, wat, s.mm_wa32[i], o, s.damp_thr,
+  m2d_pair_acc<AMOEBA>(dx, dy, dz, pt.w, ps.w, at, AMOEBA ? s.mm_a[i] : 0.0, wat, s.mm_wa32[i], o, s.damp_thr,
                              thr2m, acc);
   m2d_field<AMOEBA>(acc, e[0], e[1], e[2]);
   for (int c = 0; c < 3; ++c) sum[c] += e[c];

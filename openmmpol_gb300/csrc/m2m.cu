@@ -44,7 +44,7 @@ __device__ __noinline__ void m2m_close(const DevSites &s, int t, int i, double *
   for (int c = 0; c < LD; ++c) q[c] = s.mm_q[(size_t)i * LD + c];
   if (AMOEBA)
     for (int c = 0; c < 6; ++c) Q[c] = s.mm_q[(size_t)t * LD + 4 + c];
-  m2m_any<AMOEBA, GRAD>(q, dx, dy, dz, rinv_f64_full(r2, r2_f32(r2)), 1.0, Q, Q[0] + Q[2] + Q[5], sum);
+  m2m_any<AMOEBA, GRAD>(q, dx, dy, dz, rinv_f64(r2, r2_f32(r2)), 1.0, Q, Q[0] + Q[2] + Q[5], sum);
 }
 
 template <bool AMOEBA, bool GRAD>

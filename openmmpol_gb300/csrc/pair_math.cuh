@@ -26,34 +26,14 @@ __device__ __forceinline__ float r2_f32(double r2) {
   return __uint_as_float(hi < 0x38100000u ? 0u : f);
 }
 
-// 1/sqrt(r2) in FP64 from an FP32 value and one Newton-Raphson step
-// y <- y + (y / 2) (1 - r2 y^2).  The step squares the seed's error, so the
-// hardware estimate (~2^-22) is first refined by one FP32 Newton step to the
-// FP32 rounding level: the result is within ~1e-15 (the bare estimate left
-// ~1e-14, one-sided, which was the largest error of every FP64 pair sum:
-// T.mu of water boxes 8e-15, their permanent field 3e-14 against extended
-// precision).  GB300 runs FP64 at 1/64 of the FP32 rate, so the four FP32
-// instructions cost nothing beside the step's three FP64 ones; y and y / 2
-// are widened by integer operations (exponent rebias; infinities and NaNs
-// kept).
+// 1/sqrt(r2) in FP64 from the FP32 hardware estimate y (~2^-22) and one step to
+// second order, y (1 + e / 2 + 3 e^2 / 8), e = 1 - r2 y^2: to the last bits with
+// five FP64 operations (GB300 runs FP64 at 1/64 of the FP32 rate).  The step to
+// first order left ~1e-14, one-sided, which was the largest error of every FP64
+// pair sum: T.mu of water boxes 8e-15, their permanent field 3e-14 against
+// extended precision.  y and y / 2 are widened by integer operations (exponent
+// rebias; infinities and NaNs kept).
 __device__ __forceinline__ double rinv_f64(double r2, float r2f) {
-  const float y0 = rsqrtf(r2f);
-  const float y1 = fmaf(0.5f * y0, fmaf(-(r2f * y0), y0, 1.f), y0);
-  // outside the FP32 normal range (coincident or astronomically distant
-  // sites) the refinement is not finite: the estimate stays as it is
-  const unsigned u = __float_as_uint(fabsf(y1 - y0) < 1e-3f * y0 ? y1 : y0);
-  const bool special = (u & 0x7F800000u) == 0x7F800000u;
-  const unsigned hi = special ? (0x7FF00000u | (u >> 3)) : (u >> 3) + 0x38000000u;
-  const unsigned lo = u << 29;
-  const double y = __hiloint2double((int)hi, (int)lo);
-  const double hy = __hiloint2double((int)(special ? hi : hi - 0x00100000u), (int)lo);
-  const double e = fma(-r2, y * y, 1.0);
-  return fma(hy, e, y);
-}
-
-// The same to the last bits: the step's second-order term added, y (1 + e / 2
-// + 3 e^2 / 8), two more FP64 operations and no refinement of the estimate.
-__device__ __forceinline__ double rinv_f64_full(double r2, float r2f) {
   const unsigned u = __float_as_uint(rsqrtf(r2f));
   const bool special = (u & 0x7F800000u) == 0x7F800000u;
   const unsigned hi = special ? (0x7FF00000u | (u >> 3)) : (u >> 3) + 0x38000000u;
@@ -124,13 +104,13 @@ __device__ __forceinline__ void dd_kernel(T r2, T wt, T ws, T at, T as, T thr, T
 }
 
 // Damped r^-3 and r^-5 factors of one pair in FP64: reciprocal square root
-// from the FP32 seed plus one Newton step (FULL: to the last bits) and the
+// from the FP32 seed and one step to the last bits, and the
 // FP32 damping pre-test, so that only the arithmetic that needs FP64 runs on GB300's FP64 pipe.
-template <bool AMOEBA, bool FULL = false>
+template <bool AMOEBA>
 __device__ __forceinline__ void dd_pair_f64(double r2, double wt, double ws, double at, double as, float2 wat,
                                             float2 was, double thr, float thr2m, double &k3, double &k5) {
   const float r2f = r2_f32(r2);
-  const double rinv = FULL ? rinv_f64_full(r2, r2f) : rinv_f64(r2, r2f);
+  const double rinv = rinv_f64(r2, r2f);
   const double ir2 = rinv * rinv;
   k3 = rinv * ir2;
   k5 = k3 * ir2;
@@ -186,14 +166,14 @@ __device__ __forceinline__ void damped_factors(float r2, float wt, float ws, flo
 // Field of a static multipole (charge; + dipole and quadrupole for AMOEBA,
 // q[0..9]) at a polarizable target, d = target - source, Thole-damped
 // (elec_prop_M2D pair term, src/mod_electrostatics.F90:2579-2731).
-template <bool AMOEBA, bool FULL = false>
+template <bool AMOEBA>
 __device__ __forceinline__ void m2d_pair_f64(double dx, double dy, double dz, double wt, double ws,
                                              double at, double as, float2 wat, float2 was,
                                              const double *q, double thr, float thr2m,
                                              double &ex, double &ey, double &ez) {
   double r2 = dx * dx + dy * dy + dz * dz;
   float r2f = r2_f32(r2);
-  double rinv = FULL ? rinv_f64_full(r2, r2f) : rinv_f64(r2, r2f);
+  double rinv = rinv_f64(r2, r2f);
   double ir2 = rinv * rinv;
   double k3 = rinv * ir2;
   if (AMOEBA) {
@@ -252,13 +232,13 @@ __device__ __forceinline__ void m2d_stage(const double *q, double *o) {
   for (int c = 0; c < 6; ++c) o[7 + c] = 15.0 * q[4 + c];
 }
 
-template <bool AMOEBA, bool FULL = false>
+template <bool AMOEBA>
 __device__ __forceinline__ void m2d_pair_acc(double dx, double dy, double dz, double wt, double ws, double at,
                                              double as, float2 wat, float2 was, const double *q, double thr,
                                              float thr2m, double *acc) {
   const double r2 = dx * dx + dy * dy + dz * dz;
   const float r2f = r2_f32(r2);
-  const double rinv = FULL ? rinv_f64_full(r2, r2f) : rinv_f64(r2, r2f);
+  const double rinv = rinv_f64(r2, r2f);
   const double ir2 = rinv * rinv;
   double k3 = rinv * ir2;
   if (AMOEBA) {

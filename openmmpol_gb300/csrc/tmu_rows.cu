@@ -85,7 +85,7 @@ __device__ __forceinline__ void pair64(const RowsArgs &a, const double *x, int j
   const double dx = pt.x - ps.x, dy = pt.y - ps.y, dz = pt.z - ps.z;
   const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
   double k3, k5;
-  dd_pair_f64<AMOEBA, true>(r2, pt.w, ps.w, AMOEBA ? a.damp[j] : 0.0, AMOEBA ? a.damp[i] : 0.0, a.wa[j], a.wa[i], a.thr,
+  dd_pair_f64<AMOEBA>(r2, pt.w, ps.w, AMOEBA ? a.damp[j] : 0.0, AMOEBA ? a.damp[i] : 0.0, a.wa[j], a.wa[i], a.thr,
                             a.thr2m, k3, k5);
   k3 *= w;
   k5 *= 3.0 * w;
@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(128) k_rows_f64(int n, const Pos64 *__restrict
     const double dx = pt.x - ps.x, dy = pt.y - ps.y, dz = pt.z - ps.z;
     const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
     double k3, k5;
-    dd_pair_f64<AMOEBA, true>(r2, pt.w, ps.w, at, AMOEBA ? damp[i] : 0.0, wat, wa[i], thr, thr2m, k3, k5);
+    dd_pair_f64<AMOEBA>(r2, pt.w, ps.w, at, AMOEBA ? damp[i] : 0.0, wat, wa[i], thr, thr2m, k3, k5);
     const double k3w = k3 * w, k5w = 3.0 * w * k5;
 #pragma unroll
     for (int r = 0; r < G; ++r) {

@@ -204,7 +204,7 @@ __device__ __noinline__ void sym_queued(const unsigned short *queue, int count, 
     const double dx = pi.x - pj.x, dy = pi.y - pj.y, dz = pi.z - pj.z;
     const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
     double k3, k5;
-    dd_pair_f64<AMOEBA, true>(r2, pi.w, pj.w, AMOEBA ? jb.damp[i] : 0.0, AMOEBA ? jb.damp[j] : 0.0, jb.wa[i], jb.wa[j],
+    dd_pair_f64<AMOEBA>(r2, pi.w, pj.w, AMOEBA ? jb.damp[i] : 0.0, AMOEBA ? jb.damp[j] : 0.0, jb.wa[i], jb.wa[j],
                         jb.thr, jb.thr2m, k3, k5);
     k5 *= 3.0;
 #pragma unroll
@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(FIN_TPB) k_tmu_sym_finish(
         const double dx = pt.x - ps.x, dy = pt.y - ps.y, dz = pt.z - ps.z;
         const double r2 = fma(dx, dx, fma(dy, dy, dz * dz));
         double k3, k5;
-        dd_pair_f64<AMOEBA, true>(r2, pt.w, ps.w, at, AMOEBA ? damp[i] : 0.0, wat, wa[i], thr, thr2m, k3, k5);
+        dd_pair_f64<AMOEBA>(r2, pt.w, ps.w, at, AMOEBA ? damp[i] : 0.0, wat, wa[i], thr, thr2m, k3, k5);
         const double *mu = &x[(col + i) * 3];
         const double f = 3.0 * k5 * fma(mu[0], dx, fma(mu[1], dy, mu[2] * dz));
         const double cs = scale[k] - 1.0;
