@@ -93,14 +93,14 @@ def parse():
     ap.add_argument("--e2e-steps", type=int, default=None)
     ap.add_argument("--cpu-rows", type=int, default=0, help="target rows of the CPU sample (0 = auto)")
     ap.add_argument("--no-fp64", action="store_true")
-    ap.add_argument("--no-ds", action="store_true", help="leave out the double-single pass")
+    ap.add_argument("--no-ds", action="store_true", help="leave out the mixed-ds pass")
     ap.add_argument("--no-update", action="store_true",
                     help="leave out the strict-mode pass with the refinement residual update")
     ap.add_argument("--no-grad", action="store_true", help="leave out the polarization-gradient pass")
     ap.add_argument("--precision", default="mixed", choices=["mixed", "mixed-ds"],
-                    help="mixed: FP64 refinement residual products; mixed-ds: double-single ones")
+                    help="mixed: every refinement residual recomputed; mixed-ds: later ones updated")
     ap.add_argument("--fp32-kernel", default="auto", choices=["auto", "pairwise", "tiled", "symmetric"],
-                    help="FP32 inner T.mu kernel (auto = autotuned)")
+                    help="FP32 inner T.mu kernel (auto = by size and columns)")
     ap.add_argument("--requests", type=int, default=1024, help="s1024: requests in the mixed stream")
     ap.add_argument("--fp64-requests", type=int, default=64, help="s1024: requests in the FP64 stream")
     ap.add_argument("--slots", type=int, default=8, help="s1024: concurrent requests on the GPU")

@@ -53,8 +53,13 @@
 #endif
 
 /* precision modes of ommp_gpu_set_precision */
-#define OMMP_GPU_PREC_FP64 0  /* plain FP64 solver (default) */
-#define OMMP_GPU_PREC_MIXED 1 /* FP32 inner CG + FP64 iterative refinement */
+#define OMMP_GPU_PREC_FP64 0  /* the reference's solvers (default): FP64 vectors, pair  \
+                                 sums of FP64 accuracy: close and strongly damped pairs \
+                                 in FP64, the others in double-single arithmetic (two   \
+                                 floats, about 48 bits), errors no larger than those of \
+                                 sums in FP64 throughout */
+#define OMMP_GPU_PREC_MIXED 1 /* FP32 inner CG + iterative refinement with residuals \
+                                 of the same accuracy */
 #define OMMP_GPU_PREC_MIXED_DS 2 /* as MIXED (direct residual products whatever the \
                                     FMM setting), later residuals updated by the    \
                                     FP32 product of the correction */
@@ -279,7 +284,7 @@ int32_t ommp_gpu_set_default_matv(OMMP_SYSTEM_PRT s, int32_t matv);
 const char *ommp_gpu_last_error(void);
 
 /* solver controls; the reference hard-codes tol 1e-8 / 200 iterations
- * (src/mod_solvers.F90:30-35) */
+ * (src/mod_solvers.F90:30-35); a limit below 1 leaves the starting dipoles */
 void ommp_gpu_set_solver_tol(OMMP_SYSTEM_PRT s, double tol);
 void ommp_gpu_set_solver_maxiter(OMMP_SYSTEM_PRT s, int32_t maxiter);
 void ommp_gpu_set_precision(OMMP_SYSTEM_PRT s, int32_t mode);

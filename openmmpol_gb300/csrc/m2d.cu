@@ -5,7 +5,7 @@
 //
 // In FP64 (40 FP64 operations per pair) the field of 90,000 sites took 0.56 s,
 // the FP64 pipe 95 % busy.  All modes now form it in double-single on the FP32
-// pipes (ds_pair.cuh), about 385 FP32 operations per AMOEBA pair:
+// pipes (ds_pair.cuh), 428 FP32 operations per AMOEBA pair (ncu):
 //   E = (q G + (mu.n) F + (n.Q.n) C) n - K mu - H Q n
 // with G = y^2, F = 3 y^3, C = 15 y^4, K = y^3, H = 6 y^4 times their factors
 // in eps.  Source tiles whose box comes within the damping range test each

@@ -9,8 +9,8 @@
 // 90,000 sites with that pipe 92 % busy.  Here only the pairs that need FP64
 // use it: those that may be Thole-damped (an exponential or a polynomial in
 // r) or that are close.  All others are formed on the FP32 pipes in
-// double-single arithmetic (ds_math.cuh), ~285 FP32 operations per unordered
-// pair, with
+// double-single arithmetic (ds_math.cuh), 289 FP32 operations per unordered
+// pair (ncu), with
 //   * coordinates split on a grid into three floats (launch_split), so
 //     that the difference of two sites is exact and costs 7 operations;
 //   * the unit-length form E = K (mu.n) n - k3 mu of the dipole field
@@ -22,10 +22,10 @@
 // Errors against extended precision (2-norm, random dipoles): water boxes of
 // 900 to 90,000 sites 3.1e-15 to 4.9e-15 (the FP64 kernel: 8.1e-15 to
 // 8.7e-15), a Wang-AL system of 10,200 sites 2.1e-15 (2.9e-15).
-// Time per product (one column): 917 -> 202 us at 5,001 sites, 2.6 -> 0.50 ms
-// at 9,003, 25.6 -> 4.6 ms at 30,000, 230 -> 40.3 ms at 90,000 (4.05e9 pairs:
+// Time per product (one column): 917 -> 194 us at 5,001 sites, 2.6 -> 0.50 ms
+// at 9,003, 25.6 -> 4.6 ms at 30,000, 230 -> 40.2 ms at 90,000 (4.05e9 pairs:
 // 29 T FP32 operations/s of a measured FMA-chain rate of 36 T/s); two columns
-// 70.9 ms.  Bound by FP32 issue; 5 CTAs per SM at 96 registers with small
+// 70.5 ms.  Bound by FP32 issue; 5 CTAs per SM at 96 registers with small
 // spills beat 4 at 128 (40.9 ms).
 //
 // Schedule: sites are grouped in super-tiles of 128 (4 warps x 32 lanes).
